@@ -14,78 +14,152 @@ namespace grb {
 
 __device__ __forceinline__ const int* net_routes(const Plan& P, int id) { return P.routes + P.route_off[id]; }
 
+// A wire segment as its run of edges on a track: first slot and edge count
+// (n = 0: no wire, or a single cell), its end cells stamped by the caller.
+// `skew`: the segment runs across its layer's direction (no router emits
+// that; a caller's own routes may), so its cells are not consecutive.
+struct WireRun {
+    int first, n;
+    bool wire, skew;
+    double length;
+};
+__device__ __forceinline__ WireRun wire_run(const Tables& T, int a, int b) {
+    WireRun R{0, 0, false, false, 0.0};
+    int l, x0, y0, lb, x1, y1;
+    cell_position(T, a, l, x0, y0);
+    cell_position(T, b, lb, x1, y1);
+    R.wire = l == lb;
+    if (!R.wire) return R;
+    const bool ay = x0 == x1;
+    const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
+    R.n = hi - lo;
+    R.skew = R.n && ay != along_y(T, l);
+    R.first = slot_index(T, l, ay ? x0 : lo, ay ? lo : y0);
+    R.length = ay ? T.ydist[hi] - T.ydist[lo] : T.xdist[hi] - T.xdist[lo];
+    return R;
+}
+
+// Edge at slot c of a segment gets K; its cell is stamped.
+__device__ __forceinline__ void commit_edge(const Tables& T, int c, int stamp, int K) {
+    red_add(T.demand + c, 2 * K);
+    T.ts[c] = stamp;
+}
+
+// A skew segment, edge by edge (one thread).
+__device__ __forceinline__ void commit_skew(const Tables& T, int a, int b, int stamp, int K) {
+    int l, x0, y0, lb, x1, y1;
+    cell_position(T, a, l, x0, y0);
+    cell_position(T, b, lb, x1, y1);
+    const bool ay = x0 == x1;
+    const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
+    for (int p = lo; p < hi; ++p) {
+        const int c = slot_index(T, l, ay ? x0 : p, ay ? p : y0);
+        commit_edge(T, c, stamp, K);
+        mark_edge_dirty(T, c);
+    }
+}
+
+// Both end cells of a segment are stamped.
+__device__ __forceinline__ void stamp_ends(const Tables& T, const WireRun& R, int a, int b, int stamp) {
+    if (R.skew) {
+        int l, x, y;
+        cell_position(T, a, l, x, y);
+        T.ts[slot_index(T, l, x, y)] = stamp;
+        cell_position(T, b, l, x, y);
+        T.ts[slot_index(T, l, x, y)] = stamp;
+    } else {
+        T.ts[R.first] = stamp;
+        T.ts[R.first + R.n] = stamp;
+    }
+}
+
 // One warp commits the wire segments of net `id` (of `parts` warps sharing a
-// net, warp `part` takes every parts-th segment); lanes split each segment's
-// unit edges.  Along-y segments cover consecutive cells, so their dirty bits
-// are set a bitmap word at a time (fenwick.cuh:51-78).
+// net, warp `part` takes every parts-th group of 32 segments).  Each lane
+// decodes one segment; then the edges of all short segments are shared out
+// over the lanes together, and each long one takes the whole warp.  A run's
+// edges are consecutive slots, so its dirty bits are set a bitmap word at a
+// time by the edge that opens the word (fenwick.cuh:51-78).
+constexpr int kLongRun = 64;
 __device__ __forceinline__ void commit_net_wires(const Tables& T, const Plan& P, int id, int stamp, int K,
                                                  int lane, int part = 0, int parts = 1) {
     const int* r = net_routes(P, id);
-    const int words = r[0];
+    const int segs = (r[0] - 1) / 2;
     double length = 0;
-    for (int i = 1 + 2 * part; i < words; i += 2 * parts) {
-        const int a = r[i], b = r[i + 1], layer = a / T.XY;
-        if (layer != b / T.XY) continue;
-        const int ra = a - layer * T.XY, rb = b - layer * T.XY;
-        const int x0 = ra / T.Y, y0 = ra - x0 * T.Y, x1 = rb / T.Y, y1 = rb - x1 * T.Y;
-        const bool ay = x0 == x1;
-        const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
-        if (lane == 0) {
-            T.ts[a] = stamp;
-            T.ts[b] = stamp;
-            if (hi > lo) {
-                mark_group_dirty(T, layer, ay ? x0 : y0, lo);
-                if (ay) {
-                    const int first = layer * T.XY + x0 * T.Y + lo;
-                    mark_range(T.dirty_wire, first, first + (hi - lo) - 1);
-                    mark_range(T.dirty_via, first, first + (hi - lo));
-                }
+    for (int s0 = 32 * part; s0 < segs; s0 += 32 * parts) {
+        WireRun R{0, 0, false, false, 0.0};
+        if (s0 + lane < segs) {
+            const int a = r[1 + 2 * (s0 + lane)], b = r[2 + 2 * (s0 + lane)];
+            R = wire_run(T, a, b);
+            if (R.wire) {
+                stamp_ends(T, R, a, b, stamp);
+                length += R.length;
+                if (R.skew) commit_skew(T, a, b, stamp, K);
             }
         }
-        for (int pos = lo + lane; pos < hi; pos += 32) {
-            const int c = layer * T.XY + (ay ? x0 * T.Y + pos : pos * T.Y + y0);
-            red_add(T.demand + c, 2 * K);
-            T.ts[c] = stamp;
-            if (!ay) {
-                set_bits(T.dirty_wire, c >> 5, 1u << (c & 31));
-                set_bits(T.dirty_via, c >> 5, 1u << (c & 31));
-                if (pos + 1 < T.X) set_bits(T.dirty_via, (c + T.Y) >> 5, 1u << ((c + T.Y) & 31));
+        const int n = R.wire && !R.skew ? R.n : 0;
+        unsigned longs = __ballot_sync(0xffffffffu, n >= kLongRun);
+        while (longs) {
+            const int q = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const int first = __shfl_sync(0xffffffffu, R.first, q), last = first + __shfl_sync(0xffffffffu, n, q) - 1;
+            for (int c = first + lane; c <= last; c += 32) commit_edge(T, c, stamp, K);
+            for (int w = (first >> 5) + lane; w <= (last >> 5); w += 32) red_or(T.dirty + w, range_bits(w, first, last));
+        }
+        const int m = n < kLongRun ? n : 0;
+        int incl = m;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const int k = k0 + lane;
+            int q = 0;  // the segment of edge k: the first with incl > k
+#pragma unroll
+            for (int step = 16; step; step >>= 1) {
+                const int v = __shfl_sync(0xffffffffu, incl, q + step - 1);
+                if (v <= k) q += step;
             }
-            length += ay ? T.ylen[pos] : T.xlen[pos];
+            const int first = __shfl_sync(0xffffffffu, R.first, q), cnt = __shfl_sync(0xffffffffu, m, q);
+            const int end = __shfl_sync(0xffffffffu, incl, q);
+            if (k < total) {
+                const int c = first + (k - (end - cnt));
+                commit_edge(T, c, stamp, K);
+                if (c == first || (c & 31) == 0) red_or(T.dirty + (c >> 5), range_bits(c >> 5, first, first + cnt - 1));
+            }
         }
     }
     for (int s = 16; s; s >>= 1) length += __shfl_down_sync(0xffffffffu, length, s);
     if (lane == 0 && length != 0.0) atomicAdd(T.wirelength, length * K);
 }
 
-// Via demand on cell c, position pos of track `track` of layer l.
-__device__ __forceinline__ void add_via_demand(const Tables& T, int c, int half, int l, int track, int pos, int len,
-                                               int stride) {
+// Via demand on the edge at slot c.
+__device__ __forceinline__ void add_via_demand(const Tables& T, int c, int half) {
     red_add(T.demand + c, half);
-    mark_edge_dirty(T, c, l, track, pos, len, stride);
+    mark_edge_dirty(T, c);
 }
 
-// Demand of the via stack at (x, y) (ra = x*Y + y) between layers low and
-// high: every layer whose cell no wire of this batch stamped adds K at a track
-// end, else K/2 to the two edges it lands between.  All timestamps of the
-// stack are loaded before the first update.
-__device__ __forceinline__ void via_stack_demand(const Tables& T, int ra, int x, int y, int low, int high, int stamp,
-                                                 int K) {
+// Demand of the via stack at (x, y) between layers low and high: every layer
+// whose cell no wire of this batch stamped adds K at a track end, else K/2 to
+// the two edges it lands between.  All timestamps of the stack are loaded
+// before the first update.
+__device__ __forceinline__ void via_stack_demand(const Tables& T, int x, int y, int low, int high, int stamp, int K) {
     int ts[kMaxLayers];
 #pragma unroll
-    for (int u = 0; u < kMaxLayers; ++u) ts[u] = low + u < high ? T.ts[(low + u) * T.XY + ra] : stamp;
+    for (int u = 0; u < kMaxLayers; ++u) ts[u] = low + u < high ? T.ts[slot_index(T, low + u, x, y)] : stamp;
 #pragma unroll
     for (int u = 0; u < kMaxLayers; ++u) {
         const int layer = low + u;
         if (layer >= high || ts[u] >= stamp) continue;
-        const int c = layer * T.XY + ra;
+        const int c = slot_index(T, layer, x, y);
         const bool ay = along_y(T, layer);
-        const int pos = ay ? y : x, len = ay ? T.Y : T.X, stride = ay ? 1 : T.Y, track = ay ? x : y;
-        if (!pos) add_via_demand(T, c, 2 * K, layer, track, pos, len, stride);
-        else if (pos == len - 1) add_via_demand(T, c - stride, 2 * K, layer, track, pos - 1, len, stride);
+        const int pos = ay ? y : x, len = ay ? T.Y : T.X;
+        if (!pos) add_via_demand(T, c, 2 * K);
+        else if (pos == len - 1) add_via_demand(T, c - 1, 2 * K);
         else {
-            add_via_demand(T, c - stride, K, layer, track, pos - 1, len, stride);
-            add_via_demand(T, c, K, layer, track, pos, len, stride);
+            add_via_demand(T, c - 1, K);
+            add_via_demand(T, c, K);
         }
     }
 }
@@ -93,11 +167,11 @@ __device__ __forceinline__ void via_stack_demand(const Tables& T, int ra, int x,
 // Route segment (a, b): if it is a via, commit its stack and return the
 // number of layers it crosses, else 0.
 __device__ __forceinline__ int via_segment(const Tables& T, int a, int b, int stamp, int K) {
-    const int la = a / T.XY, lb = b / T.XY;
-    const int low = min(la, lb), high = max(la, lb);
+    int la, x, y;
+    cell_position(T, a, la, x, y);
+    const int lb = T.by_xy(b), low = min(la, lb), high = max(la, lb);
     if (low == high) return 0;
-    const int ra = a - la * T.XY, x = ra / T.Y, y = ra - x * T.Y;
-    via_stack_demand(T, ra, x, y, low, high, stamp, K);
+    via_stack_demand(T, x, y, low, high, stamp, K);
     return high - low;
 }
 
@@ -155,33 +229,16 @@ __device__ __forceinline__ void commit_thread_wires(const Tables& T, const Plan&
     const int words = r[0];
     double length = 0;
     for (int i = 1; i < words; i += 2) {
-        const int a = r[i], b = r[i + 1], layer = a / T.XY;
-        if (layer != b / T.XY) continue;
-        const int ra = a - layer * T.XY, rb = b - layer * T.XY;
-        const int x0 = ra / T.Y, y0 = ra - x0 * T.Y, x1 = rb / T.Y, y1 = rb - x1 * T.Y;
-        const bool ay = x0 == x1;
-        const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
-        T.ts[a] = stamp;
-        T.ts[b] = stamp;
-        if (hi > lo) {
-            mark_group_dirty(T, layer, ay ? x0 : y0, lo);
-            if (ay) {
-                const int first = layer * T.XY + x0 * T.Y + lo;
-                mark_range(T.dirty_wire, first, first + (hi - lo) - 1);
-                mark_range(T.dirty_via, first, first + (hi - lo));
-            }
-        }
-        for (int pos = lo; pos < hi; ++pos) {
-            const int c = layer * T.XY + (ay ? x0 * T.Y + pos : pos * T.Y + y0);
-            red_add(T.demand + c, 2 * K);
-            T.ts[c] = stamp;
-            if (!ay) {
-                set_bits(T.dirty_wire, c >> 5, 1u << (c & 31));
-                set_bits(T.dirty_via, c >> 5, 1u << (c & 31));
-                if (pos + 1 < T.X) set_bits(T.dirty_via, (c + T.Y) >> 5, 1u << ((c + T.Y) & 31));
-            }
-            length += ay ? T.ylen[pos] : T.xlen[pos];
-        }
+        const int a = r[i], b = r[i + 1];
+        const WireRun R = wire_run(T, a, b);
+        if (!R.wire) continue;
+        stamp_ends(T, R, a, b, stamp);
+        length += R.length;
+        if (R.skew) { commit_skew(T, a, b, stamp, K); continue; }
+        const int last = R.first + R.n - 1;
+        for (int c = R.first; c <= last; ++c) commit_edge(T, c, stamp, K);
+        if (R.n)
+            for (int w = R.first >> 5; w <= (last >> 5); ++w) red_or(T.dirty + w, range_bits(w, R.first, last));
     }
     if (length != 0.0) atomicAdd(T.wirelength, length * K);
 }
@@ -190,15 +247,7 @@ __device__ __forceinline__ void commit_thread_vias(const Tables& T, const Plan& 
     const int* r = net_routes(P, id);
     const int words = r[0];
     long long vias = 0;
-    for (int i = 1; i < words; i += 2) {
-        const int a = r[i], b = r[i + 1];
-        const int la = a / T.XY, lb = b / T.XY;
-        const int low = min(la, lb), high = max(la, lb);
-        if (low == high) continue;
-        const int ra = a - la * T.XY, x = ra / T.Y, y = ra - x * T.Y;
-        vias += high - low;
-        via_stack_demand(T, ra, x, y, low, high, stamp, K);
-    }
+    for (int i = 1; i < words; i += 2) vias += via_segment(T, r[i], r[i + 1], stamp, K);
     if (vias) atomicAdd(T.vias, static_cast<unsigned long long>(vias * K));
 }
 

@@ -1,10 +1,18 @@
 // common.cuh -- device-side state view and shared helpers for the routing path.
 //
-// Grid layout follows the reference router (router_state.hpp:267):
-// IDX(l,x,y) = (l*X + x)*Y + y, and layer l carries wires along y when
-// ((l & 1) ^ DIR) is 1, along x otherwise.  Demand is int32 half-units: a wire
-// edge adds 2, a split via landing adds 1 to each neighbour (demand.cuh:300-304
-// uses 1.0f and 0.5f), so demand * 0.5f reproduces the reference's float.
+// Grid positions in the ABI (tree nodes, route words, table transfers) follow
+// the reference router (router_state.hpp:267): IDX(l,x,y) = (l*X + x)*Y + y, and
+// layer l carries wires along y when ((l & 1) ^ DIR) is 1, along x otherwise.
+// Demand is int32 half-units: a wire edge adds 2, a split via landing adds 1 to
+// each neighbour (demand.cuh:300-304 uses 1.0f and 0.5f), so demand * 0.5f
+// reproduces the reference's float.
+//
+// The tables themselves are stored track by track: the cells of one wire
+// track (fixed x on layers along y, fixed y on the others) are consecutive
+// "slots", each track padded to a multiple of 32.  A wire segment, its demand
+// updates, its dirty bits, the costs they invalidate and the prefix sums over
+// them are then runs of consecutive addresses on every layer; in IDX order the
+// layers along x put every cell of a segment into a sector of its own.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -13,30 +21,55 @@ namespace grb {
 
 constexpr double kInf = 1e22;   // router_state.hpp:271
 constexpr int kMaxLayers = 10;  // lshape_warp.cuh:115 asserts L <= 10
-constexpr int kTrackGroup = 32; // tracks per prefix group (one per lane)
+constexpr int kScanBlock = 128; // positions per prefix block (four per lane)
 constexpr int kNoCapRow = 255;  // cap_id of a cell whose capacity has no table row
 
 enum : int {
     kOk = 0, kEInval = 1, kENoMem = 2, kECuda = 3, kETimedOut = 4, kELimit = 5,
 };
 
+// Division by a number fixed per context: n / d for 0 <= n < 2^31, d >= 2, as a
+// multiplication by ceil(2^p / d), p = 31 + ceil(log2 d), and a shift (Granlund
+// and Montgomery, "Division by invariant integers using multiplication").
+struct FastDiv {
+    unsigned mul;
+    int shift;
+    __device__ __forceinline__ int operator()(int n) const {
+        return static_cast<int>(__umulhi(static_cast<unsigned>(n), mul) >> shift);
+    }
+};
+inline FastDiv fast_div(int d) {
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    return FastDiv{static_cast<unsigned>(((1ull << (31 + l)) + static_cast<unsigned>(d) - 1) / static_cast<unsigned>(d)), l - 1};
+}
+
 // Device tables of one routing context.  Copied by value into every kernel.
 struct Tables {
     int L, X, Y, DIR, XY;
-    int cells;
+    int cells;             // L * X * Y
+    FastDiv by_xy, by_x, by_y;  // division by X * Y, X and Y
+    // Track layout (slot_index): padded track lengths, slots of an even layer
+    // and of an (even, odd) layer pair, all slots, all tracks.
+    int xp, yp;
+    int even_slots, pair_slots, slots, tracks;
     double unit_wire, unit_via, of_scale;
     const double* short_costs;
     const int* xlen;
     const int* ylen;
+    const double* xdist;   // [X] distance of grid line x from line 0 (sums of xlen)
+    const double* ydist;   // [Y]
     const float* capacity;
     int* demand;           // half-units
     int* ts;               // commit timestamps
     float* wcost;
     float* vcost;
     double* presum;
-    unsigned* dirty_wire;  // one bit per cell: wire cost to recompute
-    unsigned* dirty_via;   // one bit per cell: via cost to recompute
-    int words;             // bitmap words
+    // One bit per slot: the demand of the edge changed, so its wire cost, its
+    // own via cost and the via cost of the next cell along the track are to
+    // be recomputed (fenwick.cuh:27-38), and the track's prefix from there on.
+    unsigned* dirty;
+    int words;             // bitmap words (slots / 32)
     int int_wire;          // 1: wire costs clamped to [0, 1e7] and truncated (GGR build)
     // Cost-term table: row (l, k) holds, for demands h < of_dmax half-units,
     // the terms of a cell of capacity value k on layer l (cost.cuh
@@ -47,18 +80,8 @@ struct Tables {
     int of_rows;           // capacity values (rows per layer)
     int of_stride;         // entries per row
     int of_dmax;           // demands below this come from the table
-    // Prefix groups: kTrackGroup adjacent tracks of one layer.  A group's
-    // prefix is rebuilt from the first 32-position chunk where a wire cost of
-    // one of its tracks changed.
-    int group_base[kMaxLayers + 1];
-    int* group_first;      // [n_groups] first chunk with a demand change (INT_MAX: none)
-    int* first_list;       // [n_groups] group_first of each listed dirty group
-    int n_groups;
-    int* group_list;       // [n_groups] dirty groups of the current refresh
-    int* group_count;      // [1]
-    double* ptree;         // [n_groups][tree_stride][32] prefix block totals
-    int tree_stride;       // entries per group (2 * tree_chunks + 1)
-    int tree_chunks;       // 32-position chunks of the longest track
+    double* block_total;   // [tracks][track_blocks] totals of kScanBlock prefix inputs
+    int track_blocks;      // prefix blocks of the longest track
     double* wirelength;
     unsigned long long* vias;
     int* error;            // first error code
@@ -97,7 +120,40 @@ struct DpTune {
 };
 
 __device__ __forceinline__ bool along_y(const Tables& T, int l) { return ((l & 1) ^ T.DIR) != 0; }
+// Position in the ABI's IDX order (route words).
 __device__ __forceinline__ int cell_index(const Tables& T, int l, int x, int y) { return (l * T.X + x) * T.Y + y; }
+// First slot of layer l, and the slot of a cell.
+__device__ __forceinline__ int layer_base(const Tables& T, int l) {
+    return (l >> 1) * T.pair_slots + ((l & 1) ? T.even_slots : 0);
+}
+__device__ __forceinline__ int slot_index(const Tables& T, int l, int x, int y) {
+    return layer_base(T, l) + (along_y(T, l) ? x * T.yp + y : y * T.xp + x);
+}
+// Layer and grid position of an IDX position.
+__device__ __forceinline__ void cell_position(const Tables& T, int c, int& l, int& x, int& y) {
+    l = T.by_xy(c);
+    const int r = c - l * T.XY;
+    x = T.by_y(r);
+    y = r - x * T.Y;
+}
+
+// One wire track: layer, length, padded words and first slot.
+struct Track {
+    int l, len, words, base;
+};
+__device__ __forceinline__ Track track_of(const Tables& T, int t) {
+    const int pair = T.X + T.Y, p = t / pair, r = t - p * pair;
+    const int even = T.DIR ? T.X : T.Y;  // tracks of an even layer
+    const bool odd = r >= even;
+    Track K;
+    K.l = 2 * p + (odd ? 1 : 0);
+    const bool ay = along_y(T, K.l);
+    const int pad = ay ? T.yp : T.xp;
+    K.len = ay ? T.Y : T.X;
+    K.words = pad >> 5;
+    K.base = layer_base(T, K.l) + (odd ? r - even : r) * pad;
+    return K;
+}
 
 __device__ __forceinline__ void set_error(const Tables& T, int code, int info) {
     if (atomicCAS(T.error, 0, code) == 0) *T.error_info = info;
@@ -111,42 +167,16 @@ __device__ __forceinline__ void red_or(unsigned* p, unsigned v) {
 __device__ __forceinline__ void red_add(int* p, int v) {
     asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void red_min(int* p, int v) {
-    asm volatile("red.relaxed.gpu.global.min.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
+// The demand of the edge at slot c changed.
+__device__ __forceinline__ void mark_edge_dirty(const Tables& T, int c) { red_or(T.dirty + (c >> 5), 1u << (c & 31)); }
 
-__device__ __forceinline__ void set_bits(unsigned* bits, int word, unsigned mask) {
-    if (mask) red_or(bits + word, mask);
-}
-
-// A wire cost of track `track` of layer l at position `pos` changed: the
-// group's prefix must be rebuilt from that position's 32-position chunk on.
-__device__ __forceinline__ void mark_group_dirty(const Tables& T, int l, int track, int pos) {
-    red_min(T.group_first + T.group_base[l] + track / kTrackGroup, pos >> 5);
-}
-
-// A demand change on edge cell c (position pos of track `track` of layer l,
-// track length len, stride along the track) invalidates its wire cost, its
-// own via cost and the via cost of the next cell along the track
-// (fenwick.cuh:27-38).
-__device__ __forceinline__ void mark_edge_dirty(const Tables& T, int c, int l, int track, int pos, int len,
-                                                int stride) {
-    set_bits(T.dirty_wire, c >> 5, 1u << (c & 31));
-    set_bits(T.dirty_via, c >> 5, 1u << (c & 31));
-    if (pos + 1 < len) set_bits(T.dirty_via, (c + stride) >> 5, 1u << ((c + stride) & 31));
-    mark_group_dirty(T, l, track, pos);
-}
-
-// Mark cells [first, last] of a bitmap with one atomic per word
-// (fenwick.cuh:40-49).
-__device__ __forceinline__ void mark_range(unsigned* bits, int first, int last) {
-    const int a = first >> 5, b = last >> 5;
-    for (int w = a; w <= b; ++w) {
-        unsigned m = ~0u;
-        if (w == a) m &= ~0u << (first & 31);
-        if (w == b) m &= ~0u >> (31 - (last & 31));
-        set_bits(bits, w, m);
-    }
+// Bits [first, last] of bitmap word w (32-bit words, bit positions counted
+// over the whole bitmap).
+__device__ __forceinline__ unsigned range_bits(int w, int first, int last) {
+    unsigned m = ~0u;
+    if (w == (first >> 5)) m &= ~0u << (first & 31);
+    if (w == (last >> 5)) m &= ~0u >> (31 - (last & 31));
+    return m;
 }
 
 // Grid-wide barrier for cooperative launches: one monotone arrival counter

@@ -7,40 +7,43 @@
 
 namespace grb {
 
-// mark_overflow_edges (congestion.cuh:8-20): 1 where the edge of cell c
-// carries demand >= capacity + threshold (cells without an edge: 0).
-__device__ __forceinline__ void overflow_mark(const Tables& T, int threshold, int* of_sum, int c) {
-    const int l = c / T.XY, rem = c - l * T.XY, x = rem / T.Y, y = rem - x * T.Y;
-    const bool edge = along_y(T, l) ? (y + 1 < T.Y) : (x + 1 < T.X);
-    of_sum[c] = (edge && T.capacity[c] + threshold <= static_cast<float>(T.demand[c]) * 0.5f) ? 1 : 0;
+// The overflow marks and their prefix are stored track by track without
+// padding (L*X*Y entries, so the fixed scratch of the allocation-free entry
+// point holds the same grids as ever).
+__device__ __forceinline__ int mark_index(const Tables& T, int l, int x, int y) {
+    return l * T.XY + (along_y(T, l) ? x * T.Y + y : y * T.X + x);
 }
 
-// Exclusive integer prefix of the marks along track t (all layers' tracks
-// numbered consecutively; compute_presum_general, prefix_scan.cuh:42-72 --
-// integer sums are order-free).
-__device__ __forceinline__ void overflow_prefix_track(const Tables& T, int* v, int t) {
-    int l = 0, base = t;
-    for (; l < T.L; ++l) {
-        const int tracks = along_y(T, l) ? T.X : T.Y;
-        if (base < tracks) break;
-        base -= tracks;
-    }
-    if (l >= T.L) return;
+// mark_overflow_edges (congestion.cuh:8-20): 1 where the edge of mark k's
+// cell carries demand >= capacity + threshold (cells without an edge: 0).
+__device__ __forceinline__ void overflow_mark(const Tables& T, int threshold, int* of_sum, int k) {
+    const int l = T.by_xy(k), rem = k - l * T.XY;
     const bool ay = along_y(T, l);
-    const int len = ay ? T.Y : T.X, stride = ay ? 1 : T.Y;
-    const int c0 = ay ? cell_index(T, l, base, 0) : cell_index(T, l, 0, base);
-    int acc = 0;
-    for (int k = 0; k < len; ++k) {
-        const int c = c0 + k * stride, x = v[c];
-        v[c] = acc;
-        acc += x;
-    }
+    const int len = ay ? T.Y : T.X, track = ay ? T.by_y(rem) : T.by_x(rem), pos = rem - track * len;
+    const int c = layer_base(T, l) + track * (ay ? T.yp : T.xp) + pos;
+    of_sum[k] = (pos + 1 < len && T.capacity[c] + threshold <= static_cast<float>(T.demand[c]) * 0.5f) ? 1 : 0;
 }
 
-__device__ __forceinline__ int overflow_tracks(const Tables& T) {
-    int tracks = 0;
-    for (int l = 0; l < T.L; ++l) tracks += along_y(T, l) ? T.X : T.Y;
-    return tracks;
+// Exclusive integer prefix of the marks along track t, by one warp
+// (compute_presum_general, prefix_scan.cuh:42-72 -- integer sums are
+// order-free).
+__device__ __forceinline__ void overflow_prefix_track(const Tables& T, int* v, int t, int lane) {
+    const int pair = T.X + T.Y, p = t / pair, r = t - p * pair, even = T.DIR ? T.X : T.Y;
+    const int l = 2 * p + (r >= even ? 1 : 0), track = r >= even ? r - even : r;
+    const int len = along_y(T, l) ? T.Y : T.X;
+    int* a = v + l * T.XY + track * len;
+    int carry = 0;
+    for (int k0 = 0; k0 < len; k0 += 32) {
+        const int x = k0 + lane < len ? a[k0 + lane] : 0;
+        int incl = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        if (k0 + lane < len) a[k0 + lane] = carry + incl - x;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
 }
 
 // mark_overflow_nets (congestion.cuh:22-58): net `id` is flagged when its
@@ -50,10 +53,11 @@ __device__ __forceinline__ unsigned char overflow_route(const Tables& T, const i
     unsigned char flag = 0;
     if (has) {
         for (int i = 1; i < r[0]; i += 2) {
-            const int a = r[i], b = r[i + 1], l = a / T.XY, ra = a % T.XY, rb = b % T.XY;
-            const int x0 = ra / T.Y, y0 = ra % T.Y, x1 = rb / T.Y, y1 = rb % T.Y;
-            if (x0 != x1) count += of_sum[cell_index(T, l, max(x0, x1), y0)] - of_sum[cell_index(T, l, min(x0, x1), y0)];
-            if (y0 != y1) count += of_sum[cell_index(T, l, x0, max(y0, y1))] - of_sum[cell_index(T, l, x0, min(y0, y1))];
+            int l, x0, y0, lb, x1, y1;
+            cell_position(T, r[i], l, x0, y0);
+            cell_position(T, r[i + 1], lb, x1, y1);
+            if (x0 != x1) count += of_sum[mark_index(T, l, max(x0, x1), y0)] - of_sum[mark_index(T, l, min(x0, x1), y0)];
+            if (y0 != y1) count += of_sum[mark_index(T, l, x0, max(y0, y1))] - of_sum[mark_index(T, l, x0, min(y0, y1))];
             if (count > 10) { flag = 1; break; }
         }
     }
@@ -64,18 +68,46 @@ __device__ __forceinline__ void overflow_net(const Tables& T, const Plan& P, con
     is_of[id] = overflow_route(T, P.routes + P.route_off[id], P.route_off[id + 1] > P.route_off[id], of_sum);
 }
 
-// extract_congestionView (congestion.cuh:60-80) for 2-D cell i: the worst
-// demand - capacity over the layers.
-__device__ __forceinline__ void congestion_cell(const Tables& T, unsigned char* cong, float* xsum, float* ysum,
-                                                int i) {
-    double worst = 0.0;
-    for (int l = 0; l < T.L; ++l) {
-        const int e = l * T.XY + i;
-        worst = fmax(worst, static_cast<double>(static_cast<float>(T.demand[e]) * 0.5f - T.capacity[e]));
+// extract_congestionView (congestion.cuh:60-80) for the 2-D cells of 32 x 32
+// tile `tile`: the worst demand - capacity over the layers (at least 0).  One
+// CTA of a multiple of 32 threads; layers along y are read with lanes over y,
+// the others with lanes over x and transposed through shared memory, so every
+// read is a run of consecutive slots.
+constexpr int kViewTile = 32;
+__host__ __device__ __forceinline__ int view_tiles(const Tables& T) {
+    return ((T.X + kViewTile - 1) / kViewTile) * ((T.Y + kViewTile - 1) / kViewTile);
+}
+__device__ __forceinline__ void congestion_tile(const Tables& T, unsigned char* cong, float* xsum, float* ysum, int tile,
+                                                float (*across)[kViewTile + 1]) {
+    const int nty = (T.Y + kViewTile - 1) / kViewTile;
+    const int x0 = tile / nty * kViewTile, y0 = tile % nty * kViewTile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int q = warp; q < kViewTile; q += nw) {
+        const int x = x0 + lane, y = y0 + q;
+        float worst = 0.f;
+        if (x < T.X && y < T.Y)
+            for (int l = T.DIR; l < T.L; l += 2) {  // the layers along x
+                const int e = slot_index(T, l, x, y);
+                worst = fmaxf(worst, static_cast<float>(T.demand[e]) * 0.5f - T.capacity[e]);
+            }
+        across[q][lane] = worst;
     }
-    cong[i] = worst > 0.0;
-    xsum[i] = static_cast<float>(worst);
-    ysum[i] = static_cast<float>(worst);
+    __syncthreads();
+    for (int q = warp; q < kViewTile; q += nw) {
+        const int x = x0 + q, y = y0 + lane;
+        if (x < T.X && y < T.Y) {
+            float worst = across[lane][q];
+            for (int l = T.DIR ^ 1; l < T.L; l += 2) {  // the layers along y
+                const int e = slot_index(T, l, x, y);
+                worst = fmaxf(worst, static_cast<float>(T.demand[e]) * 0.5f - T.capacity[e]);
+            }
+            const int i = x * T.Y + y;
+            cong[i] = worst > 0.f;
+            xsum[i] = worst;
+            ysum[i] = worst;
+        }
+    }
+    __syncthreads();  // `across` is reused by the next tile
 }
 
 // Float prefix of one line (extract_congestionView_xsum / _ysum,
@@ -117,19 +149,19 @@ struct StageTail {
 
 // The stage tail inside a persistent kernel (grid-stride over all threads):
 // marks and per-cell view | track prefixes and line prefixes | net flags,
-// separated by grid barriers.  False when a barrier gave up.
+// separated by grid barriers.  `across`: shared memory of congestion_tile.
+// False when a barrier gave up.
 __device__ __forceinline__ bool stage_tail_persistent(const Tables& T, const Plan& P, const StageTail& tail,
-                                                      GridSync& S) {
+                                                      GridSync& S, float (*across)[kViewTile + 1]) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     if (tail.flags & kTailRipup)
         for (int c = tid; c < T.cells; c += nth) overflow_mark(T, tail.threshold, tail.of_sum, c);
     if (tail.flags & kTailView)
-        for (int i = tid; i < T.XY; i += nth) congestion_cell(T, tail.cong, tail.xsum, tail.ysum, i);
+        for (int i = blockIdx.x; i < view_tiles(T); i += gridDim.x)
+            congestion_tile(T, tail.cong, tail.xsum, tail.ysum, i, across);
     if (!grid_sync(S, T)) return false;
-    if (tail.flags & kTailRipup) {
-        const int tracks = overflow_tracks(T);
-        for (int t = tid; t < tracks; t += nth) overflow_prefix_track(T, tail.of_sum, t);
-    }
+    if (tail.flags & kTailRipup)
+        for (int t = tid >> 5; t < T.tracks; t += nth >> 5) overflow_prefix_track(T, tail.of_sum, t, threadIdx.x & 31);
     if (tail.flags & kTailView) {
         // per x along y (ysum), then per y along x (xsum), one thread per line
         for (int t = tid; t < T.X + T.Y; t += nth) {

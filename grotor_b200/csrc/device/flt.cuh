@@ -71,7 +71,7 @@ struct Flt {
 
 __device__ __forceinline__ double flt_wire(const Tables& T, int l, int xmin, int xmax, int ymin, int ymax) {
     // prefix_scan.cuh:10-40 (wire_segment_cost)
-    return T.presum[cell_index(T, l, xmax, ymax)] - T.presum[cell_index(T, l, xmin, ymin)];
+    return T.presum[slot_index(T, l, xmax, ymax)] - T.presum[slot_index(T, l, xmin, ymin)];
 }
 
 // flt_cost.cuh:25-46.
@@ -125,7 +125,7 @@ __device__ __forceinline__ void flt_edge_warp(const Tables& T, const Flt& F, int
         int bp[KV];
 #pragma unroll
         for (int ti = 0; ti < KV; ++ti) { bv[ti] = kInf; bp[ti] = -1; }
-        const double pF = T.presum[cell_index(T, fl, fromx, fromy)];
+        const double pF = T.presum[slot_index(T, fl, fromx, fromy)];
         for (int base = 0; base < ns; base += 32) {
             const int s = base + lane;
             if (s < ns) {
@@ -133,15 +133,15 @@ __device__ __forceinline__ void flt_edge_warp(const Tables& T, const Flt& F, int
                 const int sx = vertical ? fromx : sp, sy = vertical ? sp : fromy;
                 float vc[kFltLayers];
 #pragma unroll
-                for (int ll = 0; ll < kFltLayers - 1; ++ll) vc[ll] = ll < T.L ? T.vcost[cell_index(T, ll, sx, sy)] : 0.f;
-                const double pf = T.presum[cell_index(T, fl, sx, sy)];
+                for (int ll = 0; ll < kFltLayers - 1; ++ll) vc[ll] = ll < T.L ? T.vcost[slot_index(T, ll, sx, sy)] : 0.f;
+                const double pf = T.presum[slot_index(T, fl, sx, sy)];
                 const double wf = vertical ? (sy > fromy ? pf - pF : pF - pf) : (sx > fromx ? pf - pF : pF - pf);
 #pragma unroll
                 for (int ti = 0; ti < KV; ++ti) {
                     const int tl = l0 + 2 * ti;
                     if (tl >= 9 || tl >= T.L) continue;
-                    const double pT = T.presum[cell_index(T, tl, tox, toy)];
-                    const double pt = T.presum[cell_index(T, tl, vertical ? tox : sp, vertical ? sp : toy)];
+                    const double pT = T.presum[slot_index(T, tl, tox, toy)];
+                    const double pt = T.presum[slot_index(T, tl, vertical ? tox : sp, vertical ? sp : toy)];
                     const double wt = vertical ? (sy > toy ? pt - pT : pT - pt) : (sx > tox ? pt - pT : pT - pt);
                     const int lo = min(fl, tl), hi = max(fl, tl);
                     double via = 0;
@@ -210,7 +210,7 @@ __device__ __forceinline__ void flt_solve_node(const Tables& T, const Flt& F, in
     }
     float vc[kFltLayers];  // via cost of routing layer li - 2 at the node
 #pragma unroll
-    for (int li = 2; li < kFltLayers; ++li) vc[li] = li - 2 < T.L ? T.vcost[cell_index(T, li - 2, x, y)] : 0.f;
+    for (int li = 2; li < kFltLayers; ++li) vc[li] = li - 2 < T.L ? T.vcost[slot_index(T, li - 2, x, y)] : 0.f;
     double cst[kFltLayers];
 #pragma unroll
     for (int li = 0; li < kFltLayers; ++li) cst[li] = kInf;  // as flt_net left them

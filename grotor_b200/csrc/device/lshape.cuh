@@ -81,7 +81,7 @@ __device__ __forceinline__ Arena carve_arena(char* base, int L, int nmax) {
 
 __device__ __forceinline__ double wire_cost(const Tables& T, int l, int xmin, int xmax, int ymin, int ymax) {
     // prefix_scan.cuh:10-40 (wire_segment_cost)
-    return T.presum[cell_index(T, l, xmax, ymax)] - T.presum[cell_index(T, l, xmin, ymin)];
+    return T.presum[slot_index(T, l, xmax, ymax)] - T.presum[slot_index(T, l, xmin, ymin)];
 }
 
 // Route one net.  All 32 lanes of the warp call this with the same id.
@@ -92,7 +92,7 @@ __device__ __forceinline__ double wire_cost(const Tables& T, int l, int xmin, in
 template <int LC>
 __device__ __forceinline__ void lshape_net_l(const Tables& T, const Plan& P, int id, int stamp, const Arena& A,
                                              int lane, bool fuse_wires) {
-    const int L = LC > 0 ? LC : T.L, Y = T.Y, XY = T.XY, TT = tri_count(L);
+    const int L = LC > 0 ? LC : T.L, TT = tri_count(L);
     constexpr int LL = LC > 0 ? LC : kMaxLayers;  // static bound of the layer loops
     const int off = P.node_off[id], N = P.node_off[id + 1] - off;
     const int* nd = P.nodes + off;
@@ -102,8 +102,9 @@ __device__ __forceinline__ void lshape_net_l(const Tables& T, const Plan& P, int
     // sizes are not repeated per layer and step).
     int dmax = 0;
     for (int q = lane; q < N; q += 32) {
-        const int node = nd[q], l = node / XY, r = node - l * XY, x = r / Y;
-        A.xy[q] = (x << 16) | (r - x * Y);
+        int l, x, y;
+        cell_position(T, nd[q], l, x, y);
+        A.xy[q] = (x << 16) | y;
         A.lay[q] = l;
         int d = 0;
         for (int v = q; v > 0; v = par[v]) ++d;  // parents precede children
@@ -126,8 +127,8 @@ __device__ __forceinline__ void lshape_net_l(const Tables& T, const Plan& P, int
             w1[u] = w2[u] = 0.0;
             if (q >= N * L) continue;
             const int i = q / L, l = q - i * L;
-            const int x = A.xy[i] >> 16, y = A.xy[i] & 0xffff, r = x * Y + y;
-            vn[u] = T.vcost[l * XY + r];
+            const int x = A.xy[i] >> 16, y = A.xy[i] & 0xffff;
+            vn[u] = T.vcost[slot_index(T, l, x, y)];
             kind[u] = 1;
             if (i > 0) {
                 const int pxy = A.xy[par[i]], px = pxy >> 16, py = pxy & 0xffff;
@@ -140,8 +141,8 @@ __device__ __forceinline__ void lshape_net_l(const Tables& T, const Plan& P, int
                 } else {
                     w1[u] = ay ? wire_cost(T, l, x, x, miny, maxy) : wire_cost(T, l, minx, maxx, y, y);
                     w2[u] = ay ? wire_cost(T, l, px, px, miny, maxy) : wire_cost(T, l, minx, maxx, py, py);
-                    va[u] = T.vcost[cell_index(T, l, x, py)];
-                    vb[u] = T.vcost[cell_index(T, l, px, y)];
+                    va[u] = T.vcost[slot_index(T, l, x, py)];
+                    vb[u] = T.vcost[slot_index(T, l, px, y)];
                     kind[u] = 3;
                 }
             }
@@ -397,15 +398,14 @@ __device__ __forceinline__ void lshape_net_pair_l(const Tables& T, const Plan& P
     auto vN = [&](int l) -> float& { return sf[(2 * kMaxLayers + l) * 32 + lane]; };
     auto pdiag = [&](int l) -> int& { return si[(2 * kMaxLayers + l) * 32 + lane]; };       // after vN
     auto cfrom = [&](int l) -> unsigned short& { return sh[l * 32 + lane]; };
-    const int L = LC > 0 ? LC : T.L, Y = T.Y, XY = T.XY;
+    const int L = LC > 0 ? LC : T.L;
     const int off = P.node_off[id], N = P.node_off[id + 1] - off;
-    const int n0 = P.nodes[off], r0 = n0 % XY, x0 = r0 / Y, y0 = r0 - x0 * Y, fix0 = n0 / XY;
-    int x1 = 0, y1 = 0;
+    int fix0, x0, y0, x1 = 0, y1 = 0;
+    cell_position(T, P.nodes[off], fix0, x0, y0);
     bool straight = false;
     if (N == 2) {
-        const int n1 = P.nodes[off + 1], r1 = n1 % XY, fix1 = n1 / XY;
-        x1 = r1 / Y;
-        y1 = r1 - x1 * Y;
+        int fix1;
+        cell_position(T, P.nodes[off + 1], fix1, x1, y1);
         straight = x1 == x0 || y1 == y0;
         const int minx = min(x1, x0), maxx = max(x1, x0), miny = min(y1, y0), maxy = max(y1, y0);
         // Step 1 for node 1 (the child), kHalfLayers layers at a time: every
@@ -422,15 +422,15 @@ __device__ __forceinline__ void lshape_net_pair_l(const Tables& T, const Plan& P
                 a[u] = b[u] = 0.0;
                 if (l >= L) continue;
                 const bool ay = along_y(T, l);
-                vn[u] = T.vcost[l * XY + r1];
+                vn[u] = T.vcost[slot_index(T, l, x1, y1)];
                 if (straight) {
                     const bool valid = ay ? (x1 == x0) : (y1 == y0);
                     a[u] = valid ? wire_cost(T, l, minx, maxx, miny, maxy) : 0.0;
                 } else {
                     a[u] = ay ? wire_cost(T, l, x1, x1, miny, maxy) : wire_cost(T, l, minx, maxx, y1, y1);
                     b[u] = ay ? wire_cost(T, l, x0, x0, miny, maxy) : wire_cost(T, l, minx, maxx, y0, y0);
-                    va[u] = T.vcost[cell_index(T, l, x1, y0)];
-                    vb[u] = T.vcost[cell_index(T, l, x0, y1)];
+                    va[u] = T.vcost[slot_index(T, l, x1, y0)];
+                    vb[u] = T.vcost[slot_index(T, l, x0, y1)];
                 }
             }
 #pragma unroll
@@ -501,7 +501,7 @@ __device__ __forceinline__ void lshape_net_pair_l(const Tables& T, const Plan& P
     {
         float v[kMaxLayers];
 #pragma unroll
-        for (int l = 0; l < kMaxLayers; ++l) v[l] = l < L ? T.vcost[l * XY + r0] : 0.f;
+        for (int l = 0; l < kMaxLayers; ++l) v[l] = l < L ? T.vcost[slot_index(T, l, x0, y0)] : 0.f;
 #pragma unroll
         for (int l = 0; l < kMaxLayers; ++l)
             if (l < L) vA(l) = v[l];

@@ -31,11 +31,11 @@ __device__ __forceinline__ bool maze_wire_touches(const int* r, int point, int X
     return false;
 }
 
-// Edge cell c of layer l changes by `half` half-units (and is marked dirty).
+// The edge of IDX position c changes by `half` half-units (and is marked dirty).
 __device__ __forceinline__ void maze_add(const Tables& T, int c, int half) {
-    const int l = c / T.XY, r = c - l * T.XY, x = r / T.Y, y = r - x * T.Y;
-    const bool ay = along_y(T, l);
-    add_via_demand(T, c, half, l, ay ? x : y, ay ? y : x, ay ? T.Y : T.X, ay ? 1 : T.Y);
+    int l, x, y;
+    cell_position(T, c, l, x, y);
+    add_via_demand(T, slot_index(T, l, x, y), half);
 }
 
 // remove_routes for one net (one thread): route words r.
@@ -86,8 +86,10 @@ __device__ __forceinline__ void maze_score_partial(const Tables& T, double* part
     double value = 0;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < cells; i += size_t(gridDim.x) * blockDim.x) {
         const int layer = int(i / T.XY), x = int(i / T.Y % T.X), y = int(i % T.Y);
-        if (along_y(T, layer) ? y + 1 < T.Y : x + 1 < T.X)
-            value += T.short_costs[layer] * of_cost_scaled(1.0, T.capacity[i], 0.5f * static_cast<float>(T.demand[i]));
+        if (along_y(T, layer) ? y + 1 < T.Y : x + 1 < T.X) {
+            const int c = slot_index(T, layer, x, y);
+            value += T.short_costs[layer] * of_cost_scaled(1.0, T.capacity[c], 0.5f * static_cast<float>(T.demand[c]));
+        }
     }
     sums[threadIdx.x] = value;
     __syncthreads();

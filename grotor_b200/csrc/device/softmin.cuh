@@ -75,15 +75,22 @@ __device__ __forceinline__ T soft_of_dcap(const Tables& Tb, T cap, T d) {
     const T a = static_cast<T>(0.5) * (d - cap), b = scale * static_cast<T>(0.5) * (d - cap);
     return a < b ? static_cast<T>(-0.5) * s_exp<T>(a) : -scale * static_cast<T>(0.5) * s_exp<T>(b);
 }
+// Demand of the edge at IDX position c.
+template <class T>
+__device__ __forceinline__ T soft_demand(const Tables& Tb, int c) {
+    int l, x, y;
+    cell_position(Tb, c, l, x, y);
+    return static_cast<T>(Tb.demand[slot_index(Tb, l, x, y)]) * static_cast<T>(0.5);
+}
 template <class T>
 __device__ __forceinline__ T soft_incr(const Tables& Tb, const Soft<T>& S, int c, int l, T k) {
-    const T d = static_cast<T>(Tb.demand[c]) * static_cast<T>(0.5);
+    const T d = soft_demand<T>(Tb, c);
     const T v = (soft_of<T>(Tb, S.cap[c], d + k) - soft_of<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);
     return v < static_cast<T>(1e12) ? v : static_cast<T>(1e12);
 }
 template <class T>
 __device__ __forceinline__ T soft_incr_dcap(const Tables& Tb, const Soft<T>& S, int c, int l, T k) {
-    const T d = static_cast<T>(Tb.demand[c]) * static_cast<T>(0.5);
+    const T d = soft_demand<T>(Tb, c);
     const T v = (soft_of<T>(Tb, S.cap[c], d + k) - soft_of<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);
     if (!(v < static_cast<T>(1e12))) return 0;
     return (soft_of_dcap<T>(Tb, S.cap[c], d + k) - soft_of_dcap<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);

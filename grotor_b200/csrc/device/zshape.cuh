@@ -50,10 +50,10 @@ __device__ __forceinline__ int zidx(const ZTrees& Z, int i, int x, int y) {
 // positions.  The reference decodes (layer, x, y) from a plane index; the
 // loops here know the positions and read the same cells directly.
 __device__ __forceinline__ int zvia_at(const Tables& T, int i, int x, int y) {
-    return static_cast<int>(fminf(fmaxf(T.vcost[cell_index(T, i - 1, x, y)], 1.f), 1.e6f));
+    return static_cast<int>(fminf(fmaxf(T.vcost[slot_index(T, i - 1, x, y)], 1.f), 1.e6f));
 }
 __device__ __forceinline__ int zwire_at(const Tables& T, int i, int x0, int y0, int x1, int y1) {
-    return static_cast<int>(fmin(fabs(T.presum[cell_index(T, i - 1, x0, y0)] - T.presum[cell_index(T, i - 1, x1, y1)]),
+    return static_cast<int>(fmin(fabs(T.presum[slot_index(T, i - 1, x0, y0)] - T.presum[slot_index(T, i - 1, x1, y1)]),
                                  static_cast<double>(kZInf / 2)));
 }
 

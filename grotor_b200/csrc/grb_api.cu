@@ -34,60 +34,54 @@ using namespace grb;
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kRefreshThreads = 256;       // threads of a prefix-tree CTA
+constexpr int kRefreshThreads = 256;
 constexpr int kPersistentThreads = 256;
 constexpr int kDpThreads = 128;
 constexpr unsigned long long kBarrierTimeoutNs = 20ull * 1000 * 1000 * 1000;
 constexpr int kPhaseSlots = 20;  // grb_phase_times entries
 constexpr int kNetTimeSlot = 12;  // per size bucket: summed net time [12..15], longest net [16..19]
 
-// update_dirty_costs (incremental_update.cuh:62-96): recompute dirty cells.
-__global__ void k_refresh_cells(Tables T) {
+// refresh_cost (incremental_update.cuh:98-132): one warp per wire track.
+__global__ void __launch_bounds__(kRefreshThreads, 2) k_refresh_tracks(Tables T) {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    refresh_dirty_cells<4>(T, warp, nwarps, lane);
-}
-
-// Prefix rebuild of dirty groups: pass 1 and pass 2 over (group, chunk) work
-// items, one warp each; the tree with one CTA per group.
-__global__ void k_collect_groups(Tables T) { collect_dirty_groups(T); }
-__global__ void __launch_bounds__(256, 2) k_prefix_pass1(Tables T) {
-    extern __shared__ __align__(16) char xsm[];
-    void* xs = xsm + (threadIdx.x >> 5) * prefix_xpose_bytes();
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int items = *T.group_count * T.tree_chunks;
-    for (int item = warp; item < items; item += nwarps) {
-        int g, c;
-        if (prefix_item(T, item, g, c)) prefix_pass1(T, g, c, lane, xs);
-    }
-}
-__global__ void __launch_bounds__(kRefreshThreads) k_prefix_tree(Tables T) {
-    extern __shared__ __align__(16) double tree[];
-    for (int k = blockIdx.x; k < *T.group_count; k += gridDim.x) prefix_tree(T, T.group_list[k], tree);
-}
-__global__ void __launch_bounds__(256, 2) k_prefix_pass2(Tables T) {
-    extern __shared__ __align__(16) char xsm[];
-    void* xs = xsm + (threadIdx.x >> 5) * prefix_xpose_bytes();
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int items = *T.group_count * T.tree_chunks;
-    for (int item = warp; item < items; item += nwarps) {
-        int g, c;
-        if (prefix_item(T, item, g, c)) prefix_pass2(T, g, c, lane, xs);
-    }
+    for (int t = warp; t < T.tracks; t += nwarps) refresh_track<4>(T, t, lane);
 }
 
 // Everything dirty: the state of a fresh database (first refresh is full).
 __global__ void k_mark_all_dirty(Tables T) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < T.words) {
-        const int rem = T.cells - i * 32;
-        const unsigned m = rem >= 32 ? 0xffffffffu : ((1u << rem) - 1u);
-        T.dirty_wire[i] = m;
-        T.dirty_via[i] = m;
+    if (i < T.words) T.dirty[i] = 0xffffffffu;  // bits behind a track's end are ignored
+}
+
+// Tables between the track layout and IDX order, 32 x 32 tiles of layers l0 to
+// l0 + gridDim.z - 1 (threads 32 x 8).  To IDX: dst[(l - l0) * XY + x * Y + y]
+// = src[slot]; to tracks: the reverse.
+template <class V, bool kToTracks>
+__global__ void k_layout(Tables T, const V* src, V* dst, int l0) {
+    __shared__ V tile[32][33];
+    const int l = l0 + blockIdx.z, x0 = blockIdx.y * 32, y0 = blockIdx.x * 32;
+    const size_t base = size_t(blockIdx.z) * T.XY;
+    const bool ay = along_y(T, l);
+    // Reading and writing with lanes over the fastest index of each side;
+    // layers along x change that index, so they go through the tile.
+    for (int q = threadIdx.y; q < 32; q += 8) {
+        const bool by_x = kToTracks ? false : !ay;  // lanes over x while reading
+        const int x = x0 + (by_x ? int(threadIdx.x) : q), y = y0 + (by_x ? q : int(threadIdx.x));
+        if (x < T.X && y < T.Y)
+            tile[by_x ? threadIdx.x : q][by_x ? q : threadIdx.x] =
+                kToTracks ? src[base + size_t(x) * T.Y + y] : src[slot_index(T, l, x, y)];
     }
-    if (i < T.n_groups) T.group_first[i] = 0;
+    __syncthreads();
+    for (int q = threadIdx.y; q < 32; q += 8) {
+        const bool by_x = kToTracks ? !ay : false;  // lanes over x while writing
+        const int x = x0 + (by_x ? int(threadIdx.x) : q), y = y0 + (by_x ? q : int(threadIdx.x));
+        if (x < T.X && y < T.Y) {
+            const V v = tile[by_x ? threadIdx.x : q][by_x ? q : threadIdx.x];
+            if (kToTracks) dst[slot_index(T, l, x, y)] = v;
+            else dst[base + size_t(x) * T.Y + y] = v;
+        }
+    }
 }
 
 __device__ __forceinline__ Arena warp_arena(char* smem, size_t arena_b, int warp, int L, int nmax) {
@@ -189,39 +183,19 @@ __global__ void k_commit_vias(Tables T, Plan P, int b, int stamp, int K) {
 }
 
 // refresh_cost (incremental_update.cuh:98-132) inside a persistent stage
-// kernel: dirty cells (block 0 also lists the dirty groups) | prefix pass 1 |
-// trees | pass 2, each phase ended by a grid barrier.  `smem`: the block's
-// dynamic shared memory (per-warp pass scratch, or the tree of the group a
-// block builds).  False when a barrier gave up.
+// kernel: every track by one warp, ended by a grid barrier.  False when the
+// barrier gave up.
 __device__ __forceinline__ bool refresh_persistent(const Tables& T, GridSync& S, PhaseClock& clk, int gwarp,
-                                                   int nwarps, int lane, char* smem) {
-    void* xs = smem + (threadIdx.x >> 5) * prefix_xpose_bytes();
-    if (blockIdx.x == 0) collect_dirty_groups(T);
-    refresh_dirty_cells<2>(T, gwarp, nwarps, lane);
+                                                   int nwarps, int lane) {
+    for (int t = gwarp; t < T.tracks; t += nwarps) refresh_track<2>(T, t, lane);
     if (!grid_sync(S, T)) return false;
     clk.mark(S, 4);
-    const int items = *reinterpret_cast<volatile int*>(T.group_count) * T.tree_chunks;
-    for (int item = gwarp; item < items; item += nwarps) {
-        int g, c;
-        if (prefix_item(T, item, g, c)) prefix_pass1(T, g, c, lane, xs);
-    }
-    if (!grid_sync(S, T)) return false;
-    for (int k = blockIdx.x; k < *reinterpret_cast<volatile int*>(T.group_count); k += gridDim.x)
-        prefix_tree(T, T.group_list[k], reinterpret_cast<double*>(smem));
-    if (!grid_sync(S, T)) return false;
-    for (int item = gwarp; item < items; item += nwarps) {
-        int g, c;
-        if (prefix_item(T, item, g, c)) prefix_pass2(T, g, c, lane, xs);
-    }
-    if (!grid_sync(S, T)) return false;
-    clk.mark(S, 7);
     return true;
 }
 
 // Persistent stage: every batch of the plan in one cooperative launch.
-// Per batch: recompute dirty cells (block 0 also lists the dirty prefix
-// groups) -> prefix pass 1 -> prefix trees -> prefix pass 2 -> route and commit
-// wires -> commit vias, separated by bounded grid barriers.
+// Per batch: refresh the tracks -> route and commit wires -> commit vias,
+// separated by bounded grid barriers.
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tables T, Plan P, GridSync S,
         int stamp0, int nmax, size_t arena_b, char* gscratch, size_t gslot, int* work, DpTune tune, StageTail tail) {
     extern __shared__ __align__(16) char smem[];
@@ -231,7 +205,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
     clk.start(S);
     for (int b = 0; b < P.n_batches; ++b) {
         const int stamp = stamp0 + b + 1;
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane, smem)) return;
+        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
         // Route every net of the batch and commit its wires: size buckets from
         // the largest down (long nets start first), nets taken from the
         // bucket's work queue `per_grab` at a time.  (In this kernel the
@@ -291,7 +265,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
     }
     // Rip-up classification and congestion view of the final demand, in the
     // same launch (no host round trip between the stage and them).
-    if (tail.flags) stage_tail_persistent(T, P, tail, S);
+    if (tail.flags) stage_tail_persistent(T, P, tail, S, reinterpret_cast<float (*)[kViewTile + 1]>(smem));
 }
 
 // --- FLT stage kernels (flt.cuh) --------------------------------------------
@@ -317,12 +291,11 @@ __global__ void k_flt_edges(Tables T, Flt F, Plan P2, int b) {
 }
 
 // Persistent FLT stage: per batch, [remove stage-one wires -> remove their
-// vias ->] refresh cells -> prefix pass 1 -> trees -> pass 2 -> layer-change
-// tables of the batch's edges -> FLT nets and wires -> vias, separated by
-// bounded grid barriers (flt.cuh:141-168 order).
+// vias ->] refresh the tracks -> layer-change tables of the batch's edges ->
+// FLT nets and wires -> vias, separated by bounded grid barriers
+// (flt.cuh:141-168 order).
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_flt_persistent(Tables T, Flt F, Plan P1, Plan P2,
         GridSync S, int stamp0, int remove, int* work) {
-    extern __shared__ __align__(16) char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * (blockDim.x >> 5);
     PhaseClock clk;
@@ -337,7 +310,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_flt_persistent(Tables
             if (!grid_sync(S, T)) return;
             clk.mark(S, 6);
         }
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane, smem)) return;
+        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
         flt_edges_batch(T, F, P2, b, gwarp, nwarps, lane);
         if (!grid_sync(S, T)) return;
         clk.mark(S, 10);
@@ -388,11 +361,10 @@ __global__ void k_commit_thread_vias(Tables T, Plan P, int b, int stamp) {
     if (i < cnt) commit_thread_vias(T, P, P.ids[lo + i], stamp, 1);
 }
 
-// Persistent Z-shape stage: per batch, refresh cells -> prefix pass 1 ->
-// trees -> pass 2 -> Z-shape nets and their wires -> vias.
+// Persistent Z-shape stage: per batch, refresh the tracks -> Z-shape nets and
+// their wires -> vias.
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_zshape_persistent(Tables T, ZTrees Z, Plan P, GridSync S,
                                                                               int stamp0, int* work) {
-    extern __shared__ __align__(16) char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * (blockDim.x >> 5);
     __shared__ int cand[kZCand];
@@ -402,7 +374,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_zshape_persistent(Tab
     for (int b = 0; b < P.n_batches; ++b) {
         const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
         const int stamp = stamp0 + b + 1;
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane, smem)) return;
+        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
         while (true) {  // one CTA per net
             if (threadIdx.x == 0) znet = atomicAdd(work + b, 1);
             __syncthreads();
@@ -988,7 +960,10 @@ __global__ void k_mark_overflow(Tables T, int threshold, int* of_sum) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < T.cells) overflow_mark(T, threshold, of_sum, c);
 }
-__global__ void k_int_prefix(Tables T, int* v) { overflow_prefix_track(T, v, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_int_prefix(Tables T, int* v) {  // one warp per track
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t < T.tracks) overflow_prefix_track(T, v, t, threadIdx.x & 31);
+}
 __global__ void k_overflow_nets(Tables T, Plan P, int n, const int* of_sum, unsigned char* is_of) {
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id < n) overflow_net(T, P, of_sum, is_of, id);
@@ -1003,8 +978,8 @@ __global__ void k_overflow_nets2(Tables T, Plan P, Plan P2, int n, const int* of
     is_of[id] = overflow_route(T, Q.routes + Q.route_off[id], Q.route_off[id + 1] > Q.route_off[id], of_sum);
 }
 __global__ void k_congestion(Tables T, unsigned char* cong, float* xsum, float* ysum) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < T.XY) congestion_cell(T, cong, xsum, ysum, i);
+    __shared__ float across[kViewTile][kViewTile + 1];
+    congestion_tile(T, cong, xsum, ysum, blockIdx.x, across);
 }
 __global__ void k_float_line_prefix(float* v, int lines, int len, int line_stride, int elem_stride) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1073,6 +1048,8 @@ struct grb_ctx {
     std::vector<int> h_batch_off;
     int plan_version = 0;
     // scratch
+    char* stage = nullptr;            // grb_read_tables: layers in IDX order
+    size_t stage_bytes = 0;
     char* gscratch = nullptr;
     size_t gscratch_bytes = 0;
     int* work = nullptr;
@@ -1224,6 +1201,9 @@ void free_all(std::vector<void*>& v) {
     v.clear();
 }
 
+// Grid of k_layout over `layers` layers.
+dim3 layout_grid(const Tables& T, int layers) { return dim3((T.Y + 31) / 32, (T.X + 31) / 32, layers); }
+
 int check_device_error(grb_ctx* c) {
     int err[2] = {0, 0};
     GRB_CUDA(c, cudaMemcpyAsync(err, c->T.error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1352,15 +1332,9 @@ int refresh_plain(grb_ctx* c) {
     cudaEvent_t e;
     int rc = prof_begin(c, 4, &e);
     if (rc) return rc;
-    k_collect_groups<<<1, 256, 0, c->stream>>>(T);
-    k_refresh_cells<<<c->sms * 8, 256, 0, c->stream>>>(T);
+    k_refresh_tracks<<<std::min((T.tracks + 7) / 8, c->sms * 8), kRefreshThreads, 0, c->stream>>>(T);
     prof_end(c, e);
-    if ((rc = prof_begin(c, 7, &e))) return rc;
-    k_prefix_pass1<<<c->sms * 8, 256, 8 * prefix_xpose_bytes(), c->stream>>>(T);
-    k_prefix_tree<<<c->sms * 2, kRefreshThreads, prefix_smem_bytes(std::max(T.X, T.Y)), c->stream>>>(T);
-    k_prefix_pass2<<<c->sms * 8, 256, 8 * prefix_xpose_bytes(), c->stream>>>(T);
-    prof_end(c, e);
-    c->launches += 5;
+    c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     return GRB_OK;
 }
@@ -1462,16 +1436,14 @@ int launch_tail(grb_ctx* c) {
     const StageTail t = make_tail(c);
     const Tables& T = c->T;
     if (t.flags & kTailRipup) {
-        int tracks = 0;
-        for (int l = 0; l < T.L; ++l) tracks += (((l & 1) ^ T.DIR) ? T.X : T.Y);
         k_mark_overflow<<<(T.cells + 255) / 256, 256, 0, c->stream>>>(T, t.threshold, t.of_sum);
-        k_int_prefix<<<(tracks + 127) / 128, 128, 0, c->stream>>>(T, t.of_sum);
+        k_int_prefix<<<(T.tracks + 3) / 4, 128, 0, c->stream>>>(T, t.of_sum);
         if (c->n_nets)
             k_overflow_nets<<<(c->n_nets + 255) / 256, 256, 0, c->stream>>>(T, make_plan(c), c->n_nets, t.of_sum, t.is_of);
         c->launches += c->n_nets ? 3 : 2;
     }
     if (t.flags & kTailView) {
-        k_congestion<<<(T.XY + 255) / 256, 256, 0, c->stream>>>(T, t.cong, t.xsum, t.ysum);
+        k_congestion<<<view_tiles(T), 256, 0, c->stream>>>(T, t.cong, t.xsum, t.ysum);
         k_float_line_prefix<<<(T.X + 127) / 128, 128, 0, c->stream>>>(t.ysum, T.X, T.Y, T.Y, 1);  // per x, along y
         k_float_line_prefix<<<(T.Y + 127) / 128, 128, 0, c->stream>>>(t.xsum, T.Y, T.X, 1, T.Y);  // per y, along x
         c->launches += 3;
@@ -1544,11 +1516,8 @@ int ensure_work(grb_ctx* c);
 
 int z_stage_persistent(grb_ctx* c, int stamp0) {
     if (c->n_batches == 0) return GRB_OK;
-    const size_t smem = std::max(prefix_smem_bytes(std::max(c->T.X, c->T.Y)),
-                                 size_t(kPersistentThreads / 32) * prefix_xpose_bytes());
-    GRB_CUDA(c, cudaFuncSetAttribute(k_zshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
-    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, smem));
+    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, 0));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent Z-shape kernel does not fit on an SM");
     int rc = ensure_work(c);
     if (rc) return rc;
@@ -1559,7 +1528,7 @@ int z_stage_persistent(grb_ctx* c, int stamp0) {
     GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
     void* args[] = {&T, &Z, &P, &S, &stamp0, &c->work};
     GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_zshape_persistent, dim3(per_sm * c->sms), dim3(kPersistentThreads),
-                                            args, smem, c->stream));
+                                            args, 0, c->stream));
     c->launches += 1;
     return GRB_OK;
 }
@@ -1715,11 +1684,8 @@ int ensure_work(grb_ctx* c) {
 
 int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
     if (c->n_batches == 0) return GRB_OK;
-    const size_t smem = std::max(prefix_smem_bytes(std::max(c->T.X, c->T.Y)),
-                                 size_t(kPersistentThreads / 32) * prefix_xpose_bytes());
-    GRB_CUDA(c, cudaFuncSetAttribute(k_flt_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
-    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, smem));
+    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, 0));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent FLT kernel does not fit on an SM");
     int rc = ensure_work(c);
     if (rc) return rc;
@@ -1730,7 +1696,7 @@ int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
     GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
     void* args[] = {&T, &F, &P1, &P2, &S, &stamp0, &remove, &c->work};
     GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_flt_persistent, dim3(per_sm * c->sms), dim3(kPersistentThreads),
-                                            args, smem, c->stream));
+                                            args, 0, c->stream));
     c->launches += 1;
     return GRB_OK;
 }
@@ -1773,8 +1739,7 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     // A warp's arena also holds the lane-per-net scratch of the smallest nets.
     const size_t ab = std::max(arena_bytes(c->T.L, nmax), (pair_scratch_bytes() + 15) & ~size_t(15));
     const int wpb = kPersistentThreads / 32;
-    const size_t prefix_smem = prefix_smem_bytes(std::max(c->T.X, c->T.Y));  // prefix_tree
-    const size_t smem = std::max(std::max(ab * wpb, prefix_smem), size_t(wpb) * prefix_xpose_bytes());
+    const size_t smem = std::max(ab * wpb, sizeof(float) * kViewTile * (kViewTile + 1));  // the tail's view tile
     GRB_CUDA(c, cudaFuncSetAttribute(k_lshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lshape_persistent, kPersistentThreads, smem));
@@ -1864,6 +1829,32 @@ static int launch_batching(grb_ctx* c, BatchState& B, int mode, size_t smem) {
     return GRB_OK;
 }
 
+// Copy a table to the host in IDX order, some layers at a time through a
+// staging buffer kept in the context (at most kStageBytes, or one layer).
+constexpr size_t kStageBytes = size_t(64) << 20;
+template <class V>
+int read_table(grb_ctx* c, const V* table, V* host) {
+    const Tables& T = c->T;
+    const int layers = int(std::min<size_t>(T.L, std::max<size_t>(1, kStageBytes / (sizeof(V) * size_t(T.XY)))));
+    const size_t need = sizeof(V) * size_t(T.XY) * layers;
+    if (c->stage_bytes < need) {
+        if (c->stage) cudaFree(c->stage);
+        c->stage = nullptr;
+        c->stage_bytes = 0;
+        if (cudaMalloc(&c->stage, need) != cudaSuccess) { cudaGetLastError(); return fail(c, GRB_ENOMEM, "table staging"); }
+        c->stage_bytes = need;
+    }
+    for (int l0 = 0; l0 < T.L; l0 += layers) {
+        const int nl = std::min(layers, T.L - l0);
+        k_layout<V, false><<<layout_grid(T, nl), dim3(32, 8), 0, c->stream>>>(T, table, reinterpret_cast<V*>(c->stage), l0);
+        c->launches += 1;
+        GRB_CUDA(c, cudaGetLastError());
+        GRB_CUDA(c, cudaMemcpyAsync(host + size_t(l0) * T.XY, c->stage, sizeof(V) * size_t(T.XY) * nl,
+                                    cudaMemcpyDeviceToHost, c->stream));
+    }
+    return GRB_OK;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1880,8 +1871,7 @@ int grb_init_device(int32_t device) {
     // kernels every stage starts with.
     const void* kernels[] = {(const void*)k_batch_persistent<kChunkMax>, (const void*)k_lshape_persistent,
                              (const void*)k_flt_persistent, (const void*)k_zshape_persistent,
-                             (const void*)k_refresh_cells, (const void*)k_prefix_pass1, (const void*)k_prefix_pass2,
-                             (const void*)k_lshape_bucketed, (const void*)k_topo_fill, (const void*)k_out_write};
+                             (const void*)k_refresh_tracks, (const void*)k_lshape_bucketed, (const void*)k_topo_fill, (const void*)k_out_write};
     for (const void* k : kernels) {
         cudaFuncAttributes a{};
         if (cudaFuncGetAttributes(&a, k) != cudaSuccess) {
@@ -1913,49 +1903,68 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     T.unit_wire = g->unit_length_wire_cost; T.unit_via = g->unit_via_cost;
     T.of_scale = g->of_cost_scale;
     const size_t cells = T.cells;
-    T.words = int((cells + 31) / 32);
-    int ng = 0;
-    for (int l = 0; l < T.L; ++l) {
-        T.group_base[l] = ng;
-        const int tracks = (((l & 1) ^ T.DIR) ? T.X : T.Y);
-        ng += (tracks + kTrackGroup - 1) / kTrackGroup;
-    }
-    T.group_base[T.L] = ng;
-    for (int l = T.L + 1; l <= kMaxLayers; ++l) T.group_base[l] = ng;
-    T.n_groups = ng;
+    T.by_xy = fast_div(T.XY);
+    T.by_x = fast_div(T.X);
+    T.by_y = fast_div(T.Y);
+    T.xp = (T.X + 31) / 32 * 32;
+    T.yp = (T.Y + 31) / 32 * 32;
+    const int y_layer = T.X * T.yp, x_layer = T.Y * T.xp;  // slots of a layer along y, along x
+    T.even_slots = T.DIR ? y_layer : x_layer;
+    T.pair_slots = y_layer + x_layer;
+    T.slots = (T.L >> 1) * T.pair_slots + ((T.L & 1) ? T.even_slots : 0);
+    T.tracks = (T.L >> 1) * (T.X + T.Y) + ((T.L & 1) ? (T.DIR ? T.X : T.Y) : 0);
+    T.track_blocks = (std::max(T.X, T.Y) + kScanBlock - 1) / kScanBlock;
+    T.words = T.slots / 32;
+    const size_t slots = T.slots;
     grb_ctx* cp = c.get();
-    double* sc; int* xl; int* yl; float* cap;
+    double *sc, *xd, *yd; int* xl; int* yl; float* cap;
     int rc = 0;
     rc |= dalloc(cp, &sc, T.L, cp->owned);
     rc |= dalloc(cp, &xl, T.X - 1, cp->owned);
     rc |= dalloc(cp, &yl, T.Y - 1, cp->owned);
-    rc |= dalloc(cp, &cap, cells, cp->owned);
-    rc |= dalloc(cp, &T.demand, cells, cp->owned);
-    rc |= dalloc(cp, &T.ts, cells, cp->owned);
-    rc |= dalloc(cp, &T.wcost, cells, cp->owned);
-    rc |= dalloc(cp, &T.vcost, cells, cp->owned);
-    rc |= dalloc(cp, &T.presum, cells, cp->owned);
-    rc |= dalloc(cp, &T.dirty_wire, T.words, cp->owned);
-    rc |= dalloc(cp, &T.dirty_via, T.words, cp->owned);
-    rc |= dalloc(cp, &T.group_first, ng, cp->owned);
-    rc |= dalloc(cp, &T.first_list, ng, cp->owned);
-    rc |= dalloc(cp, &T.group_list, ng, cp->owned);
-    rc |= dalloc(cp, &T.group_count, 1, cp->owned);
-    T.tree_chunks = prefix_chunks(std::max(T.X, T.Y));
-    T.tree_stride = prefix_tree_entries(std::max(T.X, T.Y));
-    rc |= dalloc(cp, &T.ptree, size_t(ng) * T.tree_stride * 32, cp->owned);
-
+    rc |= dalloc(cp, &xd, T.X, cp->owned);
+    rc |= dalloc(cp, &yd, T.Y, cp->owned);
+    rc |= dalloc(cp, &cap, slots, cp->owned);
+    rc |= dalloc(cp, &T.demand, slots, cp->owned);
+    rc |= dalloc(cp, &T.ts, slots, cp->owned);
+    rc |= dalloc(cp, &T.wcost, slots, cp->owned);
+    rc |= dalloc(cp, &T.vcost, slots, cp->owned);
+    rc |= dalloc(cp, &T.presum, slots, cp->owned);
+    rc |= dalloc(cp, &T.dirty, T.words, cp->owned);
+    rc |= dalloc(cp, &T.block_total, size_t(T.tracks) * T.track_blocks, cp->owned);
     rc |= dalloc(cp, &T.wirelength, 1, cp->owned);
     rc |= dalloc(cp, &T.vias, 1, cp->owned);
     rc |= dalloc(cp, &T.error, 2, cp->owned);
     rc |= dalloc(cp, &c->sync, 2, cp->owned);
     if (rc) { free_all(cp->owned); return GRB_ENOMEM; }
     T.error_info = T.error + 1;
-    T.short_costs = sc; T.xlen = xl; T.ylen = yl; T.capacity = cap;
+    T.short_costs = sc; T.xlen = xl; T.ylen = yl; T.capacity = cap; T.xdist = xd; T.ydist = yd;
     GRB_CUDA(cp, cudaMemcpy(sc, g->unit_length_short_costs, sizeof(double) * T.L, cudaMemcpyHostToDevice));
     GRB_CUDA(cp, cudaMemcpy(xl, g->x_edge_len, sizeof(int) * (T.X - 1), cudaMemcpyHostToDevice));
     GRB_CUDA(cp, cudaMemcpy(yl, g->y_edge_len, sizeof(int) * (T.Y - 1), cudaMemcpyHostToDevice));
-    GRB_CUDA(cp, cudaMemcpy(cap, g->capacity, sizeof(float) * cells, cudaMemcpyHostToDevice));
+    for (int k = 0; k < 2; ++k) {  // distances of the grid lines (integers: exact)
+        const int n = k ? T.Y : T.X;
+        const int* len = k ? g->y_edge_len : g->x_edge_len;
+        std::vector<double> dist(n, 0.0);
+        for (int i = 1; i < n; ++i) dist[i] = dist[i - 1] + len[i - 1];
+        GRB_CUDA(cp, cudaMemcpy(k ? yd : xd, dist.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+    }
+    // The cells behind a track's end are never a cell of the grid; the prefix
+    // pass loads (and ignores) the wire costs there.
+    GRB_CUDA(cp, cudaMemset(T.wcost, 0, sizeof(float) * slots));
+    GRB_CUDA(cp, cudaMemset(cap, 0, sizeof(float) * slots));
+    {
+        std::vector<void*> up;
+        float* d_cap = nullptr;
+        if (dalloc(cp, &d_cap, cells, up)) { free_all(cp->owned); return GRB_ENOMEM; }
+        cudaError_t e = cudaMemcpy(d_cap, g->capacity, sizeof(float) * cells, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) {
+            k_layout<float, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, d_cap, cap, 0);
+            e = cudaDeviceSynchronize();
+        }
+        free_all(up);
+        GRB_CUDA(cp, e);
+    }
     GRB_CUDA(cp, cudaMemset(T.error, 0, 2 * sizeof(int)));
     {
         // Distinct capacity values (at most kNoCapRow of them get table rows;
@@ -1988,14 +1997,24 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
         T.of_dmax = caps.empty() ? 0 : kOfDmax;
         T.of_rows = rows;
         T.of_stride = kOfDmax;
-        if (dalloc(cp, &d_cid, cells, cp->owned) ||
+        std::vector<void*> up;
+        unsigned char* d_up = nullptr;
+        if (dalloc(cp, &d_cid, slots, cp->owned) || dalloc(cp, &d_up, cells, up) ||
             dalloc(cp, &d_table, size_t(T.L) * rows * T.of_stride, cp->owned) || dalloc(cp, &d_caps, rows, cp->owned)) {
+            free_all(up);
             free_all(cp->owned);
             return GRB_ENOMEM;
         }
         T.cap_id = d_cid;
         T.of_table = d_table;
-        GRB_CUDA(cp, cudaMemcpy(d_cid, cid.data(), cells, cudaMemcpyHostToDevice));
+        cudaError_t e = cudaMemcpy(d_up, cid.data(), cells, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemset(d_cid, 0, slots);
+        if (e == cudaSuccess) {
+            k_layout<unsigned char, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, d_up, d_cid, 0);
+            e = cudaDeviceSynchronize();
+        }
+        free_all(up);
+        GRB_CUDA(cp, e);
         if (!caps.empty()) {
             GRB_CUDA(cp, cudaMemcpy(d_caps, caps.data(), sizeof(float) * caps.size(), cudaMemcpyHostToDevice));
             const int n = T.L * rows * T.of_stride;
@@ -2010,10 +2029,6 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_bucketed, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_prefix_pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, int(8 * prefix_xpose_bytes())));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_prefix_pass2, cudaFuncAttributeMaxDynamicSharedMemorySize, int(8 * prefix_xpose_bytes())));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_prefix_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(prefix_smem_bytes(std::max(T.X, T.Y)))));
     const int r = grb_reset(cp);
     if (r) { const int code = r; free_all(cp->owned); return code; }
     *out = c.release();
@@ -2052,7 +2067,7 @@ void grb_destroy(grb_ctx* c) {
     if (c->ckpt_demand) cudaFree(c->ckpt_demand);
     if (c->score_partials) cudaFree(c->score_partials);
     free_all(c->owned);
-    for (void* p : {(void*)c->check, (void*)c->bucket_ids, (void*)c->bucket_off, (void*)c->ids, (void*)c->batch_off, (void*)c->gscratch, (void*)c->work, (void*)c->cellmask,
+    for (void* p : {(void*)c->check, (void*)c->stage, (void*)c->bucket_ids, (void*)c->bucket_off, (void*)c->ids, (void*)c->batch_off, (void*)c->gscratch, (void*)c->work, (void*)c->cellmask,
                     (void*)c->lmask[0], (void*)c->lmask[1], (void*)c->lmask[2], (void*)c->lmask[3], (void*)c->lmask[4],
                     (void*)c->ptchunk, (void*)c->fmask, (void*)c->pred, (void*)c->prevp,
                     (void*)c->bsolved, (void*)c->fullmask, (void*)c->bcount, (void*)c->ncolors, (void*)c->batch_of, (void*)c->brank,
@@ -2073,14 +2088,12 @@ int grb_reset(grb_ctx* c) {
     if (!c) return GRB_EINVAL;
     GRB_CUDA(c, cudaSetDevice(c->device));
     Tables& T = c->T;
-    const size_t cells = T.cells;
-    GRB_CUDA(c, cudaMemsetAsync(T.demand, 0, sizeof(int) * cells, c->stream));
-    GRB_CUDA(c, cudaMemsetAsync(T.ts, 0, sizeof(int) * cells, c->stream));
+    GRB_CUDA(c, cudaMemsetAsync(T.demand, 0, sizeof(int) * size_t(T.slots), c->stream));
+    GRB_CUDA(c, cudaMemsetAsync(T.ts, 0, sizeof(int) * size_t(T.slots), c->stream));
     GRB_CUDA(c, cudaMemsetAsync(T.wirelength, 0, sizeof(double), c->stream));
     GRB_CUDA(c, cudaMemsetAsync(T.vias, 0, sizeof(unsigned long long), c->stream));
     if (c->routes) GRB_CUDA(c, cudaMemsetAsync(c->routes, 0, sizeof(int) * std::max<long long>(c->route_words, 1), c->stream));
-    const int n = std::max(T.words, T.n_groups);
-    k_mark_all_dirty<<<(n + 255) / 256, 256, 0, c->stream>>>(T);
+    k_mark_all_dirty<<<(T.words + 255) / 256, 256, 0, c->stream>>>(T);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     c->stamp = 0;
@@ -2484,11 +2497,11 @@ int grb_routing_score(grb_ctx* c, double* score) {
 int grb_checkpoint(grb_ctx* c) {
     if (!c) return GRB_EINVAL;
     GRB_CUDA(c, cudaSetDevice(c->device));
-    if (!c->ckpt_demand && cudaMalloc(&c->ckpt_demand, sizeof(int) * size_t(c->T.cells)) != cudaSuccess) {
+    if (!c->ckpt_demand && cudaMalloc(&c->ckpt_demand, sizeof(int) * size_t(c->T.slots)) != cudaSuccess) {
         cudaGetLastError();
         return fail(c, GRB_ENOMEM, "checkpoint");
     }
-    GRB_CUDA(c, cudaMemcpyAsync(c->ckpt_demand, c->T.demand, sizeof(int) * size_t(c->T.cells), cudaMemcpyDeviceToDevice,
+    GRB_CUDA(c, cudaMemcpyAsync(c->ckpt_demand, c->T.demand, sizeof(int) * size_t(c->T.slots), cudaMemcpyDeviceToDevice,
                                 c->stream));
     GRB_CUDA(c, cudaMemcpyAsync(&c->ckpt_wirelength, c->T.wirelength, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     GRB_CUDA(c, cudaMemcpyAsync(&c->ckpt_vias, c->T.vias, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
@@ -2500,13 +2513,13 @@ int grb_restore(grb_ctx* c) {
     if (!c) return GRB_EINVAL;
     if (!c->ckpt_demand) return fail(c, GRB_EINVAL, "no checkpoint");
     GRB_CUDA(c, cudaSetDevice(c->device));
-    GRB_CUDA(c, cudaMemcpyAsync(c->T.demand, c->ckpt_demand, sizeof(int) * size_t(c->T.cells), cudaMemcpyDeviceToDevice,
+    GRB_CUDA(c, cudaMemcpyAsync(c->T.demand, c->ckpt_demand, sizeof(int) * size_t(c->T.slots), cudaMemcpyDeviceToDevice,
                                 c->stream));
     GRB_CUDA(c, cudaMemcpyAsync(c->T.wirelength, &c->ckpt_wirelength, sizeof(double), cudaMemcpyHostToDevice, c->stream));
     GRB_CUDA(c, cudaMemcpyAsync(c->T.vias, &c->ckpt_vias, sizeof(unsigned long long), cudaMemcpyHostToDevice, c->stream));
     // Every cost is recomputed at the next refresh (the reference clears
     // costs_initialized, maze_quality.cuh:100).
-    k_mark_all_dirty<<<(c->T.cells + 255) / 256, 256, 0, c->stream>>>(c->T);
+    k_mark_all_dirty<<<(c->T.words + 255) / 256, 256, 0, c->stream>>>(c->T);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -2546,8 +2559,7 @@ int grb_set_wire_cost_mode(grb_ctx* c, int32_t integer_wire) {
     GRB_CUDA(c, cudaSetDevice(c->device));
     c->T.int_wire = integer_wire ? 1 : 0;
     // Every wire cost changes: the next refresh recomputes all cells and tracks.
-    const int n = std::max(c->T.words, c->T.n_groups);
-    k_mark_all_dirty<<<(n + 255) / 256, 256, 0, c->stream>>>(c->T);
+    k_mark_all_dirty<<<(c->T.words + 255) / 256, 256, 0, c->stream>>>(c->T);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -3435,10 +3447,8 @@ static int ripup_classify(grb_ctx* c, int32_t threshold, const uint8_t* phase2, 
     }
     if (phase2 && c->n_nets)
         GRB_CUDA(c, cudaMemcpyAsync(d_phase2, phase2, size_t(c->n_nets), cudaMemcpyHostToDevice, c->stream));
-    int tracks = 0;
-    for (int l = 0; l < c->T.L; ++l) tracks += (((l & 1) ^ c->T.DIR) ? c->T.X : c->T.Y);
     k_mark_overflow<<<(c->T.cells + 255) / 256, 256, 0, c->stream>>>(c->T, threshold, of_sum);
-    k_int_prefix<<<(tracks + 127) / 128, 128, 0, c->stream>>>(c->T, of_sum);
+    k_int_prefix<<<(c->T.tracks + 3) / 4, 128, 0, c->stream>>>(c->T, of_sum);
     Plan P = make_plan(c);
     if (c->n_nets && phase2)
         k_overflow_nets2<<<(c->n_nets + 255) / 256, 256, 0, c->stream>>>(c->T, P, make_plan2(c), c->n_nets, of_sum,
@@ -3492,10 +3502,8 @@ int grb_ripup_classify_noalloc(grb_ctx* c, int32_t threshold, uint8_t* is_of) {
     // mark per cell, one flag per net), so nothing has to be cleared first.
     int* of_sum = scratch;
     unsigned char* flags = reinterpret_cast<unsigned char*>(scratch + kNoAllocCells);
-    int tracks = 0;
-    for (int l = 0; l < c->T.L; ++l) tracks += (((l & 1) ^ c->T.DIR) ? c->T.X : c->T.Y);
     k_mark_overflow<<<(c->T.cells + 255) / 256, 256, 0, c->stream>>>(c->T, threshold, of_sum);
-    k_int_prefix<<<(tracks + 127) / 128, 128, 0, c->stream>>>(c->T, of_sum);
+    k_int_prefix<<<(c->T.tracks + 3) / 4, 128, 0, c->stream>>>(c->T, of_sum);
     Plan P = make_plan(c);
     if (c->n_nets) k_overflow_nets<<<(c->n_nets + 255) / 256, 256, 0, c->stream>>>(c->T, P, c->n_nets, of_sum, flags);
     c->launches += c->n_nets ? 3 : 2;
@@ -3573,7 +3581,7 @@ int grb_congestion_view(grb_ctx* c, uint8_t* congestion, float* xsum, float* ysu
         for (void* p : {(void*)d_c, (void*)d_x, (void*)d_y}) if (p) cudaFree(p);
         return fail(c, GRB_ENOMEM, "congestion buffers");
     }
-    k_congestion<<<(XY + 255) / 256, 256, 0, c->stream>>>(c->T, d_c, d_x, d_y);
+    k_congestion<<<view_tiles(c->T), 256, 0, c->stream>>>(c->T, d_c, d_x, d_y);
     k_float_line_prefix<<<(X + 127) / 128, 128, 0, c->stream>>>(d_y, X, Y, Y, 1);   // per x, along y
     k_float_line_prefix<<<(Y + 127) / 128, 128, 0, c->stream>>>(d_x, Y, X, 1, Y);   // per y, along x
     c->launches += 3;
@@ -3590,12 +3598,12 @@ int grb_congestion_view(grb_ctx* c, uint8_t* congestion, float* xsum, float* ysu
 int grb_read_tables(grb_ctx* c, float* wcost, float* vcost, double* presum, int32_t* demand_half, int32_t* timestamp) {
     if (!c) return GRB_EINVAL;
     GRB_CUDA(c, cudaSetDevice(c->device));
-    const size_t cells = c->T.cells;
-    if (wcost) GRB_CUDA(c, cudaMemcpyAsync(wcost, c->T.wcost, 4 * cells, cudaMemcpyDeviceToHost, c->stream));
-    if (vcost) GRB_CUDA(c, cudaMemcpyAsync(vcost, c->T.vcost, 4 * cells, cudaMemcpyDeviceToHost, c->stream));
-    if (presum) GRB_CUDA(c, cudaMemcpyAsync(presum, c->T.presum, 8 * cells, cudaMemcpyDeviceToHost, c->stream));
-    if (demand_half) GRB_CUDA(c, cudaMemcpyAsync(demand_half, c->T.demand, 4 * cells, cudaMemcpyDeviceToHost, c->stream));
-    if (timestamp) GRB_CUDA(c, cudaMemcpyAsync(timestamp, c->T.ts, 4 * cells, cudaMemcpyDeviceToHost, c->stream));
+    int rc;
+    if (wcost && (rc = read_table(c, c->T.wcost, wcost))) return rc;
+    if (vcost && (rc = read_table(c, c->T.vcost, vcost))) return rc;
+    if (presum && (rc = read_table(c, c->T.presum, presum))) return rc;
+    if (demand_half && (rc = read_table(c, c->T.demand, demand_half))) return rc;
+    if (timestamp && (rc = read_table(c, c->T.ts, timestamp))) return rc;
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     return check_device_error(c);
 }
