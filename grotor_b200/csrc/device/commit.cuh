@@ -13,23 +13,25 @@
 namespace grb {
 
 __device__ __forceinline__ const int* net_routes(const Plan& P, int id) { return P.routes + P.route_off[id]; }
+// Words of the net's route in use: its count word, 0 for a net without route
+// storage, never beyond the storage.
+__device__ __forceinline__ int net_words(const Plan& P, int id) {
+    const long long off = P.route_off[id], cap = P.route_off[id + 1] - off;
+    return cap > 0 ? static_cast<int>(min(static_cast<long long>(P.routes[off]), cap)) : 0;
+}
 
 // A wire segment as its run of edges on a track: first slot and edge count
-// (n = 0: no wire, or a single cell), its end cells stamped by the caller.
-// `skew`: the segment runs across its layer's direction (no router emits
-// that; a caller's own routes may), so its cells are not consecutive.
+// (n = 0: a single cell).  `skew`: the segment runs across its layer's
+// direction (no router emits that; a caller's own routes may), so its cells
+// are not consecutive.
 struct WireRun {
-    int first, n;
-    bool wire, skew;
-    double length;
+    int first = 0, n = 0;
+    bool wire = false, skew = false;
+    double length = 0.0;
 };
-__device__ __forceinline__ WireRun wire_run(const Tables& T, int a, int b) {
-    WireRun R{0, 0, false, false, 0.0};
-    int l, x0, y0, lb, x1, y1;
-    cell_position(T, a, l, x0, y0);
-    cell_position(T, b, lb, x1, y1);
-    R.wire = l == lb;
-    if (!R.wire) return R;
+__device__ __forceinline__ WireRun run_between(const Tables& T, int l, int x0, int y0, int x1, int y1) {
+    WireRun R;
+    R.wire = true;
     const bool ay = x0 == x1;
     const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
     R.n = hi - lo;
@@ -37,6 +39,12 @@ __device__ __forceinline__ WireRun wire_run(const Tables& T, int a, int b) {
     R.first = slot_index(T, l, ay ? x0 : lo, ay ? lo : y0);
     R.length = ay ? T.ydist[hi] - T.ydist[lo] : T.xdist[hi] - T.xdist[lo];
     return R;
+}
+__device__ __forceinline__ WireRun wire_run(const Tables& T, int a, int b) {
+    int l, x0, y0, lb, x1, y1;
+    cell_position(T, a, l, x0, y0);
+    cell_position(T, b, lb, x1, y1);
+    return l == lb ? run_between(T, l, x0, y0, x1, y1) : WireRun();
 }
 
 // Edge at slot c of a segment gets K; its cell is stamped.
@@ -73,20 +81,63 @@ __device__ __forceinline__ void stamp_ends(const Tables& T, const WireRun& R, in
     }
 }
 
-// One warp commits the wire segments of net `id` (of `parts` warps sharing a
-// net, warp `part` takes every parts-th group of 32 segments).  Each lane
-// decodes one segment; then the edges of all short segments are shared out
-// over the lanes together, and each long one takes the whole warp.  A run's
-// edges are consecutive slots, so its dirty bits are set a bitmap word at a
-// time by the edge that opens the word (fenwick.cuh:51-78).
+// The edges of one run per lane (n = 0: none) are committed by the warp: those
+// of all short runs shared out over the lanes together, each long run by the
+// whole warp.  A run's edges are consecutive slots, so its dirty bits are set
+// a bitmap word at a time by the edge that opens the word
+// (fenwick.cuh:51-78).
 constexpr int kLongRun = 64;
+__device__ __forceinline__ void commit_runs(const Tables& T, int run_first, int n, int stamp, int K, int lane) {
+    unsigned longs = __ballot_sync(0xffffffffu, n >= kLongRun);
+    while (longs) {
+        const int q = __ffs(longs) - 1;
+        longs &= longs - 1;
+        const int first = __shfl_sync(0xffffffffu, run_first, q), last = first + __shfl_sync(0xffffffffu, n, q) - 1;
+        for (int c = first + lane; c <= last; c += 32) commit_edge(T, c, stamp, K);
+        for (int w = (first >> 5) + lane; w <= (last >> 5); w += 32) red_or(T.dirty + w, range_bits(w, first, last));
+    }
+    const int m = n < kLongRun ? n : 0;
+    int incl = m;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int k0 = 0; k0 < total; k0 += 32) {
+        const int k = k0 + lane;
+        int q = 0;  // the run of edge k: the first with incl > k
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+            const int v = __shfl_sync(0xffffffffu, incl, q + step - 1);
+            if (v <= k) q += step;
+        }
+        const int first = __shfl_sync(0xffffffffu, run_first, q), cnt = __shfl_sync(0xffffffffu, m, q);
+        const int end = __shfl_sync(0xffffffffu, incl, q);
+        if (k < total) {
+            const int c = first + (k - (end - cnt));
+            commit_edge(T, c, stamp, K);
+            if (c == first || (c & 31) == 0) red_or(T.dirty + (c >> 5), range_bits(c >> 5, first, first + cnt - 1));
+        }
+    }
+}
+
+// Sum of `length` over the warp into the wirelength.
+__device__ __forceinline__ void add_wirelength(const Tables& T, double length, int K, int lane) {
+    for (int s = 16; s; s >>= 1) length += __shfl_down_sync(0xffffffffu, length, s);
+    if (lane == 0 && length != 0.0) atomicAdd(T.wirelength, length * K);
+}
+
+// One warp commits the wire segments of net `id` (of `parts` warps sharing a
+// net, warp `part` takes every parts-th group of 32 segments), one segment per
+// lane.
 __device__ __forceinline__ void commit_net_wires(const Tables& T, const Plan& P, int id, int stamp, int K,
                                                  int lane, int part = 0, int parts = 1) {
     const int* r = net_routes(P, id);
-    const int segs = (r[0] - 1) / 2;
+    const int segs = (net_words(P, id) - 1) / 2;
     double length = 0;
     for (int s0 = 32 * part; s0 < segs; s0 += 32 * parts) {
-        WireRun R{0, 0, false, false, 0.0};
+        WireRun R;
         if (s0 + lane < segs) {
             const int a = r[1 + 2 * (s0 + lane)], b = r[2 + 2 * (s0 + lane)];
             R = wire_run(T, a, b);
@@ -96,42 +147,9 @@ __device__ __forceinline__ void commit_net_wires(const Tables& T, const Plan& P,
                 if (R.skew) commit_skew(T, a, b, stamp, K);
             }
         }
-        const int n = R.wire && !R.skew ? R.n : 0;
-        unsigned longs = __ballot_sync(0xffffffffu, n >= kLongRun);
-        while (longs) {
-            const int q = __ffs(longs) - 1;
-            longs &= longs - 1;
-            const int first = __shfl_sync(0xffffffffu, R.first, q), last = first + __shfl_sync(0xffffffffu, n, q) - 1;
-            for (int c = first + lane; c <= last; c += 32) commit_edge(T, c, stamp, K);
-            for (int w = (first >> 5) + lane; w <= (last >> 5); w += 32) red_or(T.dirty + w, range_bits(w, first, last));
-        }
-        const int m = n < kLongRun ? n : 0;
-        int incl = m;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += o;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        for (int k0 = 0; k0 < total; k0 += 32) {
-            const int k = k0 + lane;
-            int q = 0;  // the segment of edge k: the first with incl > k
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const int v = __shfl_sync(0xffffffffu, incl, q + step - 1);
-                if (v <= k) q += step;
-            }
-            const int first = __shfl_sync(0xffffffffu, R.first, q), cnt = __shfl_sync(0xffffffffu, m, q);
-            const int end = __shfl_sync(0xffffffffu, incl, q);
-            if (k < total) {
-                const int c = first + (k - (end - cnt));
-                commit_edge(T, c, stamp, K);
-                if (c == first || (c & 31) == 0) red_or(T.dirty + (c >> 5), range_bits(c >> 5, first, first + cnt - 1));
-            }
-        }
+        commit_runs(T, R.first, R.skew ? 0 : R.n, stamp, K, lane);
     }
-    for (int s = 16; s; s >>= 1) length += __shfl_down_sync(0xffffffffu, length, s);
-    if (lane == 0 && length != 0.0) atomicAdd(T.wirelength, length * K);
+    add_wirelength(T, length, K, lane);
 }
 
 // Via demand on the edge at slot c.
@@ -199,7 +217,7 @@ __device__ __forceinline__ void commit_vias_strided(const Tables& T, const Plan&
         {
             const int* r = P.routes + __shfl_sync(0xffffffffu, off, 0);
             const long long c = __shfl_sync(0xffffffffu, cap, 0);
-            words = r[0];
+            words = c > 0 ? static_cast<int>(min(static_cast<long long>(r[0]), c)) : 0;
             if (i0 + 1 < c) { a = r[i0]; b = r[i0 + 1]; }
         }
         for (int j = 0; j < nn; ++j) {
@@ -209,11 +227,11 @@ __device__ __forceinline__ void commit_vias_strided(const Tables& T, const Plan&
             if (j + 1 < nn) {
                 const int* rn = P.routes + __shfl_sync(0xffffffffu, off, j + 1);
                 const long long nc = __shfl_sync(0xffffffffu, cap, j + 1);
-                words = rn[0];
+                words = nc > 0 ? static_cast<int>(min(static_cast<long long>(rn[0]), nc)) : 0;
                 if (i0 + 1 < nc) { a = rn[i0]; b = rn[i0 + 1]; }
             }
-            if (i0 < cw) vias += i0 + 1 < c ? via_segment(T, ca, cb, stamp, K) : via_segment(T, r[i0], r[i0 + 1], stamp, K);
-            for (int i = i0 + 64; i < cw; i += 64) vias += via_segment(T, r[i], r[i + 1], stamp, K);
+            if (i0 + 1 < cw) vias += via_segment(T, ca, cb, stamp, K);
+            for (int i = i0 + 64; i + 1 < cw; i += 64) vias += via_segment(T, r[i], r[i + 1], stamp, K);
         }
     }
     for (int s = 16; s; s >>= 1) vias += __shfl_down_sync(0xffffffffu, vias, s);
@@ -226,9 +244,9 @@ __device__ __forceinline__ void commit_vias_strided(const Tables& T, const Plan&
 // the warp forms above.
 __device__ __forceinline__ void commit_thread_wires(const Tables& T, const Plan& P, int id, int stamp, int K) {
     const int* r = net_routes(P, id);
-    const int words = r[0];
+    const int words = net_words(P, id);
     double length = 0;
-    for (int i = 1; i < words; i += 2) {
+    for (int i = 1; i + 1 < words; i += 2) {
         const int a = r[i], b = r[i + 1];
         const WireRun R = wire_run(T, a, b);
         if (!R.wire) continue;
@@ -245,9 +263,9 @@ __device__ __forceinline__ void commit_thread_wires(const Tables& T, const Plan&
 
 __device__ __forceinline__ void commit_thread_vias(const Tables& T, const Plan& P, int id, int stamp, int K) {
     const int* r = net_routes(P, id);
-    const int words = r[0];
+    const int words = net_words(P, id);
     long long vias = 0;
-    for (int i = 1; i < words; i += 2) vias += via_segment(T, r[i], r[i + 1], stamp, K);
+    for (int i = 1; i + 1 < words; i += 2) vias += via_segment(T, r[i], r[i + 1], stamp, K);
     if (vias) atomicAdd(T.vias, static_cast<unsigned long long>(vias * K));
 }
 

@@ -361,229 +361,447 @@ __device__ __forceinline__ void lshape_net_l(const Tables& T, const Plan& P, int
     if (fuse_wires) commit_net_wires(T, P, id, stamp, 1, lane);
 }
 
-// Route one net: the layer loops unrolled for the 9 routing layers of the
-// reference's 10-layer designs, generic otherwise.
+// Route one net of any size.
 __device__ __forceinline__ void lshape_net(const Tables& T, const Plan& P, int id, int stamp, const Arena& A,
                                            int lane, bool fuse_wires) {
-    if (T.L == 9) lshape_net_l<9>(T, P, id, stamp, A, lane, fuse_wires);
-    else lshape_net_l<0>(T, P, id, stamp, A, lane, fuse_wires);
+    lshape_net_l<0>(T, P, id, stamp, A, lane, fuse_wires);
 }
 
-// Nets of one or two tree nodes, one net per lane: the lanes of a warp route
-// up to 32 such nets at once (most nets of a design), where lshape_net would
-// spend a whole warp, mostly idle, on each.  Same arithmetic, comparisons,
-// tie-breaks and emission order as lshape_net on the same net, so the routes
-// are identical.  Scratch: lane-interleaved per-warp shared memory of
-// pair_scratch_bytes().  id < 0: the lane has no net.
-constexpr int kPairD = 3 * kMaxLayers;  // doubles per lane: cur, w1, w2 (then diag)
-constexpr int kPairF = 3 * kMaxLayers;  // 4-byte words per lane: vA (then root vN), vB, vN (then choices)
-constexpr int kPairH = kMaxLayers;      // shorts per lane: best range through each layer
-__host__ __device__ __forceinline__ size_t pair_scratch_bytes() {
-    return size_t(32) * (kPairD * 8 + kPairF * 4 + kPairH * 2);
+// ---- Packs: several nets, at most 32 tree nodes, by one warp ------------------
+// The same DP with a lane per tree node for the tree's bookkeeping (coordinates,
+// parents and depths live in registers and travel by shuffle), so a warp can
+// take several small nets at once: their nodes form one forest, processed one
+// depth at a time like a single tree.  Fixed costs of a net -- the dependent
+// loads of its id, offsets, nodes and tables, the route store, the commit --
+// are paid once per pack.
+//
+// What a depth costs decides the DP's time (a batch with fewer nets than warps
+// lasts as long as its deepest net), so the step of a depth is short:
+//   * best range through each layer: a suffix minimum along each row lo (lane
+//     lo), then a minimum down each column (lane l), 18 comparisons in place of
+//     the 45 ranges;
+//   * via stacks at a corner: the difference of two prefix sums of the column
+//     wherever those are exact (below), in place of a sum per candidate;
+//   * depths by pointer jumping, a depth's nodes by one ballot.
+// Same comparisons, tie-breaks, sums and emission order as lshape_net_l, so the
+// same routes.  Warp per net at 320x320x10, 120K nets: 5.8 ms of DP in 61
+// batches, the longest net 110 us; packs: PACK_MS.
+struct PackArena {
+    double* dist;          // [nmax][TT] ranges; during a step the row minima; then what goes into the parent
+    double* w1;            // [nmax][L] first leg (or straight) wire cost
+    double* w2;            // [nmax][L] second leg wire cost
+    double* stack;         // [nmax][2][L] column sums at the corners (x, py), (px, y): entry j = sum of layers 1..j-1
+    unsigned short* from;  // [nmax][FS] column of a row minimum, then choice*L*L + curl*L + parl
+    char* rough;           // [nmax][2] the column's sums are not exact
+    double* diag;          // [32] best parent-layer cost (lane = slot * L + layer)
+    int* pdiag;            // [32]
+};
+constexpr int kPackNodes = 32;
+__host__ __device__ __forceinline__ int pack_from_stride(int L) { return (tri_count(L) + 1) & ~1; }
+__host__ __device__ __forceinline__ size_t pack_arena_bytes(int L, int nmax) {
+    const size_t per = size_t(tri_count(L)) * 8 + 4 * size_t(L) * 8 + size_t(pack_from_stride(L)) * 2 + 2;
+    return (nmax * per + 32 * 12 + 15) & ~size_t(15);
+}
+// Nodes a warp's shared-memory arena holds: 16, or what 16 warps' arenas of an
+// SM leave room for.
+__host__ __device__ __forceinline__ int pack_nmax(int L) {
+    int n = 16;
+    while (n > 2 && pack_arena_bytes(L, n) * 16 > 220 * 1024) --n;
+    return n;
+}
+__device__ __forceinline__ PackArena pack_arena(char* p, int L, int nmax) {
+    PackArena A;
+    A.dist = reinterpret_cast<double*>(p); p += size_t(nmax) * tri_count(L) * 8;
+    A.w1 = reinterpret_cast<double*>(p); p += size_t(nmax) * L * 8;
+    A.w2 = reinterpret_cast<double*>(p); p += size_t(nmax) * L * 8;
+    A.stack = reinterpret_cast<double*>(p); p += size_t(nmax) * 2 * L * 8;
+    A.diag = reinterpret_cast<double*>(p); p += 32 * 8;
+    A.pdiag = reinterpret_cast<int*>(p); p += 32 * 4;
+    A.from = reinterpret_cast<unsigned short*>(p); p += size_t(nmax) * pack_from_stride(L) * 2;
+    A.rough = p;
+    return A;
+}
+
+// The trees of a pack: lane q < nodes holds tree node q of the forest.
+struct Pack {
+    int nets, nodes;
+    int id;          // lane's net (nets without nodes appear nowhere)
+    int first, count;// lane's net: its root's lane, its nodes
+    int x, y, lay;   // lay = L: Steiner point
+    int par;         // parent's lane, -1 at a root (and beyond the nodes)
+    long long out, cap;  // lane's net: route words
+};
+// `k` <= 16 nets ids[0..k), at most 32 nodes together.
+__device__ __forceinline__ Pack load_pack(const Tables& T, const Plan& P, const int* ids, int k, int lane) {
+    Pack K;
+    K.nets = k;
+    int id = 0, off = 0, n = 0;
+    if (lane < k) {
+        id = ids[lane];
+        off = P.node_off[id];
+        n = P.node_off[id + 1] - off;
+        if (n == 0 && P.route_off[id + 1] > P.route_off[id]) P.routes[P.route_off[id]] = 1;  // an empty route
+    }
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    K.nodes = __shfl_sync(0xffffffffu, incl, k - 1);
+    int j = 0;  // the net of node `lane`: the first with incl > lane
+#pragma unroll
+    for (int step = 8; step; step >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, incl, j + step - 1);
+        if (j + step - 1 < k && v <= lane) j += step;
+    }
+    j = min(j, k - 1);
+    K.id = __shfl_sync(0xffffffffu, id, j);
+    K.count = __shfl_sync(0xffffffffu, n, j);
+    K.first = __shfl_sync(0xffffffffu, incl, j) - K.count;
+    off = __shfl_sync(0xffffffffu, off, j);
+    K.x = K.y = K.lay = 0;
+    K.par = -1;
+    K.out = K.cap = 0;
+    if (lane < K.nodes) {
+        const int v = P.nodes[off + lane - K.first], p = P.parents[off + lane - K.first];
+        K.out = P.route_off[K.id];
+        K.cap = P.route_off[K.id + 1] - K.out;
+        cell_position(T, v, K.lay, K.x, K.y);
+        if (p >= 0) K.par = K.first + p;
+    }
+    return K;
 }
 
 template <int LC>
-__device__ __forceinline__ void lshape_net_pair_l(const Tables& T, const Plan& P, int id, int stamp, char* scratch,
-                                                  int lane, bool commit) {
-    if (id < 0) return;
-    double* sd = reinterpret_cast<double*>(scratch);
-    float* sf = reinterpret_cast<float*>(scratch + size_t(32) * kPairD * 8);
-    int* si = reinterpret_cast<int*>(sf);
-    unsigned short* sh = reinterpret_cast<unsigned short*>(scratch + size_t(32) * (kPairD * 8 + kPairF * 4));
-    auto cur = [&](int l) -> double& { return sd[l * 32 + lane]; };
-    auto w1 = [&](int l) -> double& { return sd[(kMaxLayers + l) * 32 + lane]; };
-    auto w2 = [&](int l) -> double& { return sd[(2 * kMaxLayers + l) * 32 + lane]; };    // then diag
-    auto vA = [&](int l) -> float& { return sf[l * 32 + lane]; };                           // then root vN
-    auto vB = [&](int l) -> float& { return sf[(kMaxLayers + l) * 32 + lane]; };
-    auto vN = [&](int l) -> float& { return sf[(2 * kMaxLayers + l) * 32 + lane]; };
-    auto pdiag = [&](int l) -> int& { return si[(2 * kMaxLayers + l) * 32 + lane]; };       // after vN
-    auto cfrom = [&](int l) -> unsigned short& { return sh[l * 32 + lane]; };
-    const int L = LC > 0 ? LC : T.L;
-    const int off = P.node_off[id], N = P.node_off[id + 1] - off;
-    int fix0, x0, y0, x1 = 0, y1 = 0;
-    cell_position(T, P.nodes[off], fix0, x0, y0);
-    bool straight = false;
-    if (N == 2) {
-        int fix1;
-        cell_position(T, P.nodes[off + 1], fix1, x1, y1);
-        straight = x1 == x0 || y1 == y0;
-        const int minx = min(x1, x0), maxx = max(x1, x0), miny = min(y1, y0), maxy = max(y1, y0);
-        // Step 1 for node 1 (the child), kHalfLayers layers at a time: every
-        // load of a group is issued before its stores.
-        constexpr int kHalfLayers = kMaxLayers / 2;
+__device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, const Pack& K, int stamp,
+                                             const PackArena& A, int lane, bool commit) {
+    const int L = LC > 0 ? LC : T.L, TT = tri_count(L), FS = pack_from_stride(L);
+    constexpr int LL = LC > 0 ? LC : kMaxLayers;  // static bound of the layer loops
+    constexpr unsigned kAll = 0xffffffffu;
+    const int M = K.nodes;
+    if (M == 0) return;
+    // Depths by pointer jumping (trees of at most 32 nodes: five rounds).
+    int dep = K.par >= 0 ? 1 : 0;
+    for (int anc = K.par; __any_sync(kAll, anc >= 0);) {
+        const int od = __shfl_sync(kAll, dep, anc & 31), oa = __shfl_sync(kAll, anc, anc & 31);
+        if (anc >= 0) { dep += od; anc = oa; }
+    }
+    if (lane >= M) dep = -1;
+    const int dmax = __reduce_max_sync(kAll, dep);
+    const int xy = (K.x << 16) | K.y;
+    const int pxy = __shfl_sync(kAll, xy, K.par & 31);
+    // 1. Gather every cost the DP reads.  Each lane takes two (node, layer)
+    // items per pass and issues all their loads before any arena store; the
+    // corner columns wait in the node's (still unused) range table.
+    for (int q0 = 0; q0 < M * L; q0 += 64) {
+        float vn[2], va[2], vb[2];
+        double w1[2], w2[2];
+        int kind[2];  // 0: none, 1: node only, 2: straight edge, 3: L-shaped edge
 #pragma unroll
-        for (int l0 = 0; l0 < kMaxLayers; l0 += kHalfLayers) {
-            float vn[kHalfLayers], va[kHalfLayers], vb[kHalfLayers];
-            double a[kHalfLayers], b[kHalfLayers];
-#pragma unroll
-            for (int u = 0; u < kHalfLayers; ++u) {
-                const int l = l0 + u;
-                vn[u] = va[u] = vb[u] = 0.f;
-                a[u] = b[u] = 0.0;
-                if (l >= L) continue;
-                const bool ay = along_y(T, l);
-                vn[u] = T.vcost[slot_index(T, l, x1, y1)];
-                if (straight) {
-                    const bool valid = ay ? (x1 == x0) : (y1 == y0);
-                    a[u] = valid ? wire_cost(T, l, minx, maxx, miny, maxy) : 0.0;
-                } else {
-                    a[u] = ay ? wire_cost(T, l, x1, x1, miny, maxy) : wire_cost(T, l, minx, maxx, y1, y1);
-                    b[u] = ay ? wire_cost(T, l, x0, x0, miny, maxy) : wire_cost(T, l, minx, maxx, y0, y0);
-                    va[u] = T.vcost[slot_index(T, l, x1, y0)];
-                    vb[u] = T.vcost[slot_index(T, l, x0, y1)];
+        for (int u = 0; u < 2; ++u) {
+            const int q = q0 + 32 * u + lane, i = min(q / L, M - 1), l = q - q / L * L;
+            const int c = __shfl_sync(kAll, xy, i), pc = __shfl_sync(kAll, pxy, i), pa = __shfl_sync(kAll, K.par, i);
+            kind[u] = 0;
+            vn[u] = va[u] = vb[u] = 0.f;
+            w1[u] = w2[u] = 0.0;
+            if (q >= M * L) continue;
+            const int x = c >> 16, y = c & 0xffff;
+            const bool ay = along_y(T, l);
+            const int base = layer_base(T, l);
+            vn[u] = T.vcost[base + (ay ? x * T.yp + y : y * T.xp + x)];
+            kind[u] = 1;
+            if (pa >= 0) {
+                const int px = pc >> 16, py = pc & 0xffff;
+                const int minx = min(x, px), maxx = max(x, px), miny = min(y, py), maxy = max(y, py);
+                const bool straight = x == px || y == py;
+                const int lo = ay ? miny : minx, hi = ay ? maxy : maxx;
+                const int t1 = base + (ay ? x * T.yp : y * T.xp), t2 = base + (ay ? px * T.yp : py * T.xp);
+                const bool valid = !straight || (ay ? x == px : y == py);
+                if (valid) w1[u] = T.presum[t1 + hi] - T.presum[t1 + lo];
+                kind[u] = 2;
+                if (!straight) {
+                    w2[u] = T.presum[t2 + hi] - T.presum[t2 + lo];
+                    va[u] = T.vcost[base + (ay ? x * T.yp + py : py * T.xp + x)];
+                    vb[u] = T.vcost[base + (ay ? px * T.yp + y : y * T.xp + px)];
+                    kind[u] = 3;
                 }
             }
+        }
 #pragma unroll
-            for (int u = 0; u < kHalfLayers; ++u) {
-                const int l = l0 + u;
-                if (l >= L) continue;
-                vN(l) = vn[u];
-                w1(l) = a[u];
-                w2(l) = b[u];
-                vA(l) = va[u];
-                vB(l) = vb[u];
+        for (int u = 0; u < 2; ++u) {
+            const int q = q0 + 32 * u + lane, i = q / L, l = q - i * L;
+            if (kind[u] >= 1) reinterpret_cast<float*>(A.from + i * FS)[l] = vn[u];
+            if (kind[u] >= 2) A.w1[q] = w1[u];
+            if (kind[u] == 3) {
+                A.w2[q] = w2[u];
+                float* col = reinterpret_cast<float*>(A.dist + i * TT);
+                col[l] = va[u];
+                col[L + l] = vb[u];
             }
         }
-        // Steps 2 and 3a: the child's via stacks, and its best range through
-        // each layer, first minimum in (lo, hi) order.
+    }
+    __syncwarp();
+    // 2a. Column sums at the corners.  The sum of layers a+1..b-1 is wanted as
+    // the sequential loop adds it; it is the difference of two prefix sums
+    // whenever no addition of the column rounds, which holds when the values'
+    // exponents span at most 25 bits (24-bit mantissas, at most 8 terms: every
+    // partial sum fits the 53 bits of a double).  Other columns are summed
+    // where they are used.
+    for (int q = lane; q < 2 * M; q += 32) {
+        const int i = q >> 1;
+        const float* col = reinterpret_cast<const float*>(A.dist + i * TT) + (q & 1) * L;
+        double* out = A.stack + size_t(q) * L;
+        double acc = 0;
+        unsigned emin = 255, emax = 0;
+        bool odd = false;
 #pragma unroll
-        for (int l = 0; l < L; ++l) {
-            cur(l) = kInf;
-            cfrom(l) = 0;
-        }
-#pragma unroll
-        for (int lo = 0; lo < L; ++lo) {
-            double acc = 0;
-#pragma unroll
-            for (int hi = lo; hi < L; ++hi) {
-                if (hi > lo) acc = acc + static_cast<double>(vN(hi - 1));
-                const double v = (fix1 < L && (lo > fix1 || hi < fix1)) ? kInf : acc;
-#pragma unroll
-                for (int l = lo; l <= hi; ++l)
-                    if (v < cur(l)) {
-                        cur(l) = v;
-                        cfrom(l) = static_cast<unsigned short>(lo * L + hi);
-                    }
+        for (int l = 1; l < LL; ++l) {
+            if (l >= L) continue;
+            out[l] = acc;
+            const float v = col[l];
+            const unsigned b = __float_as_uint(v), e = b >> 23;
+            if (l < L - 1 && b != 0u) {
+                odd |= e == 0 || e >= 255;  // denormal, negative, infinite or NaN
+                emin = min(emin, e);
+                emax = max(emax, e);
+                acc = acc + static_cast<double>(v);
             }
         }
-        // Step 3b: best cost of reaching the parent on each layer.
+        A.rough[q] = odd || emax > emin + 25;
+    }
+    __syncwarp();
+    // 2b. Via stacks at every node (lshape_thread.cuh:40-50).
+    for (int q0 = 0; q0 < M * L; q0 += 32) {
+        const int q = q0 + lane, i = min(q / L, M - 1), lo = q - q / L * L;
+        const int fixed = __shfl_sync(kAll, K.lay, i);
+        if (q >= M * L) continue;
+        const float* vn = reinterpret_cast<const float*>(A.from + i * FS);
+        double acc = 0;
+        double* row = A.dist + i * TT + tri(L, lo, lo) - lo;
 #pragma unroll
-        for (int pl = 0; pl < L; ++pl) {
+        for (int hi = 0; hi < LL; ++hi) {
+            if (hi < lo || hi >= L) continue;
+            if (hi > lo) acc = acc + static_cast<double>(vn[hi - 1]);
+            row[hi] = (fixed < L && (lo > fixed || hi < fixed)) ? kInf : acc;
+        }
+    }
+    __syncwarp();
+    // 3. Children into parents (lshape_thread.cuh:51-115), one depth at a time
+    // from the deepest, up to 32 / L nodes at once (lane = slot * L + layer);
+    // then every node of the depth, in descending order, adds its table into
+    // its parent: exactly the sequential loop's additions.
+    const int S = max(1, 32 / L);
+    const int slot = lane / L, sl = lane - slot * L, s0 = min(slot, S - 1) * L;
+    for (int d = dmax; d >= 1; --d) {
+        const unsigned level = __ballot_sync(kAll, dep == d);
+        for (unsigned at = level; at;) {
+            int i = -1;
+            for (int k = 0; k < S; ++k) {
+                if (k == slot && at) i = __ffs(at) - 1;
+                at &= at - 1;  // 0 stays 0
+            }
+            const bool act = i >= 0;
+            const int ii = max(i, 0);
+            const int c = __shfl_sync(kAll, xy, ii), pc = __shfl_sync(kAll, pxy, ii);
+            const int x = c >> 16, y = c & 0xffff, px = pc >> 16, py = pc & 0xffff;
+            double* dist = A.dist + ii * TT;
+            unsigned short* from = A.from + ii * FS;
+            if (act) {
+                // Row sl: its first minimum over columns hi >= h, for every h.
+                const int row = tri(L, sl, sl) - sl;
+                double best = __longlong_as_double(0x7ff0000000000000ll);
+                int bh = 0;
+#pragma unroll
+                for (int hi = LL - 1; hi >= 0; --hi) {
+                    if (hi < sl || hi >= L) continue;
+                    const double v = dist[row + hi];
+                    if (v <= best) { best = v; bh = hi; }
+                    dist[row + hi] = best;
+                    from[row + hi] = static_cast<unsigned short>(bh);
+                }
+            }
+            __syncwarp();
+            double cur = kInf;
+            int bf = 0;
+            if (act) {
+                // Column sl: the first row with the least of them.
+                int bl = -1;
+#pragma unroll
+                for (int lo = 0; lo < LL; ++lo) {
+                    if (lo > sl || lo >= L) continue;
+                    const double v = dist[tri(L, lo, sl)];
+                    if (v < cur) { cur = v; bl = lo; }
+                }
+                if (bl >= 0) bf = bl * L + from[tri(L, bl, sl)];
+            }
+            // Arrival on parent layer sl (first leg on cl, corner, second leg on sl).
+            const double reach = act ? cur + A.w1[ii * L + sl] : 0.0;
+            const bool straight = x == px || y == py;
             double best = kInf;
-            int pb = 0;
-            if (straight) {
-                const bool valid = along_y(T, pl) ? (x1 == x0) : (y1 == y0);
-                if (valid) {
-                    best = cur(pl) + w1(pl);
-                    pb = cfrom(pl) * L * L + pl * L + pl;
-                }
-            } else {
+            int bc = -1;
+            if (act && straight && (along_y(T, sl) ? x == px : y == py)) { best = reach; bc = sl; }
+            if (__any_sync(kAll, act && !straight)) {
+                const double leg2 = act ? A.w2[ii * L + sl] : 0.0;
+                // The corner column depends on the first leg's direction, the other one than sl's.
+                const int side = along_y(T, sl) ? 1 : 0;
+                const double* col = A.stack + (2 * size_t(ii) + side) * L;
+                const bool rough = act && !straight && A.rough[2 * ii + side];
+                const int cx = side ? px : x, cy = side ? y : py;
 #pragma unroll
-                for (int cl = (pl & 1) ^ 1; cl < L; cl += 2) {
-                    const double cost = cur(cl) + w1(cl);
-                    double cost2 = 0;
-                    const bool ay = along_y(T, cl);
-#pragma unroll
-                    for (int l = min(cl, pl) + 1; l < max(cl, pl); ++l)
-                        cost2 += static_cast<double>(ay ? vA(l) : vB(l));
-                    cost2 += w2(pl);
-                    if (cost + cost2 < best) {
-                        best = cost + cost2;
-                        pb = cfrom(cl) * L * L + cl * L + pl;
+                for (int cl = 0; cl < LL; ++cl) {
+                    if (cl >= L) continue;
+                    const double cost = __shfl_sync(kAll, reach, s0 + cl);
+                    if (!act || straight || ((cl ^ sl) & 1) == 0) continue;
+                    const int a = min(cl, sl), b = max(cl, sl);
+                    double cost2 = col[b] - col[a + 1];
+                    if (rough) {
+                        cost2 = 0;
+                        for (int l = a + 1; l < b; ++l)
+                            cost2 += static_cast<double>(T.vcost[slot_index(T, l, cx, cy)]);
                     }
+                    cost2 += leg2;
+                    if (cost + cost2 < best) { best = cost + cost2; bc = cl; }
                 }
             }
-            w2(pl) = best;   // w2(pl) is not read again
-            pdiag(pl) = pb;  // vN of the child is not read again
-        }
-    }
-    // The root's via-cost column (vA of the child is not read again).
-    {
-        float v[kMaxLayers];
-#pragma unroll
-        for (int l = 0; l < kMaxLayers; ++l) v[l] = l < L ? T.vcost[slot_index(T, l, x0, y0)] : 0.f;
-#pragma unroll
-        for (int l = 0; l < kMaxLayers; ++l)
-            if (l < L) vA(l) = v[l];
-    }
-    // Steps 2, 3c, 3d and 4 for the root: its via stacks plus, for a child,
-    // the range minimum of the diagonal; the first minimal range.
-    int choice = 0, bestpath = 0;
-    {
-        double best = 0;
-#pragma unroll
-        for (int lo = 0; lo < L; ++lo) {
-            double acc = 0, c = 0;
-            int path = 0;
-            if (N == 2) {
-                c = w2(lo);
-                path = pdiag(lo);
+            const int cf = __shfl_sync(kAll, bf, s0 + max(bc, 0));
+            if (act) {
+                A.diag[lane] = best;
+                A.pdiag[lane] = bc >= 0 ? cf * L * L + bc * L + sl : 0;
             }
+            __syncwarp();
+            if (act) {
+                // The node's contribution to its parent replaces its own
+                // table (read above, not needed again).
+                const int row = tri(L, sl, sl) - sl;
+                double cc = A.diag[s0 + sl];
+                int path = A.pdiag[s0 + sl];
 #pragma unroll
-            for (int hi = lo; hi < L; ++hi) {
-                if (hi > lo) acc = acc + static_cast<double>(vA(hi - 1));
-                double v = (fix0 < L && (lo > fix0 || hi < fix0)) ? kInf : acc;
-                if (N == 2) {
-                    if (hi > lo && !(c <= w2(hi))) {
-                        c = w2(hi);
-                        path = pdiag(hi);
-                    }
-                    v += c;
-                }
-                if ((lo == 0 && hi == 0) || v < best) {
-                    best = v;
-                    choice = lo * L + hi;
-                    bestpath = path;
+                for (int hi = 0; hi < LL; ++hi) {
+                    if (hi < sl || hi >= L) continue;
+                    const double v = A.diag[s0 + hi];
+                    if (hi > sl && !(cc <= v)) { cc = v; path = A.pdiag[s0 + hi]; }
+                    dist[row + hi] = cc;
+                    from[row + hi] = static_cast<unsigned short>(path);
                 }
             }
+            __syncwarp();
         }
-        if (!(best < kInf)) set_error(T, kEInval, id);
+        for (unsigned m = level; m;) {
+            const int i = 31 - __clz(m);
+            m ^= 1u << i;
+            const int p = __shfl_sync(kAll, K.par, i);
+            for (int t = lane; t < TT; t += 32) A.dist[p * TT + t] += A.dist[i * TT + t];
+        }
+        __syncwarp();
     }
-    // Step 5: segments in node order.
-    int* out = P.routes + P.route_off[id];
-    const long long cap = P.route_off[id + 1] - P.route_off[id];
-    const int minl0 = choice / L, maxl0 = choice % L;
-    int words = minl0 < maxl0 ? 2 : 0;
-    int minl1 = 0, maxl1 = 0, cl = 0, pl = 0;
-    if (N == 2) {
-        const int r1 = bestpath / (L * L);
-        minl1 = r1 / L;
-        maxl1 = r1 % L;
-        cl = bestpath / L % L;
-        pl = bestpath % L;
-        words += (minl1 < maxl1 ? 2 : 0) + (straight ? 2 : 6);
-    }
-    if (1 + words > cap) {
-        set_error(T, kELimit, id);
-        return;
-    }
-    int* w = out + 1;
-    if (minl0 < maxl0) { *w++ = cell_index(T, minl0, x0, y0); *w++ = cell_index(T, maxl0, x0, y0); }
-    if (N == 2) {
-        if (minl1 < maxl1) { *w++ = cell_index(T, minl1, x1, y1); *w++ = cell_index(T, maxl1, x1, y1); }
-        if (straight) {
-            *w++ = cell_index(T, cl, min(x1, x0), min(y1, y0));
-            *w++ = cell_index(T, cl, max(x1, x0), max(y1, y0));
-        } else if (along_y(T, cl)) {
-            *w++ = cell_index(T, cl, x1, y1);   *w++ = cell_index(T, cl, x1, y0);
-            *w++ = cell_index(T, cl, x1, y0);   *w++ = cell_index(T, pl, x1, y0);
-            *w++ = cell_index(T, pl, x1, y0);   *w++ = cell_index(T, pl, x0, y0);
-        } else {
-            *w++ = cell_index(T, cl, x1, y1);   *w++ = cell_index(T, cl, x0, y1);
-            *w++ = cell_index(T, cl, x0, y1);   *w++ = cell_index(T, pl, x0, y1);
-            *w++ = cell_index(T, pl, x0, y1);   *w++ = cell_index(T, pl, x0, y0);
+    // 4. Root ranges (lshape_thread.cuh:117-120): the first minimum in loop
+    // order (lo, then hi), lane = slot * L + lo; then the traceback one depth
+    // at a time.
+    int range = 0, f = 0;
+    for (unsigned at = __ballot_sync(kAll, dep == 0); at;) {
+        int i = -1;
+        for (int k = 0; k < S; ++k) {
+            if (k == slot && at) i = __ffs(at) - 1;
+            at &= at - 1;
+        }
+        double bv = __longlong_as_double(0x7ff0000000000000ll);
+        int br = 0;
+        if (i >= 0) {
+            const double* row = A.dist + i * TT + tri(L, sl, sl) - sl;
+#pragma unroll
+            for (int hi = 0; hi < LL; ++hi) {
+                if (hi < sl || hi >= L) continue;
+                const double v = row[hi];
+                if (v < bv) { bv = v; br = sl * L + hi; }
+            }
+        }
+        double best = __longlong_as_double(0x7ff0000000000000ll);
+        int rr = 0;  // no entry below infinity: the sequential loop keeps range (0, 0)
+#pragma unroll
+        for (int lo = 0; lo < LL; ++lo) {
+            if (lo >= L) continue;
+            const double v = __shfl_sync(kAll, bv, s0 + lo);
+            const int r = __shfl_sync(kAll, br, s0 + lo);
+            if (v < best) { best = v; rr = r; }
+        }
+        // Each slot's result to its root's lane.
+        for (int k = 0; k < S; ++k) {
+            const int to = __shfl_sync(kAll, i, k * L), r = __shfl_sync(kAll, rr, k * L);
+            const double v = __shfl_sync(kAll, best, k * L);
+            if (lane == to) {
+                range = r;
+                if (!(v < kInf)) set_error(T, kEInval, K.id);
+            }
         }
     }
-    out[0] = 1 + words;
-    if (commit) commit_thread_wires(T, P, id, stamp, 1);
+    for (int d = 1; d <= dmax; ++d) {
+        const int pr = __shfl_sync(kAll, range, K.par & 31);
+        if (dep == d) {
+            f = A.from[lane * FS + tri(L, pr / L, pr % L)];
+            range = f / (L * L);
+        }
+    }
+    // 5. Segments in node order (lshape_warp.cuh:215-240), a lane per node.
+    const int minl = range / L, maxl = range % L, cl = f / L % L, pl = f % L;
+    const int x = K.x, y = K.y, px = pxy >> 16, py = pxy & 0xffff;
+    const bool edge = K.par >= 0, straight = x == px || y == py;
+    int words = 0;
+    if (lane < M) words = (minl < maxl ? 2 : 0) + (edge ? (straight ? 2 : 6) : 0);
+    int incl = words;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(kAll, incl, d);
+        if (lane >= d) incl += o;
+    }
+    const int start = __shfl_sync(kAll, incl - words, K.first & 31);  // words of the nets before this one
+    const int total = __shfl_sync(kAll, incl, (K.first + K.count - 1) & 31) - start;
+    const bool fits = 1 + total <= K.cap;
+    const bool mine = lane < M && fits;
+    // The corner of an L-shaped edge: the end of the first leg.
+    const int cx = along_y(T, cl) ? x : px, cy = along_y(T, cl) ? py : y;
+    if (lane < M && lane == K.first) {
+        if (fits) P.routes[K.out] = 1 + total;
+        else set_error(T, kELimit, K.id);
+    }
+    if (mine) {
+        int* w = P.routes + K.out + 1 + (incl - words - start);
+        if (minl < maxl) { *w++ = cell_index(T, minl, x, y); *w++ = cell_index(T, maxl, x, y); }
+        if (edge && straight) {
+            *w++ = cell_index(T, cl, min(x, px), min(y, py));
+            *w++ = cell_index(T, cl, max(x, px), max(y, py));
+        } else if (edge) {
+            const int corner = cell_index(T, cl, cx, cy), second = cell_index(T, pl, cx, cy);
+            *w++ = cell_index(T, cl, x, y); *w++ = corner;
+            *w++ = corner;                  *w++ = second;
+            *w++ = second;                  *w++ = cell_index(T, pl, px, py);
+        }
+    }
+    if (!commit) return;
+    // The wires just emitted, from registers: the first leg (or the straight
+    // run) of every lane, then the second legs.
+    double length = 0;
+#pragma unroll
+    for (int leg = 0; leg < 2; ++leg) {
+        WireRun R;
+        if (mine && edge && (leg == 0 || !straight)) {
+            const int l = leg ? pl : cl, ax = leg ? cx : x, ay = leg ? cy : y;
+            const int bx = leg || straight ? px : cx, by = leg || straight ? py : cy;
+            R = run_between(T, l, ax, ay, bx, by);
+            const int a = cell_index(T, l, ax, ay), b = cell_index(T, l, bx, by);
+            stamp_ends(T, R, a, b, stamp);
+            length += R.length;
+            if (R.skew) commit_skew(T, a, b, stamp, 1);
+        }
+        commit_runs(T, R.first, R.skew ? 0 : R.n, stamp, 1, lane);
+    }
+    add_wirelength(T, length, 1, lane);
 }
 
-// One or two tree nodes per lane: unrolled for 9 routing layers, generic
-// otherwise.
-__device__ __forceinline__ void lshape_net_pair(const Tables& T, const Plan& P, int id, int stamp, char* scratch,
-                                                int lane, bool commit) {
-    if (T.L == 9) lshape_net_pair_l<9>(T, P, id, stamp, scratch, lane, commit);
-    else lshape_net_pair_l<0>(T, P, id, stamp, scratch, lane, commit);
+__device__ __forceinline__ void route_pack(const Tables& T, const Plan& P, const Pack& K, int stamp, const PackArena& A,
+                                           int lane, bool commit) {
+    if (T.L == 9) route_pack_l<9>(T, P, K, stamp, A, lane, commit);
+    else route_pack_l<0>(T, P, K, stamp, A, lane, commit);
 }
 
 }  // namespace grb

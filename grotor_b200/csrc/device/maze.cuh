@@ -18,10 +18,10 @@
 
 namespace grb {
 
-// A wire of route r (words [1, r[0])) on point's layer covers point.
-__device__ __forceinline__ bool maze_wire_touches(const int* r, int point, int XY, int Y) {
+// A wire of route r (words [1, words)) on point's layer covers point.
+__device__ __forceinline__ bool maze_wire_touches(const int* r, int words, int point, int XY, int Y) {
     const int layer = point / XY;
-    for (int i = 1; i < r[0]; i += 2) {
+    for (int i = 1; i + 1 < words; i += 2) {
         const int a = r[i], b = r[i + 1];
         if (a / XY != layer || b / XY != layer) continue;
         const int x = point / Y, y = point % Y;  // x carries the layer offset, as a / Y does
@@ -38,12 +38,14 @@ __device__ __forceinline__ void maze_add(const Tables& T, int c, int half) {
     add_via_demand(T, slot_index(T, l, x, y), half);
 }
 
-// remove_routes for one net (one thread): route words r.
-__device__ __forceinline__ void maze_remove_route(const Tables& T, const int* r) {
+// remove_routes for net `id` of plan P (one thread).
+__device__ __forceinline__ void maze_remove_route(const Tables& T, const Plan& P, int id) {
+    const int* r = net_routes(P, id);
+    const int words = net_words(P, id);
     const int XY = T.XY, Y = T.Y, X = T.X;
     double length = 0;
     long long vias = 0;
-    for (int i = 1; i < r[0]; i += 2) {
+    for (int i = 1; i + 1 < words; i += 2) {
         const int a = r[i], b = r[i + 1];
         const int x = a / Y % X, y = a % Y;
         if (a / XY == b / XY) {
@@ -61,7 +63,7 @@ __device__ __forceinline__ void maze_remove_route(const Tables& T, const int* r)
             vias += last - first;
             for (int layer = first; layer < last; ++layer) {
                 const int point = layer * XY + x * Y + y;
-                if (maze_wire_touches(r, point, XY, Y)) continue;
+                if (maze_wire_touches(r, words, point, XY, Y)) continue;
                 const bool vertical = along_y(T, layer);
                 const int position = vertical ? y : x, limit = vertical ? Y : X, step = vertical ? 1 : Y;
                 if (!position) maze_add(T, point, -2);

@@ -464,6 +464,10 @@ __device__ __forceinline__ void zshape_net(const Tables& T, const ZTrees& Z, con
         if (t == 0 && cap > 0) r[0] = 1;
         return;
     }
+    if (cap <= 0) {
+        if (t == 0) set_error(T, kELimit, id);
+        return;
+    }
     // reset_nodes (zshape.cuh:392-404).
     for (int k = t; k < cnt * Z.LAYER; k += nth) {
         const int pt = Z.pos[nb + k / Z.LAYER];

@@ -36,7 +36,6 @@ namespace {
 
 constexpr int kRefreshThreads = 256;
 constexpr int kPersistentThreads = 256;
-constexpr int kDpThreads = 128;
 constexpr unsigned long long kBarrierTimeoutNs = 20ull * 1000 * 1000 * 1000;
 constexpr int kPhaseSlots = 20;  // grb_phase_times entries
 constexpr int kNetTimeSlot = 12;  // per size bucket: summed net time [12..15], longest net [16..19]
@@ -84,61 +83,66 @@ __global__ void k_layout(Tables T, const V* src, V* dst, int l0) {
     }
 }
 
-__device__ __forceinline__ Arena warp_arena(char* smem, size_t arena_b, int warp, int L, int nmax) {
-    return carve_arena(smem + warp * arena_b, L, nmax);
+// Route the nets ids[0..k) with one warp: a pack in the warp's shared-memory
+// arena of nmax nodes, a single larger net in its global scratch slot (nets
+// beyond kPackNodes by the general form).
+__device__ __forceinline__ void route_nets(const Tables& T, const Plan& P, const int* ids, int k, int stamp, char* arena,
+                                           int nmax, char* slot, int lane, bool commit) {
+    const int id = ids[0], N = k == 1 ? P.node_off[id + 1] - P.node_off[id] : 0;
+    if (N > nmax && !slot) {
+        if (lane == 0) set_error(T, kELimit, id);
+    } else if (N > kPackNodes) {
+        lshape_net(T, P, id, stamp, carve_arena(slot, T.L, N), lane, commit);
+    } else {
+        const Pack K = load_pack(T, P, ids, k, lane);
+        route_pack(T, P, K, stamp, N > nmax ? pack_arena(slot, T.L, N) : pack_arena(arena, T.L, nmax), lane, commit);
+    }
 }
 
-// Plain DP launch: one warp per net of batch b (routes only).
-__global__ void __launch_bounds__(kDpThreads) k_lshape_batch(Tables T, Plan P, int b, int stamp, int nmax,
-                                                             size_t arena_b, char* gscratch, size_t gslot) {
-    extern __shared__ __align__(16) char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
-    const int k = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (k >= cnt) return;
-    const int id = P.ids[lo + k];
-    const int N = P.node_off[id + 1] - P.node_off[id];
-    Arena A;
-    if (N <= nmax) A = warp_arena(smem, arena_b, warp, T.L, nmax);
-    else if (gscratch) A = carve_arena(gscratch + size_t(blockIdx.x * (blockDim.x >> 5) + warp) * gslot, T.L, N);
-    else { if (lane == 0) set_error(T, kELimit, id); return; }
-    lshape_net(T, P, id, stamp, A, lane, false);
+// Nets per pack of each size bucket for one batch (cnt nets in the bucket):
+// `fixed` where given, else by this rule.  While every net can have a warp of
+// its own, it gets one: the batch then lasts as long as its deepest net.
+// Beyond that the smallest nets share warps first, as many as it takes for one
+// wave of `warps` or as the arena holds, then the next bucket's.
+__host__ __device__ __forceinline__ void pack_sizes(const int* cnt, const int* fixed, int warps, int nmax, int* g) {
+    int cap[kDpBuckets], total = 0;
+    for (int k = 0; k < kDpBuckets; ++k) {
+        const int nodes = dp_bucket_nodes(k);
+        cap[k] = k == kDpBuckets - 1 || nodes > nmax ? 1 : nmax / nodes;
+        g[k] = fixed[k] > 0 ? (fixed[k] < cap[k] ? fixed[k] : cap[k]) : 1;
+        total += (cnt[k] + g[k] - 1) / g[k];
+    }
+    for (int k = 0; k < kDpBuckets - 1; ++k)
+        while (fixed[k] <= 0 && total > warps && 2 * g[k] <= cap[k]) {
+            total -= (cnt[k] + g[k] - 1) / g[k];
+            g[k] *= 2;
+            total += (cnt[k] + g[k] - 1) / g[k];
+        }
 }
 
 // Per-batch DP launch over every size bucket of batch b at once: CTA ranges
-// [block_off[k], block_off[k+1]) serve bucket k with per_cta[k] nets per CTA
-// (warps beyond it return) and an arena of nmax[k] nodes per warp (global
-// scratch where nmax is 0).
+// [block_off[k], block_off[k+1]) serve bucket k with per[k] warps per CTA
+// (warps beyond it return), pack[k] nets per warp and an arena of nmax[k]
+// nodes per warp (global scratch where nmax is 0).
 struct BucketLaunch {
     int block_off[kDpBuckets + 1];
     int per[kDpBuckets];
+    int pack[kDpBuckets];
     int nmax[kDpBuckets];
     int arena[kDpBuckets];
 };
-__global__ void k_lshape_bucketed(Tables T, Plan P, int b, int stamp, BucketLaunch BL, char* gscratch,
-                                  size_t gslot) {
+__global__ void __launch_bounds__(256, 2) k_lshape_bucketed(Tables T, Plan P, int b, int stamp, BucketLaunch BL,
+                                                            char* gscratch, size_t gslot) {
     extern __shared__ __align__(16) char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int bk = 0;
     while (bk + 1 < kDpBuckets && int(blockIdx.x) >= BL.block_off[bk + 1]) ++bk;
     if (warp >= BL.per[bk]) return;
     const int lo = P.bucket_off[b * (kDpBuckets + 1) + bk], hi = P.bucket_off[b * (kDpBuckets + 1) + bk + 1];
-    const int k = (int(blockIdx.x) - BL.block_off[bk]) * BL.per[bk] + warp;
-    if (bk == 0) {
-        // Nets of one or two nodes: 32 per warp, one per lane.
-        const int q = lo + 32 * k + lane;
-        lshape_net_pair(T, P, q < hi ? P.bucket_ids[q] : -1, stamp, smem + size_t(warp) * BL.arena[0], lane, false);
-        return;
-    }
-    if (lo + k >= hi) return;
-    const int id = P.bucket_ids[lo + k];
-    const int N = P.node_off[id + 1] - P.node_off[id];
-    const int nmax = BL.nmax[bk];
-    Arena A;
-    if (N <= nmax) A = warp_arena(smem, BL.arena[bk], warp, T.L, nmax);
-    else if (gscratch) A = carve_arena(gscratch + size_t(k) * gslot, T.L, N);
-    else { if (lane == 0) set_error(T, kELimit, id); return; }
-    lshape_net(T, P, id, stamp, A, lane, false);
+    const int w = (int(blockIdx.x) - BL.block_off[bk]) * BL.per[bk] + warp, k = lo + w * BL.pack[bk];
+    if (k >= hi) return;
+    route_nets(T, P, P.bucket_ids + k, min(BL.pack[bk], hi - k), stamp, smem + size_t(warp) * BL.arena[bk], BL.nmax[bk],
+               gscratch ? gscratch + size_t(w) * gslot : nullptr, lane, false);
 }
 
 // Group each batch's nets by size bucket (one CTA per batch).
@@ -206,55 +210,40 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
     for (int b = 0; b < P.n_batches; ++b) {
         const int stamp = stamp0 + b + 1;
         if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
-        // Route every net of the batch and commit its wires: size buckets from
-        // the largest down (long nets start first), nets taken from the
-        // bucket's work queue `per_grab` at a time.  (In this kernel the
-        // smallest nets are the filler that evens out the warps' finish
-        // times, so they too take a warp each.)
+        // Route every net of the batch and commit its wires, in packs from the
+        // largest size bucket down (long nets start first): the first pack of
+        // every warp by its number, the others from the batch's work counter.
         const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
-        const Arena A = warp_arena(smem, arena_b, warp, T.L, nmax);
-        for (int bk = kDpBuckets - 1; bk >= 0; --bk) {
-            const int blo = P.bucket_off[b * (kDpBuckets + 1) + bk], bhi = P.bucket_off[b * (kDpBuckets + 1) + bk + 1];
-            const int g = tune.per_grab[bk];
-            if (bk == 0 && g >= 32) {
-                // Nets of one or two nodes, one per lane (lane-interleaved
-                // scratch in the warp's arena), g per grab.
-                while (true) {
-                    int k = 0;
-                    if (lane == 0) k = atomicAdd(work + b * kDpBuckets + bk, g);
-                    k = __shfl_sync(0xffffffffu, k, 0);
-                    if (blo + k >= bhi) break;
-                    const unsigned long long t0 = S.phase_ns && lane == 0 ? global_ns() : 0ull;
-                    for (int q = blo + k + lane; q < min(blo + k + g, bhi); q += 32)
-                        lshape_net_pair(T, P, P.bucket_ids[q], stamp, smem + size_t(warp) * arena_b, lane, true);
-                    __syncwarp();
-                    if (S.phase_ns && lane == 0) {
-                        const unsigned long long dt = global_ns() - t0;
-                        atomicAdd(S.phase_ns + kNetTimeSlot + bk, dt);
-                        atomicMax(S.phase_ns + kNetTimeSlot + kDpBuckets + bk, dt);
-                    }
+        const int* bo = P.bucket_off + b * (kDpBuckets + 1);
+        int cn[kDpBuckets], g[kDpBuckets], last[kDpBuckets];  // last: end of the bucket's packs
+#pragma unroll
+        for (int k = 0; k < kDpBuckets; ++k) cn[k] = bo[k + 1] - bo[k];
+        pack_sizes(cn, tune.per_grab, nwarps, nmax, g);
+        int packs = 0;
+#pragma unroll
+        for (int k = kDpBuckets - 1; k >= 0; --k) {
+            packs += (cn[k] + g[k] - 1) / g[k];
+            last[k] = packs;
+        }
+        for (int item = gwarp; item < packs;) {
+            int bk = 0, at = 0;
+#pragma unroll
+            for (int k = 0; k < kDpBuckets; ++k)
+                if (item < last[k]) {  // the largest bucket whose packs reach it
+                    const int begin = k + 1 < kDpBuckets ? last[k + 1] : 0;
+                    if (item >= begin) { bk = k; at = bo[k] + (item - begin) * g[k]; }
                 }
-                continue;
+            const unsigned long long t0 = S.phase_ns && lane == 0 ? global_ns() : 0ull;
+            route_nets(T, P, P.bucket_ids + at, min(g[bk], bo[bk + 1] - at), stamp, smem + size_t(warp) * arena_b, nmax,
+                       gscratch ? gscratch + size_t(gwarp) * gslot : nullptr, lane, true);
+            if (S.phase_ns && lane == 0) {  // profiling: warp time of every pack, by size bucket
+                const unsigned long long dt = global_ns() - t0;
+                atomicAdd(S.phase_ns + kNetTimeSlot + bk, dt);
+                atomicMax(S.phase_ns + kNetTimeSlot + kDpBuckets + bk, dt);
             }
-            while (true) {
-                int k = 0;
-                if (lane == 0) k = atomicAdd(work + b * kDpBuckets + bk, g);
-                k = __shfl_sync(0xffffffffu, k, 0);
-                if (blo + k >= bhi) break;
-                for (int q = blo + k; q < min(blo + k + g, bhi); ++q) {
-                    const int id = P.bucket_ids[q];
-                    const int N = P.node_off[id + 1] - P.node_off[id];
-                    const unsigned long long t0 = S.phase_ns && lane == 0 ? global_ns() : 0ull;
-                    if (N <= nmax) lshape_net(T, P, id, stamp, A, lane, true);
-                    else if (gscratch) lshape_net(T, P, id, stamp, carve_arena(gscratch + size_t(gwarp) * gslot, T.L, N), lane, true);
-                    else if (lane == 0) set_error(T, kELimit, id);
-                    if (S.phase_ns && lane == 0) {  // profiling: warp time of every net, by size bucket
-                        const unsigned long long dt = global_ns() - t0;
-                        atomicAdd(S.phase_ns + kNetTimeSlot + bk, dt);
-                        atomicMax(S.phase_ns + kNetTimeSlot + kDpBuckets + bk, dt);
-                    }
-                }
-            }
+            if (packs <= nwarps) break;
+            if (lane == 0) item = nwarps + atomicAdd(work + b, 1);
+            item = __shfl_sync(0xffffffffu, item, 0);
         }
         if (!grid_sync(S, T)) return;
         clk.mark(S, 5);
@@ -655,7 +644,7 @@ __global__ void k_maze_remove(Tables T, Plan P, Plan P2, RemoveList R) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= R.n) return;
     const int id = R.ids[k];
-    maze_remove_route(T, R.phase2[k] ? P2.routes + P2.route_off[id] : P.routes + P.route_off[id]);
+    maze_remove_route(T, R.phase2[k] ? P2 : P, id);
 }
 __global__ void __launch_bounds__(kScoreThreads) k_maze_score(Tables T, double* partials) { maze_score_partial(T, partials); }
 
@@ -1142,7 +1131,7 @@ struct grb_ctx {
     int* bucket_off = nullptr;
     int bucket_cap = 0, bucket_batches = 0, bucket_version = -1;
     std::vector<int> h_bucket_off;  // [n_batches][kDpBuckets+1]
-    DpTune tune{{4, 4, 4, 4}, {1, 1, 1, 1}};
+    DpTune tune{{4, 4, 4, 4}, {0, 0, 0, 0}};
     // graph cache
     cudaGraphExec_t graph = nullptr;
     int graph_version = -1, graph_stamp = -1;
@@ -1267,14 +1256,17 @@ Plan make_plan2(const grb_ctx* c) {
     return P;
 }
 
-int dp_nmax(const grb_ctx* c) { return std::min(c->max_nodes, 16); }
+// Global scratch slot of a net with more nodes than the shared-memory arena
+// holds: a pack arena up to kPackNodes nodes, the general form's beyond.
+size_t dp_slot_bytes(const grb_ctx* c) {
+    return std::max(pack_arena_bytes(c->T.L, std::min(std::max(c->max_nodes, 1), kPackNodes)),
+                    arena_bytes(c->T.L, std::max(c->max_nodes, 1)));
+}
 
-
-// Global scratch for nets with more nodes than fit a shared-memory arena of
-// `nmax` nodes.
-int ensure_gscratch(grb_ctx* c, int slots, int nmax) {
-    if (c->max_nodes <= nmax) return GRB_OK;
-    const size_t need = size_t(slots) * arena_bytes(c->T.L, c->max_nodes);
+// Global scratch of `slots` nets (none when every net fits the arena).
+int ensure_gscratch(grb_ctx* c, int slots) {
+    if (c->max_nodes <= std::min(pack_nmax(c->T.L), dp_bucket_nodes(kDpBuckets - 2))) return GRB_OK;
+    const size_t need = size_t(slots) * dp_slot_bytes(c);
     if (need <= c->gscratch_bytes) return GRB_OK;
     if (c->gscratch) cudaFree(c->gscratch);
     c->gscratch = nullptr;
@@ -1348,17 +1340,18 @@ int launch_buckets(grb_ctx* c, int b, int stamp, int only) {
     int blocks = 0, threads = 32;
     size_t smem = 0;
     int gslots = 0;
+    int cn[kDpBuckets];
+    for (int k = 0; k < kDpBuckets; ++k) cn[k] = (only < 0 || only == k) ? bo[k + 1] - bo[k] : 0;
+    const int fixed[kDpBuckets] = {0, 0, 0, 0}, nmax = dp_bucket_nodes(kDpBuckets - 2);
+    pack_sizes(cn, fixed, c->sms * 16, nmax, BL.pack);
     for (int bk = 0; bk < kDpBuckets; ++bk) {
         BL.block_off[bk] = blocks;
-        const int cnt = (only < 0 || only == bk) ? bo[bk + 1] - bo[bk] : 0;
         BL.per[bk] = c->tune.per_cta[bk];
-        BL.nmax[bk] = bk < kDpBuckets - 1 ? std::min(dp_bucket_nodes(bk), std::max(c->max_nodes, 1)) : 0;
-        BL.arena[bk] = BL.nmax[bk] ? int(arena_bytes(c->T.L, BL.nmax[bk])) : 0;
-        if (bk == 0) BL.arena[0] = int(std::max<size_t>(BL.arena[0], pair_scratch_bytes()));
-        if (cnt <= 0) continue;
-        // Bucket 0: each warp takes 32 nets (one per lane).
-        const int per_block = BL.per[bk] * (bk == 0 ? 32 : 1);
-        const int nb = (cnt + per_block - 1) / per_block;
+        BL.nmax[bk] = bk < kDpBuckets - 1 ? std::min(dp_bucket_nodes(bk) * BL.pack[bk], nmax) : 0;
+        BL.arena[bk] = BL.nmax[bk] ? int(pack_arena_bytes(c->T.L, BL.nmax[bk])) : 0;
+        if (cn[bk] <= 0) continue;
+        const int per_block = BL.per[bk] * BL.pack[bk];
+        const int nb = (cn[bk] + per_block - 1) / per_block;
         blocks += nb;
         threads = std::max(threads, 32 * BL.per[bk]);
         smem = std::max(smem, size_t(BL.per[bk]) * BL.arena[bk]);
@@ -1367,11 +1360,11 @@ int launch_buckets(grb_ctx* c, int b, int stamp, int only) {
     BL.block_off[kDpBuckets] = blocks;
     if (!blocks) return GRB_OK;
     if (gslots) {
-        const int rc = ensure_gscratch(c, gslots, dp_nmax(c));
+        const int rc = ensure_gscratch(c, gslots);
         if (rc) return rc;
     }
-    const size_t arena_slot = arena_bytes(c->T.L, std::max(c->max_nodes, 1));
-    k_lshape_bucketed<<<blocks, threads, smem, c->stream>>>(c->T, make_plan(c), b, stamp, BL, c->gscratch, arena_slot);
+    k_lshape_bucketed<<<blocks, threads, smem, c->stream>>>(c->T, make_plan(c), b, stamp, BL, c->gscratch,
+                                                            dp_slot_bytes(c));
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     return GRB_OK;
@@ -1707,7 +1700,7 @@ int stage_graph(grb_ctx* c, int stamp0) {
         // Scratch must exist before capture (no allocation while capturing).
         int maxcnt = 0;
         for (int b = 0; b < c->n_batches; ++b) maxcnt = std::max(maxcnt, c->h_batch_off[b + 1] - c->h_batch_off[b]);
-        int rc = ensure_gscratch(c, maxcnt + 8, dp_nmax(c));
+        int rc = ensure_gscratch(c, maxcnt + 8);
         if (!rc) rc = ensure_buckets(c);
         if (rc) return rc;
         const int64_t before = c->launches;
@@ -1735,9 +1728,8 @@ int stage_graph(grb_ctx* c, int stamp0) {
 
 int stage_persistent(grb_ctx* c, int stamp0) {
     if (c->n_batches == 0) return GRB_OK;
-    const int nmax = dp_nmax(c);
-    // A warp's arena also holds the lane-per-net scratch of the smallest nets.
-    const size_t ab = std::max(arena_bytes(c->T.L, nmax), (pair_scratch_bytes() + 15) & ~size_t(15));
+    const int nmax = pack_nmax(c->T.L);
+    const size_t ab = pack_arena_bytes(c->T.L, nmax);
     const int wpb = kPersistentThreads / 32;
     const size_t smem = std::max(ab * wpb, sizeof(float) * kViewTile * (kViewTile + 1));  // the tail's view tile
     GRB_CUDA(c, cudaFuncSetAttribute(k_lshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -1745,18 +1737,11 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lshape_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent kernel does not fit on an SM");
     const int blocks = per_sm * c->sms;
-    const size_t slot = arena_bytes(c->T.L, std::max(c->max_nodes, 1));
-    int rc = ensure_gscratch(c, blocks * wpb, nmax);
+    const size_t slot = dp_slot_bytes(c);
+    int rc = ensure_gscratch(c, blocks * wpb);
     if (rc) return rc;
     if ((rc = ensure_buckets(c))) return rc;
-    const int counters = c->n_batches * kDpBuckets;
-    if (c->work_cap < counters) {
-        if (c->work) cudaFree(c->work);
-        c->work = nullptr;
-        if (cudaMalloc(&c->work, sizeof(int) * counters) != cudaSuccess) { cudaGetLastError(); return fail(c, GRB_ENOMEM, "work counters"); }
-        c->work_cap = counters;
-    }
-    GRB_CUDA(c, cudaMemsetAsync(c->work, 0, sizeof(int) * counters, c->stream));
+    if ((rc = ensure_work(c))) return rc;
     GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
     Tables T = c->T;
     Plan P = make_plan(c);
@@ -2027,7 +2012,6 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_solve<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_bucketed, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const int r = grb_reset(cp);
     if (r) { const int code = r; free_all(cp->owned); return code; }
@@ -3386,12 +3370,10 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
     }
     if (what & 2) {
         // Persistent form: whole-stage runs from a reset state for each
-        // candidate set of nets per grab (small buckets take more per grab).
-        // per_grab[0] >= 32: nets of one or two nodes one per lane, that many
-        // per grab.
-        constexpr int kCands = 6;
-        const int cands[kCands][kDpBuckets] = {{1, 1, 1, 1}, {2, 1, 1, 1}, {4, 2, 1, 1}, {8, 4, 2, 1},
-                                               {32, 2, 1, 1}, {64, 4, 2, 1}};
+        // candidate set of nets per pack, the last one the rule that sets them
+        // by batch (pack_sizes).
+        constexpr int kCands = 5;
+        const int cands[kCands][kDpBuckets] = {{1, 1, 1, 1}, {2, 1, 1, 1}, {4, 2, 1, 1}, {8, 2, 1, 1}, {0, 0, 0, 0}};
         float best = 1e30f;
         int pick = 0;
         for (int k = 0; k < kCands; ++k) {
@@ -3411,9 +3393,19 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
     c->profiling = prof;
     c->graph_version = -1;  // a captured per-batch sequence bakes in the launch shapes
     if ((rc = grb_reset(c))) return rc;
+    // Reported: the nets per pack of the plan's largest batch.
+    int largest = 0;
+    for (int b = 1; b < c->n_batches; ++b)
+        if (c->h_batch_off[b + 1] - c->h_batch_off[b] > c->h_batch_off[largest + 1] - c->h_batch_off[largest]) largest = b;
+    int cn[kDpBuckets], packs[kDpBuckets];
+    for (int q = 0; q < kDpBuckets; ++q) {
+        const int* bo = c->h_bucket_off.data() + size_t(largest) * (kDpBuckets + 1);
+        cn[q] = bo[q + 1] - bo[q];
+    }
+    pack_sizes(cn, c->tune.per_grab, c->sms * 16, pack_nmax(c->T.L), packs);
     for (int q = 0; q < kDpBuckets; ++q) {
         if (per_cta) per_cta[q] = c->tune.per_cta[q];
-        if (per_grab) per_grab[q] = c->tune.per_grab[q];
+        if (per_grab) per_grab[q] = packs[q];
     }
     return GRB_OK;
 }

@@ -194,11 +194,12 @@ int grb_ripup_classify_noalloc(grb_ctx* ctx, int32_t threshold, uint8_t* is_of);
  * scheduled by size bucket (tree nodes <= 2, <= 8, <= 16, more; the
  * persistent form takes the largest bucket first).  what & 1 times the
  * per-batch DP launch of each bucket on the plan's largest batches for 1, 2,
- * 4 and 8 nets per CTA (arena sized to the bucket); what & 2 runs the
- * persistent stage from a reset state for candidate nets-per-grab sets of its
- * work queue (a nets-per-grab of 32 or more for the smallest bucket routes
- * those nets one per lane).  The choices stay in the context (and are copied to the
- * optional per_cta[4] / per_grab[4]).  Needs nets and a plan; leaves the
+ * 4 and 8 warps per CTA (arena sized to the bucket); what & 2 runs the
+ * persistent stage from a reset state for candidate nets per pack (nets routed
+ * together by one warp) by bucket, one of them the untuned rule that follows
+ * each batch's size.  The choices stay in the context (and are copied to the
+ * optional per_cta[4] / per_grab[4]; per_grab as used on the plan's largest
+ * batch).  Needs nets and a plan; leaves the
  * context reset (grb_reset).  Routes do not depend on the choices. */
 int grb_autotune(grb_ctx* ctx, int32_t what, int32_t* per_cta, int32_t* per_grab);
 
