@@ -425,22 +425,22 @@ __device__ __forceinline__ PackArena pack_arena(char* p, int L, int nmax) {
 // The trees of a pack: lane q < nodes holds tree node q of the forest.
 struct Pack {
     int nets, nodes;
-    int id;          // lane's net (nets without nodes appear nowhere)
+    int id;          // lane's net (nets without nodes have no lane)
     int first, count;// lane's net: its root's lane, its nodes
     int x, y, lay;   // lay = L: Steiner point
     int par;         // parent's lane, -1 at a root (and beyond the nodes)
     long long out, cap;  // lane's net: route words
 };
-// `k` <= 16 nets ids[0..k), at most 32 nodes together.
-__device__ __forceinline__ Pack load_pack(const Tables& T, const Plan& P, const int* ids, int k, int lane) {
+// `k` <= 16 nets -- ids[0..k), or first_id on where ids is null --, at most 32
+// nodes together.
+__device__ __forceinline__ Pack load_pack(const Tables& T, const Plan& P, const int* ids, int first_id, int k, int lane) {
     Pack K;
     K.nets = k;
     int id = 0, off = 0, n = 0;
     if (lane < k) {
-        id = ids[lane];
+        id = ids ? ids[lane] : first_id + lane;
         off = P.node_off[id];
         n = P.node_off[id + 1] - off;
-        if (n == 0 && P.route_off[id + 1] > P.route_off[id]) P.routes[P.route_off[id]] = 1;  // an empty route
     }
     int incl = n;
 #pragma unroll

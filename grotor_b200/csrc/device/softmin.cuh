@@ -21,12 +21,26 @@
 // (full_update.cuh:9-83 without the float narrowing, so FD checks in fp64 are
 // smooth).  Demand d is the context's current demand, held fixed.
 //
-// Memory: the forward keeps only each net's root value; the backward
-// recomputes each net's DP tables in a per-thread scratch slot (N * L * L
-// values for the forward ranges, as many for their adjoints), so memory is
-// bounded by the threads in flight, not by the nets.
+// B200 form: the hard DP's packs (lshape.cuh) -- one warp takes several nets,
+// at most SoftArena's nodes together, a lane per tree node for the bookkeeping
+// and lane = slot * L + layer for the steps of a depth, with every table of the
+// pack in shared memory.  A soft minimum over nested sets is accumulated as a
+// running pair (m, s) = (minimum, sum of exp(-(v - m) / tau)): suffixes of a
+// row, then a column of them, give cur[l] with 18 exponentials a lane in place
+// of up to 25 per layer twice over, and the running minimum of diag gives the
+// nine ranges of a row with nine.  The adjoint walks the same running pairs
+// backwards with the exponentials the forward walk left.  The adjoint of a
+// wire or via cost is summed over its candidates inside the warp, so a tree
+// edge updates each cell of the tables once.  All tables are track by track
+// like the routing tables; inputs and gradients are converted on the way.
+//
+// Thread per net with the tables in local arrays (the form before, 120K nets
+// at 320x320x10, fp32, tau = 1): forward 3.1 ms, adjoint 46 ms; now 0.8 and 5.1 ms.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
+#include "lshape.cuh"
 
 namespace grb {
 
@@ -41,16 +55,15 @@ template <> __device__ __forceinline__ double s_log<double>(double v) { return l
 
 template <class T>
 struct Soft {
-    const T* cap;        // [cells]
-    const T* uw;         // [cells] unit wire cost per edge
+    const T* cap;        // [slots] capacity
+    const T* uw;         // [slots] unit wire cost per edge
     T uv;                // unit via cost
-    T tau;
-    T* wc;               // [cells] wire cost
-    T* vc;               // [cells] via cost
-    T* P;                // [cells] exclusive prefix of wc along each track
-    T* dP;               // [cells] adjoint of P
-    T* dvc;              // [cells] adjoint of vc
-    T* slot;             // scratch: 2 * L * L values per node (range tables, adjoints)
+    T tau, inv_tau;
+    T* vc;               // [slots] via cost
+    T* P;                // [slots] exclusive prefix of the wire costs along each track
+    T* dP;               // [slots] adjoint of P
+    T* dvc;              // [slots] adjoint of vc
+    T* slot;             // scratch of nets beyond a pack: 2 * L * L values per node
     T* net_cost;         // [n_nets] soft root value of each net
 };
 
@@ -75,43 +88,142 @@ __device__ __forceinline__ T soft_of_dcap(const Tables& Tb, T cap, T d) {
     const T a = static_cast<T>(0.5) * (d - cap), b = scale * static_cast<T>(0.5) * (d - cap);
     return a < b ? static_cast<T>(-0.5) * s_exp<T>(a) : -scale * static_cast<T>(0.5) * s_exp<T>(b);
 }
-// Demand of the edge at IDX position c.
+// Increments of a whole and of half a unit on the edge at slot c of layer l,
+// and (deriv) their derivatives with respect to the capacity.
 template <class T>
-__device__ __forceinline__ T soft_demand(const Tables& Tb, int c) {
-    int l, x, y;
-    cell_position(Tb, c, l, x, y);
-    return static_cast<T>(Tb.demand[slot_index(Tb, l, x, y)]) * static_cast<T>(0.5);
+struct SoftTerms {
+    T one, half;
+};
+template <class T>
+__device__ __forceinline__ SoftTerms<T> soft_terms(const Tables& Tb, const Soft<T>& S, int c, int l) {
+    const T d = static_cast<T>(Tb.demand[c]) * static_cast<T>(0.5), cap = S.cap[c], w = static_cast<T>(Tb.short_costs[l]);
+    const T o0 = soft_of<T>(Tb, cap, d), top = static_cast<T>(1e12);
+    const T one = (soft_of<T>(Tb, cap, d + 1) - o0) * w, half = (soft_of<T>(Tb, cap, d + static_cast<T>(0.5)) - o0) * w;
+    return {one < top ? one : top, half < top ? half : top};
 }
 template <class T>
-__device__ __forceinline__ T soft_incr(const Tables& Tb, const Soft<T>& S, int c, int l, T k) {
-    const T d = soft_demand<T>(Tb, c);
-    const T v = (soft_of<T>(Tb, S.cap[c], d + k) - soft_of<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);
-    return v < static_cast<T>(1e12) ? v : static_cast<T>(1e12);
-}
-template <class T>
-__device__ __forceinline__ T soft_incr_dcap(const Tables& Tb, const Soft<T>& S, int c, int l, T k) {
-    const T d = soft_demand<T>(Tb, c);
-    const T v = (soft_of<T>(Tb, S.cap[c], d + k) - soft_of<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);
-    if (!(v < static_cast<T>(1e12))) return 0;
-    return (soft_of_dcap<T>(Tb, S.cap[c], d + k) - soft_of_dcap<T>(Tb, S.cap[c], d)) * static_cast<T>(Tb.short_costs[l]);
-}
-__device__ __forceinline__ int soft_edge_len(const Tables& Tb, int l, int x, int y) {
-    if (!along_y(Tb, l)) return x < Tb.X - 1 ? Tb.xlen[x] : 0;
-    return y < Tb.Y - 1 ? Tb.ylen[y] : 0;
+__device__ __forceinline__ SoftTerms<T> soft_terms_dcap(const Tables& Tb, const Soft<T>& S, int c, int l) {
+    const T d = static_cast<T>(Tb.demand[c]) * static_cast<T>(0.5), cap = S.cap[c], w = static_cast<T>(Tb.short_costs[l]);
+    const SoftTerms<T> v = soft_terms<T>(Tb, S, c, l);
+    const T o0 = soft_of_dcap<T>(Tb, cap, d), top = static_cast<T>(1e12);
+    return {v.one < top ? (soft_of_dcap<T>(Tb, cap, d + 1) - o0) * w : static_cast<T>(0),
+            v.half < top ? (soft_of_dcap<T>(Tb, cap, d + static_cast<T>(0.5)) - o0) * w : static_cast<T>(0)};
 }
 
-// Cost tables of one cell.
+// Prefix and suffix sums are accumulated beyond the working precision -- fp32 in
+// double, fp64 as an unevaluated sum of two doubles (Knuth's two-sum) -- and
+// rounded once: a wire's cost is the difference of two of them, divided by tau.
+struct WideSum {
+    double hi, lo;
+    __device__ __forceinline__ WideSum operator+(const WideSum& b) const {
+        const double s = hi + b.hi, t = s - hi;
+        const double e = (hi - (s - t)) + (b.hi - t) + (lo + b.lo);
+        WideSum r;
+        r.hi = s + e;
+        r.lo = e - (r.hi - s);
+        return r;
+    }
+};
+template <class T> struct SoftSum;
+template <> struct SoftSum<float> {
+    using V = double;
+    static __device__ __forceinline__ V of(float v) { return v; }
+    static __device__ __forceinline__ float round(V v) { return static_cast<float>(v); }
+    static __device__ __forceinline__ V up(V v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
+    static __device__ __forceinline__ V down(V v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
+    static __device__ __forceinline__ V from(V v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+};
+template <> struct SoftSum<double> {
+    using V = WideSum;
+    static __device__ __forceinline__ V of(double v) { return {v, 0.0}; }
+    static __device__ __forceinline__ double round(V v) { return v.hi + v.lo; }
+    static __device__ __forceinline__ V up(V v, int d) {
+        return {__shfl_up_sync(0xffffffffu, v.hi, d), __shfl_up_sync(0xffffffffu, v.lo, d)};
+    }
+    static __device__ __forceinline__ V down(V v, int d) {
+        return {__shfl_down_sync(0xffffffffu, v.hi, d), __shfl_down_sync(0xffffffffu, v.lo, d)};
+    }
+    static __device__ __forceinline__ V from(V v, int lane) {
+        return {__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane)};
+    }
+};
+
+// Via costs and the exclusive wire-cost prefix of one track, by one warp: lanes
+// over the positions, the prefix of each 32 by a shuffle scan.
 template <class T>
-__device__ __forceinline__ void soft_tables_cell(const Tables& Tb, const Soft<T>& S, int c) {
-    const int l = c / Tb.XY, rem = c - l * Tb.XY, x = rem / Tb.Y, y = rem - x * Tb.Y;
-    S.wc[c] = soft_incr<T>(Tb, S, c, l, 1) + S.uw[c] * static_cast<T>(soft_edge_len(Tb, l, x, y));
-    const bool ay = along_y(Tb, l);
-    const int pos = ay ? y : x, len = ay ? Tb.Y : Tb.X, stride = ay ? 1 : Tb.Y;
-    T v;
-    if (pos == 0) v = soft_incr<T>(Tb, S, c, l, 1);
-    else if (pos == len - 1) v = soft_incr<T>(Tb, S, c - stride, l, 1);
-    else v = soft_incr<T>(Tb, S, c, l, static_cast<T>(0.5)) + soft_incr<T>(Tb, S, c - stride, l, static_cast<T>(0.5));
-    S.vc[c] = v + S.uv;
+__device__ __forceinline__ void soft_tables_track(const Tables& Tb, const Soft<T>& S, int t, int lane) {
+    const Track K = track_of(Tb, t);
+    const int* elen = along_y(Tb, K.l) ? Tb.ylen : Tb.xlen;
+    using A = SoftSum<T>;
+    auto carry = A::of(0);
+    T last_one = 0, last_half = 0;
+    for (int p0 = 0; p0 < K.len; p0 += 32) {
+        const int p = p0 + lane, c = K.base + p;
+        SoftTerms<T> v{0, 0};
+        T w = 0;
+        if (p < K.len) {
+            v = soft_terms<T>(Tb, S, c, K.l);
+            w = v.one + S.uw[c] * static_cast<T>(p < K.len - 1 ? elen[p] : 0);
+        }
+        T one = __shfl_up_sync(0xffffffffu, v.one, 1), half = __shfl_up_sync(0xffffffffu, v.half, 1);
+        if (lane == 0) { one = last_one; half = last_half; }
+        last_one = __shfl_sync(0xffffffffu, v.one, 31);
+        last_half = __shfl_sync(0xffffffffu, v.half, 31);
+        auto incl = A::of(w);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const auto o = A::up(incl, d);
+            if (lane >= d) incl = incl + o;
+        }
+        auto excl = A::up(incl, 1);
+        if (lane == 0) excl = A::of(0);
+        if (p < K.len) {
+            S.vc[c] = (p == 0 ? v.one : p == K.len - 1 ? one : v.half + half) + S.uv;
+            S.P[c] = A::round(carry + excl);
+        }
+        carry = carry + A::from(incl, 31);
+    }
+}
+
+// The adjoints of one track's wire costs (dwc[j] = sum over later positions of
+// dP, since P[i] = sum over j < i of wc[j]) and via costs, through the cost
+// model to the capacity and the unit wire cost of each edge (written over vc
+// and P, which the adjoint no longer needs).  Returns the lane's part of the
+// sum of dvc, in double.
+template <class T>
+__device__ __forceinline__ double soft_chain_track(const Tables& Tb, const Soft<T>& S, int t, int lane, T* dcap, T* duw) {
+    const Track K = track_of(Tb, t);
+    const int* elen = along_y(Tb, K.l) ? Tb.ylen : Tb.xlen;
+    using A = SoftSum<T>;
+    auto carry = A::of(0);
+    double sum = 0;
+    for (int p0 = (K.len - 1) / 32 * 32; p0 >= 0; p0 -= 32) {
+        const int p = p0 + lane, c = K.base + p;
+        const bool in = p < K.len;
+        const T g = in ? S.dP[c] : static_cast<T>(0);
+        auto incl = A::of(g);  // sum over this position and the later ones of the 32
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const auto o = A::down(incl, d);
+            if (lane + d < 32) incl = incl + o;
+        }
+        auto excl = A::down(incl, 1);
+        if (lane == 31) excl = A::of(0);
+        if (in) {
+            const T dw = A::round(carry + excl), dv = S.dvc[c], next = p + 1 < K.len ? S.dvc[c + 1] : static_cast<T>(0);
+            const SoftTerms<T> e = soft_terms_dcap<T>(Tb, S, c, K.l);
+            T gc = dw * e.one;
+            if (p == 0) gc += dv * e.one;
+            else if (p < K.len - 1) gc += dv * e.half;
+            if (p + 1 == K.len - 1) gc += next * e.one;
+            else if (p + 1 < K.len - 1) gc += next * e.half;
+            dcap[c] = gc;
+            duw[c] = dw * static_cast<T>(p < K.len - 1 ? elen[p] : 0);
+            sum += static_cast<double>(dv);
+        }
+        carry = carry + A::from(incl, 0);
+    }
+    return sum;
 }
 
 // Soft minimum of v[0..n) (entries >= kSoftAbsent do not exist); writes the
@@ -134,14 +246,14 @@ __device__ __forceinline__ T smin(const T* v, int n, T tau, T* w) {
 
 template <class T>
 __device__ __forceinline__ T soft_wire(const Tables& Tb, const Soft<T>& S, int l, int xmin, int xmax, int ymin, int ymax) {
-    return S.P[cell_index(Tb, l, xmax, ymax)] - S.P[cell_index(Tb, l, xmin, ymin)];
+    return S.P[slot_index(Tb, l, xmax, ymax)] - S.P[slot_index(Tb, l, xmin, ymin)];
 }
 template <class T>
 __device__ __forceinline__ void soft_wire_adj(const Tables& Tb, const Soft<T>& S, int l, int xmin, int xmax, int ymin,
                                               int ymax, T g) {
     if (g == 0 || (xmin == xmax && ymin == ymax)) return;
-    atomicAdd(S.dP + cell_index(Tb, l, xmax, ymax), g);
-    atomicAdd(S.dP + cell_index(Tb, l, xmin, ymin), -g);
+    atomicAdd(S.dP + slot_index(Tb, l, xmax, ymax), g);
+    atomicAdd(S.dP + slot_index(Tb, l, xmin, ymin), -g);
 }
 
 // Candidate set of one tree edge: the arrival on parent layer pl from child
@@ -168,7 +280,7 @@ __device__ __forceinline__ T soft_leg(const Tables& Tb, const Soft<T>& S, const 
                              : soft_wire<T>(Tb, S, cl, E.minx, E.maxx, E.y, E.y);
     T cost2 = 0;
     for (int l = min(cl, pl) + 1; l < max(cl, pl); ++l)
-        cost2 += along_y(Tb, cl) ? S.vc[cell_index(Tb, l, E.x, E.py)] : S.vc[cell_index(Tb, l, E.px, E.y)];
+        cost2 += along_y(Tb, cl) ? S.vc[slot_index(Tb, l, E.x, E.py)] : S.vc[slot_index(Tb, l, E.px, E.y)];
     cost2 += along_y(Tb, pl) ? soft_wire<T>(Tb, S, pl, E.px, E.px, E.miny, E.maxy)
                              : soft_wire<T>(Tb, S, pl, E.minx, E.maxx, E.py, E.py);
     return cost + cost2;
@@ -183,7 +295,7 @@ __device__ __forceinline__ void soft_leg_adj(const Tables& Tb, const Soft<T>& S,
     if (along_y(Tb, cl)) soft_wire_adj<T>(Tb, S, cl, E.x, E.x, E.miny, E.maxy, g);
     else soft_wire_adj<T>(Tb, S, cl, E.minx, E.maxx, E.y, E.y, g);
     for (int l = min(cl, pl) + 1; l < max(cl, pl); ++l)
-        atomicAdd(S.dvc + (along_y(Tb, cl) ? cell_index(Tb, l, E.x, E.py) : cell_index(Tb, l, E.px, E.y)), g);
+        atomicAdd(S.dvc + (along_y(Tb, cl) ? slot_index(Tb, l, E.x, E.py) : slot_index(Tb, l, E.px, E.y)), g);
     if (along_y(Tb, pl)) soft_wire_adj<T>(Tb, S, pl, E.px, E.px, E.miny, E.maxy, g);
     else soft_wire_adj<T>(Tb, S, pl, E.minx, E.maxx, E.py, E.py, g);
 }
@@ -209,7 +321,7 @@ __device__ T soft_net_forward(const Tables& Tb, const Soft<T>& S, const Plan& P,
         T* d = dist + size_t(i) * LL;
         for (int lo = 0; lo < L; ++lo) {
             d[lo * L + lo] = 0;
-            for (int hi = lo + 1; hi < L; ++hi) d[lo * L + hi] = d[lo * L + hi - 1] + S.vc[cell_index(Tb, hi - 1, x, y)];
+            for (int hi = lo + 1; hi < L; ++hi) d[lo * L + hi] = d[lo * L + hi - 1] + S.vc[slot_index(Tb, hi - 1, x, y)];
             for (int hi = 0; hi < lo; ++hi) d[lo * L + hi] = absent;
             if (lp < L)
                 for (int hi = lo; hi < L; ++hi)
@@ -326,7 +438,376 @@ __device__ void soft_net_backward(const Tables& Tb, const Soft<T>& S, const Plan
             for (int lo = 0; lo <= l; ++lo)
                 for (int hi = l + 1; hi < L; ++hi)
                     if (di[lo * L + hi] < static_cast<T>(kSoftAbsent)) acc += gi[lo * L + hi];
-            if (acc != 0) atomicAdd(S.dvc + cell_index(Tb, l, x, y), acc);
+            if (acc != 0) atomicAdd(S.dvc + slot_index(Tb, l, x, y), acc);
+        }
+    }
+}
+
+// ---- packs -------------------------------------------------------------------
+// Shared memory of one warp.
+template <class T>
+struct SoftArena {
+    T* D;   // [nmax][TT] range tables
+    T* G;   // [nmax][TT] their adjoints (backward)
+    T* w1;  // [nmax][L] first leg (or straight) wire cost
+    T* w2;  // [nmax][L] second leg
+    T* col; // [nmax][2][L] via costs at the corners (x, py) and (px, y)
+    T* X;   // [32][L][2] exchange between the lanes of a slot
+};
+__host__ __device__ __forceinline__ size_t soft_arena_values(int L, int nmax, bool backward) {
+    return size_t(nmax) * ((backward ? 2 : 1) * tri_count(L) + 4 * L) + size_t(32) * L * 2;
+}
+template <class T>
+__device__ __forceinline__ SoftArena<T> soft_arena(T* p, int L, int nmax, bool backward) {
+    SoftArena<T> A;
+    A.D = p; p += size_t(nmax) * tri_count(L);
+    A.G = p; if (backward) p += size_t(nmax) * tri_count(L);
+    A.w1 = p; p += size_t(nmax) * L;
+    A.w2 = p; p += size_t(nmax) * L;
+    A.col = p; p += size_t(nmax) * 2 * L;
+    A.X = p;
+    return A;
+}
+
+// A running soft minimum: m the least value, s the sum of exp(-(v - m) / tau).
+// add() returns what the adjoint needs: e = exp(-|difference| / tau) and
+// whether the added value became the minimum.
+template <class T>
+struct SoftRun {
+    T m, s;
+    __device__ __forceinline__ T add(T m2, T s2, T inv_tau, bool& less) {
+        const T d = m2 - m;
+        less = d < 0;
+        const T e = s_exp<T>(-(less ? -d : d) * inv_tau);
+        s = less ? s * e + s2 : s + s2 * e;
+        m = less ? m2 : m;
+        return e;
+    }
+    __device__ __forceinline__ T value(T tau) const { return m - tau * s_log<T>(s); }
+};
+
+// Forward DP of a pack (net_cost of its nets), and with kBackward the adjoint
+// of g * (their sum) into dP and dvc.
+template <class T, int LC, bool kBackward>
+__device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, const Pack& K, const SoftArena<T>& A, T g,
+                                          int lane) {
+    const int L = LC > 0 ? LC : Tb.L, TT = tri_count(L);
+    constexpr int LL = LC > 0 ? LC : kMaxLayers;
+    constexpr unsigned kAll = 0xffffffffu;
+    const T absent = static_cast<T>(kSoftAbsent) * 10, tau = S.tau, inv = S.inv_tau;
+    constexpr T kNone = static_cast<T>(1e30);  // no value yet: above any sum of absent candidates
+    const int M = K.nodes;
+    if (M == 0) return;
+    int dep = K.par >= 0 ? 1 : 0;
+    for (int anc = K.par; __any_sync(kAll, anc >= 0);) {
+        const int od = __shfl_sync(kAll, dep, anc & 31), oa = __shfl_sync(kAll, anc, anc & 31);
+        if (anc >= 0) { dep += od; anc = oa; }
+    }
+    if (lane >= M) dep = -1;
+    const int dmax = __reduce_max_sync(kAll, dep);
+    const int xy = (K.x << 16) | K.y;
+    const int pxy = __shfl_sync(kAll, xy, K.par & 31);
+    // Costs of every (node, layer); the node's own column waits in its table.
+    for (int q0 = 0; q0 < M * L; q0 += 32) {
+        const int q = q0 + lane, i = min(q / L, M - 1), l = q - q / L * L;
+        const int c = __shfl_sync(kAll, xy, i), pc = __shfl_sync(kAll, pxy, i), pa = __shfl_sync(kAll, K.par, i);
+        if (q >= M * L) continue;
+        const int x = c >> 16, y = c & 0xffff, px = pc >> 16, py = pc & 0xffff;
+        const bool ay = along_y(Tb, l);
+        const int base = layer_base(Tb, l);
+        A.D[i * TT + l] = S.vc[base + (ay ? x * Tb.yp + y : y * Tb.xp + x)];
+        if (pa < 0) continue;
+        const bool straight = x == px || y == py;
+        const int lo = ay ? min(y, py) : min(x, px), hi = ay ? max(y, py) : max(x, px);
+        const int t1 = base + (ay ? x * Tb.yp : y * Tb.xp), t2 = base + (ay ? px * Tb.yp : py * Tb.xp);
+        A.w1[q] = !straight || (ay ? x == px : y == py) ? S.P[t1 + hi] - S.P[t1 + lo] : absent;
+        if (straight) continue;
+        A.w2[q] = S.P[t2 + hi] - S.P[t2 + lo];
+        A.col[(2 * i) * L + l] = S.vc[base + (ay ? x * Tb.yp + py : py * Tb.xp + x)];
+        A.col[(2 * i + 1) * L + l] = S.vc[base + (ay ? px * Tb.yp + y : y * Tb.xp + px)];
+    }
+    __syncwarp();
+    // Via stacks: row lo of every node's table.  The columns move to registers
+    // (a lane per node) before the tables overwrite them.
+    {
+        T vn[LL];
+#pragma unroll
+        for (int l = 0; l < LL; ++l) vn[l] = lane < M && l < L ? A.D[lane * TT + l] : static_cast<T>(0);
+        __syncwarp();
+        if (lane < M) {
+#pragma unroll
+            for (int lo = 0; lo < LL; ++lo) {
+                T acc = 0;
+#pragma unroll
+                for (int hi = lo; hi < LL; ++hi) {
+                    if (hi >= L) continue;
+                    if (hi > lo) acc += vn[hi - 1];
+                    A.D[lane * TT + tri(L, lo, hi)] = (K.lay < L && (lo > K.lay || hi < K.lay)) ? absent : acc;
+                }
+            }
+        }
+    }
+    __syncwarp();
+    const int NS = max(1, 32 / L);
+    const int slot = lane / L, sl = lane - slot * L, s0 = min(slot, NS - 1) * L;
+    T* X = A.X + size_t(s0) * L * 2;  // the slot's exchange: [L][L][2]
+    const int row = tri(L, sl, sl) - sl;
+    // Nodes of a depth in descending order, NS at a time; mode 0: forward,
+    // children into parents; mode 1: the adjoint, parents to children.
+    auto edges = [&](unsigned level, auto backward) {
+        constexpr bool kAdj = decltype(backward)::value;
+        for (unsigned at = level; at;) {
+            int i = -1;
+            for (int k = 0; k < NS; ++k) {
+                if (!at) break;
+                const int top = 31 - __clz(at);
+                if (k == slot) i = top;
+                at ^= 1u << top;
+            }
+            const bool act = i >= 0;
+            const int ii = max(i, 0);
+            const int c = __shfl_sync(kAll, xy, ii), pc = __shfl_sync(kAll, pxy, ii), p = __shfl_sync(kAll, K.par, ii) & 31;
+            const int x = c >> 16, y = c & 0xffff, px = pc >> 16, py = pc & 0xffff;
+            const bool straight = x == px || y == py;
+            const T* Di = A.D + ii * TT;
+            // Row sl: running soft minimum of columns 8 down to hi.
+            SoftRun<T> R{kNone, 0};
+            T re[LL], rs[LL];
+            unsigned rless = 0;
+            if (act) {
+#pragma unroll
+                for (int hi = LL - 1; hi >= 0; --hi) {
+                    if (hi < sl || hi >= L) continue;
+                    bool less;
+                    const T e = R.add(Di[row + hi], 1, inv, less);
+                    if (kAdj) { re[hi] = e; rs[hi] = R.s; rless |= unsigned(less) << hi; }
+                    X[(sl * L + hi) * 2] = R.m;
+                    X[(sl * L + hi) * 2 + 1] = R.s;
+                }
+            }
+            __syncwarp();
+            // Column sl: over the rows lo <= sl.
+            SoftRun<T> C{kNone, 0};
+            T ce[LL], cs[LL], cw[LL];
+            unsigned cless = 0;
+            if (act) {
+#pragma unroll
+                for (int lo = 0; lo < LL; ++lo) {
+                    if (lo > sl || lo >= L) continue;
+                    bool less;
+                    const T w = X[(lo * L + sl) * 2 + 1];
+                    const T e = C.add(X[(lo * L + sl) * 2], w, inv, less);
+                    if (kAdj) { ce[lo] = e; cs[lo] = C.s; cw[lo] = w; cless |= unsigned(less) << lo; }
+                }
+            }
+            __syncwarp();  // X is reused
+            const T reach = act ? C.value(tau) + A.w1[ii * L + sl] : absent;
+            // Arrival on parent layer sl: the candidates cl of the other parity
+            // (or cl = sl along a straight edge).
+            constexpr int NC = (LL + 1) / 2;
+            const int odd = (sl & 1) ^ 1;
+            const int side = along_y(Tb, sl) ? 1 : 0;  // the corner is the end of the first leg
+            const T* col = A.col + (2 * ii + side) * L;
+            const T leg2 = act && !straight ? A.w2[ii * L + sl] : static_cast<T>(0);
+            T v[NC];
+            T dm = absent, ds = 0;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const int cl = 2 * j + odd;
+                const T r = __shfl_sync(kAll, reach, s0 + min(cl, L - 1));
+                v[j] = absent;
+                if (!act || straight || cl >= L) continue;
+                T via = 0;
+                for (int l = min(cl, sl) + 1; l < max(cl, sl); ++l) via += col[l];
+                v[j] = r + (via + leg2);
+                dm = v[j] < dm ? v[j] : dm;
+            }
+            T diag = absent;
+            T vw[NC];
+            if (act && straight) {
+                diag = reach;
+            } else if (act) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j) {
+                    vw[j] = 2 * j + odd < L ? s_exp<T>(-(v[j] - dm) * inv) : static_cast<T>(0);
+                    ds += vw[j];
+                }
+                diag = dm < static_cast<T>(kSoftAbsent) ? dm - tau * s_log<T>(ds) : absent;
+            }
+            // Row sl of the contribution: running soft minimum of diag[sl..hi].
+            SoftRun<T> B{kNone, 0};
+            T be[LL], bs[LL];
+            unsigned bless = 0;
+            T* Dp = A.D + p * TT;
+            T out[LL];
+#pragma unroll
+            for (int hi = 0; hi < LL; ++hi) {
+                if (hi >= L) continue;
+                const T dv = __shfl_sync(kAll, diag, s0 + hi);
+                if (!act || hi < sl) continue;
+                bool less;
+                const T e = B.add(dv, 1, inv, less);
+                if (kAdj) { be[hi] = e; bs[hi] = B.s; bless |= unsigned(less) << hi; }
+                else out[hi] = B.value(tau);
+            }
+            if (!kAdj) {
+                for (int k = 0; k < NS; ++k) {  // slots in turn: a parent's children in descending order
+                    if (act && slot == k) {
+#pragma unroll
+                        for (int hi = 0; hi < LL; ++hi)
+                            if (hi >= sl && hi < L) Dp[row + hi] += out[hi];
+                    }
+                    __syncwarp();
+                }
+                continue;
+            }
+            // Adjoint.  Contribution: back along the running minimum.
+            const T* Gp = A.G + p * TT;
+            T carry = 0;
+            if (act) {
+#pragma unroll
+                for (int hi = LL - 1; hi >= 0; --hi) {
+                    if (hi < sl || hi >= L) continue;
+                    const T acc = Gp[row + hi] + carry, is = static_cast<T>(1) / bs[hi], e = be[hi];
+                    const bool less = (bless >> hi) & 1u;
+                    X[sl * L + hi] = acc * (less ? is : e * is);
+                    carry = hi > sl ? acc * (less ? bs[hi - 1] * e * is : bs[hi - 1] * is) : static_cast<T>(0);
+                }
+            }
+            __syncwarp();
+            T gd = 0;  // adjoint of diag[sl]
+            if (act) {
+#pragma unroll
+                for (int lo = 0; lo < LL; ++lo)
+                    if (lo <= sl && lo < L) gd += X[lo * L + sl];
+            }
+            __syncwarp();
+            // Arrival: X[pl][cl] = adjoint of candidate (cl, pl).
+            T gcur = 0, gleg2 = 0;
+            if (act && straight) gcur = gd;
+            if (act && !straight) {
+                const T is = ds > 0 ? static_cast<T>(1) / ds : static_cast<T>(0);
+#pragma unroll
+                for (int j = 0; j < NC; ++j) {
+                    const int cl = 2 * j + odd;
+                    if (cl >= L) continue;
+                    const T w = gd * (vw[j] * is);
+                    X[sl * L + cl] = w;
+                    gleg2 += w;
+                }
+            }
+            __syncwarp();
+            if (act && !straight) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j)
+                    if (2 * j + odd < L) gcur += X[(2 * j + odd) * L + sl];
+                // Via cells of layer sl at the two corners: every candidate
+                // whose layers enclose it; the corner by the first leg cl.
+                T va = 0, vb = 0;
+                for (int a = 0; a < sl; ++a)
+                    for (int b = a + 1; b < L; b += 2) {
+                        if (b <= sl) continue;
+                        const T up = X[b * L + a], down = X[a * L + b];  // cl = a, pl = b; cl = b, pl = a
+                        if (along_y(Tb, a)) { va += up; vb += down; }
+                        else { vb += up; va += down; }
+                    }
+                if (va != 0) atomicAdd(S.dvc + slot_index(Tb, sl, x, py), va);
+                if (vb != 0) atomicAdd(S.dvc + slot_index(Tb, sl, px, y), vb);
+            }
+            if (act && (!straight || (along_y(Tb, sl) ? x == px : y == py))) {
+                // First leg on sl (at the child's end), second leg on sl (at the parent's).
+                const bool ay = along_y(Tb, sl);
+                const int base = layer_base(Tb, sl);
+                const int lo = ay ? min(y, py) : min(x, px), hi = ay ? max(y, py) : max(x, px);
+                const int t1 = base + (ay ? x * Tb.yp : y * Tb.xp), t2 = base + (ay ? px * Tb.yp : py * Tb.xp);
+                if (gcur != 0 && lo != hi) { atomicAdd(S.dP + t1 + hi, gcur); atomicAdd(S.dP + t1 + lo, -gcur); }
+                if (gleg2 != 0 && lo != hi) { atomicAdd(S.dP + t2 + hi, gleg2); atomicAdd(S.dP + t2 + lo, -gleg2); }
+            }
+            __syncwarp();
+            // Column sl back to the rows' running minima, then row sl back to
+            // the ranges.
+            if (act) {
+                carry = gcur;
+#pragma unroll
+                for (int lo = LL - 1; lo >= 0; --lo) {
+                    if (lo > sl || lo >= L) continue;
+                    const T is = static_cast<T>(1) / cs[lo], e = ce[lo];
+                    const bool less = (cless >> lo) & 1u;
+                    X[lo * L + sl] = carry * (less ? cw[lo] * is : cw[lo] * e * is);
+                    carry = lo > 0 ? carry * (less ? cs[lo > 0 ? lo - 1 : 0] * e * is : cs[lo > 0 ? lo - 1 : 0] * is)
+                                   : static_cast<T>(0);
+                }
+            }
+            __syncwarp();
+            if (act) {
+                T* Gi = A.G + ii * TT;
+                carry = 0;
+#pragma unroll
+                for (int hi = 0; hi < LL; ++hi) {
+                    if (hi < sl || hi >= L) continue;
+                    const T acc = X[sl * L + hi] + carry, is = static_cast<T>(1) / rs[hi], e = re[hi];
+                    const bool less = (rless >> hi) & 1u;
+                    Gi[row + hi] = acc * (less ? is : e * is);
+                    const T below = hi + 1 < L ? rs[hi + 1 < LL ? hi + 1 : hi] : static_cast<T>(0);
+                    carry = acc * (less ? below * e * is : below * is);
+                }
+            }
+            __syncwarp();
+        }
+    };
+    for (int d = dmax; d >= 1; --d) edges(__ballot_sync(kAll, dep == d), std::integral_constant<bool, false>{});
+    // Root values, lane = slot * L + lo.
+    for (unsigned at = __ballot_sync(kAll, dep == 0); at;) {
+        int i = -1;
+        for (int k = 0; k < NS; ++k) {
+            if (!at) break;
+            const int top = 31 - __clz(at);
+            if (k == slot) i = top;
+            at ^= 1u << top;
+        }
+        const bool act = i >= 0;
+        const int ii = max(i, 0), id = __shfl_sync(kAll, K.id, ii);
+        const T* Di = A.D + ii * TT;
+        T m = absent;
+        if (act) {
+#pragma unroll
+            for (int hi = 0; hi < LL; ++hi)
+                if (hi >= sl && hi < L) m = Di[row + hi] < m ? Di[row + hi] : m;
+        }
+        T best = absent;
+        for (int l = 0; l < L; ++l) {
+            const T o = __shfl_sync(kAll, m, s0 + l);
+            best = o < best ? o : best;
+        }
+        T part = 0, w[LL];
+        if (act) {
+#pragma unroll
+            for (int hi = 0; hi < LL; ++hi)
+                if (hi >= sl && hi < L) { w[hi] = s_exp<T>(-(Di[row + hi] - best) * inv); part += w[hi]; }
+        }
+        T sum = 0;
+        for (int l = 0; l < L; ++l) sum += __shfl_sync(kAll, part, s0 + l);
+        const bool feasible = best < static_cast<T>(kSoftAbsent);
+        if (act && sl == 0 && S.net_cost) S.net_cost[id] = feasible ? best - tau * s_log<T>(sum) : absent;
+        if (kBackward && act) {
+#pragma unroll
+            for (int hi = 0; hi < LL; ++hi)
+                if (hi >= sl && hi < L) A.G[ii * TT + row + hi] = feasible ? g * (w[hi] / sum) : static_cast<T>(0);
+        }
+    }
+    __syncwarp();
+    if constexpr (kBackward) {
+        for (int d = 1; d <= dmax; ++d) edges(__ballot_sync(kAll, dep == d), std::integral_constant<bool, true>{});
+        // Via stacks of every node's ranges: range [lo, hi] holds vc[lo..hi-1].
+        for (int q0 = 0; q0 < M * L; q0 += 32) {
+            const int q = q0 + lane, i = min(q / L, M - 1), l = q - q / L * L;
+            const int c = __shfl_sync(kAll, xy, i);
+            if (q >= M * L || l + 1 >= L) continue;
+            const T* Gi = A.G + i * TT;
+            T acc = 0;
+            for (int lo = 0; lo <= l; ++lo)
+                for (int hi = l + 1; hi < L; ++hi) acc += Gi[tri(L, lo, hi)];
+            if (acc != 0) atomicAdd(S.dvc + slot_index(Tb, l, c >> 16, c & 0xffff), acc);
         }
     }
 }

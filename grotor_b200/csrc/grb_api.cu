@@ -94,7 +94,11 @@ __device__ __forceinline__ void route_nets(const Tables& T, const Plan& P, const
     } else if (N > kPackNodes) {
         lshape_net(T, P, id, stamp, carve_arena(slot, T.L, N), lane, commit);
     } else {
-        const Pack K = load_pack(T, P, ids, k, lane);
+        const Pack K = load_pack(T, P, ids, 0, k, lane);
+        if (lane < k) {  // nets without nodes: an empty route
+            const int e = ids[lane];
+            if (P.node_off[e + 1] == P.node_off[e] && P.route_off[e + 1] > P.route_off[e]) P.routes[P.route_off[e]] = 1;
+        }
         route_pack(T, P, K, stamp, N > nmax ? pack_arena(slot, T.L, N) : pack_arena(arena, T.L, nmax), lane, commit);
     }
 }
@@ -491,89 +495,74 @@ __global__ void k_bbox_scatter(const int* batch_off, const int* tmp, const int* 
     }
 }
 
+constexpr int kSoftParts = 256;  // partial sums of the nets' costs
 // --- soft-min DAG and adjoint (softmin.cuh) ---------------------------------
 constexpr int kSoftThreads = 128;
 
 template <class T>
-__global__ void k_soft_tables(Tables Tb, Soft<T> S) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < Tb.cells) soft_tables_cell<T>(Tb, S, c);
+__global__ void k_soft_tables(Tables Tb, Soft<T> S) {  // one warp per track
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t < Tb.tracks) soft_tables_track<T>(Tb, S, t, threadIdx.x & 31);
 }
-// Track k of layer l (one thread each): first cell, stride and length.
-__device__ __forceinline__ bool soft_track(const Tables& Tb, int t, int& base, int& stride, int& len) {
-    const int M = max(Tb.X, Tb.Y), l = t / M, k = t - l * M;
-    if (l >= Tb.L) return false;
-    if (along_y(Tb, l)) {
-        if (k >= Tb.X) return false;
-        base = cell_index(Tb, l, k, 0); stride = 1; len = Tb.Y;
-    } else {
-        if (k >= Tb.Y) return false;
-        base = cell_index(Tb, l, 0, k); stride = Tb.Y; len = Tb.X;
-    }
-    return true;
-}
-template <class T>
-__global__ void k_soft_prefix(Tables Tb, Soft<T> S) {
-    int base, stride, len;
-    if (!soft_track(Tb, blockIdx.x * blockDim.x + threadIdx.x, base, stride, len)) return;
-    T acc = 0;
-    for (int q = 0; q < len; ++q) {
-        S.P[base + q * stride] = acc;
-        acc += S.wc[base + q * stride];
-    }
-}
-// One thread per net; a net's range tables (and their adjoints) sit in the
-// scratch at twice its first node's index times L*L, so every net of the
-// design runs at once.
-template <class T>
-__global__ void __launch_bounds__(kSoftThreads) k_soft_forward(Tables Tb, Soft<T> S, Plan P, int n) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    T* dist = S.slot + size_t(2) * P.node_off[id] * Tb.L * Tb.L;
-    S.net_cost[id] = P.node_off[id + 1] > P.node_off[id] ? soft_net_forward<T>(Tb, S, P, id, dist) : T(0);
-}
-template <class T>
-__global__ void __launch_bounds__(kSoftThreads) k_soft_backward(Tables Tb, Soft<T> S, Plan P, int n, T g) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const int N = P.node_off[id + 1] - P.node_off[id];
-    T* dist = S.slot + size_t(2) * P.node_off[id] * Tb.L * Tb.L;
-    T* gd = dist + size_t(N) * Tb.L * Tb.L;
-    if (N > 0) soft_net_backward<T>(Tb, S, P, id, dist, gd, g);
-}
-// dwc[j] = sum over later track positions of dP (presum[i] = sum_{j<i} wc[j]).
-template <class T>
-__global__ void k_soft_suffix(Tables Tb, Soft<T> S, T* dwc) {
-    int base, stride, len;
-    if (!soft_track(Tb, blockIdx.x * blockDim.x + threadIdx.x, base, stride, len)) return;
-    T acc = 0;
-    for (int q = len - 1; q >= 0; --q) {
-        dwc[base + q * stride] = acc;
-        acc += S.dP[base + q * stride];
+// Forward DP (net_cost) or adjoint of every net: a warp takes `span`
+// consecutive nets, as many at a time as its arena of nmax nodes holds; nets
+// beyond kPackNodes are walked by one thread in global scratch.
+template <class T, int LC, bool kBackward>
+__global__ void __launch_bounds__(kSoftThreads, sizeof(T) == 4 ? 3 : 2) k_soft_packs(Tables Tb, Soft<T> S, Plan P, int n, int span, int nmax, T g) {
+    extern __shared__ __align__(16) char smem[];
+    const int lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const SoftArena<T> A = soft_arena(reinterpret_cast<T*>(smem) + (threadIdx.x >> 5) * soft_arena_values(Tb.L, nmax, kBackward),
+                                      Tb.L, nmax, kBackward);
+    const long long first = (long long)w * span;
+    const int end = int(min(first + span, (long long)n));
+    for (int at = int(min(first, (long long)n)); at < end;) {
+        int incl = lane < 16 && at + lane < end ? P.node_off[at + lane + 1] - P.node_off[at] : 0x7fffffff;
+        const int k = __popc(__ballot_sync(0xffffffffu, incl <= nmax));  // offsets do not decrease: the first k nets fit
+        if (!k) {
+            if (lane == 0) {
+                const int N = P.node_off[at + 1] - P.node_off[at];
+                T* dist = S.slot + size_t(2) * P.node_off[at] * Tb.L * Tb.L;
+                if (kBackward) soft_net_backward<T>(Tb, S, P, at, dist, dist + size_t(N) * Tb.L * Tb.L, g);
+                else S.net_cost[at] = soft_net_forward<T>(Tb, S, P, at, dist);
+            }
+            ++at;
+            continue;
+        }
+        if (!kBackward && lane < k && P.node_off[at + lane + 1] == P.node_off[at + lane]) S.net_cost[at + lane] = 0;
+        const Pack K = load_pack(Tb, P, nullptr, at, k, lane);
+        soft_pack<T, LC, kBackward>(Tb, S, K, A, g, lane);
+        __syncwarp();
+        at += k;
+// Adjoints of the tracks' costs into gradients (one warp per track), and each
+// track's part of the via cost's.
     }
 }
-// Chain rule to capacity and the per-edge unit wire cost.
 template <class T>
-__global__ void k_soft_chain(Tables Tb, Soft<T> S, const T* dwc, T* dcap, T* duw) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= Tb.cells) return;
-    const int l = c / Tb.XY, rem = c - l * Tb.XY, x = rem / Tb.Y, y = rem - x * Tb.Y;
-    const bool ay = along_y(Tb, l);
-    const int pos = ay ? y : x, len = ay ? Tb.Y : Tb.X, stride = ay ? 1 : Tb.Y;
-    T g = dwc[c] * soft_incr_dcap<T>(Tb, S, c, l, 1);
-    if (pos == 0) g += S.dvc[c] * soft_incr_dcap<T>(Tb, S, c, l, 1);
-    else if (pos < len - 1) g += S.dvc[c] * soft_incr_dcap<T>(Tb, S, c, l, static_cast<T>(0.5));
-    if (pos + 1 == len - 1) g += S.dvc[c + stride] * soft_incr_dcap<T>(Tb, S, c, l, 1);
-    else if (pos + 1 < len - 1) g += S.dvc[c + stride] * soft_incr_dcap<T>(Tb, S, c, l, static_cast<T>(0.5));
-    dcap[c] = g;
-    duw[c] = dwc[c] * static_cast<T>(soft_edge_len(Tb, l, x, y));
+__global__ void k_soft_chain(Tables Tb, Soft<T> S, T* dcap, T* duw, double* parts) {
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (t >= Tb.tracks) return;
+    double sum = soft_chain_track<T>(Tb, S, t, lane, dcap, duw);
+    for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if (lane == 0) parts[t] = sum;
 }
-// Deterministic sum of v[0..n) into *out (one CTA).
+// Deterministic sums: parts[block] of v[0..n), and one CTA's total of parts.
 template <class T>
-__global__ void __launch_bounds__(1024) k_soft_sum(const T* v, int n, double* out) {
+__global__ void __launch_bounds__(256) k_soft_parts(const T* v, int n, double* parts) {
+    __shared__ double ws[8];
+    double acc = 0;
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) acc += static_cast<double>(v[k]);
+    for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) acc += ws[k];
+        parts[blockIdx.x] = acc;
+    }
+}
+__global__ void __launch_bounds__(1024) k_soft_total(const double* parts, int n, double* out) {
     __shared__ double part[1024];
     double acc = 0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) acc += static_cast<double>(v[k]);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) acc += parts[k];
     part[threadIdx.x] = acc;
     __syncthreads();
     for (int w = blockDim.x / 2; w; w >>= 1) {
@@ -1121,10 +1110,10 @@ struct grb_ctx {
     int64_t z_graph_kernels = 0;
     // soft-min workspace (grb_softmin_forward / backward)
     std::vector<void*> soft_bufs;
-    char* soft_cells = nullptr;       // 6 arrays of cells doubles
+    char* soft_cells = nullptr;       // 6 tables of doubles
     char* soft_slot = nullptr;
     size_t soft_slot_bytes = 0;
-    double* soft_scalar = nullptr;
+    double* soft_parts = nullptr;     // total, then partial sums
     int* check = nullptr;             // [3] upload validation status
     // size-bucketed plan and tuned launch shapes
     int* bucket_ids = nullptr;
@@ -1528,51 +1517,79 @@ int z_stage_persistent(grb_ctx* c, int stamp0) {
 
 // --- soft-min executors ------------------------------------------------------
 int soft_workspace(grb_ctx* c) {
-    const size_t cells = c->T.cells;
-    // Range tables and adjoints of every node: 2 * nodes * L * L values.
-    const size_t slot = 2 * size_t(std::max(c->topo_sizes[0], 1ll)) * c->T.L * c->T.L * sizeof(double);
+    const size_t slots = c->T.slots;
+    // Six tables; partial sums by track; and for nets beyond a pack the range
+    // tables and adjoints of every node (2 * nodes * L * L values).
+    const size_t slot = c->max_nodes > kPackNodes
+        ? 2 * size_t(std::max(c->topo_sizes[0], 1ll)) * c->T.L * c->T.L * sizeof(double) : 0;
     if (c->soft_cells && c->soft_slot_bytes >= slot) return GRB_OK;
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
-    free_all(c->used_bufs);
     free_all(c->soft_bufs);
     int rc = 0;
-    rc |= dalloc(c, &c->soft_cells, 6 * cells * sizeof(double), c->soft_bufs);
-    rc |= dalloc(c, &c->soft_slot, slot, c->soft_bufs);
-    rc |= dalloc(c, &c->soft_scalar, 2, c->soft_bufs);
+    rc |= dalloc(c, &c->soft_cells, 6 * slots * sizeof(double), c->soft_bufs);
+    if (slot) rc |= dalloc(c, &c->soft_slot, slot, c->soft_bufs);
+    rc |= dalloc(c, &c->soft_parts, size_t(std::max(c->T.tracks, kSoftParts)) + 1, c->soft_bufs);
+    c->soft_cells = nullptr;
+    c->soft_slot = nullptr;
+    c->soft_slot_bytes = 0;
     if (rc) { free_all(c->soft_bufs); c->soft_cells = nullptr; return GRB_ENOMEM; }
     c->soft_slot_bytes = slot;
     return GRB_OK;
 }
 
 template <class T>
-Soft<T> soft_view(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost) {
-    const size_t cells = c->T.cells;
+Soft<T> soft_tables(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost) {
+    const Tables& Tb = c->T;
+    const size_t slots = Tb.slots;
     T* a = reinterpret_cast<T*>(c->soft_cells);
+// The inputs track by track, and the cost tables of the context's demand.
     Soft<T> S{};
-    S.cap = static_cast<const T*>(cap);
-    S.uw = static_cast<const T*>(uw);
+    S.cap = a;
+    S.uw = a + slots;
     S.uv = static_cast<T>(uv);
+    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(cap), a, 0);
+    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(uw), a + slots, 0);
     S.tau = static_cast<T>(tau);
-    S.wc = a; S.vc = a + cells; S.P = a + 2 * cells; S.dP = a + 3 * cells; S.dvc = a + 4 * cells;
+    S.inv_tau = static_cast<T>(1.0 / static_cast<double>(S.tau));
+    S.vc = a + 2 * slots; S.P = a + 3 * slots; S.dP = a + 4 * slots; S.dvc = a + 5 * slots;
     S.slot = reinterpret_cast<T*>(c->soft_slot);
     S.net_cost = net_cost;
     return S;
 }
 
 template <class T>
+    k_soft_tables<T><<<(Tb.tracks + 3) / 4, 128, 0, c->stream>>>(Tb, S);
+    c->launches += 3;
 int soft_forward(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost, double* total) {
     const Tables& Tb = c->T;
     const int n = c->n_nets;
-    Soft<T> S = soft_view<T>(c, tau, cap, uw, uv, net_cost);
-    const int M = std::max(Tb.X, Tb.Y);
-    k_soft_tables<T><<<(Tb.cells + 255) / 256, 256, 0, c->stream>>>(Tb, S);
-    k_soft_prefix<T><<<(Tb.L * M + 127) / 128, 128, 0, c->stream>>>(Tb, S);
-    k_soft_forward<T><<<std::max(1, (n + kSoftThreads - 1) / kSoftThreads), kSoftThreads, 0, c->stream>>>(
-        Tb, S, make_plan(c), n);
-    k_soft_sum<T><<<1, 1024, 0, c->stream>>>(net_cost, n, c->soft_scalar);
-    c->launches += 4;
+// Every net's DP, forward or adjoint.  A warp takes several nets once there are
+// more nets than warps on the GPU.
+template <class T, bool kBackward>
+int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
+    const int n = c->n_nets;
+    if (!n) return GRB_OK;
+    const int nmax = std::min(kPackNodes, std::max(16, c->max_nodes));
+    const int warps = kSoftThreads / 32, span = std::min(16, std::max(1, n / (c->sms * 16)));
+    const size_t smem = warps * soft_arena_values(c->T.L, nmax, kBackward) * sizeof(T);
+    const long long blocks = (n + (long long)span * warps - 1) / ((long long)span * warps);
+    // The layer loops unrolled for the 9 routing layers of 10-layer designs.
+    void (*kernel)(Tables, Soft<T>, Plan, int, int, int, T) =
+        c->T.L == 9 ? k_soft_packs<T, 9, kBackward> : k_soft_packs<T, 0, kBackward>;
+    GRB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    kernel<<<unsigned(blocks), kSoftThreads, smem, c->stream>>>(c->T, S, make_plan(c), n, span, nmax, g);
+    c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
-    GRB_CUDA(c, cudaMemcpyAsync(total, c->soft_scalar, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    return GRB_OK;
+}
+
+    const Soft<T> S = soft_tables<T>(c, tau, cap, uw, uv, net_cost);
+    if (int rc = soft_nets<T, false>(c, S, T(0))) return rc;
+    k_soft_parts<T><<<kSoftParts, 256, 0, c->stream>>>(net_cost, n, c->soft_parts + 1);
+    k_soft_total<<<1, 1024, 0, c->stream>>>(c->soft_parts + 1, kSoftParts, c->soft_parts);
+    c->launches += 2;
+    GRB_CUDA(c, cudaGetLastError());
+    GRB_CUDA(c, cudaMemcpyAsync(total, c->soft_parts, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     return GRB_OK;
 }
@@ -1580,24 +1597,18 @@ int soft_forward(grb_ctx* c, double tau, const void* cap, const void* uw, double
 template <class T>
 int soft_backward(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, double g, T* dcap, T* duw,
                   double* duv) {
-    const Tables& Tb = c->T;
-    const int n = c->n_nets;
-    const size_t cells = Tb.cells;
-    Soft<T> S = soft_view<T>(c, tau, cap, uw, uv, nullptr);
-    T* dwc = reinterpret_cast<T*>(c->soft_cells) + 5 * cells;
-    const int M = std::max(Tb.X, Tb.Y);
-    k_soft_tables<T><<<(Tb.cells + 255) / 256, 256, 0, c->stream>>>(Tb, S);
-    k_soft_prefix<T><<<(Tb.L * M + 127) / 128, 128, 0, c->stream>>>(Tb, S);
-    GRB_CUDA(c, cudaMemsetAsync(S.dP, 0, sizeof(T) * cells, c->stream));
-    GRB_CUDA(c, cudaMemsetAsync(S.dvc, 0, sizeof(T) * cells, c->stream));
-    k_soft_backward<T><<<std::max(1, (n + kSoftThreads - 1) / kSoftThreads), kSoftThreads, 0, c->stream>>>(
-        Tb, S, make_plan(c), n, static_cast<T>(g));
-    k_soft_suffix<T><<<(Tb.L * M + 127) / 128, 128, 0, c->stream>>>(Tb, S, dwc);
-    k_soft_chain<T><<<(Tb.cells + 255) / 256, 256, 0, c->stream>>>(Tb, S, dwc, dcap, duw);
-    k_soft_sum<T><<<1, 1024, 0, c->stream>>>(S.dvc, int(cells), c->soft_scalar + 1);
-    c->launches += 6;
+    const size_t slots = Tb.slots;
+    const Soft<T> S = soft_tables<T>(c, tau, cap, uw, uv, nullptr);
+    GRB_CUDA(c, cudaMemsetAsync(S.dP, 0, 2 * sizeof(T) * slots, c->stream));  // dP and dvc
+    if (int rc = soft_nets<T, true>(c, S, static_cast<T>(g))) return rc;
+    // The gradients, track by track, over the tables the adjoint has read.
+    k_soft_chain<T><<<(Tb.tracks + 3) / 4, 128, 0, c->stream>>>(Tb, S, S.vc, S.P, c->soft_parts + 1);
+    k_layout<T, false><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, S.vc, dcap, 0);
+    k_layout<T, false><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, S.P, duw, 0);
+    k_soft_total<<<1, 1024, 0, c->stream>>>(c->soft_parts + 1, Tb.tracks, c->soft_parts);
+    c->launches += 4;
     GRB_CUDA(c, cudaGetLastError());
-    GRB_CUDA(c, cudaMemcpyAsync(duv, c->soft_scalar + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    GRB_CUDA(c, cudaMemcpyAsync(duv, c->soft_parts, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     return GRB_OK;
 }
@@ -2034,6 +2045,7 @@ void grb_destroy(grb_ctx* c) {
     free_all(c->box_bufs);
     free_all(c->net_bufs);
     free_all(c->geom_bufs);
+    free_all(c->used_bufs);
     free_all(c->flt_bufs);
     free_all(c->topo_bufs);
     if (c->out_stream) cudaStreamSynchronize(c->out_stream);
