@@ -333,13 +333,16 @@ constexpr int kZThreads = 256;
 constexpr int kBoxThreads = 256;
 constexpr int kMaxBoxBatch = 256;
 
-constexpr int kZCand = 2 * (kMaxLayers + 1) * (kMaxLayers + 1);  // node-DP ranges per warp
+constexpr int kZFit = 96;  // nodes of a net whose arrays may sit in shared memory
 // One CTA per net of batch b (solve<4>, zshape.cuh:62-388, with the route
 // conversion of convert_routes fused into the traceback).
 __global__ void __launch_bounds__(kZThreads) k_zshape_batch(Tables T, ZTrees Z, Plan P, int b) {
-    __shared__ int cand[kZCand];
-    const int lo = P.batch_off[b];
-    zshape_net(T, Z, P, P.ids[lo + blockIdx.x], 0, threadIdx.x, blockDim.x, false, cand);
+    extern __shared__ __align__(16) int zsm[];
+    const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
+    for (int k = blockIdx.x; k < cnt; k += gridDim.x) {
+        zshape_net(T, Z, P, P.ids[lo + k], 0, false, zsm);
+        __syncthreads();
+    }
 }
 // Thread-per-net commit (commit_wire_demand / commit_via_demand,
 // demand.cuh:129-232), the Z-shape pipeline's form (pipeline_ggr.hpp:132-133).
@@ -357,24 +360,19 @@ __global__ void k_commit_thread_vias(Tables T, Plan P, int b, int stamp) {
 // Persistent Z-shape stage: per batch, refresh the tracks -> Z-shape nets and
 // their wires -> vias.
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_zshape_persistent(Tables T, ZTrees Z, Plan P, GridSync S,
-                                                                              int stamp0, int* work) {
+                                                                              int stamp0) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * (blockDim.x >> 5);
-    __shared__ int cand[kZCand];
-    __shared__ int znet;
+    extern __shared__ __align__(16) int zsm[];
     PhaseClock clk;
     clk.start(S);
     for (int b = 0; b < P.n_batches; ++b) {
         const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
         const int stamp = stamp0 + b + 1;
         if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
-        while (true) {  // one CTA per net
-            if (threadIdx.x == 0) znet = atomicAdd(work + b, 1);
+        for (int k = blockIdx.x; k < cnt; k += gridDim.x) {  // one CTA per net
+            zshape_net(T, Z, P, P.ids[lo + k], stamp, true, zsm);
             __syncthreads();
-            const int k = znet;
-            __syncthreads();
-            if (k >= cnt) break;
-            zshape_net(T, Z, P, P.ids[lo + k], stamp, threadIdx.x, blockDim.x, true, cand);
         }
         if (!grid_sync(S, T)) return;
         clk.mark(S, 5);
@@ -495,9 +493,9 @@ __global__ void k_bbox_scatter(const int* batch_off, const int* tmp, const int* 
     }
 }
 
-constexpr int kSoftParts = 256;  // partial sums of the nets' costs
 // --- soft-min DAG and adjoint (softmin.cuh) ---------------------------------
 constexpr int kSoftThreads = 128;
+constexpr int kSoftParts = 256;  // partial sums of the nets' costs
 
 template <class T>
 __global__ void k_soft_tables(Tables Tb, Soft<T> S) {  // one warp per track
@@ -533,10 +531,10 @@ __global__ void __launch_bounds__(kSoftThreads, sizeof(T) == 4 ? 3 : 2) k_soft_p
         soft_pack<T, LC, kBackward>(Tb, S, K, A, g, lane);
         __syncwarp();
         at += k;
-// Adjoints of the tracks' costs into gradients (one warp per track), and each
-// track's part of the via cost's.
     }
 }
+// Adjoints of the tracks' costs into gradients (one warp per track), and each
+// track's part of the via cost's.
 template <class T>
 __global__ void k_soft_chain(Tables Tb, Soft<T> S, T* dcap, T* duw, double* parts) {
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -1446,6 +1444,12 @@ int stage_plain(grb_ctx* c, int stamp0) {
 }
 
 // --- Z-shape stage executors (pipeline_ggr.hpp:119-134) ---------------------
+int z_blocks(const grb_ctx* c) { return c->sms * 8; }  // CTAs with a scratch slot
+size_t z_smem(const grb_ctx* c) {
+    const int LY = c->Z.LAYER;
+    return sizeof(int) * (size_t(kZThreads / 32) * 2 * LY * LY + size_t(c->Z.fit) * znet_ints(LY));
+}
+
 int z_stage_plain(grb_ctx* c, int stamp0) {
     const Plan P = make_plan(c);
     for (int b = 0; b < c->n_batches; ++b) {
@@ -1456,7 +1460,7 @@ int z_stage_plain(grb_ctx* c, int stamp0) {
         if ((rc = refresh_plain(c))) return rc;
         cudaEvent_t e;
         if ((rc = prof_begin(c, 5, &e))) return rc;
-        k_zshape_batch<<<cnt, kZThreads, 0, c->stream>>>(c->T, c->Z, P, b);
+        k_zshape_batch<<<std::min(cnt, z_blocks(c)), kZThreads, z_smem(c), c->stream>>>(c->T, c->Z, P, b);
         prof_end(c, e);
         if ((rc = prof_begin(c, 6, &e))) return rc;
         k_commit_thread_wires<<<(cnt + 255) / 256, 256, 0, c->stream>>>(c->T, P, b, stamp);
@@ -1499,18 +1503,18 @@ int ensure_work(grb_ctx* c);
 int z_stage_persistent(grb_ctx* c, int stamp0) {
     if (c->n_batches == 0) return GRB_OK;
     int per_sm = 0;
-    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, 0));
+    const size_t smem = z_smem(c);
+    GRB_CUDA(c, cudaFuncSetAttribute(k_zshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent Z-shape kernel does not fit on an SM");
-    int rc = ensure_work(c);
-    if (rc) return rc;
     GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
     Tables T = c->T;
     ZTrees Z = c->Z;
     Plan P = make_plan(c);
     GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
-    void* args[] = {&T, &Z, &P, &S, &stamp0, &c->work};
-    GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_zshape_persistent, dim3(per_sm * c->sms), dim3(kPersistentThreads),
-                                            args, 0, c->stream));
+    void* args[] = {&T, &Z, &P, &S, &stamp0};
+    GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_zshape_persistent, dim3(std::min(per_sm * c->sms, z_blocks(c))),
+                                            dim3(kPersistentThreads), args, smem, c->stream));
     c->launches += 1;
     return GRB_OK;
 }
@@ -1525,44 +1529,40 @@ int soft_workspace(grb_ctx* c) {
     if (c->soft_cells && c->soft_slot_bytes >= slot) return GRB_OK;
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     free_all(c->soft_bufs);
+    c->soft_cells = nullptr;
+    c->soft_slot = nullptr;
+    c->soft_slot_bytes = 0;
     int rc = 0;
     rc |= dalloc(c, &c->soft_cells, 6 * slots * sizeof(double), c->soft_bufs);
     if (slot) rc |= dalloc(c, &c->soft_slot, slot, c->soft_bufs);
     rc |= dalloc(c, &c->soft_parts, size_t(std::max(c->T.tracks, kSoftParts)) + 1, c->soft_bufs);
-    c->soft_cells = nullptr;
-    c->soft_slot = nullptr;
-    c->soft_slot_bytes = 0;
     if (rc) { free_all(c->soft_bufs); c->soft_cells = nullptr; return GRB_ENOMEM; }
     c->soft_slot_bytes = slot;
     return GRB_OK;
 }
 
+// The inputs track by track, and the cost tables of the context's demand.
 template <class T>
 Soft<T> soft_tables(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost) {
     const Tables& Tb = c->T;
     const size_t slots = Tb.slots;
     T* a = reinterpret_cast<T*>(c->soft_cells);
-// The inputs track by track, and the cost tables of the context's demand.
+    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(cap), a, 0);
+    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(uw), a + slots, 0);
     Soft<T> S{};
     S.cap = a;
     S.uw = a + slots;
     S.uv = static_cast<T>(uv);
-    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(cap), a, 0);
-    k_layout<T, true><<<layout_grid(Tb, Tb.L), dim3(32, 8), 0, c->stream>>>(Tb, static_cast<const T*>(uw), a + slots, 0);
     S.tau = static_cast<T>(tau);
     S.inv_tau = static_cast<T>(1.0 / static_cast<double>(S.tau));
     S.vc = a + 2 * slots; S.P = a + 3 * slots; S.dP = a + 4 * slots; S.dvc = a + 5 * slots;
     S.slot = reinterpret_cast<T*>(c->soft_slot);
     S.net_cost = net_cost;
+    k_soft_tables<T><<<(Tb.tracks + 3) / 4, 128, 0, c->stream>>>(Tb, S);
+    c->launches += 3;
     return S;
 }
 
-template <class T>
-    k_soft_tables<T><<<(Tb.tracks + 3) / 4, 128, 0, c->stream>>>(Tb, S);
-    c->launches += 3;
-int soft_forward(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost, double* total) {
-    const Tables& Tb = c->T;
-    const int n = c->n_nets;
 // Every net's DP, forward or adjoint.  A warp takes several nets once there are
 // more nets than warps on the GPU.
 template <class T, bool kBackward>
@@ -1583,6 +1583,9 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
     return GRB_OK;
 }
 
+template <class T>
+int soft_forward(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, T* net_cost, double* total) {
+    const int n = c->n_nets;
     const Soft<T> S = soft_tables<T>(c, tau, cap, uw, uv, net_cost);
     if (int rc = soft_nets<T, false>(c, S, T(0))) return rc;
     k_soft_parts<T><<<kSoftParts, 256, 0, c->stream>>>(net_cost, n, c->soft_parts + 1);
@@ -1597,6 +1600,7 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
 template <class T>
 int soft_backward(grb_ctx* c, double tau, const void* cap, const void* uw, double uv, double g, T* dcap, T* duw,
                   double* duv) {
+    const Tables& Tb = c->T;
     const size_t slots = Tb.slots;
     const Soft<T> S = soft_tables<T>(c, tau, cap, uw, uv, nullptr);
     GRB_CUDA(c, cudaMemsetAsync(S.dP, 0, 2 * sizeof(T) * slots, c->stream));  // dP and dvc
@@ -2041,11 +2045,11 @@ void grb_destroy(grb_ctx* c) {
     if (c->flt_graph) cudaGraphExecDestroy(c->flt_graph);
     if (c->z_graph) cudaGraphExecDestroy(c->z_graph);
     free_all(c->soft_bufs);
+    free_all(c->used_bufs);
     free_all(c->z_bufs);
     free_all(c->box_bufs);
     free_all(c->net_bufs);
     free_all(c->geom_bufs);
-    free_all(c->used_bufs);
     free_all(c->flt_bufs);
     free_all(c->topo_bufs);
     if (c->out_stream) cudaStreamSynchronize(c->out_stream);
@@ -2598,17 +2602,8 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
         box[id] = bb;
     }
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
-    const bool planes = c->Z.map != nullptr && c->Z.LNN == LNN;
-    std::vector<void*> keep;
-    if (planes) {  // keep the (large) planes, replace the per-node arrays
-        for (void* p : c->z_bufs)
-            if (p == c->Z.map || p == c->Z.prev) keep.push_back(p);
-            else cudaFree(p);
-        c->z_bufs = keep;
-    } else {
-        free_all(c->z_bufs);
-    }
-    ZTrees Z = c->Z;
+    free_all(c->z_bufs);
+    ZTrees Z{};
     int *noff, *dpos, *dpin, *dch;
     int4* dbox;
     int rc = 0;
@@ -2617,10 +2612,11 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     rc |= dalloc(c, &dpin, nn, c->z_bufs);
     rc |= dalloc(c, &dch, 3 * nn, c->z_bufs);
     rc |= dalloc(c, &dbox, std::max(n, 1), c->z_bufs);
-    if (!planes) {
-        rc |= dalloc(c, &Z.map, size_t(6) * LNN, c->z_bufs);
-        rc |= dalloc(c, &Z.prev, size_t(16) * LNN, c->z_bufs);
-    }
+    int most = 1;
+    for (int i = 0; i < n; ++i) most = std::max(most, t->node_off[i + 1] - t->node_off[i]);
+    Z.fit = std::min(most, kZFit);
+    Z.scratch_ints = most > Z.fit ? (long long)most * znet_ints(LAYER) : 0;
+    if (Z.scratch_ints) rc |= dalloc(c, &Z.scratch, size_t(z_blocks(c)) * Z.scratch_ints, c->z_bufs);
     if (rc) { free_all(c->z_bufs); c->Z = ZTrees{}; c->z_n = -1; return GRB_ENOMEM; }
     auto h2d = [&](void* dst, const void* src, size_t bytes) {
         return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
@@ -2630,13 +2626,12 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     GRB_CUDA(c, h2d(dpin, pin.data(), 4 * size_t(nn)));
     GRB_CUDA(c, h2d(dch, t->child, 12 * size_t(nn)));
     GRB_CUDA(c, h2d(dbox, box.data(), sizeof(int4) * box.size()));
-    if (!planes) {
-        GRB_CUDA(c, cudaMemsetAsync(Z.map, 0, sizeof(int) * 6 * LNN, c->stream));
-        GRB_CUDA(c, cudaMemsetAsync(Z.prev, 0, sizeof(int) * 16 * LNN, c->stream));
-    }
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     Z.node_off = noff; Z.pos = dpos; Z.pin = dpin; Z.child = dch;
-    Z.N = N; Z.LAYER = LAYER; Z.D = T.DIR ^ 1; Z.NN = NN; Z.LNN = LNN;
+    Z.N = N; Z.NN = int(NN); Z.LAYER = LAYER; Z.D = T.DIR ^ 1;
+    Z.by_n = fast_div(N); Z.by_nn = fast_div(Z.NN);
+    GRB_CUDA(c, cudaFuncSetAttribute(k_zshape_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(sizeof(int) * (size_t(kZThreads / 32) * 2 * LAYER * LAYER + size_t(Z.fit) * znet_ints(LAYER)))));
     c->Z = Z;
     c->z_box = dbox;
     c->z_n = n;
