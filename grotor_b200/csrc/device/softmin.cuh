@@ -35,7 +35,7 @@
 // like the routing tables; inputs and gradients are converted on the way.
 //
 // Thread per net with the tables in local arrays (the form before, 120K nets
-// at 320x320x10, fp32, tau = 1): forward 3.1 ms, adjoint 46 ms; now 0.8 and 5.1 ms.
+// at 320x320x10, fp32, tau = 1): forward 3.1 ms, adjoint 46 ms; now 0.7 and 2.3 ms.
 #pragma once
 #include <type_traits>
 
@@ -110,43 +110,35 @@ __device__ __forceinline__ SoftTerms<T> soft_terms_dcap(const Tables& Tb, const 
             v.half < top ? (soft_of_dcap<T>(Tb, cap, d + static_cast<T>(0.5)) - o0) * w : static_cast<T>(0)};
 }
 
-// Prefix and suffix sums are accumulated beyond the working precision -- fp32 in
-// double, fp64 as an unevaluated sum of two doubles (Knuth's two-sum) -- and
-// rounded once: a wire's cost is the difference of two of them, divided by tau.
-struct WideSum {
-    double hi, lo;
-    __device__ __forceinline__ WideSum operator+(const WideSum& b) const {
-        const double s = hi + b.hi, t = s - hi;
-        const double e = (hi - (s - t)) + (b.hi - t) + (lo + b.lo);
-        WideSum r;
-        r.hi = s + e;
-        r.lo = e - (r.hi - s);
-        return r;
+// Exclusive prefix (kUp) or suffix sums of the warp's v behind `carry`, which
+// moves on by the warp's total.  fp32: accumulated in double, rounded once (a
+// wire's cost is the difference of two sums, divided by tau).  fp64: added one
+// by one in position order, whose rounding errors stay common to the sums of
+// neighbouring positions.
+template <bool kUp>
+__device__ __forceinline__ float soft_scan(float v, double& carry, int lane) {
+    double incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double o = kUp ? __shfl_up_sync(0xffffffffu, incl, d) : __shfl_down_sync(0xffffffffu, incl, d);
+        if (kUp ? lane >= d : lane + d < 32) incl += o;
     }
-};
-template <class T> struct SoftSum;
-template <> struct SoftSum<float> {
-    using V = double;
-    static __device__ __forceinline__ V of(float v) { return v; }
-    static __device__ __forceinline__ float round(V v) { return static_cast<float>(v); }
-    static __device__ __forceinline__ V up(V v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-    static __device__ __forceinline__ V down(V v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
-    static __device__ __forceinline__ V from(V v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
-};
-template <> struct SoftSum<double> {
-    using V = WideSum;
-    static __device__ __forceinline__ V of(double v) { return {v, 0.0}; }
-    static __device__ __forceinline__ double round(V v) { return v.hi + v.lo; }
-    static __device__ __forceinline__ V up(V v, int d) {
-        return {__shfl_up_sync(0xffffffffu, v.hi, d), __shfl_up_sync(0xffffffffu, v.lo, d)};
+    const double next = kUp ? __shfl_up_sync(0xffffffffu, incl, 1) : __shfl_down_sync(0xffffffffu, incl, 1);
+    const float out = static_cast<float>(lane == (kUp ? 0 : 31) ? carry : carry + next);
+    carry += __shfl_sync(0xffffffffu, incl, kUp ? 31 : 0);
+    return out;
+}
+template <bool kUp>
+__device__ __forceinline__ double soft_scan(double v, double& carry, int lane) {
+    double out = 0;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        const int j = kUp ? k : 31 - k;
+        if (lane == j) out = carry;
+        carry += __shfl_sync(0xffffffffu, v, j);
     }
-    static __device__ __forceinline__ V down(V v, int d) {
-        return {__shfl_down_sync(0xffffffffu, v.hi, d), __shfl_down_sync(0xffffffffu, v.lo, d)};
-    }
-    static __device__ __forceinline__ V from(V v, int lane) {
-        return {__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane)};
-    }
-};
+    return out;
+}
 
 // Via costs and the exclusive wire-cost prefix of one track, by one warp: lanes
 // over the positions, the prefix of each 32 by a shuffle scan.
@@ -154,8 +146,7 @@ template <class T>
 __device__ __forceinline__ void soft_tables_track(const Tables& Tb, const Soft<T>& S, int t, int lane) {
     const Track K = track_of(Tb, t);
     const int* elen = along_y(Tb, K.l) ? Tb.ylen : Tb.xlen;
-    using A = SoftSum<T>;
-    auto carry = A::of(0);
+    double carry = 0;
     T last_one = 0, last_half = 0;
     for (int p0 = 0; p0 < K.len; p0 += 32) {
         const int p = p0 + lane, c = K.base + p;
@@ -169,19 +160,11 @@ __device__ __forceinline__ void soft_tables_track(const Tables& Tb, const Soft<T
         if (lane == 0) { one = last_one; half = last_half; }
         last_one = __shfl_sync(0xffffffffu, v.one, 31);
         last_half = __shfl_sync(0xffffffffu, v.half, 31);
-        auto incl = A::of(w);
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const auto o = A::up(incl, d);
-            if (lane >= d) incl = incl + o;
-        }
-        auto excl = A::up(incl, 1);
-        if (lane == 0) excl = A::of(0);
+        const T before = soft_scan<true>(w, carry, lane);
         if (p < K.len) {
             S.vc[c] = (p == 0 ? v.one : p == K.len - 1 ? one : v.half + half) + S.uv;
-            S.P[c] = A::round(carry + excl);
+            S.P[c] = before;
         }
-        carry = carry + A::from(incl, 31);
     }
 }
 
@@ -194,23 +177,14 @@ template <class T>
 __device__ __forceinline__ double soft_chain_track(const Tables& Tb, const Soft<T>& S, int t, int lane, T* dcap, T* duw) {
     const Track K = track_of(Tb, t);
     const int* elen = along_y(Tb, K.l) ? Tb.ylen : Tb.xlen;
-    using A = SoftSum<T>;
-    auto carry = A::of(0);
-    double sum = 0;
+    double carry = 0, sum = 0;
     for (int p0 = (K.len - 1) / 32 * 32; p0 >= 0; p0 -= 32) {
         const int p = p0 + lane, c = K.base + p;
         const bool in = p < K.len;
         const T g = in ? S.dP[c] : static_cast<T>(0);
-        auto incl = A::of(g);  // sum over this position and the later ones of the 32
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const auto o = A::down(incl, d);
-            if (lane + d < 32) incl = incl + o;
-        }
-        auto excl = A::down(incl, 1);
-        if (lane == 31) excl = A::of(0);
+        const T dw = soft_scan<false>(g, carry, lane);
         if (in) {
-            const T dw = A::round(carry + excl), dv = S.dvc[c], next = p + 1 < K.len ? S.dvc[c + 1] : static_cast<T>(0);
+            const T dv = S.dvc[c], next = p + 1 < K.len ? S.dvc[c + 1] : static_cast<T>(0);
             const SoftTerms<T> e = soft_terms_dcap<T>(Tb, S, c, K.l);
             T gc = dw * e.one;
             if (p == 0) gc += dv * e.one;
@@ -221,7 +195,6 @@ __device__ __forceinline__ double soft_chain_track(const Tables& Tb, const Soft<
             duw[c] = dw * static_cast<T>(p < K.len - 1 ? elen[p] : 0);
             sum += static_cast<double>(dv);
         }
-        carry = carry + A::from(incl, 0);
     }
     return sum;
 }
@@ -452,10 +425,11 @@ struct SoftArena {
     T* w1;  // [nmax][L] first leg (or straight) wire cost
     T* w2;  // [nmax][L] second leg
     T* col; // [nmax][2][L] via costs at the corners (x, py) and (px, y)
-    T* X;   // [32][L][2] exchange between the lanes of a slot
+    T* X;   // [2][32][L] exchange between the lanes of a slot
+    T* Y;   // [3][32][L] running minima of the rows and columns (backward)
 };
 __host__ __device__ __forceinline__ size_t soft_arena_values(int L, int nmax, bool backward) {
-    return size_t(nmax) * ((backward ? 2 : 1) * tri_count(L) + 4 * L) + size_t(32) * L * 2;
+    return size_t(nmax) * ((backward ? 2 : 1) * tri_count(L) + 4 * L) + size_t(32) * L * (backward ? 5 : 2);
 }
 template <class T>
 __device__ __forceinline__ SoftArena<T> soft_arena(T* p, int L, int nmax, bool backward) {
@@ -465,7 +439,8 @@ __device__ __forceinline__ SoftArena<T> soft_arena(T* p, int L, int nmax, bool b
     A.w1 = p; p += size_t(nmax) * L;
     A.w2 = p; p += size_t(nmax) * L;
     A.col = p; p += size_t(nmax) * 2 * L;
-    A.X = p;
+    A.X = p; p += size_t(2) * 32 * L;
+    A.Y = p;
     return A;
 }
 
@@ -487,12 +462,14 @@ struct SoftRun {
 };
 
 // Forward DP of a pack (net_cost of its nets), and with kBackward the adjoint
-// of g * (their sum) into dP and dvc.
-template <class T, int LC, bool kBackward>
+// of g * (their sum) into dP and dvc.  The loops over layers stay rolled, their
+// state in shared memory: unrolled, the adjoint was several times the
+// instruction cache and waited for instructions 11 cycles of every 17 (5.1 ms
+// at 320x320x10, 120K nets, fp32; rolled 2.3 ms).
+template <class T, bool kBackward>
 __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, const Pack& K, const SoftArena<T>& A, T g,
                                           int lane) {
-    const int L = LC > 0 ? LC : Tb.L, TT = tri_count(L);
-    constexpr int LL = LC > 0 ? LC : kMaxLayers;
+    const int L = Tb.L, TT = tri_count(L);
     constexpr unsigned kAll = 0xffffffffu;
     const T absent = static_cast<T>(kSoftAbsent) * 10, tau = S.tau, inv = S.inv_tau;
     constexpr T kNone = static_cast<T>(1e30);  // no value yet: above any sum of absent candidates
@@ -507,7 +484,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
     const int dmax = __reduce_max_sync(kAll, dep);
     const int xy = (K.x << 16) | K.y;
     const int pxy = __shfl_sync(kAll, xy, K.par & 31);
-    // Costs of every (node, layer); the node's own column waits in its table.
+    // Costs of every (node, layer); the nodes' own columns in X.
     for (int q0 = 0; q0 < M * L; q0 += 32) {
         const int q = q0 + lane, i = min(q / L, M - 1), l = q - q / L * L;
         const int c = __shfl_sync(kAll, xy, i), pc = __shfl_sync(kAll, pxy, i), pa = __shfl_sync(kAll, K.par, i);
@@ -515,7 +492,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
         const int x = c >> 16, y = c & 0xffff, px = pc >> 16, py = pc & 0xffff;
         const bool ay = along_y(Tb, l);
         const int base = layer_base(Tb, l);
-        A.D[i * TT + l] = S.vc[base + (ay ? x * Tb.yp + y : y * Tb.xp + x)];
+        A.X[q] = S.vc[base + (ay ? x * Tb.yp + y : y * Tb.xp + x)];
         if (pa < 0) continue;
         const bool straight = x == px || y == py;
         const int lo = ay ? min(y, py) : min(x, px), hi = ay ? max(y, py) : max(x, px);
@@ -527,33 +504,28 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
         A.col[(2 * i + 1) * L + l] = S.vc[base + (ay ? px * Tb.yp + y : y * Tb.xp + px)];
     }
     __syncwarp();
-    // Via stacks: row lo of every node's table.  The columns move to registers
-    // (a lane per node) before the tables overwrite them.
-    {
-        T vn[LL];
-#pragma unroll
-        for (int l = 0; l < LL; ++l) vn[l] = lane < M && l < L ? A.D[lane * TT + l] : static_cast<T>(0);
-        __syncwarp();
-        if (lane < M) {
-#pragma unroll
-            for (int lo = 0; lo < LL; ++lo) {
-                T acc = 0;
-#pragma unroll
-                for (int hi = lo; hi < LL; ++hi) {
-                    if (hi >= L) continue;
-                    if (hi > lo) acc += vn[hi - 1];
-                    A.D[lane * TT + tri(L, lo, hi)] = (K.lay < L && (lo > K.lay || hi < K.lay)) ? absent : acc;
-                }
-            }
+    // Via stacks: row lo of every node's table.
+    for (int q0 = 0; q0 < M * L; q0 += 32) {
+        const int q = q0 + lane, i = min(q / L, M - 1), lo = q - q / L * L;
+        const int lay = __shfl_sync(kAll, K.lay, i);
+        if (q >= M * L) continue;
+        T acc = 0;
+        T* row = A.D + i * TT + tri(L, lo, lo) - lo;
+#pragma unroll 1
+        for (int hi = lo; hi < L; ++hi) {
+            if (hi > lo) acc += A.X[i * L + hi - 1];
+            row[hi] = (lay < L && (lo > lay || hi < lay)) ? absent : acc;
         }
     }
     __syncwarp();
     const int NS = max(1, 32 / L);
-    const int slot = lane / L, sl = lane - slot * L, s0 = min(slot, NS - 1) * L;
-    T* X = A.X + size_t(s0) * L * 2;  // the slot's exchange: [L][L][2]
+    const int slot = lane / L, sl = lane - slot * L, s0 = min(slot, NS - 1) * L, own = lane * L;
+    // The slot's exchange, [L][L] twice; the lane's running minima.
+    T *X = A.X + size_t(s0) * L, *X2 = X + size_t(32) * L;
+    T *Re = A.Y + own, *Rs = Re + size_t(32) * L, *Ce = Rs + size_t(32) * L;
     const int row = tri(L, sl, sl) - sl;
-    // Nodes of a depth in descending order, NS at a time; mode 0: forward,
-    // children into parents; mode 1: the adjoint, parents to children.
+    // Nodes of a depth in descending order, NS at a time: forward, children
+    // into parents; or the adjoint, parents to children.
     auto edges = [&](unsigned level, auto backward) {
         constexpr bool kAdj = decltype(backward)::value;
         for (unsigned at = level; at;) {
@@ -570,41 +542,32 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             const int x = c >> 16, y = c & 0xffff, px = pc >> 16, py = pc & 0xffff;
             const bool straight = x == px || y == py;
             const T* Di = A.D + ii * TT;
-            // Row sl: running soft minimum of columns 8 down to hi.
+            // Row sl: running soft minimum of columns L-1 down to hi.
             SoftRun<T> R{kNone, 0};
-            T re[LL], rs[LL];
             unsigned rless = 0;
-            if (act) {
-#pragma unroll
-                for (int hi = LL - 1; hi >= 0; --hi) {
-                    if (hi < sl || hi >= L) continue;
-                    bool less;
-                    const T e = R.add(Di[row + hi], 1, inv, less);
-                    if (kAdj) { re[hi] = e; rs[hi] = R.s; rless |= unsigned(less) << hi; }
-                    X[(sl * L + hi) * 2] = R.m;
-                    X[(sl * L + hi) * 2 + 1] = R.s;
-                }
+#pragma unroll 1
+            for (int hi = act ? L - 1 : -1; hi >= sl; --hi) {
+                bool less;
+                const T e = R.add(Di[row + hi], 1, inv, less);
+                if (kAdj) { Re[hi] = e; Rs[hi] = R.s; rless |= unsigned(less) << hi; }
+                X[sl * L + hi] = R.m;
+                X2[sl * L + hi] = R.s;
             }
             __syncwarp();
             // Column sl: over the rows lo <= sl.
             SoftRun<T> C{kNone, 0};
-            T ce[LL], cs[LL], cw[LL];
             unsigned cless = 0;
-            if (act) {
-#pragma unroll
-                for (int lo = 0; lo < LL; ++lo) {
-                    if (lo > sl || lo >= L) continue;
-                    bool less;
-                    const T w = X[(lo * L + sl) * 2 + 1];
-                    const T e = C.add(X[(lo * L + sl) * 2], w, inv, less);
-                    if (kAdj) { ce[lo] = e; cs[lo] = C.s; cw[lo] = w; cless |= unsigned(less) << lo; }
-                }
+#pragma unroll 1
+            for (int lo = 0; lo <= (act ? sl : -1); ++lo) {
+                bool less;
+                const T e = C.add(X[lo * L + sl], X2[lo * L + sl], inv, less);
+                if (kAdj) { Ce[lo] = e; cless |= unsigned(less) << lo; }
             }
             __syncwarp();  // X is reused
             const T reach = act ? C.value(tau) + A.w1[ii * L + sl] : absent;
             // Arrival on parent layer sl: the candidates cl of the other parity
             // (or cl = sl along a straight edge).
-            constexpr int NC = (LL + 1) / 2;
+            constexpr int NC = (kMaxLayers + 1) / 2;
             const int odd = (sl & 1) ^ 1;
             const int side = along_y(Tb, sl) ? 1 : 0;  // the corner is the end of the first leg
             const T* col = A.col + (2 * ii + side) * L;
@@ -618,98 +581,93 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
                 v[j] = absent;
                 if (!act || straight || cl >= L) continue;
                 T via = 0;
+#pragma unroll 1
                 for (int l = min(cl, sl) + 1; l < max(cl, sl); ++l) via += col[l];
                 v[j] = r + (via + leg2);
                 dm = v[j] < dm ? v[j] : dm;
             }
             T diag = absent;
-            T vw[NC];
             if (act && straight) {
                 diag = reach;
             } else if (act) {
 #pragma unroll
                 for (int j = 0; j < NC; ++j) {
-                    vw[j] = 2 * j + odd < L ? s_exp<T>(-(v[j] - dm) * inv) : static_cast<T>(0);
-                    ds += vw[j];
+                    v[j] = 2 * j + odd < L ? s_exp<T>(-(v[j] - dm) * inv) : static_cast<T>(0);  // from here on: weights
+                    ds += v[j];
                 }
                 diag = dm < static_cast<T>(kSoftAbsent) ? dm - tau * s_log<T>(ds) : absent;
             }
             // Row sl of the contribution: running soft minimum of diag[sl..hi].
             SoftRun<T> B{kNone, 0};
-            T be[LL], bs[LL];
             unsigned bless = 0;
-            T* Dp = A.D + p * TT;
-            T out[LL];
-#pragma unroll
-            for (int hi = 0; hi < LL; ++hi) {
-                if (hi >= L) continue;
+#pragma unroll 1
+            for (int hi = 0; hi < L; ++hi) {
                 const T dv = __shfl_sync(kAll, diag, s0 + hi);
                 if (!act || hi < sl) continue;
                 bool less;
                 const T e = B.add(dv, 1, inv, less);
-                if (kAdj) { be[hi] = e; bs[hi] = B.s; bless |= unsigned(less) << hi; }
-                else out[hi] = B.value(tau);
+                if (kAdj) { X[sl * L + hi] = e; X2[sl * L + hi] = B.s; bless |= unsigned(less) << hi; }
+                else X[sl * L + hi] = B.value(tau);
             }
             if (!kAdj) {
+                T* Dp = A.D + p * TT;
                 for (int k = 0; k < NS; ++k) {  // slots in turn: a parent's children in descending order
-                    if (act && slot == k) {
-#pragma unroll
-                        for (int hi = 0; hi < LL; ++hi)
-                            if (hi >= sl && hi < L) Dp[row + hi] += out[hi];
-                    }
+                    if (act && slot == k)
+#pragma unroll 1
+                        for (int hi = sl; hi < L; ++hi) Dp[row + hi] += X[sl * L + hi];
                     __syncwarp();
                 }
                 continue;
             }
-            // Adjoint.  Contribution: back along the running minimum.
+            // Adjoint.  Back along a running minimum: U is what a value v gets for
+            // each unit of exp(-(v - m) / tau), m the minimum of that step, so a
+            // step adds its adjoint over its sum, and going below the value that
+            // made the minimum scales U by that value's e.  Contribution (the
+            // lane's own row of X, its result in place):
             const T* Gp = A.G + p * TT;
-            T carry = 0;
-            if (act) {
-#pragma unroll
-                for (int hi = LL - 1; hi >= 0; --hi) {
-                    if (hi < sl || hi >= L) continue;
-                    const T acc = Gp[row + hi] + carry, is = static_cast<T>(1) / bs[hi], e = be[hi];
-                    const bool less = (bless >> hi) & 1u;
-                    X[sl * L + hi] = acc * (less ? is : e * is);
-                    carry = hi > sl ? acc * (less ? bs[hi - 1] * e * is : bs[hi - 1] * is) : static_cast<T>(0);
-                }
+            T U = 0;
+#pragma unroll 1
+            for (int hi = act ? L - 1 : -1; hi >= sl; --hi) {
+                const T e = X[sl * L + hi];
+                const bool less = (bless >> hi) & 1u;
+                U += Gp[row + hi] / X2[sl * L + hi];
+                X[sl * L + hi] = less ? U : U * e;
+                U = less ? U * e : U;
             }
             __syncwarp();
             T gd = 0;  // adjoint of diag[sl]
-            if (act) {
-#pragma unroll
-                for (int lo = 0; lo < LL; ++lo)
-                    if (lo <= sl && lo < L) gd += X[lo * L + sl];
-            }
+#pragma unroll 1
+            for (int lo = 0; lo <= (act ? sl : -1); ++lo) gd += X[lo * L + sl];
             __syncwarp();
             // Arrival: X[pl][cl] = adjoint of candidate (cl, pl).
             T gcur = 0, gleg2 = 0;
             if (act && straight) gcur = gd;
             if (act && !straight) {
-                const T is = ds > 0 ? static_cast<T>(1) / ds : static_cast<T>(0);
+                const T scale = ds > 0 ? gd / ds : static_cast<T>(0);
 #pragma unroll
                 for (int j = 0; j < NC; ++j) {
                     const int cl = 2 * j + odd;
                     if (cl >= L) continue;
-                    const T w = gd * (vw[j] * is);
+                    const T w = scale * v[j];
                     X[sl * L + cl] = w;
                     gleg2 += w;
                 }
             }
             __syncwarp();
             if (act && !straight) {
-#pragma unroll
-                for (int j = 0; j < NC; ++j)
-                    if (2 * j + odd < L) gcur += X[(2 * j + odd) * L + sl];
+#pragma unroll 1
+                for (int cl = odd; cl < L; cl += 2) gcur += X[cl * L + sl];
                 // Via cells of layer sl at the two corners: every candidate
                 // whose layers enclose it; the corner by the first leg cl.
                 T va = 0, vb = 0;
+#pragma unroll 1
                 for (int a = 0; a < sl; ++a)
-                    for (int b = a + 1; b < L; b += 2) {
-                        if (b <= sl) continue;
+#pragma unroll 1
+                    for (int b = a + 1 + (((sl - a + 1) >> 1) << 1); b < L; b += 2) {  // the other parity, above sl
                         const T up = X[b * L + a], down = X[a * L + b];  // cl = a, pl = b; cl = b, pl = a
-                        if (along_y(Tb, a)) { va += up; vb += down; }
-                        else { vb += up; va += down; }
+                        const bool ay = along_y(Tb, a);
+                        va += ay ? up : down;
+                        vb += ay ? down : up;
                     }
                 if (va != 0) atomicAdd(S.dvc + slot_index(Tb, sl, x, py), va);
                 if (vb != 0) atomicAdd(S.dvc + slot_index(Tb, sl, px, y), vb);
@@ -724,33 +682,26 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
                 if (gleg2 != 0 && lo != hi) { atomicAdd(S.dP + t2 + hi, gleg2); atomicAdd(S.dP + t2 + lo, -gleg2); }
             }
             __syncwarp();
-            // Column sl back to the rows' running minima, then row sl back to
-            // the ranges.
-            if (act) {
-                carry = gcur;
-#pragma unroll
-                for (int lo = LL - 1; lo >= 0; --lo) {
-                    if (lo > sl || lo >= L) continue;
-                    const T is = static_cast<T>(1) / cs[lo], e = ce[lo];
-                    const bool less = (cless >> lo) & 1u;
-                    X[lo * L + sl] = carry * (less ? cw[lo] * is : cw[lo] * e * is);
-                    carry = lo > 0 ? carry * (less ? cs[lo > 0 ? lo - 1 : 0] * e * is : cs[lo > 0 ? lo - 1 : 0] * is)
-                                   : static_cast<T>(0);
-                }
+            // Column sl back to the rows' running minima (a row's sum at column
+            // sl is in its lane's Rs), then row sl back to the ranges.
+            U = act ? gcur / C.s : static_cast<T>(0);
+#pragma unroll 1
+            for (int lo = act ? sl : -1; lo >= 0; --lo) {
+                const T e = Ce[lo], w = A.Y[size_t(32 + s0 + lo) * L + sl];
+                const bool less = (cless >> lo) & 1u;
+                X[lo * L + sl] = less ? U * w : U * e * w;
+                U = less ? U * e : U;
             }
             __syncwarp();
-            if (act) {
-                T* Gi = A.G + ii * TT;
-                carry = 0;
-#pragma unroll
-                for (int hi = 0; hi < LL; ++hi) {
-                    if (hi < sl || hi >= L) continue;
-                    const T acc = X[sl * L + hi] + carry, is = static_cast<T>(1) / rs[hi], e = re[hi];
-                    const bool less = (rless >> hi) & 1u;
-                    Gi[row + hi] = acc * (less ? is : e * is);
-                    const T below = hi + 1 < L ? rs[hi + 1 < LL ? hi + 1 : hi] : static_cast<T>(0);
-                    carry = acc * (less ? below * e * is : below * is);
-                }
+            T* Gi = A.G + ii * TT;
+            U = 0;
+#pragma unroll 1
+            for (int hi = sl; hi < (act ? L : 0); ++hi) {
+                const T e = Re[hi];
+                const bool less = (rless >> hi) & 1u;
+                U += X[sl * L + hi] / Rs[hi];
+                Gi[row + hi] = less ? U : U * e;
+                U = less ? U * e : U;
             }
             __syncwarp();
         }
@@ -769,31 +720,30 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
         const int ii = max(i, 0), id = __shfl_sync(kAll, K.id, ii);
         const T* Di = A.D + ii * TT;
         T m = absent;
-        if (act) {
-#pragma unroll
-            for (int hi = 0; hi < LL; ++hi)
-                if (hi >= sl && hi < L) m = Di[row + hi] < m ? Di[row + hi] : m;
-        }
+#pragma unroll 1
+        for (int hi = sl; hi < (act ? L : 0); ++hi) m = Di[row + hi] < m ? Di[row + hi] : m;
         T best = absent;
+#pragma unroll 1
         for (int l = 0; l < L; ++l) {
             const T o = __shfl_sync(kAll, m, s0 + l);
             best = o < best ? o : best;
         }
-        T part = 0, w[LL];
-        if (act) {
-#pragma unroll
-            for (int hi = 0; hi < LL; ++hi)
-                if (hi >= sl && hi < L) { w[hi] = s_exp<T>(-(Di[row + hi] - best) * inv); part += w[hi]; }
+        T part = 0;
+#pragma unroll 1
+        for (int hi = sl; hi < (act ? L : 0); ++hi) {
+            const T w = s_exp<T>(-(Di[row + hi] - best) * inv);
+            X[sl * L + hi] = w;
+            part += w;
         }
         T sum = 0;
+#pragma unroll 1
         for (int l = 0; l < L; ++l) sum += __shfl_sync(kAll, part, s0 + l);
         const bool feasible = best < static_cast<T>(kSoftAbsent);
         if (act && sl == 0 && S.net_cost) S.net_cost[id] = feasible ? best - tau * s_log<T>(sum) : absent;
-        if (kBackward && act) {
-#pragma unroll
-            for (int hi = 0; hi < LL; ++hi)
-                if (hi >= sl && hi < L) A.G[ii * TT + row + hi] = feasible ? g * (w[hi] / sum) : static_cast<T>(0);
-        }
+        if (kBackward)
+#pragma unroll 1
+            for (int hi = sl; hi < (act ? L : 0); ++hi)
+                A.G[ii * TT + row + hi] = feasible ? g * (X[sl * L + hi] / sum) : static_cast<T>(0);
     }
     __syncwarp();
     if constexpr (kBackward) {
@@ -805,7 +755,9 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             if (q >= M * L || l + 1 >= L) continue;
             const T* Gi = A.G + i * TT;
             T acc = 0;
+#pragma unroll 1
             for (int lo = 0; lo <= l; ++lo)
+#pragma unroll 1
                 for (int hi = l + 1; hi < L; ++hi) acc += Gi[tri(L, lo, hi)];
             if (acc != 0) atomicAdd(S.dvc + slot_index(Tb, l, c >> 16, c & 0xffff), acc);
         }

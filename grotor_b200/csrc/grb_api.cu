@@ -505,8 +505,8 @@ __global__ void k_soft_tables(Tables Tb, Soft<T> S) {  // one warp per track
 // Forward DP (net_cost) or adjoint of every net: a warp takes `span`
 // consecutive nets, as many at a time as its arena of nmax nodes holds; nets
 // beyond kPackNodes are walked by one thread in global scratch.
-template <class T, int LC, bool kBackward>
-__global__ void __launch_bounds__(kSoftThreads, sizeof(T) == 4 ? 3 : 2) k_soft_packs(Tables Tb, Soft<T> S, Plan P, int n, int span, int nmax, T g) {
+template <class T, bool kBackward>
+__global__ void __launch_bounds__(kSoftThreads, 4) k_soft_packs(Tables Tb, Soft<T> S, Plan P, int n, int span, int nmax, T g) {
     extern __shared__ __align__(16) char smem[];
     const int lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const SoftArena<T> A = soft_arena(reinterpret_cast<T*>(smem) + (threadIdx.x >> 5) * soft_arena_values(Tb.L, nmax, kBackward),
@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(kSoftThreads, sizeof(T) == 4 ? 3 : 2) k_soft_p
         }
         if (!kBackward && lane < k && P.node_off[at + lane + 1] == P.node_off[at + lane]) S.net_cost[at + lane] = 0;
         const Pack K = load_pack(Tb, P, nullptr, at, k, lane);
-        soft_pack<T, LC, kBackward>(Tb, S, K, A, g, lane);
+        soft_pack<T, kBackward>(Tb, S, K, A, g, lane);
         __syncwarp();
         at += k;
     }
@@ -1570,14 +1570,12 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
     const int n = c->n_nets;
     if (!n) return GRB_OK;
     const int nmax = std::min(kPackNodes, std::max(16, c->max_nodes));
-    const int warps = kSoftThreads / 32, span = std::min(16, std::max(1, n / (c->sms * 16)));
+    // Three warps a CTA in fp64: two CTAs of the adjoint share an SM.
+    const int warps = sizeof(T) == 8 ? 3 : kSoftThreads / 32, span = std::min(16, std::max(1, n / (c->sms * 16)));
     const size_t smem = warps * soft_arena_values(c->T.L, nmax, kBackward) * sizeof(T);
     const long long blocks = (n + (long long)span * warps - 1) / ((long long)span * warps);
-    // The layer loops unrolled for the 9 routing layers of 10-layer designs.
-    void (*kernel)(Tables, Soft<T>, Plan, int, int, int, T) =
-        c->T.L == 9 ? k_soft_packs<T, 9, kBackward> : k_soft_packs<T, 0, kBackward>;
-    GRB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    kernel<<<unsigned(blocks), kSoftThreads, smem, c->stream>>>(c->T, S, make_plan(c), n, span, nmax, g);
+    GRB_CUDA(c, cudaFuncSetAttribute(k_soft_packs<T, kBackward>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    k_soft_packs<T, kBackward><<<unsigned(blocks), 32 * warps, smem, c->stream>>>(c->T, S, make_plan(c), n, span, nmax, g);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
     return GRB_OK;
