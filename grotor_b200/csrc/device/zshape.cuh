@@ -15,18 +15,21 @@
 // they are small per-net arrays in shared memory (nodes at one position share
 // their cells, as on the planes), and no plane exists.
 //
-// B200 form: one CTA per net, a warp per tree edge.  A two-bend candidate of an
-// edge runs from the child along one side of the box, changes layer, crosses
-// the box, changes layer again and runs to the node: everything between the
-// child and the node depends on one position of that side only.  So a lane
-// takes a position and walks the five steps in registers (zedge_chunk) --
-// all its table reads issued at once, no barrier and no memory in between --
-// and a warp minimum per layer joins the edge's other positions by a minimum in
-// shared memory.  The positions of all edges into the nodes of one depth are
-// dealt out to the CTA's warps, 32 at a time; two barriers per depth.  A net takes as long
-// as its depths; the phases over planes in HBM, six barriers an edge and a
-// serial traceback from global memory, took 136 us of DP a batch of 127 nets
-// (320x320x10, 60K nets), this form 87 us.
+// B200 form: one CTA per net.  A two-bend candidate of an edge runs from the
+// child along one side of the box, changes layer, crosses the box, changes
+// layer again and runs to the node: everything between the child and the node
+// depends on one position of that side only.  So a warp takes as many
+// positions as it holds columns (a lane per position and layer) and walks the
+// five steps in registers (zedge_chunk): one round of table reads, layer
+// changes as prefix minima by shuffle, no barrier and no memory in between; a
+// minimum in shared memory joins the positions.  The positions of all edges
+// into the nodes of one depth are dealt out to the CTA's warps; two barriers
+// per depth.  A batch lasts as long as its largest net, a few dozen short
+// dependent steps: phases over planes in HBM, six barriers an edge and a serial
+// traceback from global memory, took 136 us of DP a batch of 127 nets
+// (320x320x10, 60K nets); a lane per position with its column in registers, 87
+// us (2,500 instructions of straight-line code, fetched anew by every warp);
+// this form 68 us.
 #pragma once
 #include "commit.cuh"
 #include "common.cuh"
@@ -94,24 +97,44 @@ __device__ __forceinline__ ZNet znet(int* a, int cnt, int LY) {
     return W;
 }
 
-// viaSweep (zshape.cuh:42-61) on one position's column, layers 1..LAYER-1: up,
-// then down; q: the layer the value came from in this sweep.
-template <int K>
-__device__ __forceinline__ void zsweep(int (&m)[K], int (&p)[K], int (&q)[K], const int (&via)[K], int LAYER) {
+// viaSweep (zshape.cuh:42-61) over one position's column, a lane per layer (the
+// `width` lanes from lane - r on hold layers 1..width, r = layer - 1): up, then
+// down, each keeping strict improvements.  In either direction a layer takes
+// the least m[j] + (vias between), the nearest j on ties, which is a prefix
+// minimum of m[j] - V[j], V the running via sum.  Sums stay below 2^31 (values
+// at most 1.5e9, vias 1e6 each).  src: the layer offset whose back-pointer the
+// value carries; q: the layer offset the value came from in its last step.
+__device__ __forceinline__ void zsweep(int& m, int& src, int& q, int V, int r, int width, int lane) {
+    const int lo = lane - r;
+    int val = m - V, at = r;
 #pragma unroll
-    for (int i = 1; i < K; ++i) q[i] = i;
-#pragma unroll
-    for (int i = 2; i < K; ++i) {
-        if (i >= LAYER) continue;
-        const int v = zadd(m[i - 1], via[i - 1]);
-        if (m[i] > v) { m[i] = v; p[i] = p[i - 1]; q[i] = i - 1; }
+    for (int d = 1; d < 16; d <<= 1) {
+        const int ov = __shfl_sync(0xffffffffu, val, max(lane - d, 0)), oa = __shfl_sync(0xffffffffu, at, max(lane - d, 0));
+        if (r >= d && ov < val) { val = ov; at = oa; }
     }
+    q = at == r ? r : r - 1;
+    src = __shfl_sync(0xffffffffu, src, (lo + at) & 31);
+    m = val + V;
+    val = m + V;
+    at = r;
 #pragma unroll
-    for (int i = K - 2; i >= 1; --i) {
-        if (i > LAYER - 2) continue;
-        const int v = zadd(m[i + 1], via[i]);
-        if (m[i] > v) { m[i] = v; p[i] = p[i + 1]; q[i] = i + 1; }
+    for (int d = 1; d < 16; d <<= 1) {
+        const int ov = __shfl_sync(0xffffffffu, val, min(lane + d, 31)), oa = __shfl_sync(0xffffffffu, at, min(lane + d, 31));
+        if (r + d < width && ov < val) { val = ov; at = oa; }
     }
+    if (at != r) q = r + 1;
+    src = __shfl_sync(0xffffffffu, src, (lo + at) & 31);
+    m = val - V;
+}
+// Exclusive sum of v over the layers below (same lanes).
+__device__ __forceinline__ int zbelow(int v, int r, int lane) {
+    int incl = v;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const int o = __shfl_sync(0xffffffffu, incl, max(lane - d, 0));
+        if (r >= d) incl += o;
+    }
+    return incl - v;
 }
 
 // Geometry of the edge from child c to node v.
@@ -150,76 +173,55 @@ __device__ __forceinline__ void zedge_straight(const Tables& T, const ZTrees& Z,
     }
 }
 
-// 32 positions from k0 on of a bent edge into child slot j of node v
-// (zshape.cuh:87-212), one per lane.
+// Positions k0, k0 + 1, ... (`rounds` times the S a warp holds) of a bent edge
+// into child slot j of node v (zshape.cuh:87-212); lane = position * width +
+// (layer - 1).
 __device__ __forceinline__ void zedge_chunk(const Tables& T, const ZTrees& Z, const ZNet& W, const ZEdge& E, int j, int c,
-                                            int v, int k0, int lane) {
-    const int LAYER = W.LY, D = Z.D, k = k0 + lane;
-    constexpr int K = kMaxLayers + 1;
-    const int* base = W.m0 + W.rep[c] * LAYER;
-    const bool in = k < E.items, isx = k < E.nx;
-    const int f = isx ? E.fromx : E.fromy;
-    int b = (isx ? min(E.fromx, E.tox) : min(E.fromy, E.toy)) + (isx ? k : k - E.nx);
-    if (b >= f) ++b;
-    if (!in) b = f;  // any position of the box
-    // At the box corner the run already ends on the node's other line: no
-    // crossing, and the way goes on across the line's direction.
-    const bool corner = b == (isx ? E.tox : E.toy);
-    const int x1 = isx ? b : E.fromx, y1 = isx ? E.fromy : b, x2 = isx ? b : E.tox, y2 = isx ? E.toy : b;
-    int m[K], p[K], q[K], via[K], wc[K], we[K];  // wc: crossing, we: last run
-    {
-        double s1[K], s2[K];
-        int v2[K];
-#pragma unroll
-        for (int i = 1; i < K; ++i) {
-            if (i >= LAYER) continue;
-            const int a1 = slot_index(T, i - 1, x1, y1), a2 = slot_index(T, i - 1, x2, y2);
-            s1[i] = T.presum[a1];
-            s2[i] = T.presum[a2];
-            via[i] = static_cast<int>(fminf(fmaxf(T.vcost[a1], 1.f), 1.e6f));
-            v2[i] = static_cast<int>(fminf(fmaxf(T.vcost[corner ? a1 : a2], 1.f), 1.e6f));
+                                            int v, int k0, int rounds, int lane) {
+    const int width = W.LY - 1, S = 32 / width, D = Z.D;
+    const int s = lane / width, r = lane - s * width, i = r + 1;  // plane layer i, routing layer r
+    const bool on = s < S, ay = ((i & 1) ^ D) != 0;
+    const int base = on ? W.m0[W.rep[c] * W.LY + i] : 0;
+    const int lb = layer_base(T, on ? r : 0);
+    auto slot = [&](int x, int y) { return lb + (ay ? x * T.yp + y : y * T.xp + x); };
+    const double pf = on ? T.presum[slot(E.fromx, E.fromy)] : 0.0, pt = on ? T.presum[slot(E.tox, E.toy)] : 0.0;
+    int best = 0x7fffffff;
+    unsigned code = ~0u;
+    for (int n = 0; n < rounds; ++n) {
+        const int k = k0 + n * S + s;
+        if (k0 + n * S >= E.items) break;
+        const bool in = on && k < E.items, isx = k < E.nx;
+        const int f = isx ? E.fromx : E.fromy;
+        int b = (isx ? min(E.fromx, E.tox) : min(E.fromy, E.toy)) + (isx ? k : k - E.nx);
+        if (b >= f) ++b;
+        if (!in) b = f;  // any position of the box
+        // At the box corner the run already ends on the node's other line: no
+        // crossing, and the way goes on across the line's direction.
+        const bool corner = b == (isx ? E.tox : E.toy);
+        const int a1 = slot(isx ? b : E.fromx, isx ? E.fromy : b), a2 = slot(isx ? b : E.tox, isx ? E.toy : b);
+        const double p1 = on ? T.presum[a1] : 0.0, p2 = on ? T.presum[a2] : 0.0;
+        const int v1 = on ? static_cast<int>(fminf(fmaxf(T.vcost[a1], 1.f), 1.e6f)) : 0;
+        const int v2 = on ? static_cast<int>(fminf(fmaxf(T.vcost[corner ? a1 : a2], 1.f), 1.e6f)) : 0;
+        const bool own = ay != isx;  // the layer runs along this line
+        int m = own ? zadd(base, zwire_of(pf, p1)) : kZInf, src = r, q;
+        zsweep(m, src, q, zbelow(v1, r, lane), r, width, lane);
+        const int step = own ? zwire_of(p2, pt) : zwire_of(p1, p2);  // the last run; the crossing
+        if (!corner) {
+            const int x = zadd(m, step);
+            m = !own && x < kZInf ? x : kZInf;
         }
-#pragma unroll
-        for (int i = 1; i < K; ++i) {
-            if (i >= LAYER) continue;
-            const bool own = (((i & 1) ^ D) != 0) != isx;  // the layer runs along this line
-            const double sf = own ? T.presum[slot_index(T, i - 1, E.fromx, E.fromy)] : 0.0;
-            const double st = own ? T.presum[slot_index(T, i - 1, E.tox, E.toy)] : 0.0;
-            wc[i] = own ? 0 : zwire_of(s1[i], s2[i]);
-            we[i] = own ? zwire_of(s2[i], st) : 0;
-            m[i] = own ? zadd(base[i], zwire_of(sf, s1[i])) : kZInf;
-            p[i] = i;
-        }
-        zsweep<K>(m, p, q, via, LAYER);
-#pragma unroll
-        for (int i = 1; i < K; ++i) via[i] = v2[i];
-    }
-    if (!corner) {
-#pragma unroll
-        for (int i = 1; i < K; ++i) {
-            if (i >= LAYER) continue;
-            const bool own = (((i & 1) ^ D) != 0) != isx;
-            const int x = zadd(m[i], wc[i]);
-            m[i] = !own && x < kZInf ? x : kZInf;
+        zsweep(m, src, q, zbelow(v2, r, lane), r, width, lane);
+        if (in && own != corner) {  // ends across the line at the corner, along it elsewhere
+            const int x = zadd(m, step);
+            const unsigned xc = unsigned((corner ? (isx ? E.fromy : E.fromx) : b) << 8) | unsigned((src + 1) << 4) | unsigned(q + 1);
+            if (x < best || (x == best && xc < code)) { best = x; code = xc; }
         }
     }
-    zsweep<K>(m, p, q, via, LAYER);
     // Per layer the first minimum over the positions (the reference scans them
-    // in order keeping strict improvements); ends across the line at the
-    // corner, along it elsewhere.
-    unsigned long long* key = W.key + (j * W.cnt + W.rep[v]) * LAYER;
-    const int at = corner ? (isx ? E.fromy : E.fromx) : b;
-#pragma unroll
-    for (int i = 1; i < K; ++i) {
-        if (i >= LAYER) continue;
-        const bool own = (((i & 1) ^ D) != 0) != isx, ends = in && own != corner;
-        const int x = zadd(m[i], corner ? wc[i] : we[i]);
-        const int best = __reduce_min_sync(0xffffffffu, ends ? x : 0x7fffffff);
-        const unsigned code = __reduce_min_sync(
-            0xffffffffu, ends && x == best ? unsigned(at << 8) | unsigned(p[i] << 4) | unsigned(q[i]) : ~0u);
-        if (lane == i && code != ~0u)
-            atomicMin(key + i, (static_cast<unsigned long long>(static_cast<unsigned>(best) ^ 0x80000000u) << 32) | code);
-    }
+    // in order keeping strict improvements).
+    if (on && code != ~0u)
+        atomicMin(W.key + (j * W.cnt + W.rep[v]) * W.LY + i,
+                  (static_cast<unsigned long long>(static_cast<unsigned>(best) ^ 0x80000000u) << 32) | code);
 }
 
 // The finished edge into child slot j of node v: its least arrival per layer,
@@ -436,9 +438,17 @@ __device__ __forceinline__ void zshape_net(const Tables& T, const ZTrees& Z, con
         atomicMax(&zdeep, d);
     }
     __syncthreads();
+    const int S = 32 / (LY - 1);  // positions a warp takes at once
     for (int d = zdeep; d >= 0; --d) {
-        for (int pass = 0; pass < 2; ++pass) {  // the depth's edges, then its nodes
-            int turn = 0;
+        // The depth's edges: how many positions, so that every warp gets a share.
+        int positions = 0, turn = 0;
+        for (int u = lane; u < cnt; u += 32)
+            if (W.dep[u] == d)
+                for (int j = 0; j < 3; ++j)
+                    if (W.child[3 * u + j] != -1) positions += zedge(Z, W, W.child[3 * u + j], u).items;
+        positions = __reduce_add_sync(0xffffffffu, positions);
+        const int rounds = max(1, (positions + nw * S - 1) / (nw * S));
+        for (int pass = positions ? 0 : 1; pass < 2; ++pass) {  // edges, then nodes
             for (int u0 = 0; u0 < cnt; u0 += 32) {
                 unsigned at = __ballot_sync(0xffffffffu, u0 + lane < cnt && W.dep[min(u0 + lane, cnt - 1)] == d);
                 for (; at; at &= at - 1) {
@@ -451,9 +461,9 @@ __device__ __forceinline__ void zshape_net(const Tables& T, const ZTrees& Z, con
                         if (pass) {
                             if (E.bent) zedge_apply(Z, W, E, j, v, lane);
                         } else {
-                            for (int k0 = 0; k0 < E.items; k0 += 32) {
+                            for (int k0 = 0; k0 < E.items; k0 += rounds * S) {
                                 if (turn++ % nw != warp) continue;
-                                if (E.bent) zedge_chunk(T, Z, W, E, j, c, v, k0, lane);
+                                if (E.bent) zedge_chunk(T, Z, W, E, j, c, v, k0, rounds, lane);
                                 else zedge_straight(T, Z, W, E, j, c, v, lane);
                             }
                         }
