@@ -273,32 +273,40 @@ __device__ __forceinline__ void refresh_track(const Tables& T, int t, int lane) 
         }
         if (!started) continue;
         const int pad = K.words * 32;
-        float4 next = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b * kScanBlock + 4 * lane < pad)
-            next = *reinterpret_cast<const float4*>(T.wcost + K.base + b * kScanBlock + 4 * lane);
-        for (; b < bend; ++b) {
-            const float4 v = next;
-            const int p = b * kScanBlock + 4 * lane;
-            if (b + 1 < bend && p + kScanBlock < pad)
-                next = *reinterpret_cast<const float4*>(T.wcost + K.base + p + kScanBlock);
-            float before = __shfl_up_sync(0xffffffffu, v.w, 1);
-            if (lane == 0) before = edge;
-            edge = __shfl_sync(0xffffffffu, v.w, 31);
-            double a[4] = {before, v.x, v.y, v.z};
-            block_prefix(a, lane);
-            const double total = __shfl_sync(0xffffffffu, a[3], 31);
-            if (lane == 0) totals[b] = total;
+        // Four blocks at a time, their loads issued together (one in flight a
+        // warp left HBM reads at a quarter of what they can be).
+        for (; b < bend; b += 4) {
+            float4 in[4];
 #pragma unroll
-            for (int e = 0; e < kScanLevels; ++e)
-                if ((b >> e) & 1) {
+            for (int u = 0; u < 4; ++u) {
+                const int p = (b + u) * kScanBlock + 4 * lane;
+                in[u] = b + u < bend && p < pad ? *reinterpret_cast<const float4*>(T.wcost + K.base + p)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) a[j] = a[j] + S.t[e];
+            for (int u = 0; u < 4; ++u) {
+                if (b + u >= bend) continue;
+                const float4 v = in[u];
+                const int p = (b + u) * kScanBlock + 4 * lane;
+                float before = __shfl_up_sync(0xffffffffu, v.w, 1);
+                if (lane == 0) before = edge;
+                edge = __shfl_sync(0xffffffffu, v.w, 31);
+                double a[4] = {before, v.x, v.y, v.z};
+                block_prefix(a, lane);
+                const double total = __shfl_sync(0xffffffffu, a[3], 31);
+                if (lane == 0) totals[b + u] = total;
+#pragma unroll
+                for (int e = 0; e < kScanLevels; ++e)
+                    if (((b + u) >> e) & 1) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) a[j] = a[j] + S.t[e];
+                    }
+                S.push(b + u, total);
+                if (p < pad) {
+                    double2* out = reinterpret_cast<double2*>(T.presum + K.base + p);
+                    out[0] = make_double2(a[0], a[1]);
+                    out[1] = make_double2(a[2], a[3]);
                 }
-            S.push(b, total);
-            if (p < pad) {
-                double2* out = reinterpret_cast<double2*>(T.presum + K.base + p);
-                out[0] = make_double2(a[0], a[1]);
-                out[1] = make_double2(a[2], a[3]);
             }
         }
     }

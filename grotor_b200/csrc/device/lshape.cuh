@@ -473,6 +473,7 @@ __device__ __forceinline__ Pack load_pack(const Tables& T, const Plan& P, const 
     return K;
 }
 
+constexpr int kUnroll = 3;
 template <int LC>
 __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, const Pack& K, int stamp,
                                              const PackArena& A, int lane, bool commit) {
@@ -555,7 +556,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
         double acc = 0;
         unsigned emin = 255, emax = 0;
         bool odd = false;
-#pragma unroll
+#pragma unroll kUnroll
         for (int l = 1; l < LL; ++l) {
             if (l >= L) continue;
             out[l] = acc;
@@ -579,7 +580,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
         const float* vn = reinterpret_cast<const float*>(A.from + i * FS);
         double acc = 0;
         double* row = A.dist + i * TT + tri(L, lo, lo) - lo;
-#pragma unroll
+#pragma unroll kUnroll
         for (int hi = 0; hi < LL; ++hi) {
             if (hi < lo || hi >= L) continue;
             if (hi > lo) acc = acc + static_cast<double>(vn[hi - 1]);
@@ -648,7 +649,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
                 const double* col = A.stack + (2 * size_t(ii) + side) * L;
                 const bool rough = act && !straight && A.rough[2 * ii + side];
                 const int cx = side ? px : x, cy = side ? y : py;
-#pragma unroll
+#pragma unroll kUnroll
                 for (int cl = 0; cl < LL; ++cl) {
                     if (cl >= L) continue;
                     const double cost = __shfl_sync(kAll, reach, s0 + cl);
@@ -676,7 +677,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
                 const int row = tri(L, sl, sl) - sl;
                 double cc = A.diag[s0 + sl];
                 int path = A.pdiag[s0 + sl];
-#pragma unroll
+#pragma unroll kUnroll
                 for (int hi = 0; hi < LL; ++hi) {
                     if (hi < sl || hi >= L) continue;
                     const double v = A.diag[s0 + hi];
@@ -709,7 +710,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
         int br = 0;
         if (i >= 0) {
             const double* row = A.dist + i * TT + tri(L, sl, sl) - sl;
-#pragma unroll
+#pragma unroll kUnroll
             for (int hi = 0; hi < LL; ++hi) {
                 if (hi < sl || hi >= L) continue;
                 const double v = row[hi];
@@ -718,7 +719,7 @@ __device__ __forceinline__ void route_pack_l(const Tables& T, const Plan& P, con
         }
         double best = __longlong_as_double(0x7ff0000000000000ll);
         int rr = 0;  // no entry below infinity: the sequential loop keeps range (0, 0)
-#pragma unroll
+#pragma unroll kUnroll
         for (int lo = 0; lo < LL; ++lo) {
             if (lo >= L) continue;
             const double v = __shfl_sync(kAll, bv, s0 + lo);
