@@ -68,10 +68,12 @@ struct BatchState {
     unsigned* cellmask;         // [W][X*Y]: word w of every cell contiguous, so the
                                 // colour ORs of consecutive cells share sectors
     unsigned* localmask[5];     // [X*Y][CH/32], chunk k in buffer k % 5
+    unsigned* localset[5];      // [X*Y] which words of the cell's record are nonzero
     unsigned* ptchunk;          // [X*Y] bit k % 32: the cell is a query point of chunk k
     unsigned* fmask;            // [2][W][CH] forbidden colours, by chunk parity
     unsigned* pred;             // [2][CH/32][CH] predecessors inside the chunk
     unsigned* prevp;            // [2][CH/32][CH] marking nets of the previous chunk
+    unsigned* words;            // [2][2][CH] per net, which words of its pred and prevp columns are set
     unsigned* fullmask;         // [W]
     int* count;                 // [32*W]
     int* n_colors;              // [1]
@@ -177,6 +179,9 @@ __device__ __forceinline__ void flat_fill(const BatchState& B, int p) {
 
 constexpr int kLocalMasks = 5;
 __device__ __forceinline__ unsigned* chunk_mask(const BatchState& B, int chunk) { return B.localmask[chunk % kLocalMasks]; }
+// A cell's record is a few bits in 128 bytes (a chunk marks a cell a handful of
+// times); one word per cell says which of its words to read or to clear.
+__device__ __forceinline__ unsigned* chunk_set(const BatchState& B, int chunk) { return B.localset[chunk % kLocalMasks]; }
 
 // Query-point bits of the chunk at s: bit (chunk % 32) of every query point
 // cell of the chunk is set (set) or cleared.
@@ -202,7 +207,7 @@ __device__ __forceinline__ void batch_raster(const BatchState& B, int s, int ahe
     const int m = min(CH, B.n - s), chunk = s / CH;
     unsigned want = 0u;
     for (int a = 0; a <= ahead; ++a) want |= 1u << ((chunk + a) & 31);
-    unsigned* lm = chunk_mask(B, chunk);
+    unsigned *lm = chunk_mask(B, chunk), *ls = chunk_set(B, chunk);
     const long long a = B.mark_off[s], b = B.mark_off[s + m];
     // Four marks per thread and pass, every load of a pass issued first.
     for (long long k0 = a + t; k0 < b; k0 += 4 * nt) {
@@ -218,25 +223,26 @@ __device__ __forceinline__ void batch_raster(const BatchState& B, int s, int ahe
         for (int u = 0; u < 4; ++u) bits[u] = jj[u] >= 0 ? __ldcg(B.ptchunk + q[u]) : 0u;
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (bits[u] & want) red_or(lm + size_t(q[u]) * (CH / 32) + (jj[u] >> 5), 1u << (jj[u] & 31));
+            if (bits[u] & want) {
+                red_or(lm + size_t(q[u]) * (CH / 32) + (jj[u] >> 5), 1u << (jj[u] & 31));
+                red_or(ls + q[u], 1u << (jj[u] >> 5));
+            }
     }
 }
 
 // The chunk-local mask of the chunk at s is nonzero only at query points of
-// this chunk and the `ahead` chunks after it: zero the whole record of each of
-// those cells.
+// this chunk and the `ahead` chunks after it: zero those cells' words.
 template <int CH>
 __device__ __forceinline__ void batch_clear(const BatchState& B, int s, int ahead, long long t, long long nt) {
-    unsigned* lm = chunk_mask(B, s / CH);
+    unsigned *lm = chunk_mask(B, s / CH), *ls = chunk_set(B, s / CH);
     const long long a = B.pt_off[s];
     const long long b = B.pt_off[min(s + (ahead + 1) * CH, B.n)];
-    constexpr int kParts = (CH / 32) / 4;  // 16-byte groups of a record
-    const long long items = (b - a) * kParts;
-    for (long long k = t; k < items; k += nt) {
-        const long long pi = a + k / kParts;
-        const int part = int(k % kParts);
-        uint4* rec = reinterpret_cast<uint4*>(lm + size_t(__ldg(B.pt_cell + pi)) * (CH / 32));
-        rec[part] = make_uint4(0u, 0u, 0u, 0u);
+    for (long long k = a + t; k < b; k += nt) {
+        const unsigned q = __ldg(B.pt_cell + k);
+        unsigned set = __ldcg(ls + q);  // several points may share the cell: whoever sees a set bit clears its word
+        if (!set) continue;
+        for (; set; set &= set - 1) lm[size_t(q) * (CH / 32) + __ffs(set) - 1] = 0u;
+        ls[q] = 0u;
     }
 }
 
@@ -245,69 +251,59 @@ __device__ __forceinline__ void batch_clear(const BatchState& B, int s, int ahea
 // previous chunk's nets (resolved by the solver, which knows their colours);
 // with lookback 2 also the colours of the nets two chunks back that mark the
 // cell (that chunk is solved, its colours published or being published).
-// Each item is a 16-byte group of one record (W and (CH / 32) are
-// multiples of 4).
+// An item is four colour words or one chunk's record at a point; of a record
+// only the words its set word names are read (with whole records, 26 items a
+// point at 8 colour words instead of 5, the gather was the longest task of a
+// round).  Consecutive lanes take the items of one point.
 template <int CH>
 __device__ __forceinline__ void batch_gather(const BatchState& B, int s, int lookback, long long t, long long nt) {
     const int chunk = s / CH, m = min(CH, B.n - s), W = B.W;
-    const unsigned* lm = chunk_mask(B, chunk);
-    const unsigned* lp = lookback >= 1 ? chunk_mask(B, chunk - 1) : nullptr;
-    const unsigned* lp2 = lookback >= 2 ? chunk_mask(B, chunk - 2) : nullptr;
     unsigned* F = B.fmask + size_t(chunk & 1) * W * CH;
     unsigned* P = B.pred + size_t(chunk & 1) * (CH / 32) * CH;
     unsigned* Q = B.prevp + size_t(chunk & 1) * (CH / 32) * CH;
-    const int gw = W / 4, gl = (CH / 32) / 4;
-    const int per = gw + gl * (1 + lookback);
+    unsigned* words = B.words + size_t(chunk & 1) * 2 * CH;
+    const int gw = W / 4, per = gw + 1 + lookback, shift = 32 - __clz(per - 1);  // 2^shift lanes a point
     const long long a = B.pt_off[s], b = B.pt_off[s + m];
-    const long long items = (b - a) * per;
+    const long long items = (b - a) << shift;
+    const size_t XY = size_t(B.X) * B.Y;
     for (long long k = t; k < items; k += nt) {
-        const long long pi = k / per;
-        const int g = int(k - pi * per);
-        const unsigned q = __ldg(B.pt_cell + a + pi);
-        const int jj = __ldg(B.pt_jj + a + pi) & (CH - 1);
-        uint4 v;
-        unsigned* dst;
-        int w0;
+        const int g = int(k) & ((1 << shift) - 1);
+        if (g >= per) continue;
+        const long long pi = a + (k >> shift);
+        const unsigned q = __ldg(B.pt_cell + pi);
+        const int jj = __ldg(B.pt_jj + pi) & (CH - 1);
         if (g < gw) {
-            w0 = 4 * g;
-            const size_t XY = size_t(B.X) * B.Y;
-            v.x = __ldcg(B.cellmask + (4 * g) * XY + q);
-            v.y = __ldcg(B.cellmask + (4 * g + 1) * XY + q);
-            v.z = __ldcg(B.cellmask + (4 * g + 2) * XY + q);
-            v.w = __ldcg(B.cellmask + (4 * g + 3) * XY + q);
-            dst = F;
-        } else if (g < gw + gl) {
-            w0 = 4 * (g - gw);
-            if (w0 > (jj >> 5)) continue;
-            v = __ldcg(reinterpret_cast<const uint4*>(lm + size_t(q) * (CH / 32)) + (g - gw));
-            const unsigned own = (1u << (jj & 31)) - 1u;  // earlier nets of the own word
-            const int ow = (jj >> 5) - w0;
-            if (ow == 0) { v.x &= own; v.y = v.z = v.w = 0u; }
-            else if (ow == 1) { v.y &= own; v.z = v.w = 0u; }
-            else if (ow == 2) { v.z &= own; v.w = 0u; }
-            else if (ow == 3) v.w &= own;
-            dst = P;
-        } else if (g < gw + 2 * gl) {
-            w0 = 4 * (g - gw - gl);
-            v = __ldcg(reinterpret_cast<const uint4*>(lp + size_t(q) * (CH / 32)) + (g - gw - gl));
-            dst = Q;
-        } else {
-            w0 = 4 * (g - gw - 2 * gl);
-            v = __ldcg(reinterpret_cast<const uint4*>(lp2 + size_t(q) * (CH / 32)) + (g - gw - 2 * gl));
-            const unsigned vw[4] = {v.x, v.y, v.z, v.w};
-            const int* col2 = B.batch_of + size_t(chunk - 2) * CH;
+            unsigned v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = __ldcg(B.cellmask + (4 * g + u) * XY + q);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                for (unsigned bits = vw[u]; bits; bits &= bits - 1) {
-                    const int c = __ldcg(col2 + (w0 + u) * 32 + __ffs(bits) - 1);
-                    red_or(F + size_t(c >> 5) * CH + jj, 1u << (c & 31));
-                }
+                if (v[u]) red_or(F + size_t(4 * g + u) * CH + jj, v[u]);
             continue;
         }
-        if (v.x) red_or(dst + size_t(w0) * CH + jj, v.x);
-        if (v.y) red_or(dst + size_t(w0 + 1) * CH + jj, v.y);
-        if (v.z) red_or(dst + size_t(w0 + 2) * CH + jj, v.z);
-        if (v.w) red_or(dst + size_t(w0 + 3) * CH + jj, v.w);
+        const int back = g - gw;  // the record of chunk - back
+        unsigned set = __ldcg(chunk_set(B, chunk - back) + q);
+        if (back == 0) set &= (2u << (jj >> 5)) - 1u;  // words of earlier nets
+        if (!set) continue;
+        const unsigned* rec = chunk_mask(B, chunk - back) + size_t(q) * (CH / 32);
+        unsigned found = 0u;
+        for (; set; set &= set - 1) {
+            const int w = __ffs(set) - 1;
+            unsigned bits = __ldcg(rec + w);
+            if (back == 0 && w == (jj >> 5)) bits &= (1u << (jj & 31)) - 1u;  // earlier nets of the own word
+            if (!bits) continue;
+            if (back < 2) {
+                found |= 1u << w;
+                red_or((back ? Q : P) + size_t(w) * CH + jj, bits);
+            } else {
+                const int* col2 = B.batch_of + size_t(chunk - 2) * CH + w * 32;
+                for (; bits; bits &= bits - 1) {
+                    const int c = __ldcg(col2 + __ffs(bits) - 1);
+                    red_or(F + size_t(c >> 5) * CH + jj, 1u << (c & 31));
+                }
+            }
+        }
+        if (found) red_or(words + (back ? CH : 0) + jj, found);
     }
 }
 
@@ -316,11 +312,21 @@ template <int CH>
 __device__ __forceinline__ void batch_publish(const BatchState& B, int s, long long t, long long nt) {
     const int m = min(CH, B.n - s);
     const long long a = B.mark_off[s], b = B.mark_off[s + m];
-    for (long long k = a + t; k < b; k += nt) {
-        const unsigned q = __ldg(B.mark_cell + k);
-        const int jj = __ldg(B.mark_jj + k) & (CH - 1);
-        const int c = __ldcg(B.batch_of + s + jj);
-        red_or(B.cellmask + size_t(c >> 5) * B.X * B.Y + q, 1u << (c & 31));
+    // Four marks per thread and pass, every load of a pass issued first.
+    for (long long k0 = a + t; k0 < b; k0 += 4 * nt) {
+        unsigned q[4];
+        int jj[4], c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const long long k = k0 + u * nt;
+            q[u] = k < b ? __ldg(B.mark_cell + k) : 0u;
+            jj[u] = k < b ? (__ldg(B.mark_jj + k) & (CH - 1)) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = jj[u] >= 0 ? __ldcg(B.batch_of + s + jj[u]) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (jj[u] >= 0) red_or(B.cellmask + size_t(c[u] >> 5) * B.X * B.Y + q[u], 1u << (c[u] & 31));
     }
 }
 
@@ -414,6 +420,67 @@ __device__ __forceinline__ bool solve_sync_or(bool v) {
     return r != 0;
 }
 
+// First-fit of the chunk's nets from `fixed` on, warp after warp (32 nets in
+// order): a warp settles its nets by sweeps among themselves once every earlier
+// warp is final, and after a barrier the later warps add its colours to those
+// their nets may not take.  Each predecessor is looked at once, where a sweep
+// over the whole chunk looks at all of them again: for chunks whose nets depend
+// on one another in long chains (small grids).  For W == 8.  Leaves the colours
+// in S.col; false if a net finds none.
+template <int CH>
+__device__ __forceinline__ bool colours_in_order(const SolveSmem& S, int m, int fixed, unsigned pmask) {
+    constexpr int W = 8;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    unsigned no[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) no[w] = tid < m ? S.U[w * CH + tid] : 0u;
+    const bool open = tid < m && tid >= fixed;
+    bool fits = true;
+    for (int k = 0; 32 * k < m; ++k) {
+        const unsigned preds = tid < m && ((pmask >> k) & 1u) ? S.P[k * CH + tid] : 0u;
+        if (warp == k) {
+            int mine = tid < m ? (open ? -1 : S.col[tid]) : -1;
+            if (tid < m) S.col[tid] = mine;
+            while (true) {
+                __syncwarp();
+                int next = mine;
+                if (open) {
+                    unsigned used[W];
+#pragma unroll
+                    for (int w = 0; w < W; ++w) used[w] = no[w];
+                    for (unsigned b = preds; b; b &= b - 1) {
+                        const int c = S.col[32 * k + __ffs(b) - 1];  // -1 (not yet coloured) is in no word
+#pragma unroll
+                        for (int w = 0; w < W; ++w) used[w] |= (c >> 5) == w ? 1u << (c & 31) : 0u;
+                    }
+                    next = 32 * W;
+#pragma unroll
+                    for (int w = W - 1; w >= 0; --w)
+                        if (used[w] != 0xffffffffu) next = 32 * w + __ffs(~used[w]) - 1;
+                    fits = next < 32 * W;
+                    next = min(next, 32 * W - 1);
+                }
+                const bool again = __any_sync(0xffffffffu, next != mine);
+                if (tid < m) S.col[tid] = next;
+                mine = next;
+                if (!again) break;
+            }
+        }
+        solve_sync<CH>();
+        if (warp > k)
+            for (unsigned b = preds; b; b &= b - 1) {
+                const int c = S.col[32 * k + __ffs(b) - 1];
+#pragma unroll
+                for (int w = 0; w < W; ++w) no[w] |= (c >> 5) == w ? 1u << (c & 31) : 0u;
+            }
+    }
+    return fits;
+}
+// Sweeps over the whole chunk before it is coloured in order: most chunks of
+// large designs settle in two or three (0.5 us each at 3 predecessors a net);
+// in order a chunk takes about 60 us whatever its chains (64x64x5: 86 against 106).
+constexpr int kSweeps = 6;
+
 // Step 3 (threads 0..CH-1 of a CTA): first-fit of the chunk at order
 // position s.  S.cnt and S.full hold the state of the chunks before it;
 // with `lookback`, S.colp holds the previous chunk's colours.  The chunk's
@@ -429,9 +496,12 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
     unsigned* Qg = B.prevp + size_t(chunk & 1) * (CH / 32) * CH;
     __shared__ int first_bad, overflow;
     if (tid == 0) overflow = 0;
-    unsigned pmask = 0;
+    unsigned* set = B.words + size_t(chunk & 1) * 2 * CH;
+    unsigned pmask = 0, qmask = 0;
     int c0 = 0;  // first colour not in U
     if (tid < m) {
+        pmask = __ldcg(set + tid);
+        if (lookback) qmask = __ldcg(set + CH + tid);
         // Every load of a group is issued before its stores, so the round
         // trips overlap (the tables were just written by other SMs).
         for (int w0 = 0; w0 < W; w0 += 8) {
@@ -445,45 +515,58 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
                 S.U[(w0 + k) * CH + tid] = v[k] | S.full[w0 + k];
             }
         }
-        {
-            unsigned v[(CH / 32)];
+        // Only the words the gather has set are read (a net has a few earlier
+        // neighbours, in a few words of the 32), four at a time.
+        auto words = [&](unsigned left, unsigned* table, auto use) {
+            while (left) {
+                int w[4];
+                unsigned v[4];
 #pragma unroll
-            for (int w = 0; w < (CH / 32); ++w) v[w] = w <= (tid >> 5) ? __ldcg(Pg + w * CH + tid) : 0u;
+                for (int k = 0; k < 4; ++k) {
+                    w[k] = left ? __ffs(left) - 1 : -1;
+                    left &= left - 1;  // 0 stays 0
+                }
 #pragma unroll
-            for (int w = 0; w < (CH / 32); ++w) {
-                S.P[w * CH + tid] = v[w];
-                if (v[w]) { Pg[w * CH + tid] = 0u; pmask |= 1u << w; }
+                for (int k = 0; k < 4; ++k) v[k] = w[k] >= 0 ? __ldcg(table + w[k] * CH + tid) : 0u;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (w[k] >= 0) {
+                        table[w[k] * CH + tid] = 0u;
+                        use(w[k], v[k]);
+                    }
             }
-        }
+        };
+        if (pmask) set[tid] = 0u;
+        words(pmask, Pg, [&](int w, unsigned bits) { S.P[w * CH + tid] = bits; });
         if (lookback) {
-            unsigned v[(CH / 32)];
-#pragma unroll
-            for (int w = 0; w < (CH / 32); ++w) v[w] = __ldcg(Qg + w * CH + tid);
-#pragma unroll
-            for (int w = 0; w < (CH / 32); ++w) {
-                unsigned bits = v[w];
-                if (bits) Qg[w * CH + tid] = 0u;
+            if (qmask) set[CH + tid] = 0u;
+            words(qmask, Qg, [&](int w, unsigned bits) {
                 while (bits) {
                     const int c = S.colp[w * 32 + __ffs(bits) - 1];
                     bits &= bits - 1;
                     S.U[(c >> 5) * CH + tid] |= 1u << (c & 31);
                 }
-            }
+            });
         }
         c0 = first_fit<CH>(S, tid, W, 0u, 0);
     }
-    S.col[tid] = -1;
+    // The first sweep, in which no net has a colour yet, gives every net c0.
+    S.col[tid] = tid < m ? c0 : -1;
     solve_sync<CH>();
     int fixed = 0;  // nets below `fixed` are final
     int rank = 0;
-    bool counted = false;  // this chunk's nets are in S.cnt already
     __shared__ int tight;
     while (true) {
         // Jacobi sweeps until the colouring is a fixed point.
-        while (true) {
+        for (int sweep = 0;; ++sweep) {
+            if (sweep == kSweeps && W == 8) {
+                if (!colours_in_order<CH>(S, m, fixed, pmask)) overflow = 1;
+                solve_sync<CH>();
+                break;
+            }
             int mine = tid < m ? S.col[tid] : -1;
             if (tid < m && tid >= fixed) {
-                mine = first_fit<CH>(S, tid, W, pmask, c0);
+                mine = pmask ? first_fit<CH>(S, tid, W, pmask, c0) : c0;
                 if (mine >= C) { overflow = 1; mine = C - 1; }
             }
             solve_sync<CH>();
@@ -492,37 +575,35 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
             if (!solve_sync_or<CH>(changed)) break;
         }
         if (overflow) break;
-        // Position of every net inside its batch, in chunk order: colour
-        // counts of the earlier warps plus the rank inside the own warp.
-        if (tid == 0) first_bad = m;
+        // While no batch reaches its limit, no position inside a batch is
+        // needed here (the rank pass after the run assigns them): the chunk's
+        // nets are added to the per-colour totals.  Else the positions, in
+        // chunk order -- colour counts of the earlier warps plus the rank inside
+        // the own warp -- find the first net that does not fit.
+        if (tid == 0) { first_bad = m; tight = 0; }
         const int c = tid < m ? S.col[tid] : -1 - lane;  // distinct dummies for idle lanes
-        const unsigned peers = __match_any_sync(0xffffffffu, c);
-        const bool leader = tid < m && lane == __ffs(peers) - 1;
-        const int within = __popc(peers & ((1u << lane) - 1u));
-        if (S.per_warp) {
-            if (leader) S.wh[warp * C + c] = __popc(peers);
+        if (tid < m) atomicAdd(S.cnt + c, 1);
+        solve_sync<CH>();
+        if (tid < m && S.cnt[c] > B.limit) tight = 1;
+        solve_sync<CH>();
+        const bool counted = !tight;
+        if (!counted) {
+            if (tid < m) atomicSub(S.cnt + c, 1);
+            const unsigned peers = __match_any_sync(0xffffffffu, c);
+            const bool leader = tid < m && lane == __ffs(peers) - 1;
+            const int within = __popc(peers & ((1u << lane) - 1u));
+            if (S.per_warp && leader) S.wh[warp * C + c] = __popc(peers);
             solve_sync<CH>();
-            if (tid < m) {
-                int r = S.cnt[c] + within;
-                for (int w = 0; w < warp; ++w) r += S.wh[w * C + c];
-                rank = r;
-                if (r >= B.limit) atomicMin(&first_bad, tid);
-            }
-            solve_sync<CH>();
-            if (leader) S.wh[warp * C + c] = 0;
-        } else {
-            // Per-colour totals first: while no batch reaches the limit, no
-            // position inside a batch is needed here (the rank pass after the
-            // run assigns them); else warps add their counts in turn.
-            if (tid == 0) tight = 0;
-            solve_sync<CH>();
-            if (leader && atomicAdd(S.cnt + c, __popc(peers)) + __popc(peers) > B.limit) tight = 1;
-            solve_sync<CH>();
-            if (!tight) {
-                counted = true;
-            } else {
-                if (leader) atomicSub(S.cnt + c, __popc(peers));
+            if (S.per_warp) {
+                if (tid < m) {
+                    int r = S.cnt[c] + within;
+                    for (int w = 0; w < warp; ++w) r += S.wh[w * C + c];
+                    rank = r;
+                    if (r >= B.limit) atomicMin(&first_bad, tid);
+                }
                 solve_sync<CH>();
+                if (leader) S.wh[warp * C + c] = 0;
+            } else {
                 for (int k = tid; k < C; k += CH) S.wh[k] = S.cnt[k];
                 solve_sync<CH>();
                 for (int w = 0; w < (m + 31) / 32; ++w) {
@@ -537,7 +618,7 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
         }
         const int bad = first_bad;
         if (bad >= m) {
-            if (leader && !counted) atomicAdd(S.cnt + c, __popc(peers));
+            if (!counted && tid < m) atomicAdd(S.cnt + c, 1);
             break;
         }
         // Net `bad` finds its colour full; so does every later net.
@@ -561,7 +642,7 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
         S.colp[tid] = c;
         top = c + 1;
     }
-    for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    top = __reduce_max_sync(0xffffffffu, top);
     if (lane == 0 && top) atomicMax(B.n_colors, top);
     solve_sync<CH>();
     return true;

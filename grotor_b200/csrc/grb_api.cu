@@ -792,18 +792,22 @@ __global__ void k_batch_publish(BatchState B, int s) {
 // and releases `solved` = r + 1.  The other CTAs set the query-point bits of
 // chunks 0-4 | raster chunks 0 and 1 | gather chunk 0 | and then run, per
 // round r, one phase and one barrier:
-//   wait for chunk r-1's colours; publish chunk r-1 and clear its query-point
-//   bits; empty chunk r-2's chunk-local mask; set the query-point bits of
-//   chunk r+5; gather chunk r+1 (cellmask as of chunk r-2 at least, chunk r-1
-//   through its chunk-local mask and its colours, chunk r through the
-//   previous-chunk bits the solver resolves); raster chunk r+2, keeping the
-//   marks on query points of chunks r+2 to r+4              | barrier
+//   some warps wait for chunk r-1's colours, then gather chunk r+1 (cellmask as
+//   of chunk r-2 at least, chunk r-1 through its chunk-local mask and its
+//   colours, chunk r through the previous-chunk bits the solver resolves) or
+//   publish chunk r-1 and clear its query-point bits; the others, without
+//   waiting, raster chunk r+2, keeping the marks on query points of chunks r+2
+//   to r+4, empty chunk r-2's chunk-local mask and set the query-point bits of
+//   chunk r+5                                                       | barrier
 // A chunk's local mask (five buffers, chunk k in buffer k % 5) is written by
 // its raster in round k-2, read by the gathers of chunks k, k+1 and k+2
 // (rounds k-1 to k+1) and emptied in round k+2, before the raster of chunk
 // k+5 in round k+3.  The barrier of round r is what the solver waits for
 // before chunk r+1 (counter (3 + (r + 1)) * G).
 constexpr int kPersistThreads = kChunkMax;
+// A worker CTA's threads per task of a round: gather; publish; the others
+// raster, empty and set bits.
+constexpr int kGatherThreads = 320, kPublishThreads = 320;
 template <int CH>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_batch_persistent(BatchState B, GridSync S, Tables T) {
     extern __shared__ __align__(16) unsigned bsm[];
@@ -845,19 +849,36 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_batch_persistent(BatchSt
     batch_gather<CH>(B, 0, 0, t, nt);
     if (!grid_sync_of(S, T, G)) return;
     clk.mark(S, 1);
+    // The tasks of a round are independent, and each is a chain of dependent
+    // loads: the CTA's warps are split among them, so a round costs the longest
+    // chain and not their sum.  The raster, the emptying and the next bits wait
+    // for no colours.
+    const int role = threadIdx.x < kGatherThreads ? 0 : threadIdx.x < kGatherThreads + kPublishThreads ? 1 : 2;
+    const int in_role = threadIdx.x - (role == 0 ? 0 : role == 1 ? kGatherThreads : kGatherThreads + kPublishThreads);
+    const int of_role = role == 0 ? kGatherThreads : role == 1 ? kPublishThreads
+                                                               : kPersistThreads - kGatherThreads - kPublishThreads;
+    const long long rt = (blockIdx.x - 1) * (long long)of_role + in_role, rn = (long long)G * of_role;
     for (int r = 0; r < chunks; ++r) {
-        if (r >= 1) {
-            if (threadIdx.x == 0) go = wait_at_least(B.solved, unsigned(r), S.timeout_ns, T, true);
-            __syncthreads();
-            if (!go) return;
-            clk.mark(S, 9);
-            batch_publish<CH>(B, (r - 1) * CH, t, nt);
-            batch_point_bits<CH>(B, (r - 1) * CH, false, t, nt);
+        if (role == 2) {
+            if (r + 2 < chunks) batch_raster<CH>(B, (r + 2) * CH, 2, rt, rn);
+            if (r >= 2) batch_clear<CH>(B, (r - 2) * CH, 2, rt, rn);
+            if (r + 5 < chunks) batch_point_bits<CH>(B, (r + 5) * CH, true, rt, rn);
+        } else {
+            bool on = true;
+            if (r >= 1) {
+                if (threadIdx.x == 0) go = wait_at_least(B.solved, unsigned(r), S.timeout_ns, T, true);
+                asm volatile("bar.sync 2, %0;" ::"n"(kGatherThreads + kPublishThreads) : "memory");
+                on = go != 0;
+                clk.mark(S, 9);
+            }
+            if (on && role == 0 && r + 1 < chunks) batch_gather<CH>(B, (r + 1) * CH, min(r + 1, 2), rt, rn);
+            if (on && role == 1 && r >= 1) {
+                batch_publish<CH>(B, (r - 1) * CH, rt, rn);
+                batch_point_bits<CH>(B, (r - 1) * CH, false, rt, rn);
+            }
         }
-        if (r >= 2) batch_clear<CH>(B, (r - 2) * CH, 2, t, nt);
-        if (r + 5 < chunks) batch_point_bits<CH>(B, (r + 5) * CH, true, t, nt);
-        if (r + 1 < chunks) batch_gather<CH>(B, (r + 1) * CH, min(r + 1, 2), t, nt);
-        if (r + 2 < chunks) batch_raster<CH>(B, (r + 2) * CH, 2, t, nt);
+        __syncthreads();
+        if (r >= 1 && !go) return;
         if (!grid_sync_of(S, T, G)) return;
         clk.mark(S, 1);
     }
@@ -1034,8 +1055,9 @@ struct grb_ctx {
     // batching buffers
     unsigned *cellmask = nullptr, *fmask = nullptr, *fullmask = nullptr;
     unsigned* lmask[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // chunk-local masks
+    unsigned* lset = nullptr;                           // [5][X*Y] nonzero words of each record
     unsigned* ptchunk = nullptr;                        // [X*Y] query-point bits by chunk % 32
-    unsigned *pred = nullptr, *prevp = nullptr, *bsolved = nullptr;
+    unsigned *pred = nullptr, *prevp = nullptr, *pwords = nullptr, *bsolved = nullptr;
     bool lmask_dirty = false;          // a run stopped before clearing them
     int *bcount = nullptr, *ncolors = nullptr, *batch_of = nullptr, *brank = nullptr, *order = nullptr;
     int* rank_tiles = nullptr;         // [tiles][colours] scratch of the rank pass
@@ -2067,7 +2089,7 @@ void grb_destroy(grb_ctx* c) {
     free_all(c->owned);
     for (void* p : {(void*)c->check, (void*)c->stage, (void*)c->bucket_ids, (void*)c->bucket_off, (void*)c->ids, (void*)c->batch_off, (void*)c->gscratch, (void*)c->work, (void*)c->cellmask,
                     (void*)c->lmask[0], (void*)c->lmask[1], (void*)c->lmask[2], (void*)c->lmask[3], (void*)c->lmask[4],
-                    (void*)c->ptchunk, (void*)c->fmask, (void*)c->pred, (void*)c->prevp,
+                    (void*)c->lset, (void*)c->ptchunk, (void*)c->fmask, (void*)c->pred, (void*)c->prevp, (void*)c->pwords,
                     (void*)c->bsolved, (void*)c->fullmask, (void*)c->bcount, (void*)c->ncolors, (void*)c->batch_of, (void*)c->brank,
                     (void*)c->order, (void*)c->rank_tiles, (void*)c->mark_off, (void*)c->pt_off, (void*)c->scan_sums, (void*)c->mark_cell,
                     (void*)c->pt_cell, (void*)c->mark_jj, (void*)c->pt_jj})
@@ -2986,15 +3008,16 @@ int grb_plan_batches(grb_ctx* c, const int32_t* order, int32_t n, int32_t limit,
     GRB_CUDA(c, cudaSetDevice(c->device));
     const size_t xy = size_t(c->T.XY);
     const size_t lm_bytes = xy * kChunkMaxWords * 4;
-    const size_t pq_bytes = 2 * size_t(kChunkMax) * kChunkMaxWords * 4;
+    const size_t pq_bytes = 2 * size_t(kChunkMax) * kChunkMaxWords * 4, pw_bytes = 2 * 2 * size_t(kChunkMax) * 4;
     int W = std::max(c->bW, 8);
     int rc = ensure_plan_capacity(c, n, n);
     if (rc) return rc;
     if (!c->lmask[0]) {
         if (cudaMalloc(&c->lmask[0], lm_bytes) || cudaMalloc(&c->lmask[1], lm_bytes) || cudaMalloc(&c->lmask[2], lm_bytes) ||
             cudaMalloc(&c->lmask[3], lm_bytes) || cudaMalloc(&c->lmask[4], lm_bytes) ||
-            cudaMalloc(&c->ptchunk, xy * 4) ||
-            cudaMalloc(&c->pred, pq_bytes) || cudaMalloc(&c->prevp, pq_bytes) || cudaMalloc(&c->bsolved, 4) ||
+            cudaMalloc(&c->lset, 5 * xy * 4) || cudaMalloc(&c->ptchunk, xy * 4) ||
+            cudaMalloc(&c->pred, pq_bytes) || cudaMalloc(&c->prevp, pq_bytes) || cudaMalloc(&c->pwords, pw_bytes) ||
+            cudaMalloc(&c->bsolved, 4) ||
             cudaMalloc(&c->ncolors, 4)) {
             cudaGetLastError();
             return fail(c, GRB_ENOMEM, "batching buffers");
@@ -3028,6 +3051,7 @@ int grb_plan_batches(grb_ctx* c, const int32_t* order, int32_t n, int32_t limit,
         if (smem > kSolveSmemLimit) return fail(c, GRB_ELIMIT, "too many batch colours");
         if (c->lmask_dirty) {
             for (unsigned* lm : c->lmask) GRB_CUDA(c, cudaMemsetAsync(lm, 0, lm_bytes, c->stream));
+            GRB_CUDA(c, cudaMemsetAsync(c->lset, 0, 5 * xy * 4, c->stream));
             GRB_CUDA(c, cudaMemsetAsync(c->ptchunk, 0, xy * 4, c->stream));
             c->lmask_dirty = false;
         }
@@ -3035,15 +3059,19 @@ int grb_plan_batches(grb_ctx* c, const int32_t* order, int32_t n, int32_t limit,
         GRB_CUDA(c, cudaMemsetAsync(c->fmask, 0, 2 * size_t(kChunkMax) * W * 4, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->pred, 0, pq_bytes, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->prevp, 0, pq_bytes, c->stream));
+        GRB_CUDA(c, cudaMemsetAsync(c->pwords, 0, pw_bytes, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->fullmask, 0, W * 4, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->bcount, 0, size_t(32) * W * 4, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->ncolors, 0, 4, c->stream));
         GRB_CUDA(c, cudaMemsetAsync(c->bsolved, 0, 4, c->stream));
         B.W = W;
         B.cellmask = c->cellmask;
-        for (int k = 0; k < 5; ++k) B.localmask[k] = c->lmask[k];
+        for (int k = 0; k < 5; ++k) {
+            B.localmask[k] = c->lmask[k];
+            B.localset[k] = c->lset + k * xy;
+        }
         B.ptchunk = c->ptchunk;
-        B.fmask = c->fmask; B.pred = c->pred; B.prevp = c->prevp;
+        B.fmask = c->fmask; B.pred = c->pred; B.prevp = c->prevp; B.words = c->pwords;
         B.fullmask = c->fullmask; B.count = c->bcount; B.n_colors = c->ncolors;
         B.solved = c->bsolved;
         c->lmask_dirty = true;  // until the run completes
