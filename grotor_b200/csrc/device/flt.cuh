@@ -12,11 +12,17 @@
 // each node's via stack.
 //
 // B200 form: the layer-change tables of all the batch's edges are one
-// grid-wide pass, a thread per (edge, from-layer, to-layer) entry (the
-// reference launches a thread per (edge, from-layer)); then one warp per net
-// (the reference uses a 128-thread CTA); lanes take the nodes of one depth
-// level, __syncwarp separates levels; the packed keys live in a per-stage
-// workspace in HBM (mostly L2-resident per batch).
+// grid-wide pass, a warp per edge (the reference launches a thread per (edge,
+// from-layer)).  Then a net is walked by one warp, or by a CTA where its levels
+// are wide; its topology, candidate keys and choices sit in shared memory.  A
+// warp solves three nodes of a level at once, a lane per (node, layer): lane
+// `low` walks its range tops, a column minimum per top picks the range, and a
+// lane per target layer offers the node to each parent slot (the reference and
+// the earlier form here give a node to one thread, which walks the ranges of
+// all layers in thread-local arrays).  A batch lasts as long as its largest
+// net's levels one after the other, so it is a level's latency that counts:
+// 2,400 nets in 35 batches at 320x320x10 took 18 ms of solve and trace by a
+// thread per node, 4.6 ms in this form.
 // Node numbering is net-local: candidates for a slot always belong to one
 // net, so the batch-global numbering of the reference orders them the same.
 // Segments are appended in level order, ascending node index within a level,
@@ -186,144 +192,215 @@ __device__ __forceinline__ void flt_edges_batch(const Tables& T, const Flt& F, c
     }
 }
 
-// solve_flt_node (flt_block.cuh:6-142) for net-local node `i`.  The node's
-// inputs -- its children's candidate keys and the via costs of its column --
-// are loaded once, and its range costs and choices are kept in registers and
-// thread-local arrays until the end (in HBM they would cost a round trip per
-// read after a write); the loops and comparisons are the reference's.
-__device__ __forceinline__ void flt_solve_node(const Tables& T, const Flt& F, int nb, int eb, int i) {
-    const int g = nb + i;
-    const int c0 = F.coord[g];
-    const int flow = 1 + c0 / T.XY, x = c0 / T.Y % T.X, y = c0 % T.Y;
-    const int fhigh = flow == kFltLayers ? 0 : flow;
-    const int nc = F.children[g];
-    unsigned long long* cbp = F.best + size_t(F.child_off[g]) * kFltLayers;
-    const unsigned long long* cpk = F.packed + size_t(F.child_off[g]) * kFltLayers;
-    double* cst_g = F.costs + size_t(g) * kFltLayers;
-    unsigned long long pk[kFltMaxChildren][kFltLayers];  // children's keys
-    for (int c = 0; c < nc; ++c) {
-        unsigned long long v[kFltLayers];
-#pragma unroll
-        for (int li = 0; li < kFltLayers; ++li) v[li] = cpk[c * kFltLayers + li];
-#pragma unroll
-        for (int li = 0; li < kFltLayers; ++li) pk[c][li] = v[li];
+// One net as its warp or CTA walks it: topology, candidate keys, choices, in
+// shared memory where they fit, else in HBM.
+struct FltNet {
+    int N, nb, eb;
+    const int *coord, *children, *coff, *pend, *order;  // per node; coff: first child slot in packed / best
+    const int *epar, *eslot;                            // per edge of the net
+    unsigned long long *packed, *best;                  // [child slots][kFltLayers]
+    int* lo;                                            // [N] chosen layer (1-based), -1 unused
+};
+constexpr int kFltArena = 10240;  // shared memory of a net's arrays, per warp
+constexpr int kFltRow = kFltLayers - 1;  // layers 1..9: lanes of a slot
+constexpr int kFltSlots = 3;             // nodes a warp solves at once
+constexpr int kFltScratch = kFltSlots * kFltRow * kFltRow * 8 + 256;  // range costs and tops, per warp
+
+// Sets up net `id` for threads t of nth (a warp, or a CTA), its arrays in
+// `arena` when they fit `bytes`.  The caller synchronises before the next use.
+__device__ __forceinline__ FltNet flt_open(const Flt& F, int id, char* arena, int bytes, int t, int nth) {
+    FltNet W;
+    W.nb = F.node_off[id];
+    W.N = F.node_off[id + 1] - W.nb;
+    W.eb = F.edge_off[id];
+    const int E = F.edge_off[id + 1] - W.eb, N = W.N;
+    W.coord = F.coord + W.nb;
+    W.children = F.children + W.nb;
+    W.coff = F.child_off + W.nb;
+    W.pend = F.pend + W.nb;
+    W.order = F.order + W.nb;
+    W.epar = F.eparent + W.eb;
+    W.eslot = F.eslot + W.eb;
+    W.packed = F.packed;
+    W.best = F.best;
+    W.lo = F.lo + W.nb;
+    if (N <= 0) return W;
+    const int cb = W.coff[0], C = W.coff[N - 1] + W.children[N - 1] - cb;
+    const long long need = 16ll * kFltLayers * C + 24ll * N + 8ll * E;
+    if (need > bytes) {
+        for (int k = t; k < C * kFltLayers; k += nth) W.packed[size_t(cb) * kFltLayers + k] = kFltInit;
+        return W;
     }
-    float vc[kFltLayers];  // via cost of routing layer li - 2 at the node
+    unsigned long long* packed = reinterpret_cast<unsigned long long*>(arena);
+    int* p = reinterpret_cast<int*>(packed + 2 * size_t(C) * kFltLayers);
+    int *coord = p, *children = p + N, *coff = p + 2 * N, *pend = p + 3 * N, *order = p + 4 * N, *lo = p + 5 * N,
+        *epar = p + 6 * N, *eslot = epar + E;
+    for (int k = t; k < C * kFltLayers; k += nth) packed[k] = kFltInit;
+    for (int k = t; k < N; k += nth) {
+        coord[k] = W.coord[k];
+        children[k] = W.children[k];
+        coff[k] = W.coff[k] - cb;
+        pend[k] = W.pend[k];
+        order[k] = W.order[k];
+    }
+    for (int k = t; k < E; k += nth) {
+        epar[k] = W.epar[k];
+        eslot[k] = W.eslot[k];
+    }
+    W.packed = packed;
+    W.best = packed + size_t(C) * kFltLayers;
+    W.coord = coord; W.children = children; W.coff = coff; W.pend = pend; W.order = order;
+    W.epar = epar; W.eslot = eslot; W.lo = lo;
+    return W;
+}
+
+// solve_flt_node (flt_block.cuh:6-142) for one node per slot (lane = slot * 9 +
+// layer - 1; i < 0: none), by one warp.  `scratch`: kFltScratch bytes of the
+// warp's shared memory.
+//
+// The sequential loops keep, per range top, the first strict minimum over the
+// range bottoms in ascending order and, at one bottom, over the tops from it
+// up: lane `low` forms its bottom's costs and their suffix minima (lowest top
+// on ties), then lane `top` takes the first minimum over the bottoms.
+__device__ __forceinline__ void flt_solve_group(const Tables& T, const Flt& F, const FltNet& W, int i, int lane,
+                                                char* scratch) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int slot = min(lane / kFltRow, kFltSlots - 1), s0 = slot * kFltRow, li = lane - lane / kFltRow * kFltRow + 1;
+    const bool on = lane < kFltSlots * kFltRow && i >= 0;
+    const int ii = on ? i : 0;
+    double* cs = reinterpret_cast<double*>(scratch) + s0 * kFltRow;
+    unsigned char* hs = reinterpret_cast<unsigned char*>(scratch) + kFltSlots * kFltRow * kFltRow * 8 + s0 * kFltRow;
+    int l0, x, y;
+    cell_position(T, W.coord[ii], l0, x, y);
+    const int flow = 1 + l0, fhigh = flow == kFltLayers ? 0 : flow, nc = on ? W.children[ii] : 0;
+    const unsigned long long* keys = W.packed + size_t(W.coff[ii]) * kFltLayers;
+    // Via cost below layer li (between routing layers li - 2 and li - 1).
+    const float below = on && li >= 2 && li - 2 < T.L ? T.vcost[slot_index(T, li - 2, x, y)] : 0.f;
+    {
+        double mcc[kFltMaxChildren], via = 0;
 #pragma unroll
-    for (int li = 2; li < kFltLayers; ++li) vc[li] = li - 2 < T.L ? T.vcost[slot_index(T, li - 2, x, y)] : 0.f;
-    double cst[kFltLayers];
+        for (int c = 0; c < kFltMaxChildren; ++c) mcc[c] = kInf;
+#pragma unroll 1
+        for (int h = 1; h <= kFltRow; ++h) {
+            const float v = __shfl_sync(kAll, below, s0 + h - 1);
+            if (!on || h < li || li > flow) continue;
+            if (h > li) via += v;
+            double cost = via;
 #pragma unroll
-    for (int li = 0; li < kFltLayers; ++li) cst[li] = kInf;  // as flt_net left them
-    unsigned long long chosen[kFltMaxChildren][kFltLayers];  // chosen child candidate per range top
-    unsigned written = 0;                                    // range tops whose choices were set
-    double mcc[kFltMaxChildren];
-    unsigned long long bp[kFltMaxChildren];
-    for (int c = 0; c < kFltMaxChildren; ++c) bp[c] = 0;
-    for (int low = 1; low <= flow; ++low) {
-        for (int c = 0; c < nc; ++c) mcc[c] = kInf;
-        double via = 0;
-#pragma unroll
-        for (int li = 1; li < kFltLayers; ++li) {
-            if (li < low || li >= T.L + 1) continue;
-            if (li > low) via += vc[li];
-            for (int c = 0; c < nc; ++c) {
-                const unsigned long long pv = pk[c][li];
+            for (int c = 0; c < kFltMaxChildren; ++c) {
+                if (c >= nc) continue;
+                const double cc = flt_cost(keys[c * kFltLayers + h]);
+                if (cc < mcc[c]) mcc[c] = cc;
+                cost += mcc[c];
+            }
+            cs[(li - 1) * kFltRow + h - 1] = h >= fhigh && cost < kInf && h < T.L + 1 ? cost : kInf;
+        }
+        double best = kInf;
+        int top = 0;
+#pragma unroll 1
+        for (int h = on && li <= flow ? kFltRow : 0; h >= li; --h) {
+            const double v = cs[(li - 1) * kFltRow + h - 1];
+            if (v <= best) { best = v; top = h; }
+            cs[(li - 1) * kFltRow + h - 1] = best;
+            hs[(li - 1) * kFltRow + h - 1] = static_cast<unsigned char>(top);
+        }
+    }
+    __syncwarp();
+    double cst = kInf;
+    int low = 0;
+#pragma unroll 1
+    for (int l = 1; l <= (on ? min(li, flow) : 0); ++l) {
+        const double v = cs[(l - 1) * kFltRow + li - 1];
+        if (v < cst) { cst = v; low = l; }
+    }
+    if (low) {
+        // The cheapest candidate of every child slot inside the chosen range.
+        const int top = hs[(low - 1) * kFltRow + li - 1];
+        unsigned long long* chosen = W.best + size_t(W.coff[ii]) * kFltLayers;
+#pragma unroll 1
+        for (int c = 0; c < nc; ++c) {
+            double m = kInf;
+            unsigned long long bp = 0;
+#pragma unroll 1
+            for (int h = low; h <= top; ++h) {
+                const unsigned long long pv = keys[c * kFltLayers + h];
                 const double cc = flt_cost(pv);
-                if (cc < mcc[c]) { mcc[c] = cc; bp[c] = static_cast<unsigned long long>(static_cast<unsigned>(pv)) * kFltLayers + li; }
+                if (cc < m) { m = cc; bp = static_cast<unsigned long long>(static_cast<unsigned>(pv)) * kFltLayers + h; }
             }
-            if (li >= fhigh) {
-                double cost = via;
-                for (int c = 0; c < nc; ++c) cost += mcc[c];
-                if (cost < kInf && cost < cst[li]) {
-                    cst[li] = cost;
-                    for (int c = 0; c < nc; ++c) chosen[c][li] = bp[c];
-                    written |= 1u << li;
-                }
-            }
-        }
-#pragma unroll
-        for (int li = kFltLayers - 2; li >= 1; --li) {
-            if (li < low || li > T.L - 1) continue;
-            if (cst[li + 1] < cst[li]) {
-                cst[li] = cst[li + 1];
-                for (int c = 0; c < nc; ++c) chosen[c][li] = chosen[c][li + 1];
-                written |= 1u << li;
-            }
+            chosen[c * kFltLayers + li] = bp;
         }
     }
-#pragma unroll
-    for (int li = 0; li < kFltLayers; ++li) cst_g[li] = cst[li];
-    for (int c = 0; c < nc; ++c)
-#pragma unroll
-        for (int li = 0; li < kFltLayers; ++li)
-            if (written >> li & 1u) cbp[c * kFltLayers + li] = chosen[c][li];
-    const int pb = i ? F.pend[g - 1] : 0, pe = F.pend[g];
-    for (int e = eb + pb; e < eb + pe; ++e) {
-        const int par = nb + F.eparent[e], slot = F.eslot[e] % 10;
-        unsigned long long* ppk = F.packed + size_t(F.child_off[par]) * kFltLayers + slot * kFltLayers;
-        const int cp = F.coord[par], px = cp / T.Y % T.X, py = cp % T.Y;
-        const int minx = min(x, px), maxx = max(x, px), miny = min(y, py), maxy = max(y, py);
+    const int pb = on && ii ? W.pend[ii - 1] : 0, pe = on ? W.pend[ii] : 0;
+    if (on && pb == pe) {  // a root: its layer is chosen from its costs
+        F.costs[size_t(W.nb + ii) * kFltLayers + li] = cst;
+        if (li == 1) F.costs[size_t(W.nb + ii) * kFltLayers] = kInf;
+    }
+    // Offers to the parents' slots, lane = target layer; sources are the layers
+    // of the edge's direction (all of the target's parity).
+    for (int e = pb; __any_sync(kAll, e < pe); ++e) {
+        const bool live = e < pe;
+        const int par = live ? W.epar[e] : 0;
+        int pl, px, py;
+        cell_position(T, W.coord[par], pl, px, py);
+        const bool ay = ((li & 1) ^ T.DIR) == 1;  // 1-based layer index
+        const bool use = live && (ay ? y == py : x == px);
         const bool far = abs(x - px) + abs(y - py) > 4;
-        unsigned long long cache[kFltLayers];
-        for (int t = 0; t < kFltLayers; ++t) cache[t] = kFltInit;
+        double ce[(kFltRow + 1) / 2];
 #pragma unroll
-        for (int layer = 1; layer < kFltLayers; ++layer) {
-            const bool ay = ((layer & 1) ^ T.DIR) == 1;  // 1-based layer index
-            if (ay && y != py) continue;
-            if (!ay && x != px) continue;
-            const double cb = cst[layer];
-            for (int tl = 1 + (1 - layer % 2); tl < kFltLayers; tl += 2) {
-                double c2;
-                int choice = kFltStraight;
-                if (tl == layer) {
-                    c2 = cb + flt_wire(T, layer - 1, minx, maxx, miny, maxy);
-                } else if (far) {
-                    const int seq = (layer - 1) * 9 + (tl - 1);
-                    const double c_e = F.ce[size_t(e) * 81 + seq];
-                    if (!(c_e < kInf)) continue;
-                    c2 = cb + c_e;
-                    choice = seq;
-                } else {
-                    continue;
-                }
-                const unsigned long long v = flt_pack(static_cast<float>(c2), i * 100 + choice);
-                if (v < cache[tl]) cache[tl] = v;
-            }
+        for (int k = 0; k < (kFltRow + 1) / 2; ++k) {
+            const int layer = ((li - 1) & 1) + 1 + 2 * k;
+            ce[k] = use && far && layer != li && layer <= kFltRow
+                        ? F.ce[size_t(W.eb + e) * 81 + (layer - 1) * 9 + li - 1] : kInf;
         }
-        for (int tl = 1; tl < kFltLayers; ++tl) atomicMin(ppk + tl, cache[tl]);
+        unsigned long long offer = kFltInit;
+        if (use) {
+            const double c2 = cst + flt_wire(T, li - 1, min(x, px), max(x, px), min(y, py), max(y, py));
+            offer = min(offer, flt_pack(static_cast<float>(c2), ii * 100 + kFltStraight));
+        }
+#pragma unroll
+        for (int k = 0; k < (kFltRow + 1) / 2; ++k) {
+            const int layer = ((li - 1) & 1) + 1 + 2 * k;
+            const double cb = __shfl_sync(kAll, cst, (s0 + min(layer, kFltRow) - 1) & 31);
+            if (ce[k] < kInf)
+                offer = min(offer, flt_pack(static_cast<float>(cb + ce[k]), ii * 100 + (layer - 1) * 9 + li - 1));
+        }
+        if (live && offer != kFltInit)
+            atomicMin(W.packed + size_t(W.coff[par] + W.eslot[e] % 10) * kFltLayers + li, offer);
     }
+    __syncwarp();
 }
 
 // trace_flt_node (flt_block.cuh:144-331) for net-local node `i`: sets lo[i]
 // and writes up to 4 segments (8 words) into `w`; returns the word count.
-__device__ __forceinline__ int flt_trace_node(const Tables& T, const Flt& F, int nb, int eb, int i, int* w) {
-    const int g = nb + i;
-    const int c0 = F.coord[g];
-    const int cx = c0 / T.Y % T.X, cy = c0 % T.Y, l = c0 / T.XY;
-    const int pb = i ? F.pend[g - 1] : 0, pe = F.pend[g];
+__device__ __forceinline__ int flt_trace_node(const Tables& T, const Flt& F, const FltNet& W, int i, int* w) {
+    int l, cx, cy;
+    cell_position(T, W.coord[i], l, cx, cy);
+    const int pb = i ? W.pend[i - 1] : 0, pe = W.pend[i];
     int n = 0;
     int me;
     if (pb == pe) {
+        const double* costs = F.costs + size_t(W.nb + i) * kFltLayers;
         int ml = 0;
-        double mc = F.costs[size_t(g) * kFltLayers];
+        double mc = costs[0];
         for (int layer = 1; layer < kFltLayers; ++layer) {
-            const double v = F.costs[size_t(g) * kFltLayers + layer];
+            const double v = costs[layer];
             if (v < mc) { mc = v; ml = layer; }
         }
         me = ml;
     } else {
         int par_layer = -1, par_idx = -1, par_edge = -1;
         me = -1;
-        for (int e = eb + pb; e < eb + pe; ++e) {
-            const int pn = nb + F.eparent[e];
-            const int pl = F.lo[pn];
+        for (int e = pb; e < pe; ++e) {
+            const int pn = W.epar[e];
+            const int pl = W.lo[pn];
             if (pl <= 0) continue;
             par_idx = pn; par_edge = e; par_layer = pl;
-            const unsigned long long path = F.best[(size_t(F.child_off[pn]) + F.eslot[e] % 10) * kFltLayers + pl];
+            const unsigned long long path = W.best[size_t(W.coff[pn] + W.eslot[e] % 10) * kFltLayers + pl];
             const unsigned long long cidx = path / kFltLayers / 100, choice = (path / kFltLayers) % 100;
             if (cidx != static_cast<unsigned long long>(i)) { me = -1; continue; }
             me = choice == kFltStraight ? int(path % kFltLayers) : int(choice / 9 + 1);
-            const int cpp = F.coord[pn], px = cpp / T.Y % T.X, py = cpp % T.Y;
+            int pq, px, py;
+            cell_position(T, W.coord[pn], pq, px, py);
             const bool vert = px == cx && cy != py, horz = py == cy && cx != px;
             if (vert || horz) {
                 if (choice == kFltStraight) {
@@ -332,7 +409,7 @@ __device__ __forceinline__ int flt_trace_node(const Tables& T, const Flt& F, int
                     else { w[n++] = cell_index(T, ll, min(px, cx), py); w[n++] = cell_index(T, ll, max(px, cx), py); }
                 } else {
                     const int fl = int(choice / 9), tl = int(choice % 9);
-                    const int cp = F.bc[size_t(e) * 81 + fl * 9 + tl];
+                    const int cp = F.bc[size_t(W.eb + e) * 81 + fl * 9 + tl];
                     if (vert) {
                         w[n++] = cell_index(T, fl, cx, min(cy, cp)); w[n++] = cell_index(T, fl, cx, max(cy, cp));
                         w[n++] = cell_index(T, min(fl, tl), cx, cp); w[n++] = cell_index(T, max(fl, tl), cx, cp);
@@ -346,18 +423,17 @@ __device__ __forceinline__ int flt_trace_node(const Tables& T, const Flt& F, int
             }
             break;
         }
-        if (par_layer == -1) { F.lo[g] = -1; return 0; }
-        const unsigned long long path =
-            F.best[(size_t(F.child_off[par_idx]) + F.eslot[par_edge] % 10) * kFltLayers + par_layer];
-        if (path / kFltLayers / 100 != static_cast<unsigned long long>(i)) { F.lo[g] = -1; return 0; }
+        if (par_layer == -1) { W.lo[i] = -1; return 0; }
+        const unsigned long long path = W.best[size_t(W.coff[par_idx] + W.eslot[par_edge] % 10) * kFltLayers + par_layer];
+        if (path / kFltLayers / 100 != static_cast<unsigned long long>(i)) { W.lo[i] = -1; return 0; }
     }
-    F.lo[g] = me;
+    W.lo[i] = me;
     int minl = l + 1, maxl = (l + 1) == kFltLayers ? 1 : minl;
     minl = min(minl, me);
     maxl = max(maxl, me);
-    const int nc = F.children[g];
+    const int nc = W.children[i];
     for (int c = 0; c < nc; ++c) {
-        const int lc = int(F.best[(size_t(F.child_off[g]) + c) * kFltLayers + me] % kFltLayers);
+        const int lc = int(W.best[size_t(W.coff[i] + c) * kFltLayers + me] % kFltLayers);
         minl = min(lc, minl);
         maxl = max(lc, maxl);
     }
@@ -366,24 +442,25 @@ __device__ __forceinline__ int flt_trace_node(const Tables& T, const Flt& F, int
     return n;
 }
 
-// Route net `id` with one warp: tables, solve, trace into the phase-two
-// routes, then (if `commit`) its wire demand.  P2 is the phase-two view of the
-// plan (routes = routes2).  All 32 lanes call with the same id.
+// Route net `id` with one warp: solve, trace into the phase-two routes, then
+// (if `commit`) its wire demand.  P2 is the phase-two view of the plan (routes
+// = routes2).  All 32 lanes call with the same id; `smem`: the CTA's shared
+// memory (the warps' arenas, then their scratch).
 __device__ __forceinline__ void flt_net(const Tables& T, const Flt& F, const Plan& P2, int id, int stamp, int lane,
-                                        bool commit) {
-    const int nb = F.node_off[id], N = F.node_off[id + 1] - nb;
-    const int eb = F.edge_off[id];
-    if (N <= 0) return;
-    for (int k = lane; k < N * kFltLayers; k += 32) F.costs[size_t(nb) * kFltLayers + k] = kInf;
-    const int cb = F.child_off[nb], cn = F.child_off[nb + N - 1] + F.children[nb + N - 1] - cb;
-    for (int k = lane; k < cn * kFltLayers; k += 32) F.packed[size_t(cb) * kFltLayers + k] = kFltInit;
+                                        bool commit, char* smem) {
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    char* scratch = smem + size_t(nw) * kFltArena + size_t(warp) * kFltScratch;
+    const FltNet W = flt_open(F, id, smem + size_t(warp) * kFltArena, kFltArena, lane, 32);
+    if (W.N <= 0) return;
     __syncwarp();
     const int* lev = F.level + F.lvl_off[id];
     const int nl = F.lvl_off[id + 1] - F.lvl_off[id] - 1;
-    const int* ord = F.order + nb;
     for (int d = nl - 1; d >= 0; --d) {
-        for (int k = lev[d] + lane; k < lev[d + 1]; k += 32) flt_solve_node(T, F, nb, eb, ord[k]);
-        __syncwarp();
+        const int end = lev[d + 1];
+        for (int k = lev[d]; k < end; k += kFltSlots) {
+            const int at = k + lane / kFltRow;
+            flt_solve_group(T, F, W, at < end && lane < kFltSlots * kFltRow ? W.order[at] : -1, lane, scratch);
+        }
     }
     int* r = F.routes2 + P2.route_off[id];
     const long long cap = P2.route_off[id + 1] - P2.route_off[id];
@@ -393,7 +470,7 @@ __device__ __forceinline__ void flt_net(const Tables& T, const Flt& F, const Pla
         for (int base = lev[d]; base < lev[d + 1]; base += 32) {
             int w[8];
             int n = 0;
-            if (base + lane < lev[d + 1]) n = flt_trace_node(T, F, nb, eb, ord[base + lane], w);
+            if (base + lane < lev[d + 1]) n = flt_trace_node(T, F, W, W.order[base + lane], w);
             if (__any_sync(0xffffffffu, n < 0)) { bad = true; n = max(n, 0); }
             int off = n;
             for (int s = 1; s < 32; s <<= 1) {
@@ -417,27 +494,27 @@ __device__ __forceinline__ void flt_net(const Tables& T, const Flt& F, const Pla
     if (commit && !bad) commit_net_wires(T, P2, id, stamp, 1, lane);
 }
 
-// Route net `id` with the whole CTA: flt_net for nets whose DAG has a level
-// wider than a warp, the CTA's threads over a level's nodes.  The words go
-// out in the same order (level by level, ascending node index, each node's
-// wires before its via stack): a block scan of the words per node replaces
-// the warp scan.  All threads of the CTA call with the same id.
+// Route net `id` with the whole CTA: flt_net for nets with wide DAG levels, a
+// level's nodes dealt to the warps.  The words go out in the same order (level
+// by level, ascending node index, each node's wires before its via stack): a
+// block scan of the words per node replaces the warp scan.  All threads of the
+// CTA call with the same id.
 __device__ __forceinline__ void flt_net_block(const Tables& T, const Flt& F, const Plan& P2, int id, int stamp,
-                                              bool commit) {
+                                              bool commit, char* smem) {
     __shared__ int wsum[32];
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
-    const int nb = F.node_off[id], N = F.node_off[id + 1] - nb;
-    const int eb = F.edge_off[id];
-    if (N <= 0) return;
-    for (int k = tid; k < N * kFltLayers; k += nth) F.costs[size_t(nb) * kFltLayers + k] = kInf;
-    const int cb = F.child_off[nb], cn = F.child_off[nb + N - 1] + F.children[nb + N - 1] - cb;
-    for (int k = tid; k < cn * kFltLayers; k += nth) F.packed[size_t(cb) * kFltLayers + k] = kFltInit;
+    char* scratch = smem + size_t(nw) * kFltArena + size_t(warp) * kFltScratch;
+    const FltNet W = flt_open(F, id, smem, nw * kFltArena, tid, nth);
+    if (W.N <= 0) return;
     __syncthreads();
     const int* lev = F.level + F.lvl_off[id];
     const int nl = F.lvl_off[id + 1] - F.lvl_off[id] - 1;
-    const int* ord = F.order + nb;
     for (int d = nl - 1; d >= 0; --d) {
-        for (int k = lev[d] + tid; k < lev[d + 1]; k += nth) flt_solve_node(T, F, nb, eb, ord[k]);
+        const int end = lev[d + 1];
+        for (int k = lev[d] + kFltSlots * warp; k < end; k += kFltSlots * nw) {
+            const int at = k + lane / kFltRow;
+            flt_solve_group(T, F, W, at < end && lane < kFltSlots * kFltRow ? W.order[at] : -1, lane, scratch);
+        }
         __syncthreads();
     }
     int* r = F.routes2 + P2.route_off[id];
@@ -448,7 +525,7 @@ __device__ __forceinline__ void flt_net_block(const Tables& T, const Flt& F, con
         for (int base = lev[d]; base < lev[d + 1]; base += nth) {
             int w[8];
             int n = 0;
-            if (base + tid < lev[d + 1]) n = flt_trace_node(T, F, nb, eb, ord[base + tid], w);
+            if (base + tid < lev[d + 1]) n = flt_trace_node(T, F, W, W.order[base + tid], w);
             const bool neg = n < 0;
             n = max(n, 0);
             int off = n;  // inclusive scan inside the warp
@@ -482,6 +559,7 @@ __device__ __forceinline__ void flt_net_block(const Tables& T, const Flt& F, con
     }
     __syncthreads();
     if (commit && !bad) commit_net_wires(T, P2, id, stamp, 1, lane, warp, nw);
+    __syncthreads();  // the arrays are reused by the CTA's next net
 }
 
 }  // namespace grb

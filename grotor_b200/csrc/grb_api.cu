@@ -264,17 +264,18 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
 // --- FLT stage kernels (flt.cuh) --------------------------------------------
 constexpr int kFltThreads = 128;
 
-// One warp per net of batch b: layer-change tables, solve, trace, wires.
-// Blocks below `nw` take the batch's wide nets, a CTA each.
+// One warp per net of batch b: solve, trace, wires.  Blocks below `nw` take
+// the batch's wide nets, a CTA each.
 __global__ void __launch_bounds__(kFltThreads) k_flt_batch(Tables T, Flt F, Plan P2, int b, int stamp, int nw) {
+    extern __shared__ __align__(16) char smem[];
     const int lane = threadIdx.x & 31;
     const int lo = P2.batch_off[b], cnt = P2.batch_off[b + 1] - lo;
     if (int(blockIdx.x) < nw) {
-        flt_net_block(T, F, P2, P2.ids[F.border[lo + blockIdx.x]], stamp, true);
+        flt_net_block(T, F, P2, P2.ids[F.border[lo + blockIdx.x]], stamp, true, smem);
         return;
     }
     const int k = nw + (((blockIdx.x - nw) * blockDim.x + threadIdx.x) >> 5);
-    if (k < cnt) flt_net(T, F, P2, P2.ids[F.border[lo + k]], stamp, lane, true);
+    if (k < cnt) flt_net(T, F, P2, P2.ids[F.border[lo + k]], stamp, lane, true, smem);
 }
 
 // Layer-change tables of batch b's edges (flt_edges_batch).
@@ -288,7 +289,8 @@ __global__ void k_flt_edges(Tables T, Flt F, Plan P2, int b) {
 // FLT nets and wires -> vias, separated by bounded grid barriers
 // (flt.cuh:141-168 order).
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_flt_persistent(Tables T, Flt F, Plan P1, Plan P2,
-        GridSync S, int stamp0, int remove, int* work) {
+        GridSync S, int stamp0, int remove) {
+    extern __shared__ __align__(16) char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * (blockDim.x >> 5);
     PhaseClock clk;
@@ -310,16 +312,15 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_flt_persistent(Tables
         // The batch's wide nets a CTA each, from block 0; the others a warp
         // each, to global warps in block-major order over the remaining blocks
         // (warp 0 of every block first, so a batch's nets -- often fewer than
-        // the blocks -- land on different SMs, each with its L1 to itself for
-        // the nets' thread-local arrays).  With at least as many wide nets as
-        // blocks, every block takes wide nets in turn and then every warp the
+        // the blocks -- land on different SMs).  With at least as many wide nets
+        // as blocks, every block takes wide nets in turn and then every warp the
         // others.
         const int nw = F.nwide[b], G = gridDim.x, wpb = blockDim.x >> 5;
-        for (int k = blockIdx.x; k < nw; k += G) flt_net_block(T, F, P2, P2.ids[F.border[lo + k]], stamp, true);
+        for (int k = blockIdx.x; k < nw; k += G) flt_net_block(T, F, P2, P2.ids[F.border[lo + k]], stamp, true, smem);
         const int G2 = nw < G ? G - nw : G, b2 = nw < G ? int(blockIdx.x) - nw : int(blockIdx.x);
         if (b2 >= 0)
             for (int k = nw + warp * G2 + b2; k < cnt; k += G2 * wpb)
-                flt_net(T, F, P2, P2.ids[F.border[lo + k]], stamp, lane, true);
+                flt_net(T, F, P2, P2.ids[F.border[lo + k]], stamp, lane, true, smem);
         if (!grid_sync(S, T)) return;
         clk.mark(S, 5);
         commit_vias_strided(T, P2, P2.ids + lo, cnt, gwarp, nwarps, stamp, 1, lane);
@@ -1020,6 +1021,12 @@ static __device__ __align__(256) int g_noalloc_scratch[kNoAllocWords];
 // ---------------------------------------------------------------------------
 // Host context
 // ---------------------------------------------------------------------------
+// Until grb_set_flt_block_width is called the width follows the batch: while
+// every net can have a CTA to itself, one pays as soon as a level is more than
+// two rounds of a warp's kFltSlots nodes; beyond that only for the widest.
+constexpr int kFltWidthAuto = INT_MAX;
+constexpr int kFltNarrow = 2 * kFltSlots, kFltWide = 32;
+
 struct grb_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -1102,7 +1109,7 @@ struct grb_ctx {
     long long* used_sums = nullptr;
     int* used_pack = nullptr;
     std::vector<int> h_flt_width;     // per net: nodes of its widest DAG level
-    int flt_block_width = 32;         // wider nets are routed by a whole CTA (< 0: none)
+    int flt_block_width = kFltWidthAuto;  // wider nets are routed by a whole CTA (< 0: none)
     int* flt_border = nullptr;        // plan positions, each batch's wide nets first
     int* flt_nwide = nullptr;         // wide nets per batch
     long long flt_border_cap = 0, flt_nwide_cap = 0;
@@ -1661,8 +1668,8 @@ int flt_stage_plain(grb_ctx* c, int stamp0, int remove) {
         k_flt_edges<<<c->sms * 8, 256, 0, c->stream>>>(c->T, c->F, P2, b);
         c->launches += 1;
         const int nw = c->h_flt_nwide[b];
-        k_flt_batch<<<nw + (cnt - nw + kFltThreads / 32 - 1) / (kFltThreads / 32), kFltThreads, 0, c->stream>>>(
-            c->T, c->F, P2, b, stamp, nw);
+        k_flt_batch<<<nw + (cnt - nw + kFltThreads / 32 - 1) / (kFltThreads / 32), kFltThreads,
+                      (kFltThreads / 32) * (kFltArena + kFltScratch), c->stream>>>(c->T, c->F, P2, b, stamp, nw);
         prof_end(c, e);
         if ((rc = prof_begin(c, 6, &e))) return rc;
         k_commit_vias<<<cblocks, 128, 0, c->stream>>>(c->T, P2, b, stamp, 1);
@@ -1713,18 +1720,18 @@ int ensure_work(grb_ctx* c) {
 int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
     if (c->n_batches == 0) return GRB_OK;
     int per_sm = 0;
-    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, 0));
+    const size_t smem = size_t(kPersistentThreads / 32) * (kFltArena + kFltScratch);
+    GRB_CUDA(c, cudaFuncSetAttribute(k_flt_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent FLT kernel does not fit on an SM");
-    int rc = ensure_work(c);
-    if (rc) return rc;
     GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
     Tables T = c->T;
     Flt F = c->F;
     Plan P1 = make_plan(c), P2 = make_plan2(c);
     GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
-    void* args[] = {&T, &F, &P1, &P2, &S, &stamp0, &remove, &c->work};
+    void* args[] = {&T, &F, &P1, &P2, &S, &stamp0, &remove};
     GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_flt_persistent, dim3(per_sm * c->sms), dim3(kPersistentThreads),
-                                            args, 0, c->stream));
+                                            args, smem, c->stream));
     c->launches += 1;
     return GRB_OK;
 }
@@ -1973,18 +1980,11 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     // pass loads (and ignores) the wire costs there.
     GRB_CUDA(cp, cudaMemset(T.wcost, 0, sizeof(float) * slots));
     GRB_CUDA(cp, cudaMemset(cap, 0, sizeof(float) * slots));
-    {
-        std::vector<void*> up;
-        float* d_cap = nullptr;
-        if (dalloc(cp, &d_cap, cells, up)) { free_all(cp->owned); return GRB_ENOMEM; }
-        cudaError_t e = cudaMemcpy(d_cap, g->capacity, sizeof(float) * cells, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) {
-            k_layout<float, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, d_cap, cap, 0);
-            e = cudaDeviceSynchronize();
-        }
-        free_all(up);
-        GRB_CUDA(cp, e);
-    }
+    // Uploads in IDX order pass through the prefix table (8 bytes a slot), which
+    // the first refresh writes anew.
+    GRB_CUDA(cp, cudaMemcpy(T.presum, g->capacity, sizeof(float) * cells, cudaMemcpyHostToDevice));
+    k_layout<float, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, reinterpret_cast<const float*>(T.presum), cap, 0);
+    GRB_CUDA(cp, cudaGetLastError());
     GRB_CUDA(cp, cudaMemset(T.error, 0, 2 * sizeof(int)));
     {
         // Distinct capacity values (at most kNoCapRow of them get table rows;
@@ -2017,24 +2017,18 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
         T.of_dmax = caps.empty() ? 0 : kOfDmax;
         T.of_rows = rows;
         T.of_stride = kOfDmax;
-        std::vector<void*> up;
-        unsigned char* d_up = nullptr;
-        if (dalloc(cp, &d_cid, slots, cp->owned) || dalloc(cp, &d_up, cells, up) ||
+        if (dalloc(cp, &d_cid, slots, cp->owned) ||
             dalloc(cp, &d_table, size_t(T.L) * rows * T.of_stride, cp->owned) || dalloc(cp, &d_caps, rows, cp->owned)) {
-            free_all(up);
             free_all(cp->owned);
             return GRB_ENOMEM;
         }
         T.cap_id = d_cid;
         T.of_table = d_table;
-        cudaError_t e = cudaMemcpy(d_up, cid.data(), cells, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(d_cid, 0, slots);
-        if (e == cudaSuccess) {
-            k_layout<unsigned char, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, d_up, d_cid, 0);
-            e = cudaDeviceSynchronize();
-        }
-        free_all(up);
-        GRB_CUDA(cp, e);
+        unsigned char* up = reinterpret_cast<unsigned char*>(T.presum);
+        GRB_CUDA(cp, cudaMemcpy(up, cid.data(), cells, cudaMemcpyHostToDevice));  // (after the layout of the capacities)
+        GRB_CUDA(cp, cudaMemset(d_cid, 0, slots));
+        k_layout<unsigned char, true><<<layout_grid(T, T.L), dim3(32, 8)>>>(T, up, d_cid, 0);
+        GRB_CUDA(cp, cudaGetLastError());
         if (!caps.empty()) {
             GRB_CUDA(cp, cudaMemcpy(d_caps, caps.data(), sizeof(float) * caps.size(), cudaMemcpyHostToDevice));
             const int n = T.L * rows * T.of_stride;
@@ -2048,6 +2042,9 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
     GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_bucketed, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    GRB_CUDA(cp, cudaFuncSetAttribute(k_flt_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (kFltThreads / 32) * (kFltArena + kFltScratch)));
+    GRB_CUDA(cp, cudaDeviceSynchronize());  // the tables above were laid out on the default stream
     const int r = grb_reset(cp);
     if (r) { const int code = r; free_all(cp->owned); return code; }
     *out = c.release();
@@ -3180,7 +3177,7 @@ int grb_lshape_stage(grb_ctx* c, int32_t mode, grb_stats* stats) {
 
 int grb_set_flt_block_width(grb_ctx* c, int32_t width) {
     if (!c) return GRB_EINVAL;
-    c->flt_block_width = width;
+    c->flt_block_width = std::min(width, kFltWidthAuto - 1);
     return GRB_OK;
 }
 
@@ -3236,9 +3233,11 @@ int grb_flt_stage(grb_ctx* c, int32_t remove_phase_one, int32_t mode, grb_stats*
         std::vector<int> border(std::max(c->plan_n, 1)), nwide(std::max(c->n_batches, 1), 0);
         for (int b = 0; b < c->n_batches; ++b) {
             int w = c->h_batch_off[b];
+            const int limit = c->flt_block_width != kFltWidthAuto ? c->flt_block_width
+                              : c->h_batch_off[b + 1] - c->h_batch_off[b] <= 2 * c->sms ? kFltNarrow : kFltWide;
             for (int pass = 0; pass < 2; ++pass)
                 for (int k = c->h_batch_off[b]; k < c->h_batch_off[b + 1]; ++k) {
-                    const bool wide = c->flt_block_width >= 0 && c->h_flt_width[ids[k]] > c->flt_block_width;
+                    const bool wide = limit >= 0 && c->h_flt_width[ids[k]] > limit;
                     if (wide == (pass == 0)) border[w++] = k;
                     if (wide && pass == 0) ++nwide[b];
                 }

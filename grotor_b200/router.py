@@ -299,7 +299,8 @@ class Router:
 
     def set_flt_block_width(self, width: int):
         """Nets whose widest FLT DAG level holds more than `width` nodes are
-        routed by a whole CTA (default 32; negative: every net by one warp)."""
+        routed by a whole CTA (negative: every net by one warp).  Until this is
+        called the width follows each batch's size."""
         self._check(self._lib.grb_set_flt_block_width(self._ctx, int(width)))
 
     def read_routes2(self) -> np.ndarray:
@@ -430,8 +431,8 @@ class Router:
         return _stats_dict(st)
 
     # Batching: plain form raster / gather / solve / publish; persistent form
-    # publish / gather / solve, plus the waits and the raster it overlaps
-    # with the solve.  L-shape stage: the next four.
+    # a worker round / solve and the waits.  Stages: cost refresh (cost_pass1),
+    # DP, commit.
     PHASES = ("batch_raster", "batch_gather", "batch_solve", "batch_publish", "cost_pass1", "dp", "commit",
               "prefix_tree_pass2", "batch_solver_wait", "batch_worker_wait", "flt_edge_tables", "unused11",
               "net_ms_bucket0", "net_ms_bucket1", "net_ms_bucket2", "net_ms_bucket3",

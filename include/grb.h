@@ -248,9 +248,11 @@ int grb_upload_flt(grb_ctx* ctx, const grb_flt_dags* dags);
 int grb_flt_stage(grb_ctx* ctx, int32_t remove_phase_one, int32_t mode, grb_stats* stats);
 
 /* Nets whose widest FLT DAG level holds more than `width` nodes are solved
- * and traced by a whole CTA (its threads over a level's nodes), the others by
- * one warp each; routes, demand and statistics are the same either way.
- * Default 32; a negative width routes every net with one warp. */
+ * and traced by a whole CTA (a level's nodes dealt to its warps), the others
+ * by one warp each; routes, demand and statistics are the same either way.
+ * Until this is called the width follows the batch (6 while every net of the
+ * batch can have a CTA to itself, else 32); a negative width routes every net
+ * with one warp. */
 int grb_set_flt_block_width(grb_ctx* ctx, int32_t width);
 
 /* ---- Maze stage of the CUGR2 pipeline (pipeline_cugr2.hpp:90-117) -------- */
@@ -468,16 +470,15 @@ int grb_set_wait_limit(grb_ctx* ctx, double seconds);
  * group with CUDA events and the persistent kernels time each phase between
  * grid barriers (global timer, thread 0 of one block).  grb_phase_times
  * returns accumulated milliseconds per phase (up to 20 entries):
- * batching [0] raster (persistent: publish of the previous chunk), [1]
- * gather of forbidden colours and predecessors (persistent: gather of the
- * next chunk and raster of the one after), [2] in-chunk solve, [3] publish
- * (plain form only); stages [4] cost recompute of the dirty chunks with
- * prefix pass 1, [5] DP (persistent: + wire commit), [6] commit
- * (persistent: vias), [7] prefix trees and pass 2; persistent batching [8]
+ * batching [0] raster (persistent: unused), [1]
+ * gather of forbidden colours and predecessors (persistent: a whole round of
+ * the other blocks), [2] in-chunk solve, [3] publish
+ * (plain form only); stages [4] cost refresh, [5] DP (persistent: + wire
+ * commit), [6] commit (persistent: vias), [7] unused; persistent batching [8]
  * solver waiting for a gathered chunk, [9] other blocks waiting for a solved
  * chunk; [10] and [11] unused; persistent L-shape stage, per size bucket k of
  * the DP (tree nodes <= 2, <= 8, <= 16, more): [12+k] warp time summed over
- * its nets, [16+k] the longest single net (a maximum, not a sum).  The reference prints its stage timings as BATCH_TIMING /
+ * its packs, [16+k] the longest single pack (a maximum, not a sum).  The reference prints its stage timings as BATCH_TIMING /
  * DAG_TIMING records (router_state.hpp:259-264). */
 int grb_set_profiling(grb_ctx* ctx, int32_t on);
 int grb_phase_times(grb_ctx* ctx, double* ms, int32_t n, int32_t reset);
