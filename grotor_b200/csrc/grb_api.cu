@@ -807,8 +807,11 @@ __global__ void k_batch_publish(BatchState B, int s) {
 // before chunk r+1 (counter (3 + (r + 1)) * G).
 constexpr int kPersistThreads = kChunkMax;
 // A worker CTA's threads per task of a round: gather; publish; the others
-// raster, empty and set bits.
-constexpr int kGatherThreads = 320, kPublishThreads = 320;
+// raster, empty and set bits.  k_batch_persistent with gather/publish threads
+// of 256/256, 320/320, 448/192, 512/256, 576/256, 640/192, 640/256: 800x800x10
+// (900K nets) 8.3, 7.7, 7.3, 7.1, 7.0, 6.9, 7.0 ms; 1600x1600x10 (1.5M nets)
+// 20.2, 19.4, 20.1, 17.9, 18.4, 18.5, 20.8 ms.
+constexpr int kGatherThreads = 512, kPublishThreads = 256;
 template <int CH>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_batch_persistent(BatchState B, GridSync S, Tables T) {
     extern __shared__ __align__(16) unsigned bsm[];

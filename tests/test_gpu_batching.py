@@ -50,6 +50,21 @@ def test_medium_many_chunks(mode):
     r.close()
 
 
+@pytest.mark.parametrize("mode", ["plain", "persistent"])
+@pytest.mark.parametrize("n,limit", [(2500, 1000000), (2500, 3), (1250, 1000000), (240, 1000000)])
+def test_nets_that_all_meet(n, limit, mode):
+    """A grid so small that nearly every net meets every other: a colour per
+    net or so (few and many words of colours), chains of conflicts as long as a
+    chunk, with and without a tight limit."""
+    from grotor_b200 import Router
+    from grotor_b200.synth import WORKLOADS, Design
+    d = Design(WORKLOADS["small_64x64x5"].scaled(n, seed=33, X=9, Y=8, bbox_median=4.0))
+    r = Router(d.grid)
+    r.upload_nets(d.nets)
+    _check(r, d.order, d.nets, d.grid.X, d.grid.Y, limit, 1, mode)
+    r.close()
+
+
 @pytest.mark.parametrize("name", ["ref_64x64x10_2k", "ref_32x32x10_400"])
 def test_reference_geometry(name):
     """On the reference's own FLUTE geometry the GPU reproduces the
