@@ -193,9 +193,9 @@ __global__ void k_commit_vias(Tables T, Plan P, int b, int stamp, int K) {
 // refresh_cost (incremental_update.cuh:98-132) inside a persistent stage
 // kernel: every track by one warp, ended by a grid barrier.  False when the
 // barrier gave up.
-__device__ __forceinline__ bool refresh_persistent(const Tables& T, GridSync& S, PhaseClock& clk, int gwarp,
-                                                   int nwarps, int lane) {
-    for (int t = gwarp; t < T.tracks; t += nwarps) refresh_track<2>(T, t, lane);
+template <bool kListed>
+__device__ __forceinline__ bool refresh_persistent(const Tables& T, GridSync& S, PhaseClock& clk) {
+    refresh_tracks<2, kListed>(T);
     if (!grid_sync(S, T)) return false;
     clk.mark(S, 4);
     return true;
@@ -204,6 +204,8 @@ __device__ __forceinline__ bool refresh_persistent(const Tables& T, GridSync& S,
 // Persistent stage: every batch of the plan in one cooperative launch.
 // Per batch: refresh the tracks -> route and commit wires -> commit vias,
 // separated by bounded grid barriers.
+// kListed: refresh_tracks.
+template <bool kListed>
 __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tables T, Plan P, GridSync S,
         int stamp0, int nmax, size_t arena_b, char* gscratch, size_t gslot, int* work, DpTune tune, StageTail tail) {
     extern __shared__ __align__(16) char smem[];
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
     clk.start(S);
     for (int b = 0; b < P.n_batches; ++b) {
         const int stamp = stamp0 + b + 1;
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
+        if (!refresh_persistent<kListed>(T, S, clk)) return;
         // Route every net of the batch and commit its wires, in packs from the
         // largest size bucket down (long nets start first): the first pack of
         // every warp by its number, the others from the batch's work counter.
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_flt_persistent(Tables
             if (!grid_sync(S, T)) return;
             clk.mark(S, 6);
         }
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
+        if (!refresh_persistent<false>(T, S, clk)) return;
         flt_edges_batch(T, F, P2, b, gwarp, nwarps, lane);
         if (!grid_sync(S, T)) return;
         clk.mark(S, 10);
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_zshape_persistent(Tab
     for (int b = 0; b < P.n_batches; ++b) {
         const int lo = P.batch_off[b], cnt = P.batch_off[b + 1] - lo;
         const int stamp = stamp0 + b + 1;
-        if (!refresh_persistent(T, S, clk, gwarp, nwarps, lane)) return;
+        if (!refresh_persistent<false>(T, S, clk)) return;
         for (int k = blockIdx.x; k < cnt; k += gridDim.x) {  // one CTA per net
             zshape_net(T, Z, P, P.ids[lo + k], stamp, true, zsm);
             __syncthreads();
@@ -1777,9 +1779,12 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     const size_t ab = pack_arena_bytes(c->T.L, nmax);
     const int wpb = kPersistentThreads / 32;
     const size_t smem = std::max(ab * wpb, sizeof(float) * kViewTile * (kViewTile + 1));  // the tail's view tile
-    GRB_CUDA(c, cudaFuncSetAttribute(k_lshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    // Tracks enough for the refresh's list (refresh_tracks), at two CTAs per SM.
+    const bool listed = c->T.tracks > kListedPerWarp * 2 * c->sms * wpb;
+    const void* kernel = listed ? (const void*)k_lshape_persistent<true> : (const void*)k_lshape_persistent<false>;
+    GRB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
-    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lshape_persistent, kPersistentThreads, smem));
+    GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent kernel does not fit on an SM");
     const int blocks = per_sm * c->sms;
     const size_t slot = dp_slot_bytes(c);
@@ -1796,7 +1801,7 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     if ((rc = ensure_tail(c))) return rc;
     StageTail tail = make_tail(c);
     void* args[] = {&T, &P, &S, &stamp0, (void*)&nmax, (void*)&ab, &gs, (void*)&slot, &c->work, &tune, &tail};
-    GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_lshape_persistent, dim3(blocks), dim3(kPersistentThreads), args, smem, c->stream));
+    GRB_CUDA(c, cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kPersistentThreads), args, smem, c->stream));
     c->launches += 1;
     return GRB_OK;
 }
@@ -1899,7 +1904,7 @@ int grb_init_device(int32_t device) {
     }
     // Loading a kernel's code is deferred to its first use; these are the
     // kernels every stage starts with.
-    const void* kernels[] = {(const void*)k_batch_persistent<kChunkMax>, (const void*)k_lshape_persistent,
+    const void* kernels[] = {(const void*)k_batch_persistent<kChunkMax>, (const void*)k_lshape_persistent<false>,
                              (const void*)k_flt_persistent, (const void*)k_zshape_persistent,
                              (const void*)k_refresh_tracks, (const void*)k_lshape_bucketed, (const void*)k_topo_fill, (const void*)k_out_write};
     for (const void* k : kernels) {

@@ -89,3 +89,29 @@ def test_refresh_equals_recomputation(X, Y, L, DIR, skew):
             oracle.commit_batch(og, order[off[b]:off[b + 1]], nets.route_off, routes, step + 1, k, demand, ts, st)
         s = r.stats()
         assert s["wirelength"] == st["wirelength"] and s["vias"] == st["vias"]
+
+
+@pytest.mark.parametrize("X,Y", [(2500, 24), (8000, 16)])
+def test_listed_refresh_of_the_persistent_stage(X, Y):
+    """Grids with so many tracks that a persistent stage's CTAs list the dirty
+    ones (below and above what is listed at once): routes, demand and costs
+    equal the per-batch launches', which take every track in turn."""
+    from grotor_b200 import Router
+    from grotor_b200.synth import WORKLOADS, Design
+    d = Design(WORKLOADS["small_64x64x5"].scaled(4000, seed=78, X=X, Y=Y, cap_layers=11, cap_lo=1, cap_hi=4))
+    tracks = (d.grid.L + 1) // 2 * (X + Y)
+    assert tracks > 5 * 2 * 148 * 8 and (tracks > 128 * 2 * 148) == (X > 7000)
+    out = []
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order, 1000000)
+        for mode in ("plain", "persistent"):
+            r.reset()
+            st = r.lshape_route(mode)
+            r.refresh_cost()
+            out.append((r.read_routes(), r.read_tables(), st["wirelength"], st["vias"]))
+    (a, ta, wa, va), (b, tb, wb, vb) = out
+    np.testing.assert_array_equal(a, b)
+    for k in ta:
+        np.testing.assert_array_equal(ta[k], tb[k])
+    assert (wa, va) == (wb, vb)
