@@ -768,9 +768,9 @@ def softmin_measure(args, workload="softmin_320x320x10", taus=(1.0, 0.1, 0.01), 
         ba = bwd_bytes / (np.mean(bw) / 1e3) / 1e9
         out[f"tau_{tau:g}"] = {
             "forward_ms": float(np.mean(fw)), "backward_ms": float(np.mean(bw)), "total_cost": float(F.item()),
-            "roofline_forward": {"kernel": "k_soft_forward (+ tables, prefix)", "bound": "hbm", "achieved": fa,
+            "roofline_forward": {"kernel": "k_soft_packs (+ tables)", "bound": "hbm", "achieved": fa,
                                  "peak": peak, "unit": "GB/s", "frac": fa / peak, "peak_source": f"{kind} hbm_gbs"},
-            "roofline_backward": {"kernel": "k_soft_backward (+ tables, prefix, suffix, chain)", "bound": "hbm",
+            "roofline_backward": {"kernel": "k_soft_packs, adjoint (+ tables, chain)", "bound": "hbm",
                                   "achieved": ba, "peak": peak, "unit": "GB/s", "frac": ba / peak,
                                   "peak_source": f"{kind} hbm_gbs"}}
     r.close()
