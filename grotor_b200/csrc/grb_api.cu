@@ -1199,9 +1199,10 @@ struct grb_ctx {
     int bucket_cap = 0, bucket_batches = 0, bucket_version = -1;
     std::vector<int> h_bucket_off;  // [n_batches][kDpBuckets+1]
     DpTune tune{{4, 4, 4, 4}, {0, 0, 0, 0}};
-    // graph cache
+    // graph cache; the key names everything of the context that the captured
+    // launches hold by value (graph_key)
     cudaGraphExec_t graph = nullptr;
-    int graph_version = -1, graph_stamp = -1;
+    long long graph_key[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
     int64_t graph_kernels = 0;
     // timing
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1788,14 +1789,19 @@ int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
 }
 
 int stage_graph(grb_ctx* c, int stamp0) {
-    if (!c->graph || c->graph_version != c->plan_version || c->graph_stamp != stamp0) {
+    // Scratch must exist before capture (no allocation while capturing), and a
+    // kept graph runs on the scratch it was captured with: another executor's
+    // larger need may have replaced it since.
+    int maxcnt = 0;
+    for (int b = 0; b < c->n_batches; ++b) maxcnt = std::max(maxcnt, c->h_batch_off[b + 1] - c->h_batch_off[b]);
+    int rc = ensure_gscratch(c, maxcnt + 8);
+    if (!rc) rc = ensure_buckets(c);
+    if (rc) return rc;
+    const long long key[8] = {c->plan_version, stamp0, (long long)reinterpret_cast<uintptr_t>(c->gscratch),
+                              (long long)dp_slot_bytes(c), c->tune.per_cta[0], c->tune.per_cta[1], c->tune.per_cta[2],
+                              c->tune.per_cta[3]};
+    if (!c->graph || !std::equal(key, key + 8, c->graph_key)) {
         if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
-        // Scratch must exist before capture (no allocation while capturing).
-        int maxcnt = 0;
-        for (int b = 0; b < c->n_batches; ++b) maxcnt = std::max(maxcnt, c->h_batch_off[b + 1] - c->h_batch_off[b]);
-        int rc = ensure_gscratch(c, maxcnt + 8);
-        if (!rc) rc = ensure_buckets(c);
-        if (rc) return rc;
         const int64_t before = c->launches;
         const bool prof = c->profiling;
         c->profiling = false;
@@ -1811,8 +1817,7 @@ int stage_graph(grb_ctx* c, int stamp0) {
         if (ei != cudaSuccess) return cuda_fail(c, ei, "cudaGraphInstantiate");
         c->graph_kernels = c->launches - before;
         c->launches = before;
-        c->graph_version = c->plan_version;
-        c->graph_stamp = stamp0;
+        std::copy(key, key + 8, c->graph_key);
     }
     GRB_CUDA(c, cudaGraphLaunch(c->graph, c->stream));
     c->launches += c->graph_kernels;
@@ -3477,7 +3482,6 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
         for (int q = 0; q < kDpBuckets; ++q) c->tune.per_grab[q] = cands[pick][q];
     }
     c->profiling = prof;
-    c->graph_version = -1;  // a captured per-batch sequence bakes in the launch shapes
     if ((rc = grb_reset(c))) return rc;
     // Reported: the nets per pack of the plan's largest batch.
     int largest = 0;
