@@ -1100,6 +1100,7 @@ struct grb_ctx {
     // plan
     int *ids = nullptr, *batch_off = nullptr;
     int plan_n = 0, n_batches = 0, plan_cap = 0;
+    int plan_nets = 0;                // every id of the plan is below this
     std::vector<int> h_batch_off;
     int plan_version = 0;
     // scratch
@@ -1286,7 +1287,22 @@ Plan make_plan(const grb_ctx* c) {
     return P;
 }
 
-// The plan grouped by size bucket, rebuilt when the plan changes (one launch).
+// The plan outlives an upload of other nets (the same ids may be routed again)
+// but not the nets it names: with fewer nets now than the plan was made for,
+// its ids are looked at.
+int check_plan(grb_ctx* c) {
+    if (c->n_nets >= c->plan_nets || !c->plan_n) return GRB_OK;
+    std::vector<int> ids(c->plan_n);
+    GRB_CUDA(c, cudaMemcpyAsync(ids.data(), c->ids, sizeof(int) * c->plan_n, cudaMemcpyDeviceToHost, c->stream));
+    GRB_CUDA(c, cudaStreamSynchronize(c->stream));
+    const int top = *std::max_element(ids.begin(), ids.end()) + 1;
+    if (top > c->n_nets) return fail(c, GRB_EINVAL, "the plan names nets that are no longer uploaded");
+    c->plan_nets = top;
+    return GRB_OK;
+}
+
+// The plan grouped by size bucket, rebuilt when the plan or the nets change
+// (one launch).
 int ensure_buckets(grb_ctx* c) {
     if (c->bucket_version == c->plan_version && c->bucket_ids) return GRB_OK;
     if (c->bucket_cap < c->plan_n || c->bucket_batches < c->n_batches || !c->bucket_ids) {
@@ -2222,6 +2238,7 @@ static int validate_net_store(grb_ctx* c, int n, int nn, long long rw, int np, i
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
     c->flt_n = -1;  // FLT DAGs and Z-shape trees refer to the previous nets
     c->z_n = -1;
+    ++c->plan_version;  // so do the plan's size buckets and captured graphs
     if (status[0]) {
         static const char* what[] = {"", "offsets must be non-decreasing and within the arrays", "tree node outside the grid",
                                      "parents must precede children", "batching geometry outside the grid"};
@@ -2721,6 +2738,7 @@ int grb_plan_bbox_batches(grb_ctx* c, const int32_t* bbox, int32_t max_batch, in
     if (max_batch < 1 || max_batch > kMaxBoxBatch) return fail(c, GRB_EINVAL, "max_batch must be in [1, 256]");
     if (!bbox && c->z_n != c->n_nets) return fail(c, GRB_EINVAL, "no boxes given and no Z-shape trees uploaded");
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     const int n = c->plan_n, G = c->n_batches;
     if (n == 0) { if (n_batches) *n_batches = 0; return GRB_OK; }
     std::vector<void*> tmpb;
@@ -2961,6 +2979,7 @@ int grb_set_plan(grb_ctx* c, const int32_t* ids, int32_t n, const int32_t* batch
     GRB_CUDA(c, cudaMemcpyAsync(c->batch_off, batch_off, sizeof(int) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
     c->h_batch_off.assign(batch_off, batch_off + nb + 1);
     c->plan_n = n;
+    c->plan_nets = c->n_nets;
     c->n_batches = nb;
     ++c->plan_version;
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -3181,6 +3200,7 @@ int grb_plan_batches(grb_ctx* c, const int32_t* order, int32_t n, int32_t limit,
         c->batching_ms = ms;
         if ((rc = prof_collect(c))) return rc;
         c->plan_n = n;
+        c->plan_nets = c->n_nets;
         c->n_batches = nb;
         ++c->plan_version;
         if (n_batches) *n_batches = nb;
@@ -3198,12 +3218,14 @@ int grb_refresh_cost(grb_ctx* c) {
 int grb_route_batch(grb_ctx* c, int32_t b, int32_t stamp) {
     if (!c || b < 0 || b >= c->n_batches) return c ? fail(c, GRB_EINVAL, "batch out of range") : GRB_EINVAL;
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     return route_plain(c, b, stamp);
 }
 
 int grb_commit_batch(grb_ctx* c, int32_t b, int32_t stamp, int32_t K) {
     if (!c || b < 0 || b >= c->n_batches || (K != 1 && K != -1)) return c ? fail(c, GRB_EINVAL, "bad commit arguments") : GRB_EINVAL;
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     return commit_plain(c, b, stamp, K);
 }
 
@@ -3211,6 +3233,7 @@ int grb_lshape_stage(grb_ctx* c, int32_t mode, grb_stats* stats) {
     if (!c) return GRB_EINVAL;
     if (!c->node_off) return fail(c, GRB_EINVAL, "no nets uploaded");
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     const int stamp0 = c->stamp;
     GRB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     int rc;
@@ -3244,6 +3267,7 @@ int grb_flt_stage(grb_ctx* c, int32_t remove_phase_one, int32_t mode, grb_stats*
     if (!c) return GRB_EINVAL;
     if (c->flt_n != c->n_nets || c->flt_n < 0) return fail(c, GRB_EINVAL, "no FLT DAGs uploaded for the current nets");
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     std::vector<int> ids(c->plan_n);
     if (c->plan_n) {
         GRB_CUDA(c, cudaMemcpyAsync(ids.data(), c->ids, sizeof(int) * c->plan_n, cudaMemcpyDeviceToHost, c->stream));
@@ -3384,6 +3408,7 @@ int grb_zshape_stage(grb_ctx* c, int32_t mode, grb_stats* stats) {
     if (!c) return GRB_EINVAL;
     if (c->z_n != c->n_nets || c->z_n < 0) return fail(c, GRB_EINVAL, "no Z-shape trees uploaded for the current nets");
     GRB_CUDA(c, cudaSetDevice(c->device));
+    if (int rc = check_plan(c)) return rc;
     const int stamp0 = c->stamp;
     GRB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     int rc;
@@ -3422,7 +3447,8 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
     if (!c->node_off) return fail(c, GRB_EINVAL, "no nets uploaded");
     if (!c->n_batches) return fail(c, GRB_EINVAL, "no plan to tune on");
     GRB_CUDA(c, cudaSetDevice(c->device));
-    int rc = ensure_buckets(c);
+    int rc = check_plan(c);
+    if (!rc) rc = ensure_buckets(c);
     if (rc) return rc;
     const bool prof = c->profiling;
     c->profiling = false;

@@ -1,6 +1,7 @@
-"""A captured stage stays right when the context changes around it: scratch that
-another executor has replaced by a larger one.  The plain executor, which
-captures nothing, gives the expected routes."""
+"""A plan and what is derived from it -- size buckets, captured stages -- stay
+right when the context changes around them: scratch that another executor has
+replaced by a larger one; other nets uploaded under the same plan.  A fresh
+context's plain executor, which keeps nothing, gives the expected routes."""
 import numpy as np
 import pytest
 
@@ -48,3 +49,49 @@ def test_graph_after_the_scratch_grew(big_nets):
         r.generate_batches_rsmt(d.order, 1000000)
         for mode in ("graph", "persistent", "graph", "plain", "graph"):
             _same(_stage(r, mode), want)
+
+
+@pytest.mark.parametrize("mode", ["plain", "graph", "persistent"])
+def test_plan_kept_over_an_upload_of_other_nets(big_nets, mode):
+    """The same ids under the same plan, first with two-pin trees and then with
+    trees of up to dozens of nodes (other size buckets, other arenas)."""
+    from grotor_b200 import Router
+    from grotor_b200.synth import WORKLOADS, Design
+    small = Design(WORKLOADS["medium_320x320x10"].scaled(big_nets.nets.n, seed=46, two_pin_frac=1.0))
+    assert small.nets.n == big_nets.nets.n
+    ids = np.random.default_rng(1).permutation(small.nets.n).astype(np.int32)
+    off = np.array([0, 7, 200, len(ids)], np.int32)
+
+    def fresh(d):
+        with Router(d.grid) as r:
+            r.upload_nets(d.nets)
+            r.set_plan(ids, off)
+            return _stage(r, "plain")
+    with Router(big_nets.grid) as r:
+        r.upload_nets(small.nets)
+        r.set_plan(ids, off)
+        _stage(r, mode)
+        r.upload_nets(big_nets.nets)
+        _same(_stage(r, mode), fresh(big_nets))
+
+
+def test_plan_of_nets_that_are_gone(big_nets):
+    """Fewer nets than the plan names: every use of the plan is refused; a plan
+    whose ids are all still there is not."""
+    from grotor_b200 import GrbError, Router
+    from grotor_b200.synth import WORKLOADS, Design
+    d = big_nets
+    few = Design(WORKLOADS["medium_320x320x10"].scaled(50, seed=47, two_pin_frac=1.0))
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order, 1000000)
+        r.upload_nets(few.nets)
+        for call in (lambda: r.lshape_route("plain"), lambda: r.lshape_route("graph"),
+                     lambda: r.lshape_route("persistent"), lambda: r.route_batch(0, 1),
+                     lambda: r.commit_batch_demand(0, 1, 1), lambda: r.autotune()):
+            with pytest.raises(GrbError, match="no longer uploaded"):
+                call()
+        r.upload_nets(d.nets)
+        r.set_plan(np.arange(40, dtype=np.int32), np.array([0, 40], np.int32))
+        r.upload_nets(few.nets)
+        assert r.lshape_route("plain")["wirelength"] > 0
