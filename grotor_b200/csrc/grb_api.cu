@@ -1877,9 +1877,14 @@ int ensure_plan_capacity(grb_ctx* c, int n, int nb) {
     if (c->ids && n <= c->plan_cap && nb + 1 <= c->plan_cap + 1) {
         return GRB_OK;
     }
+    // The plan goes with its buffers: a call that is refused after this leaves
+    // the context without one.
     if (c->ids) cudaFree(c->ids);
     if (c->batch_off) cudaFree(c->batch_off);
     c->ids = nullptr; c->batch_off = nullptr;
+    c->plan_cap = c->plan_n = c->n_batches = 0;
+    c->h_batch_off.assign(1, 0);
+    ++c->plan_version;
     const int cap = std::max(n, 1);
     if (cudaMalloc(&c->ids, sizeof(int) * cap) != cudaSuccess ||
         cudaMalloc(&c->batch_off, sizeof(int) * (size_t(cap) + 1)) != cudaSuccess) {

@@ -95,3 +95,24 @@ def test_plan_of_nets_that_are_gone(big_nets):
         r.set_plan(np.arange(40, dtype=np.int32), np.array([0, 40], np.int32))
         r.upload_nets(few.nets)
         assert r.lshape_route("plain")["wirelength"] > 0
+
+
+@pytest.mark.parametrize("mode", ["plain", "graph", "persistent"])
+def test_refused_planning_leaves_no_plan_behind(big_nets, mode):
+    """A longer order than the plan's buffers hold, with an id that is not
+    uploaded: the buffers grow, the call is refused, and a stage then has
+    nothing to route."""
+    from grotor_b200 import GrbError, Router
+    d = big_nets
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order[:20], 1000000)
+        bad = d.order.copy()
+        bad[-1] = d.nets.n
+        with pytest.raises(GrbError, match="out of range"):
+            r.generate_batches_rsmt(bad, 1000000)
+        ids, off = r.plan()
+        assert len(ids) == 0 and off.tolist() == [0]
+        assert r.lshape_route(mode)["wirelength"] == 0
+        r.generate_batches_rsmt(d.order, 1000000)
+        assert r.lshape_route(mode)["wirelength"] > 0
