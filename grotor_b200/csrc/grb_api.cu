@@ -2197,6 +2197,21 @@ int grb_reset(grb_ctx* c) {
     return GRB_OK;
 }
 
+// The net store or a part of it is gone: no net id is accepted, and nothing
+// reads its arrays, until a valid upload.
+static void drop_nets(grb_ctx* c) {
+    free_all(c->net_bufs);
+    free_all(c->geom_bufs);
+    c->node_off = c->nodes = c->parents = c->routes = nullptr;
+    c->route_off = nullptr;
+    c->point_off = c->points = c->hseg_off = c->hsegs = c->vseg_off = c->vsegs = nullptr;
+    c->n_nets = c->max_nodes = 0;
+    c->route_words = 0;
+    c->topo_sizes[0] = -1;
+    c->flt_n = c->z_n = -1;
+    ++c->plan_version;
+}
+
 // Device buffers of the net store, reused while every array still fits
 // (need: nets, nodes, route words, points, h-segments, v-segments).
 static int net_buffers(grb_ctx* c, const long long need[6]) {
@@ -2221,7 +2236,7 @@ static int net_buffers(grb_ctx* c, const long long need[6]) {
     rc |= dalloc(c, &c->hsegs, 2 * size_t(nh), c->net_bufs);
     rc |= dalloc(c, &c->vseg_off, n + 1, c->net_bufs);
     rc |= dalloc(c, &c->vsegs, 2 * size_t(nv), c->net_bufs);
-    if (rc) { free_all(c->net_bufs); return fail(c, GRB_ENOMEM, "net buffers"); }
+    if (rc) { drop_nets(c); return fail(c, GRB_ENOMEM, "net buffers"); }
     for (int k = 0; k < 6; ++k) c->net_cap[k] = need[k];
     return GRB_OK;
 }
@@ -2248,6 +2263,7 @@ static int validate_net_store(grb_ctx* c, int n, int nn, long long rw, int np, i
         static const char* what[] = {"", "offsets must be non-decreasing and within the arrays", "tree node outside the grid",
                                      "parents must precede children", "batching geometry outside the grid"};
         c->n_nets = 0;  // no net id is accepted until a valid upload
+        c->route_words = 0;  // the route storage may be this upload's, smaller than the last one's
         c->topo_sizes[0] = -1;
         return fail(c, GRB_EINVAL, std::string(what[status[0]]) + " (item " + std::to_string(status[1]) + ")");
     }
@@ -2836,7 +2852,7 @@ int grb_upload_geometry(grb_ctx* c, const int32_t* point_off, const int32_t* poi
     rc |= dalloc(c, &d[3], 2 * size_t(hseg_off[n]), c->geom_bufs);
     rc |= dalloc(c, &d[4], n + 1, c->geom_bufs);
     rc |= dalloc(c, &d[5], 2 * size_t(vseg_off[n]), c->geom_bufs);
-    if (rc) { free_all(c->geom_bufs); return GRB_ENOMEM; }
+    if (rc) { drop_nets(c); return GRB_ENOMEM; }  // the geometry in use before went with geom_bufs
     for (int k = 0; k < 3; ++k) {
         GRB_CUDA(c, cudaMemcpyAsync(d[2 * k], offs[k], sizeof(int) * (n + 1), cudaMemcpyHostToDevice, c->stream));
         if (offs[k][n])

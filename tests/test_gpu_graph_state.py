@@ -116,3 +116,51 @@ def test_refused_planning_leaves_no_plan_behind(big_nets, mode):
         assert r.lshape_route(mode)["wirelength"] == 0
         r.generate_batches_rsmt(d.order, 1000000)
         assert r.lshape_route(mode)["wirelength"] > 0
+
+
+def test_upload_beyond_the_memory_leaves_no_nets_behind(big_nets):
+    """An upload whose route storage no GPU holds (2^44 words) is refused and
+    leaves the context without nets; a valid upload makes it usable again."""
+    from dataclasses import replace
+    from grotor_b200 import GrbError, Router
+    from grotor_b200._abi import GRB_ENOMEM
+    d = big_nets
+    too_much = d.nets.route_off.copy()
+    too_much[-1] = 1 << 44
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order, 1000000)
+        want = _stage(r, "plain")
+        ids, off = r.plan()
+        with pytest.raises(GrbError) as e:
+            r.upload_nets(replace(d.nets, route_off=too_much))
+        assert e.value.code == GRB_ENOMEM
+        r.reset()
+        for call in (lambda: r.lshape_route("plain"), lambda: r.lshape_route("persistent"), lambda: r.route_batch(0, 1),
+                     lambda: r.generate_batches_rsmt(d.order, 1000000)):
+            with pytest.raises(GrbError):
+                call()
+        r.upload_nets(d.nets)
+        r.set_plan(ids, off)
+        _same(_stage(r, "plain"), want)
+
+
+def test_refused_upload_with_less_route_storage(big_nets):
+    """An invalid upload of more nets than before with less route storage (the
+    buffers are replaced, then the trees are refused): a reset clears the storage
+    there is, not the last upload's."""
+    from grotor_b200 import GrbError, Router
+    from grotor_b200.router import NetArrays
+    d = big_nets
+    n = 2 * d.nets.n
+    z, e = np.zeros(n + 1, np.int32), np.zeros(0, np.int32)
+    bad = NetArrays(np.arange(n + 1, dtype=np.int32), np.full(n, -1, np.int32), np.full(n, -1, np.int32),
+                    np.zeros(n + 1, np.int64), z, e, z, e, z, e)
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        with pytest.raises(GrbError, match="outside the grid"):
+            r.upload_nets(bad)
+        r.reset()
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order, 1000000)
+        assert r.lshape_route("plain")["wirelength"] > 0
