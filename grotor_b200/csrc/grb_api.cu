@@ -2993,6 +2993,8 @@ int grb_set_plan(grb_ctx* c, const int32_t* ids, int32_t n, const int32_t* batch
     if (batch_off[0] != 0 || batch_off[nb] != n) return fail(c, GRB_EINVAL, "batch offsets must span the ids");
     for (int i = 0; i < n; ++i)
         if (ids[i] < 0 || ids[i] >= c->n_nets) return fail(c, GRB_EINVAL, "net id out of range");
+    for (int b = 0; b < nb; ++b)
+        if (batch_off[b] > batch_off[b + 1]) return fail(c, GRB_EINVAL, "batch offsets must not decrease");
     int rc = ensure_plan_capacity(c, n, nb);
     if (rc) return rc;
     if (nb + 1 > c->plan_cap + 1) return fail(c, GRB_EINVAL, "more batches than nets");

@@ -164,3 +164,14 @@ def test_refused_upload_with_less_route_storage(big_nets):
         r.upload_nets(d.nets)
         r.generate_batches_rsmt(d.order, 1000000)
         assert r.lshape_route("plain")["wirelength"] > 0
+
+
+@pytest.mark.parametrize("off", [[0, 60, 20, 40], [0, -1, 40], [0, 41, 40]])
+def test_plan_offsets_that_decrease_are_refused(big_nets, off):
+    from grotor_b200 import GrbError, Router
+    with Router(big_nets.grid) as r:
+        r.upload_nets(big_nets.nets)
+        with pytest.raises(GrbError, match="must not decrease"):
+            r.set_plan(np.arange(40, dtype=np.int32), np.array(off, np.int32))
+        r.set_plan(np.arange(40, dtype=np.int32), np.array([0, 20, 20, 40], np.int32))
+        assert r.lshape_route("plain")["wirelength"] > 0
