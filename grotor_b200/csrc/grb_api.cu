@@ -1169,7 +1169,7 @@ struct grb_ctx {
     std::vector<int> h_flt_nwide;
     int flt_version = 0;
     cudaGraphExec_t flt_graph = nullptr;
-    long long flt_graph_key[5] = {-1, -1, -1, -1, -1};
+    long long flt_graph_key[6] = {-1, -1, -1, -1, -1, -1};
     int64_t flt_graph_kernels = 0;
     // Z-shape stage (grb_upload_zshape)
     std::vector<void*> z_bufs;
@@ -1185,7 +1185,7 @@ struct grb_ctx {
     std::vector<int> h_z_node_off;
     int z_version = 0;
     cudaGraphExec_t z_graph = nullptr;
-    long long z_graph_key[3] = {-1, -1, -1};
+    long long z_graph_key[4] = {-1, -1, -1, -1};
     int64_t z_graph_kernels = 0;
     // soft-min workspace (grb_softmin_forward / backward)
     std::vector<void*> soft_bufs;
@@ -1201,9 +1201,9 @@ struct grb_ctx {
     std::vector<int> h_bucket_off;  // [n_batches][kDpBuckets+1]
     DpTune tune{{4, 4, 4, 4}, {0, 0, 0, 0}};
     // graph cache; the key names everything of the context that the captured
-    // launches hold by value (graph_key)
+    // launches hold by value
     cudaGraphExec_t graph = nullptr;
-    long long graph_key[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+    long long graph_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
     int64_t graph_kernels = 0;
     // timing
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1570,8 +1570,8 @@ int z_stage_plain(grb_ctx* c, int stamp0) {
 }
 
 int z_stage_graph(grb_ctx* c, int stamp0) {
-    const long long key[3] = {c->plan_version, c->z_version, stamp0};
-    if (!c->z_graph || !std::equal(key, key + 3, c->z_graph_key)) {
+    const long long key[4] = {c->plan_version, c->z_version, stamp0, c->T.int_wire};
+    if (!c->z_graph || !std::equal(key, key + 4, c->z_graph_key)) {
         if (c->z_graph) { cudaGraphExecDestroy(c->z_graph); c->z_graph = nullptr; }
         const int64_t before = c->launches;
         const bool prof = c->profiling;
@@ -1588,7 +1588,7 @@ int z_stage_graph(grb_ctx* c, int stamp0) {
         if (ei != cudaSuccess) return cuda_fail(c, ei, "cudaGraphInstantiate");
         c->z_graph_kernels = c->launches - before;
         c->launches = before;
-        std::copy(key, key + 3, c->z_graph_key);
+        std::copy(key, key + 4, c->z_graph_key);
     }
     GRB_CUDA(c, cudaGraphLaunch(c->z_graph, c->stream));
     c->launches += c->z_graph_kernels;
@@ -1749,8 +1749,8 @@ int flt_stage_plain(grb_ctx* c, int stamp0, int remove) {
 }
 
 int flt_stage_graph(grb_ctx* c, int stamp0, int remove) {
-    const long long key[5] = {c->plan_version, c->flt_version, stamp0, remove, c->flt_block_width};
-    if (!c->flt_graph || !std::equal(key, key + 5, c->flt_graph_key)) {
+    const long long key[6] = {c->plan_version, c->flt_version, stamp0, remove, c->flt_block_width, c->T.int_wire};
+    if (!c->flt_graph || !std::equal(key, key + 6, c->flt_graph_key)) {
         if (c->flt_graph) { cudaGraphExecDestroy(c->flt_graph); c->flt_graph = nullptr; }
         const int64_t before = c->launches;
         const bool prof = c->profiling;
@@ -1767,7 +1767,7 @@ int flt_stage_graph(grb_ctx* c, int stamp0, int remove) {
         if (ei != cudaSuccess) return cuda_fail(c, ei, "cudaGraphInstantiate");
         c->flt_graph_kernels = c->launches - before;
         c->launches = before;
-        std::copy(key, key + 5, c->flt_graph_key);
+        std::copy(key, key + 6, c->flt_graph_key);
     }
     GRB_CUDA(c, cudaGraphLaunch(c->flt_graph, c->stream));
     c->launches += c->flt_graph_kernels;
@@ -1813,10 +1813,10 @@ int stage_graph(grb_ctx* c, int stamp0) {
     int rc = ensure_gscratch(c, maxcnt + 8);
     if (!rc) rc = ensure_buckets(c);
     if (rc) return rc;
-    const long long key[8] = {c->plan_version, stamp0, (long long)reinterpret_cast<uintptr_t>(c->gscratch),
+    const long long key[9] = {c->plan_version, stamp0, c->T.int_wire, (long long)reinterpret_cast<uintptr_t>(c->gscratch),
                               (long long)dp_slot_bytes(c), c->tune.per_cta[0], c->tune.per_cta[1], c->tune.per_cta[2],
                               c->tune.per_cta[3]};
-    if (!c->graph || !std::equal(key, key + 8, c->graph_key)) {
+    if (!c->graph || !std::equal(key, key + 9, c->graph_key)) {
         if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
         const int64_t before = c->launches;
         const bool prof = c->profiling;
@@ -1833,7 +1833,7 @@ int stage_graph(grb_ctx* c, int stamp0) {
         if (ei != cudaSuccess) return cuda_fail(c, ei, "cudaGraphInstantiate");
         c->graph_kernels = c->launches - before;
         c->launches = before;
-        std::copy(key, key + 8, c->graph_key);
+        std::copy(key, key + 9, c->graph_key);
     }
     GRB_CUDA(c, cudaGraphLaunch(c->graph, c->stream));
     c->launches += c->graph_kernels;

@@ -1,9 +1,12 @@
 """A plan and what is derived from it -- size buckets, captured stages -- stay
 right when the context changes around them: scratch that another executor has
-replaced by a larger one; other nets uploaded under the same plan.  A fresh
+replaced by a larger one; other nets uploaded under the same plan; the other
+wire-cost rule.  A fresh
 context's plain executor, which keeps nothing, gives the expected routes."""
 import numpy as np
 import pytest
+
+from helpers import flt_by_net, golden_grid, golden_nets, load_golden
 
 pytestmark = pytest.mark.gpu
 
@@ -175,3 +178,63 @@ def test_plan_offsets_that_decrease_are_refused(big_nets, off):
             r.set_plan(np.arange(40, dtype=np.int32), np.array(off, np.int32))
         r.set_plan(np.arange(40, dtype=np.int32), np.array([0, 20, 20, 40], np.int32))
         assert r.lshape_route("plain")["wirelength"] > 0
+
+
+def _modes_in_turn(r, run):
+    """The graph executor under one wire-cost rule, the other, the first again:
+    each equals the plain executor under that rule, and the rules differ."""
+    want = {}
+    for rule in (False, True):
+        r.set_wire_cost_mode(rule)
+        want[rule] = run("plain")
+    assert not np.array_equal(want[False][0], want[True][0])
+    for rule in (False, True, False):
+        r.set_wire_cost_mode(rule)
+        _same(run("graph"), want[rule])
+
+
+def test_graph_after_a_wire_cost_mode_switch():
+    from grotor_b200 import Router
+    from grotor_b200.synth import WORKLOADS, Design
+    d = Design(WORKLOADS["small_64x64x5"].scaled(2500, seed=48, cap_lo=1, cap_hi=4))
+    with Router(d.grid) as r:
+        r.upload_nets(d.nets)
+        r.generate_batches_rsmt(d.order, 1000000)
+        _modes_in_turn(r, lambda mode: _stage(r, mode))
+
+
+def test_zshape_graph_after_a_wire_cost_mode_switch():
+    from grotor_b200 import Router
+    from grotor_b200.router import NetArrays
+    from grotor_b200.synth import WORKLOADS, Design
+    d = Design(WORKLOADS["small_64x64x5"].scaled(1500, seed=49, cap_lo=1, cap_hi=4))
+    n, z = d.nets, d.zshape_trees()
+    room = np.concatenate([[0], np.cumsum(1 + 64 * np.diff(z["node_off"]).astype(np.int64))])
+    nets = NetArrays(n.node_off, n.nodes, n.parents, room, n.point_off, n.points, n.hseg_off, n.hsegs, n.vseg_off, n.vsegs)
+
+    def run(mode):
+        r.reset()
+        st = r.zshape_route(mode)
+        return r.read_routes(), r.read_tables()["demand_half"], st["wirelength"], st["vias"]
+    with Router(d.grid) as r:
+        r.upload_nets(nets)
+        r.upload_zshape(z)
+        r.generate_batches_rsmt(d.order, 1000000)
+        r.plan_bbox_batches(250)
+        _modes_in_turn(r, run)
+
+
+def test_flt_graph_after_a_wire_cost_mode_switch():
+    from grotor_b200 import Router
+    g = load_golden("ref_flt_48x48x10_1500")
+    dags, _, route2_off = flt_by_net(g)
+
+    def run(mode):
+        r.reset()
+        st = r.flt_route(mode, remove_phase_one=False)
+        return r.read_routes2(), r.read_tables()["demand_half"], st["wirelength"], st["vias"]
+    with Router(golden_grid(g)) as r:
+        r.upload_nets(golden_nets(g))
+        r.upload_flt(dags, route2_off)
+        r.set_plan(g["flt_batch_ids"], g["flt_batch_off"])
+        _modes_in_turn(r, run)
