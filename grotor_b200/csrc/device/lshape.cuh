@@ -404,9 +404,10 @@ __host__ __device__ __forceinline__ size_t pack_arena_bytes(int L, int nmax) {
 }
 // Nodes a warp's shared-memory arena holds: 16, or what 16 warps' arenas of an
 // SM leave room for.
+constexpr size_t kPackSmemLimit = 220 * 1024;
 __host__ __device__ __forceinline__ int pack_nmax(int L) {
     int n = 16;
-    while (n > 2 && pack_arena_bytes(L, n) * 16 > 220 * 1024) --n;
+    while (n > 2 && pack_arena_bytes(L, n) * 16 > kPackSmemLimit) --n;
     return n;
 }
 __device__ __forceinline__ PackArena pack_arena(char* p, int L, int nmax) {

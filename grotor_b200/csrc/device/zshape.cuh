@@ -76,7 +76,7 @@ struct ZNet {
     int* via;        // [cnt][LY] via cost at the node
     int *pos, *pin, *child, *rep, *dep, *par, *lay;  // child [3 * cnt]; lay: chosen layer
 };
-__host__ __device__ __forceinline__ int znet_ints(int LY) { return 18 * LY + 10; }  // per node (even: 8-byte keys)
+__host__ __device__ constexpr int znet_ints(int LY) { return 18 * LY + 10; }  // per node (even: 8-byte keys)
 __device__ __forceinline__ ZNet znet(int* a, int cnt, int LY) {
     ZNet W;
     W.cnt = cnt; W.LY = LY;

@@ -1259,6 +1259,14 @@ void free_all(std::vector<void*>& v) {
     v.clear();
 }
 
+// Lets kernel `f` be launched with up to `bytes` of dynamic shared memory.  The
+// limit belongs to the function, not to a context, so `bytes` is always the most
+// that any context asks of it: a second context or thread that sets it again
+// changes nothing.
+cudaError_t allow_smem(const void* f, size_t bytes) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+}
+
 // Grid of k_layout over `layers` layers.
 dim3 layout_grid(const Tables& T, int layers) { return dim3((T.Y + 31) / 32, (T.X + 31) / 32, layers); }
 
@@ -1542,10 +1550,11 @@ int stage_plain(grb_ctx* c, int stamp0) {
 
 // --- Z-shape stage executors (pipeline_ggr.hpp:119-134) ---------------------
 int z_blocks(const grb_ctx* c) { return c->sms * 8; }  // CTAs with a scratch slot
-size_t z_smem(const grb_ctx* c) {
-    const int LY = c->Z.LAYER;
-    return sizeof(int) * (size_t(kZThreads / 32) * 2 * LY * LY + size_t(c->Z.fit) * znet_ints(LY));
+constexpr size_t z_smem_bytes(int LY, int fit) {
+    return sizeof(int) * (size_t(kZThreads / 32) * 2 * LY * LY + size_t(fit) * znet_ints(LY));
 }
+constexpr size_t kZSmemMax = z_smem_bytes(kMaxLayers + 1, kZFit);
+size_t z_smem(const grb_ctx* c) { return z_smem_bytes(c->Z.LAYER, c->Z.fit); }
 
 int z_stage_plain(grb_ctx* c, int stamp0) {
     const Plan P = make_plan(c);
@@ -1601,7 +1610,7 @@ int z_stage_persistent(grb_ctx* c, int stamp0) {
     if (c->n_batches == 0) return GRB_OK;
     int per_sm = 0;
     const size_t smem = z_smem(c);
-    GRB_CUDA(c, cudaFuncSetAttribute(k_zshape_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, allow_smem((const void*)k_zshape_persistent, kZSmemMax));
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent Z-shape kernel does not fit on an SM");
     GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
@@ -1671,7 +1680,8 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
     const int warps = sizeof(T) == 8 ? 3 : kSoftThreads / 32, span = std::min(16, std::max(1, n / (c->sms * 16)));
     const size_t smem = warps * soft_arena_values(c->T.L, nmax, kBackward) * sizeof(T);
     const long long blocks = (n + (long long)span * warps - 1) / ((long long)span * warps);
-    GRB_CUDA(c, cudaFuncSetAttribute(k_soft_packs<T, kBackward>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, allow_smem((const void*)k_soft_packs<T, kBackward>,
+                           warps * soft_arena_values(kMaxLayers, kPackNodes, kBackward) * sizeof(T)));
     k_soft_packs<T, kBackward><<<unsigned(blocks), 32 * warps, smem, c->stream>>>(c->T, S, make_plan(c), n, span, nmax, g);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
@@ -1789,7 +1799,7 @@ int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
     if (c->n_batches == 0) return GRB_OK;
     int per_sm = 0;
     const size_t smem = size_t(kPersistentThreads / 32) * (kFltArena + kFltScratch);
-    GRB_CUDA(c, cudaFuncSetAttribute(k_flt_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, allow_smem((const void*)k_flt_persistent, smem));
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent FLT kernel does not fit on an SM");
     GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
@@ -1849,7 +1859,7 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     // Tracks enough for the refresh's list (refresh_tracks), at two CTAs per SM.
     const bool listed = c->T.tracks > kListedPerWarp * 2 * c->sms * wpb;
     const void* kernel = listed ? (const void*)k_lshape_persistent<true> : (const void*)k_lshape_persistent<false>;
-    GRB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GRB_CUDA(c, allow_smem(kernel, kPackSmemLimit / 16 * wpb));
     int per_sm = 0;
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent kernel does not fit on an SM");
@@ -2117,13 +2127,12 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
             GRB_CUDA(cp, cudaDeviceSynchronize());
         }
     }
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_solve<kChunkMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_solve<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_batch_persistent<kChunkMax / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSolveSmemLimit)));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_lshape_bucketed, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GRB_CUDA(cp, cudaFuncSetAttribute(k_flt_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (kFltThreads / 32) * (kFltArena + kFltScratch)));
+    GRB_CUDA(cp, allow_smem((const void*)k_batch_solve<kChunkMax>, kSolveSmemLimit));
+    GRB_CUDA(cp, allow_smem((const void*)k_batch_solve<kChunkMax / 2>, kSolveSmemLimit));
+    GRB_CUDA(cp, allow_smem((const void*)k_batch_persistent<kChunkMax>, kSolveSmemLimit));
+    GRB_CUDA(cp, allow_smem((const void*)k_batch_persistent<kChunkMax / 2>, kSolveSmemLimit));
+    GRB_CUDA(cp, allow_smem((const void*)k_lshape_bucketed, 200 * 1024));
+    GRB_CUDA(cp, allow_smem((const void*)k_flt_batch, (kFltThreads / 32) * (kFltArena + kFltScratch)));
     GRB_CUDA(cp, cudaDeviceSynchronize());  // the tables above were laid out on the default stream
     const int r = grb_reset(cp);
     if (r) { const int code = r; free_all(cp->owned); return code; }
@@ -2744,8 +2753,7 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     Z.node_off = noff; Z.pos = dpos; Z.pin = dpin; Z.child = dch;
     Z.N = N; Z.NN = int(NN); Z.LAYER = LAYER; Z.D = T.DIR ^ 1;
     Z.by_n = fast_div(N); Z.by_nn = fast_div(Z.NN);
-    GRB_CUDA(c, cudaFuncSetAttribute(k_zshape_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(sizeof(int) * (size_t(kZThreads / 32) * 2 * LAYER * LAYER + size_t(Z.fit) * znet_ints(LAYER)))));
+    GRB_CUDA(c, allow_smem((const void*)k_zshape_batch, kZSmemMax));
     c->Z = Z;
     c->z_box = dbox;
     c->z_n = n;
