@@ -444,22 +444,33 @@ __device__ __forceinline__ SoftArena<T> soft_arena(T* p, int L, int nmax, bool b
     return A;
 }
 
-// A running soft minimum: m the least value, s the sum of exp(-(v - m) / tau).
-// add() returns what the adjoint needs: e = exp(-|difference| / tau) and
-// whether the added value became the minimum.
+// A candidate that exists: NaN, infinities and kSoftAbsent or more do not (smin).
+template <class T>
+__device__ __forceinline__ bool soft_exists(T v) { return v < static_cast<T>(kSoftAbsent); }
+
+// A running soft minimum: m the least value, s the sum of exp(-(v - m) / tau);
+// s = 0 while no value exists.  add() returns what the adjoint needs:
+// e = exp(-|difference| / tau), 0 for a value that does not exist, and whether
+// the added value became the minimum.
 template <class T>
 struct SoftRun {
     T m, s;
     __device__ __forceinline__ T add(T m2, T s2, T inv_tau, bool& less) {
         const T d = m2 - m;
-        less = d < 0;
-        const T e = s_exp<T>(-(less ? -d : d) * inv_tau);
-        s = less ? s * e + s2 : s + s2 * e;
+        const bool exists = soft_exists<T>(m2);
+        less = exists && d < 0;
+        const T e = exists ? s_exp<T>(-(less ? -d : d) * inv_tau) : static_cast<T>(0);
+        s = less ? s * e + s2 : exists ? s + s2 * e : s;
         m = less ? m2 : m;
         return e;
     }
-    __device__ __forceinline__ T value(T tau) const { return m - tau * s_log<T>(s); }
+    __device__ __forceinline__ T value(T tau) const {
+        return s > 0 ? m - tau * s_log<T>(s) : static_cast<T>(kSoftAbsent) * 10;
+    }
 };
+// Adjoint of a running sum: nothing reaches one that holds no value.
+template <class T>
+__device__ __forceinline__ T soft_share(T g, T s) { return s > 0 ? g / s : static_cast<T>(0); }
 
 // Forward DP of a pack (net_cost of its nets), and with kBackward the adjoint
 // of g * (their sum) into dP and dvc.  The loops over layers stay rolled, their
@@ -588,14 +599,14 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             }
             T diag = absent;
             if (act && straight) {
-                diag = reach;
+                if (soft_exists<T>(reach)) diag = reach;
             } else if (act) {
 #pragma unroll
                 for (int j = 0; j < NC; ++j) {
-                    v[j] = 2 * j + odd < L ? s_exp<T>(-(v[j] - dm) * inv) : static_cast<T>(0);  // from here on: weights
+                    v[j] = soft_exists<T>(v[j]) ? s_exp<T>(-(v[j] - dm) * inv) : static_cast<T>(0);  // from here on: weights
                     ds += v[j];
                 }
-                diag = dm < static_cast<T>(kSoftAbsent) ? dm - tau * s_log<T>(ds) : absent;
+                if (soft_exists<T>(dm)) diag = dm - tau * s_log<T>(ds);
             }
             // Row sl of the contribution: running soft minimum of diag[sl..hi].
             SoftRun<T> B{kNone, 0};
@@ -630,7 +641,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             for (int hi = act ? L - 1 : -1; hi >= sl; --hi) {
                 const T e = X[sl * L + hi];
                 const bool less = (bless >> hi) & 1u;
-                U += Gp[row + hi] / X2[sl * L + hi];
+                U += soft_share<T>(Gp[row + hi], X2[sl * L + hi]);
                 X[sl * L + hi] = less ? U : U * e;
                 U = less ? U * e : U;
             }
@@ -643,7 +654,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             T gcur = 0, gleg2 = 0;
             if (act && straight) gcur = gd;
             if (act && !straight) {
-                const T scale = ds > 0 ? gd / ds : static_cast<T>(0);
+                const T scale = soft_share<T>(gd, ds);
 #pragma unroll
                 for (int j = 0; j < NC; ++j) {
                     const int cl = 2 * j + odd;
@@ -684,7 +695,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             __syncwarp();
             // Column sl back to the rows' running minima (a row's sum at column
             // sl is in its lane's Rs), then row sl back to the ranges.
-            U = act ? gcur / C.s : static_cast<T>(0);
+            U = act ? soft_share<T>(gcur, C.s) : static_cast<T>(0);
 #pragma unroll 1
             for (int lo = act ? sl : -1; lo >= 0; --lo) {
                 const T e = Ce[lo], w = A.Y[size_t(32 + s0 + lo) * L + sl];
@@ -699,7 +710,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             for (int hi = sl; hi < (act ? L : 0); ++hi) {
                 const T e = Re[hi];
                 const bool less = (rless >> hi) & 1u;
-                U += X[sl * L + hi] / Rs[hi];
+                U += soft_share<T>(X[sl * L + hi], Rs[hi]);
                 Gi[row + hi] = less ? U : U * e;
                 U = less ? U * e : U;
             }
@@ -731,14 +742,14 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
         T part = 0;
 #pragma unroll 1
         for (int hi = sl; hi < (act ? L : 0); ++hi) {
-            const T w = s_exp<T>(-(Di[row + hi] - best) * inv);
+            const T w = soft_exists<T>(Di[row + hi]) ? s_exp<T>(-(Di[row + hi] - best) * inv) : static_cast<T>(0);
             X[sl * L + hi] = w;
             part += w;
         }
         T sum = 0;
 #pragma unroll 1
         for (int l = 0; l < L; ++l) sum += __shfl_sync(kAll, part, s0 + l);
-        const bool feasible = best < static_cast<T>(kSoftAbsent);
+        const bool feasible = soft_exists<T>(best);
         if (act && sl == 0 && S.net_cost) S.net_cost[id] = feasible ? best - tau * s_log<T>(sum) : absent;
         if (kBackward)
 #pragma unroll 1
