@@ -7,6 +7,7 @@
 #include <climits>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -1660,7 +1661,9 @@ Soft<T> soft_tables(grb_ctx* c, double tau, const void* cap, const void* uw, dou
     S.uw = a + slots;
     S.uv = static_cast<T>(uv);
     S.tau = static_cast<T>(tau);
-    S.inv_tau = static_cast<T>(1.0 / static_cast<double>(S.tau));
+    // Finite also for the smallest tau: a difference of 0 times it stays 0.
+    S.inv_tau = static_cast<T>(std::min(1.0 / static_cast<double>(S.tau),
+                                        static_cast<double>(std::numeric_limits<T>::max())));
     S.vc = a + 2 * slots; S.P = a + 3 * slots; S.dP = a + 4 * slots; S.dvc = a + 5 * slots;
     S.slot = reinterpret_cast<T*>(c->soft_slot);
     S.net_cost = net_cost;

@@ -1,7 +1,8 @@
 """Soft-min inputs that are not finite.  A candidate whose cost is NaN, infinite
 or at least 1e21 does not exist, whatever the size of its net: edges of infinite
 and of NaN unit wire cost (every run over or behind one on its track drops out)
-and an infinite via cost (only single-layer ranges are left).  In fp64 against
+and an infinite via cost (only single-layer ranges are left).  A temperature whose
+reciprocal is infinite is the hard minimum.  In fp64 against
 the dense reference with such candidates dropped from every minimum; 1e-9 on the
 cost and 1e-7 on the gradients as for finite inputs."""
 import numpy as np
@@ -76,3 +77,23 @@ def test_candidates_that_do_not_exist(kind, case, monkeypatch):
     for a, b in zip(got, want):
         assert bool(torch.isfinite(a).all())
         torch.testing.assert_close(a.cpu(), b.reshape(a.shape), rtol=1e-7, atol=1e-7 * float(b.abs().max()) + 1e-12)
+
+
+@pytest.mark.parametrize("dtype,tau", [(torch.float32, 1e-40), (torch.float64, 1e-310)])
+def test_temperature_below_the_reciprocal(dtype, tau):
+    """Below any difference of two costs of the working precision the soft minimum
+    is the hard one (ties apart: their count's logarithm is times tau)."""
+    from grotor_b200 import Router
+    from grotor_b200.softmin import routing_cost
+    d = _design("packs")
+    g = d.grid
+    rng = np.random.default_rng(10)
+    p = [torch.tensor(np.asarray(v, np.float64)) for v in (g.capacity.reshape(-1), rng.uniform(0.5, 1.5, g.cells), 2.0)]
+    want = R.total_cost(g, np.zeros(g.cells, np.int32), d.nets, *p, 0).item()
+    q = [v.to(dtype).cuda().requires_grad_(True) for v in p]
+    with Router(g) as r:
+        r.upload_nets(d.nets)
+        F = routing_cost(r, *q, tau)
+        got = torch.autograd.grad(F, q)
+    assert F.item() == pytest.approx(want, rel=1e-5 if dtype == torch.float32 else 1e-12)
+    assert all(bool(torch.isfinite(v).all()) for v in got)
