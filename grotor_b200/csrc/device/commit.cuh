@@ -22,8 +22,8 @@ __device__ __forceinline__ int net_words(const Plan& P, int id) {
 
 // A wire segment as its run of edges on a track: first slot and edge count
 // (n = 0: a single cell).  `skew`: the segment runs across its layer's
-// direction (no router emits that; a caller's own routes may), so its cells
-// are not consecutive.
+// direction or between two tracks (no router emits that; a caller's own routes
+// may), so its cells are not consecutive.
 struct WireRun {
     int first = 0, n = 0;
     bool wire = false, skew = false;
@@ -35,7 +35,7 @@ __device__ __forceinline__ WireRun run_between(const Tables& T, int l, int x0, i
     const bool ay = x0 == x1;
     const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
     R.n = hi - lo;
-    R.skew = R.n && ay != along_y(T, l);
+    R.skew = R.n && (ay != along_y(T, l) || (!ay && y0 != y1));
     R.first = slot_index(T, l, ay ? x0 : lo, ay ? lo : y0);
     R.length = ay ? T.ydist[hi] - T.ydist[lo] : T.xdist[hi] - T.xdist[lo];
     return R;

@@ -115,3 +115,36 @@ def test_listed_refresh_of_the_persistent_stage(X, Y):
     for k in ta:
         np.testing.assert_array_equal(ta[k], tb[k])
     assert (wa, va) == (wb, vb)
+
+
+@pytest.mark.parametrize("DIR", [0, 1])
+def test_segments_between_two_tracks(DIR):
+    """A caller's segment whose ends differ in x and in y, on layers of either
+    direction: both end cells are stamped where they are, the edges are those
+    along x at the first end's y, as the oracle commits them."""
+    from grotor_b200 import Router
+    from grotor_b200.router import NetArrays
+    rng = np.random.default_rng(DIR)
+    g = _grid(40, 37, 4, DIR, rng)
+    XY, n = g.X * g.Y, 30
+    rec = []
+    for _ in range(n):
+        l, (x0, x1), (y0, y1) = int(rng.integers(g.L)), rng.choice(g.X, 2, False), rng.choice(g.Y, 2, False)
+        rec.append([3, l * XY + x0 * g.Y + y0, l * XY + x1 * g.Y + y1])
+    routes = np.concatenate(rec).astype(np.int32)
+    z, e = np.zeros(n + 1, np.int32), np.zeros(0, np.int32)
+    nets = NetArrays(z, e, e, 3 * np.arange(n + 1, dtype=np.int64), z, e, z, e, z, e)
+    og, ids = orc_grid(g), np.arange(n, dtype=np.int32)
+    demand, ts = np.zeros(g.cells, np.int32), np.zeros(g.cells, np.int32)
+    st = {"wirelength": 0.0, "vias": 0}
+    with Router(g) as r:
+        r.upload_nets(nets)
+        r.set_plan(ids, np.arange(n + 1, dtype=np.int32))
+        r.write_routes_used(routes)
+        for b in range(n):
+            r.commit_batch_demand(b, b + 1, 1)
+            oracle.commit_batch(og, ids[b:b + 1], nets.route_off, routes, b + 1, 1, demand, ts, st)
+        t = r.read_tables()
+        np.testing.assert_array_equal(t["demand_half"], demand)
+        np.testing.assert_array_equal(t["timestamp"], ts)
+        assert r.stats()["wirelength"] == st["wirelength"]
