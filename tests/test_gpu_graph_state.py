@@ -232,7 +232,11 @@ def test_flt_graph_after_a_wire_cost_mode_switch():
     def run(mode):
         r.reset()
         st = r.flt_route(mode, remove_phase_one=False)
-        return r.read_routes2(), r.read_tables()["demand_half"], st["wirelength"], st["vias"]
+        routes = r.read_routes2()
+        for a, b in zip(route2_off[:-1], route2_off[1:]):  # words behind a route's own are an earlier run's
+            if b > a:
+                routes[a + routes[a]:b] = 0
+        return routes, r.read_tables()["demand_half"], st["wirelength"], st["vias"]
     with Router(golden_grid(g)) as r:
         r.upload_nets(golden_nets(g))
         r.upload_flt(dags, route2_off)

@@ -73,7 +73,7 @@ def test_candidates_that_do_not_exist(kind, case, monkeypatch):
         got = torch.autograd.grad(F, q)
     # A net without a route counts 1e22 each.
     lost = len(costs) - len(left)
-    assert F.item() == pytest.approx(float(total) + 1e22 * lost, rel=1e-9)
+    assert F.item() == pytest.approx(total.item() + 1e22 * lost, rel=1e-9)
     for a, b in zip(got, want):
         assert bool(torch.isfinite(a).all())
         torch.testing.assert_close(a.cpu(), b.reshape(a.shape), rtol=1e-7, atol=1e-7 * float(b.abs().max()) + 1e-12)
