@@ -557,24 +557,27 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
     int rank = 0;
     __shared__ int tight;
     while (true) {
-        // Jacobi sweeps until the colouring is a fixed point.
+        // Jacobi sweeps until the colouring is a fixed point.  A net may find no
+        // colour on the way, while its predecessors' are provisional: only the
+        // settled colouring says whether the colours suffice.
+        bool none = false;
         for (int sweep = 0;; ++sweep) {
             if (sweep == kSweeps && W == 8) {
-                if (!colours_in_order<CH>(S, m, fixed, pmask)) overflow = 1;
-                solve_sync<CH>();
+                none = !colours_in_order<CH>(S, m, fixed, pmask);
                 break;
             }
             int mine = tid < m ? S.col[tid] : -1;
             if (tid < m && tid >= fixed) {
                 mine = pmask ? first_fit<CH>(S, tid, W, pmask, c0) : c0;
-                if (mine >= C) { overflow = 1; mine = C - 1; }
+                none = mine >= C;
+                mine = min(mine, C - 1);
             }
             solve_sync<CH>();
             const bool changed = tid < m && S.col[tid] != mine;
             if (tid < m) S.col[tid] = mine;
             if (!solve_sync_or<CH>(changed)) break;
         }
-        if (overflow) break;
+        if (none) overflow = 1;
         // While no batch reaches its limit, no position inside a batch is
         // needed here (the rank pass after the run assigns them): the chunk's
         // nets are added to the per-colour totals.  Else the positions, in
@@ -584,6 +587,7 @@ __device__ __forceinline__ bool batch_solve(const BatchState& B, int s, bool loo
         const int c = tid < m ? S.col[tid] : -1 - lane;  // distinct dummies for idle lanes
         if (tid < m) atomicAdd(S.cnt + c, 1);
         solve_sync<CH>();
+        if (overflow) break;
         if (tid < m && S.cnt[c] > B.limit) tight = 1;
         solve_sync<CH>();
         const bool counted = !tight;

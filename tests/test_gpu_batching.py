@@ -94,3 +94,52 @@ def test_empty_and_single():
     bo, nb = r.generate_batches_rsmt(d.order[:1], 10)
     assert nb == 1 and bo.tolist() == [0]
     r.close()
+
+
+@pytest.mark.parametrize("mode", ["plain", "persistent"])
+def test_colours_that_run_out_only_on_the_way(mode):
+    """256 colours, 254 of them taken by earlier nets that all meet.  Of the next
+    chunk's nets a takes 254, e (meets a) 255, d (meets e) and b 254, c (meets b
+    and d) 255.  While d still counts with 255, c has no colour left; the colouring
+    that settles fits, so nothing is run again with more colours."""
+    from grotor_b200 import Router
+    from grotor_b200.router import GridArrays, NetArrays
+    X, Y, L = 64, 64, 3
+    g = GridArrays(L, X, Y, 1, 1.0, 2.0, np.ones(L), np.ones(X - 1, np.int32), np.ones(Y - 1, np.int32),
+                   np.ones(L * X * Y, np.float32))
+    row, meet = 40, 60  # the clique's marks run along y = row
+
+    def nets(edges):
+        points, marks = [], []
+        for _ in range(254):
+            points.append([2 * Y + 2])
+            marks.append([(0 * Y + row, (X - 1) * Y + row)])
+        while len(points) < 1024:  # the rest of the first chunk meets nothing
+            points.append([(20 + 4 * (len(points) % 8)) * Y + 10 + 3 * (len(points) // 8 % 7)])
+            marks.append([])
+        names = "aedbc"
+        for k, name in enumerate(names):
+            points.append([4 * (k + 1) * Y + row])
+            marks.append([])
+        for k, (u, v) in enumerate(edges):  # v looks where u marks
+            cell = 4 * (k + 1) * Y + meet
+            marks[1024 + names.index(u)].append((cell, cell))
+            points[1024 + names.index(v)].append(cell)
+        n = len(points)
+        off = lambda lists: np.cumsum([0] + [len(v) for v in lists]).astype(np.int32)
+        z, e = np.zeros(n + 1, np.int32), np.zeros(0, np.int32)
+        return NetArrays(z, e, e, np.zeros(n + 1, np.int64), off(points), np.concatenate(points).astype(np.int32), off(marks),
+                         np.array([c for m in marks for s in m for c in s], np.int32), z, e)
+    launches = []
+    for edges in (["ae", "ed", "bc", "dc"], ["ae", "ed", "bc"]):
+        m = nets(edges)
+        order = np.arange(m.n, dtype=np.int32)
+        with Router(g) as r:
+            r.upload_nets(m)
+            before = r.kernel_launches
+            _check(r, order, m, X, Y, 1000000, 1, mode)
+            launches.append(r.kernel_launches - before)
+            colours, _ = oracle.batches(X, Y, order, m.point_off, m.points, m.hseg_off, m.hsegs, m.vseg_off, m.vsegs,
+                                        1000000, 1)
+            assert colours[-5:].tolist() == [254, 255, 254, 254, 255]
+    assert launches[0] == launches[1]
