@@ -448,29 +448,26 @@ __device__ __forceinline__ SoftArena<T> soft_arena(T* p, int L, int nmax, bool b
 template <class T>
 __device__ __forceinline__ bool soft_exists(T v) { return v < static_cast<T>(kSoftAbsent); }
 
-// A running soft minimum: m the least value, s the sum of exp(-(v - m) / tau);
-// s = 0 while no value exists.  add() returns what the adjoint needs:
-// e = exp(-|difference| / tau), 0 for a value that does not exist, and whether
-// the added value became the minimum.
+// A running soft minimum: m the least value, s the sum of exp(-(v - m) / tau).
+// A value that does not exist counts as kSoftNone, far above those that do: it
+// weighs exactly 0 beside any of them, and nothing asks for the weights among
+// values none of which exists.  add() returns what the adjoint needs: e =
+// exp(-|difference| / tau) and whether the added value became the minimum.
+constexpr double kSoftNone = 1e30;
 template <class T>
 struct SoftRun {
     T m, s;
     __device__ __forceinline__ T add(T m2, T s2, T inv_tau, bool& less) {
+        m2 = soft_exists<T>(m2) ? m2 : static_cast<T>(kSoftNone);
         const T d = m2 - m;
-        const bool exists = soft_exists<T>(m2);
-        less = exists && d < 0;
-        const T e = exists ? s_exp<T>(-(less ? -d : d) * inv_tau) : static_cast<T>(0);
-        s = less ? s * e + s2 : exists ? s + s2 * e : s;
+        less = d < 0;
+        const T e = s_exp<T>(-(less ? -d : d) * inv_tau);
+        s = less ? s * e + s2 : s + s2 * e;
         m = less ? m2 : m;
         return e;
     }
-    __device__ __forceinline__ T value(T tau) const {
-        return s > 0 ? m - tau * s_log<T>(s) : static_cast<T>(kSoftAbsent) * 10;
-    }
+    __device__ __forceinline__ T value(T tau) const { return m - tau * s_log<T>(s); }
 };
-// Adjoint of a running sum: nothing reaches one that holds no value.
-template <class T>
-__device__ __forceinline__ T soft_share(T g, T s) { return s > 0 ? g / s : static_cast<T>(0); }
 
 // Forward DP of a pack (net_cost of its nets), and with kBackward the adjoint
 // of g * (their sum) into dP and dvc.  The loops over layers stay rolled, their
@@ -483,7 +480,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
     const int L = Tb.L, TT = tri_count(L);
     constexpr unsigned kAll = 0xffffffffu;
     const T absent = static_cast<T>(kSoftAbsent) * 10, tau = S.tau, inv = S.inv_tau;
-    constexpr T kNone = static_cast<T>(1e30);  // no value yet: above any sum of absent candidates
+    constexpr T kNone = static_cast<T>(kSoftNone);
     const int M = K.nodes;
     if (M == 0) return;
     int dep = K.par >= 0 ? 1 : 0;
@@ -641,7 +638,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             for (int hi = act ? L - 1 : -1; hi >= sl; --hi) {
                 const T e = X[sl * L + hi];
                 const bool less = (bless >> hi) & 1u;
-                U += soft_share<T>(Gp[row + hi], X2[sl * L + hi]);
+                U += Gp[row + hi] / X2[sl * L + hi];
                 X[sl * L + hi] = less ? U : U * e;
                 U = less ? U * e : U;
             }
@@ -654,7 +651,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             T gcur = 0, gleg2 = 0;
             if (act && straight) gcur = gd;
             if (act && !straight) {
-                const T scale = soft_share<T>(gd, ds);
+                const T scale = ds > 0 ? gd / ds : static_cast<T>(0);
 #pragma unroll
                 for (int j = 0; j < NC; ++j) {
                     const int cl = 2 * j + odd;
@@ -695,7 +692,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             __syncwarp();
             // Column sl back to the rows' running minima (a row's sum at column
             // sl is in its lane's Rs), then row sl back to the ranges.
-            U = act ? soft_share<T>(gcur, C.s) : static_cast<T>(0);
+            U = act ? gcur / C.s : static_cast<T>(0);
 #pragma unroll 1
             for (int lo = act ? sl : -1; lo >= 0; --lo) {
                 const T e = Ce[lo], w = A.Y[size_t(32 + s0 + lo) * L + sl];
@@ -710,7 +707,7 @@ __device__ __forceinline__ void soft_pack(const Tables& Tb, const Soft<T>& S, co
             for (int hi = sl; hi < (act ? L : 0); ++hi) {
                 const T e = Re[hi];
                 const bool less = (rless >> hi) & 1u;
-                U += soft_share<T>(X[sl * L + hi], Rs[hi]);
+                U += X[sl * L + hi] / Rs[hi];
                 Gi[row + hi] = less ? U : U * e;
                 U = less ? U * e : U;
             }
