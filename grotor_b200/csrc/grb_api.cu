@@ -552,9 +552,9 @@ __global__ void k_soft_tables(Tables Tb, Soft<T> S) {  // one warp per track
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t < Tb.tracks) soft_tables_track<T>(Tb, S, t, threadIdx.x & 31);
 }
-// Forward DP (net_cost) or adjoint of every net: a warp takes `span`
-// consecutive nets, as many at a time as its arena of nmax nodes holds; nets
-// beyond kPackNodes are walked by one thread in global scratch.
+// Forward DP (net_cost) or adjoint of every net of at most nmax nodes: a warp
+// takes `span` consecutive nets, as many at a time as its arena of nmax nodes
+// holds.
 template <class T, bool kBackward>
 __global__ void __launch_bounds__(kSoftThreads, 4) k_soft_packs(Tables Tb, Soft<T> S, Plan P, int n, int span, int nmax, T g) {
     extern __shared__ __align__(16) char smem[];
@@ -566,13 +566,7 @@ __global__ void __launch_bounds__(kSoftThreads, 4) k_soft_packs(Tables Tb, Soft<
     for (int at = int(min(first, (long long)n)); at < end;) {
         int incl = lane < 16 && at + lane < end ? P.node_off[at + lane + 1] - P.node_off[at] : 0x7fffffff;
         const int k = __popc(__ballot_sync(0xffffffffu, incl <= nmax));  // offsets do not decrease: the first k nets fit
-        if (!k) {
-            if (lane == 0) {
-                const int N = P.node_off[at + 1] - P.node_off[at];
-                T* dist = S.slot + size_t(2) * P.node_off[at] * Tb.L * Tb.L;
-                if (kBackward) soft_net_backward<T>(Tb, S, P, at, dist, dist + size_t(N) * Tb.L * Tb.L, g);
-                else S.net_cost[at] = soft_net_forward<T>(Tb, S, P, at, dist);
-            }
+        if (!k) {  // k_soft_wide's
             ++at;
             continue;
         }
@@ -582,6 +576,24 @@ __global__ void __launch_bounds__(kSoftThreads, 4) k_soft_packs(Tables Tb, Soft<
         __syncwarp();
         at += k;
     }
+}
+// The nets beyond nmax nodes, each by one thread in global scratch; a warp looks
+// at `span` consecutive nets, so that its wide ones run side by side.  Bound by
+// the longest net's chain of dependent local loads, so as many warps as the GPU
+// holds share the nets.  Forward and adjoint of 10K nets at 320x320x10, 4,690 of
+// them of 33 to 95 nodes, fp32 / fp64: 155 / 248 ms with 32 nets of any size a
+// warp, 202 / 362 where a warp of packs met them one after the other, 97 / 169
+// this way.  (On a stream beside the packs: 108 / 181 and less even.)
+template <class T, bool kBackward>
+__global__ void __launch_bounds__(kSoftThreads) k_soft_wide(Tables Tb, Soft<T> S, Plan P, int n, int span, int nmax, T g) {
+    const int lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long id = (long long)w * span + lane;
+    if (lane >= span || id >= n) return;
+    const int nb = P.node_off[id], N = P.node_off[id + 1] - nb;
+    if (N <= nmax) return;
+    T* dist = S.slot + size_t(2) * nb * Tb.L * Tb.L;
+    if (kBackward) soft_net_backward<T>(Tb, S, P, int(id), dist, dist + size_t(N) * Tb.L * Tb.L, g);
+    else S.net_cost[id] = soft_net_forward<T>(Tb, S, P, int(id), dist);
 }
 // Adjoints of the tracks' costs into gradients (one warp per track), and each
 // track's part of the via cost's.
@@ -1679,7 +1691,9 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
     const int n = c->n_nets;
     if (!n) return GRB_OK;
     const int nmax = std::min(kPackNodes, std::max(16, c->max_nodes));
-    // Three warps a CTA in fp64: two CTAs of the adjoint share an SM.
+    // Three warps a CTA in fp64: two CTAs of the adjoint share an SM while no net
+    // has more than 26 nodes (nine layers); a larger arena leaves one.  (20K nets of
+    // up to 31 nodes at 320x320x10: 12 ms forward and adjoint.)
     const int warps = sizeof(T) == 8 ? 3 : kSoftThreads / 32, span = std::min(16, std::max(1, n / (c->sms * 16)));
     const size_t smem = warps * soft_arena_values(c->T.L, nmax, kBackward) * sizeof(T);
     const long long blocks = (n + (long long)span * warps - 1) / ((long long)span * warps);
@@ -1688,6 +1702,13 @@ int soft_nets(grb_ctx* c, const Soft<T>& S, T g) {
     k_soft_packs<T, kBackward><<<unsigned(blocks), 32 * warps, smem, c->stream>>>(c->T, S, make_plan(c), n, span, nmax, g);
     c->launches += 1;
     GRB_CUDA(c, cudaGetLastError());
+    if (c->max_nodes > nmax) {
+        const int each = std::min(32, std::max(1, n / (c->sms * 16))), per = each * (kSoftThreads / 32);
+        k_soft_wide<T, kBackward><<<unsigned((n + (long long)per - 1) / per), kSoftThreads, 0, c->stream>>>(
+            c->T, S, make_plan(c), n, each, nmax, g);
+        c->launches += 1;
+        GRB_CUDA(c, cudaGetLastError());
+    }
     return GRB_OK;
 }
 
