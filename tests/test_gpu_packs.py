@@ -73,3 +73,37 @@ def test_packs_equal_oracle(case):
         np.testing.assert_array_equal(r.read_routes(), routes)
         np.testing.assert_array_equal(r.read_tables()["demand_half"], dem)
         assert sp["wirelength"] == st["wirelength"] and sp["vias"] == st["vias"]
+
+
+@pytest.mark.parametrize("cap_layers", [10, 6, 11])
+def test_trees_beyond_a_pack_equal_oracle(cap_layers):
+    """Trees of 17 to 32 nodes (packs in global scratch) and of more (the general
+    form, unrolled for nine layers), per batch and persistent."""
+    from grotor_b200 import Router
+    from grotor_b200.synth import WORKLOADS, Design
+    d = Design(WORKLOADS["small_64x64x5"].scaled(160, seed=79, X=60, Y=52, cap_layers=cap_layers, cap_lo=1, cap_hi=4,
+                                                max_pins=64, two_pin_frac=0.2, geo_p=0.05, bbox_median=25.0),
+               max_subnet_pins=64)
+    g, m = d.grid, d.nets
+    sizes = np.diff(m.node_off)
+    assert ((sizes > 16) & (sizes <= 32)).sum() > 10 and (sizes > 32).sum() > 10
+    with Router(g) as r:
+        r.upload_nets(m)
+        _, nb = r.generate_batches_rsmt(d.order, 1000000)
+        ids, off = r.plan()
+        for b in range(nb):
+            r.refresh_cost()
+            t = r.read_tables()
+            r.route_batch(b, b + 1)
+            mine, want = r.read_routes(), np.zeros(int(m.route_off[-1]), np.int32)
+            assert oracle.lshape_batch(orc_grid(g), t["vcost"], t["presum"], ids[off[b]:off[b + 1]], m.node_off, m.nodes,
+                                       m.parents, m.route_off, want) == 0
+            for i in ids[off[b]:off[b + 1]]:
+                a = m.route_off[i]
+                np.testing.assert_array_equal(mine[a:a + want[a]], want[a:a + want[a]], err_msg=f"net {i}, batch {b}")
+            r.commit_batch_demand(b, b + 1, 1)
+        routes, dem = r.read_routes(), r.read_tables()["demand_half"]
+        r.reset()
+        r.lshape_route("persistent")
+        np.testing.assert_array_equal(r.read_routes(), routes)
+        np.testing.assert_array_equal(r.read_tables()["demand_half"], dem)
