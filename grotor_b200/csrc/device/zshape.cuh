@@ -43,9 +43,11 @@ struct ZTrees {
     const int* pos;       // per node: x*N + y
     const int* pin;       // per node: pin layer + 1, -1 for Steiner points
     const int* child;     // [3 per node] net-local preorder index, -1 = none
-    int* scratch;         // per CTA: the arrays of a net beyond `fit` nodes
-    long long scratch_ints;
     int fit;              // nodes whose arrays fit the CTA's shared memory
+    int* scratch;         // the arrays of the nets beyond `fit` nodes
+    const int* wide_off;  // [n] nodes of the nets beyond `fit` before this one: a place
+                          // each; null: a place of `most` nodes per CTA
+    int most;             // nodes of the largest net
     int N, NN, LAYER, D;
     FastDiv by_n, by_nn;
 };
@@ -375,6 +377,12 @@ __device__ __forceinline__ int ztrace(const Tables& T, const ZTrees& Z, const ZN
     return status;
 }
 
+// Global scratch of net `id` (beyond Z.fit nodes).
+__device__ __forceinline__ int* zscratch(const ZTrees& Z, int id) {
+    const long long at = Z.wide_off ? Z.wide_off[id] : static_cast<long long>(blockIdx.x) * Z.most;
+    return Z.scratch + at * znet_ints(Z.LAYER);
+}
+
 // Route net `id` with the whole CTA; with `commit`, also its wire demand (warp
 // 0).  `smem`: the warps' node-DP ranges (2 * LAYER * LAYER ints each), then
 // the arrays of a net of Z.fit nodes.
@@ -394,7 +402,7 @@ __device__ __forceinline__ void zshape_net(const Tables& T, const ZTrees& Z, con
         return;
     }
     int* cand = smem + warp * 2 * LY * LY;
-    const ZNet W = znet(cnt <= Z.fit ? smem + nw * 2 * LY * LY : Z.scratch + blockIdx.x * Z.scratch_ints, cnt, LY);
+    const ZNet W = znet(cnt <= Z.fit ? smem + nw * 2 * LY * LY : zscratch(Z, id), cnt, LY);
     // reset_nodes (zshape.cuh:392-404), and everything of the net the DP reads.
     if (t == 0) zdeep = 0;
     for (int k = t; k < cnt * LY; k += nth) {

@@ -2759,11 +2759,30 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     rc |= dalloc(c, &dpin, nn, c->z_bufs);
     rc |= dalloc(c, &dch, 3 * nn, c->z_bufs);
     rc |= dalloc(c, &dbox, std::max(n, 1), c->z_bufs);
-    int most = 1;
-    for (int i = 0; i < n; ++i) most = std::max(most, t->node_off[i + 1] - t->node_off[i]);
-    Z.fit = std::min(most, kZFit);
-    Z.scratch_ints = most > Z.fit ? (long long)most * znet_ints(LAYER) : 0;
-    if (Z.scratch_ints) rc |= dalloc(c, &Z.scratch, size_t(z_blocks(c)) * Z.scratch_ints, c->z_bufs);
+    // Nets beyond the shared-memory arrays have a place each in global scratch, or
+    // where that is less, one of the largest net's size per CTA.
+    Z.most = 1;
+    long long wide = 0;  // their nodes
+    for (int i = 0; i < n; ++i) {
+        const int cnt = t->node_off[i + 1] - t->node_off[i];
+        Z.most = std::max(Z.most, cnt);
+        if (cnt > kZFit) wide += cnt;
+    }
+    Z.fit = std::min(Z.most, kZFit);
+    const long long per_cta = (long long)z_blocks(c) * Z.most;
+    std::vector<int> wide_off;
+    int* dwide = nullptr;
+    if (wide && wide <= per_cta && wide < INT_MAX) {
+        wide_off.resize(n);
+        long long at = 0;
+        for (int i = 0; i < n; ++i) {
+            const int cnt = t->node_off[i + 1] - t->node_off[i];
+            wide_off[i] = int(at);
+            if (cnt > kZFit) at += cnt;
+        }
+        rc |= dalloc(c, &dwide, n, c->z_bufs);
+    }
+    if (wide) rc |= dalloc(c, &Z.scratch, size_t(dwide ? wide : per_cta) * znet_ints(LAYER), c->z_bufs);
     if (rc) { free_all(c->z_bufs); c->Z = ZTrees{}; c->z_n = -1; return GRB_ENOMEM; }
     auto h2d = [&](void* dst, const void* src, size_t bytes) {
         return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
@@ -2773,8 +2792,9 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     GRB_CUDA(c, h2d(dpin, pin.data(), 4 * size_t(nn)));
     GRB_CUDA(c, h2d(dch, t->child, 12 * size_t(nn)));
     GRB_CUDA(c, h2d(dbox, box.data(), sizeof(int4) * box.size()));
+    GRB_CUDA(c, h2d(dwide, wide_off.data(), 4 * wide_off.size()));
     GRB_CUDA(c, cudaStreamSynchronize(c->stream));
-    Z.node_off = noff; Z.pos = dpos; Z.pin = dpin; Z.child = dch;
+    Z.node_off = noff; Z.pos = dpos; Z.pin = dpin; Z.child = dch; Z.wide_off = dwide;
     Z.N = N; Z.NN = int(NN); Z.LAYER = LAYER; Z.D = T.DIR ^ 1;
     Z.by_n = fast_div(N); Z.by_nn = fast_div(Z.NN);
     GRB_CUDA(c, allow_smem((const void*)k_zshape_batch, kZSmemMax));

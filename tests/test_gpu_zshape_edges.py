@@ -80,3 +80,42 @@ def test_bbox_rounds_equal_oracle(max_batch):
         assert nb == len(want)
         np.testing.assert_array_equal(np.diff(got), [len(w) for w in want])
         np.testing.assert_array_equal(ids, np.concatenate(want))
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_scratch_follows_the_large_nets(many):
+    """Nets of more than 96 nodes: a few of up to three hundred among small ones
+    take memory for their own arrays, not for one such net on every block; where
+    there are so many that a place per block is less, they share those."""
+    import torch
+    from grotor_b200 import Router
+    from grotor_b200.router import NetArrays
+    from grotor_b200.synth import WORKLOADS, Design
+    if many:
+        d = Design(WORKLOADS["small_64x64x5"].scaled(2400, seed=65, X=120, Y=120, cap_layers=4, two_pin_frac=0.0,
+                                                    geo_p=0.001, max_pins=100, bbox_median=40.0, cap_lo=900, cap_hi=900), max_subnet_pins=256)
+    else:
+        d = Design(WORKLOADS["small_64x64x5"].scaled(400, seed=64, X=90, Y=90, cap_layers=10, pin_model=1, max_pins=256,
+                                                    pareto_alpha=0.9, bbox_model=1, bbox_max=90), max_subnet_pins=256)
+    n, z = d.nets, d.zshape_trees()
+    zn = np.diff(z["node_off"]).astype(np.int64)
+    wide, blocks = zn[zn > 96], 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert (wide.sum() > blocks * zn.max()) == many and len(wide)
+    arrays = 4 * min(int(wide.sum()), int(blocks * zn.max())) * (18 * (d.grid.L + 1) + 10)
+    room = np.concatenate([[0], np.cumsum(1 + 64 * zn)]).astype(np.int64)
+    with Router(d.grid) as r:
+        r.upload_nets(NetArrays(n.node_off, n.nodes, n.parents, room, n.point_off, n.points, n.hseg_off, n.hsegs,
+                                n.vseg_off, n.vsegs))
+        before = torch.cuda.mem_get_info()[0]
+        r.upload_zshape(z)
+        taken = before - torch.cuda.mem_get_info()[0]
+        assert taken < arrays + (24 << 20), (taken, arrays)  # allocations come in 2 MiB pieces
+        r.generate_batches_rsmt(d.order, 1000000)
+        r.plan_bbox_batches(250)
+        out = []
+        for mode in ("persistent", "plain", "graph"):
+            r.reset()
+            r.zshape_route(mode)
+            out.append(r.read_routes())
+        np.testing.assert_array_equal(out[0], out[1])
+        np.testing.assert_array_equal(out[0], out[2])
