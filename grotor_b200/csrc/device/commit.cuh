@@ -35,7 +35,7 @@ __device__ __forceinline__ WireRun run_between(const Tables& T, int l, int x0, i
     const bool ay = x0 == x1;
     const int lo = ay ? min(y0, y1) : min(x0, x1), hi = ay ? max(y0, y1) : max(x0, x1);
     R.n = hi - lo;
-    R.skew = R.n && (ay != along_y(T, l) || (!ay && y0 != y1));
+    R.skew = along_y(T, l) ? x0 != x1 : y0 != y1;
     R.first = slot_index(T, l, ay ? x0 : lo, ay ? lo : y0);
     R.length = ay ? T.ydist[hi] - T.ydist[lo] : T.xdist[hi] - T.xdist[lo];
     return R;
