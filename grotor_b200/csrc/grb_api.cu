@@ -2009,9 +2009,10 @@ int grb_init_device(int32_t device) {
         return GRB_ECUDA;
     }
     // Loading a kernel's code is deferred to its first use; these are the
-    // kernels every stage starts with.
+    // kernels every stage starts with, the L-shape stage's in both its forms (the
+    // grid decides, and is not known here).
     const void* kernels[] = {(const void*)k_batch_persistent<kChunkMax>, (const void*)k_lshape_persistent<false>,
-                             (const void*)k_flt_persistent, (const void*)k_zshape_persistent,
+                             (const void*)k_lshape_persistent<true>, (const void*)k_flt_persistent, (const void*)k_zshape_persistent,
                              (const void*)k_refresh_tracks, (const void*)k_lshape_bucketed, (const void*)k_topo_fill, (const void*)k_out_write};
     for (const void* k : kernels) {
         cudaFuncAttributes a{};
