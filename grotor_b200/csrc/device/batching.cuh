@@ -425,8 +425,10 @@ __device__ __forceinline__ bool solve_sync_or(bool v) {
 // warp is final, and after a barrier the later warps add its colours to those
 // their nets may not take.  Each predecessor is looked at once, where a sweep
 // over the whole chunk looks at all of them again: for chunks whose nets depend
-// on one another in long chains (small grids).  For W == 8.  Leaves the colours
-// in S.col; false if a net finds none.
+// on one another in long chains (small grids).  For W == 8: a thread holds the
+// colours its net may not take in registers, twice over, and the CTA's 1024
+// threads have 64 registers each; designs that need more than 256 colours keep
+// the sweeps.  Leaves the colours in S.col; false if a net finds none.
 template <int CH>
 __device__ __forceinline__ bool colours_in_order(const SolveSmem& S, int m, int fixed, unsigned pmask) {
     constexpr int W = 8;

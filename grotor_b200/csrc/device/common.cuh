@@ -115,7 +115,7 @@ __host__ __device__ __forceinline__ int dp_bucket_nodes(int b) { return b == 0 ?
 // per-batch DP launch, nets per pack in the persistent form (0: by batch).
 struct DpTune {
     int per_cta[kDpBuckets];
-    int per_grab[kDpBuckets];
+    int per_pack[kDpBuckets];
 };
 
 __device__ __forceinline__ bool along_y(const Tables& T, int l) { return ((l & 1) ^ T.DIR) != 0; }
@@ -186,7 +186,6 @@ __device__ __forceinline__ unsigned range_bits(int w, int first, int last) {
 // callers return.  `epoch` counts this block's barriers (a kernel-local copy).
 struct GridSync {
     unsigned* count;
-    unsigned* generation;          // unused by the counter barrier
     unsigned long long timeout_ns;
     unsigned long long* phase_ns;  // optional per-phase time accumulators
     unsigned epoch;

@@ -316,9 +316,12 @@ __device__ __forceinline__ void refresh_track(const Tables& T, int t, int lane) 
 // i + gridDim.x, ...: warp w takes the w-th of every warps, or (kListed) the
 // CTA's warps list its dirty tracks first and take them from the list in turn.
 // A batch's nets dirty a minority of the tracks and by chance some warps'
-// shares are several times the mean: with 54 tracks a CTA (1600x1600x10) the
-// list takes the refresh from 122 to 99 us a batch; with 27 (800x800x10) it
-// costs what it evens out (33.6 us without, 34.0 with).
+// shares are several times the mean.  Refresh a batch without and with the list,
+// by tracks a warp (nine routing layers, 296 CTAs of 8 warps): 3.0 (800x800)
+// 33.9 and 29.9 us, 3.8 (1000x1000) 41.3 and 36.3, 4.4 (1150x1150) 56.7 and 45.8,
+// 4.9 (1300x1300) 65.1 and 54.4, 5.5 (1450x1450) 70.1 and 61.2, 6.1 (1600x1600)
+// 123 and 99.  The line was drawn between two sizes, before those in between were
+// measured: it is where the list certainly pays, not where it begins to.
 constexpr int kListTracks = 128;  // tracks of a CTA listed at once
 constexpr int kListedPerWarp = 5; // the list from this many tracks a warp on
 template <int kRounds, bool kListed>

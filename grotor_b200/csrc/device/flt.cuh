@@ -70,7 +70,8 @@ struct Flt {
     const int* eprefix;
     const int* emap;
     // per plan position, batch by batch: the batch's positions with its wide
-    // nets (a DAG level wider than a warp) first; per batch: its wide nets
+    // nets (those a CTA takes, grb_set_flt_block_width) first; per batch: its
+    // wide nets
     const int* border;
     const int* nwide;
 };

@@ -1,4 +1,5 @@
-// lshape.cuh -- L-shape pattern routing with layer assignment, one warp per net.
+// lshape.cuh -- L-shape pattern routing with layer assignment: a warp per pack of
+// small nets (route_pack), or per net beyond a pack (lshape_net).
 //
 // Semantics are those of the reference's tree DP (lshape_thread.cuh:18-171,
 // lshape_warp.cuh:8-247): per tree node a table dist[low][high] over layer
@@ -388,8 +389,8 @@ __device__ __forceinline__ void lshape_net(const Tables& T, const Plan& P, int i
 //     wherever those are exact (below), in place of a sum per candidate;
 //   * depths by pointer jumping, a depth's nodes by one ballot.
 // Same comparisons, tie-breaks, sums and emission order as lshape_net_l, so the
-// same routes.  Warp per net at 320x320x10, 120K nets: 5.8 ms of DP in 61
-// batches, the longest net 110 us; packs: PACK_MS.
+// same routes.  At 320x320x10, 120K nets, 63 batches: 5.8 ms of DP with a warp per
+// net, the longest net 110 us; 2.7 ms with packs, the longest of them 65 us.
 struct PackArena {
     double* dist;          // [nmax][TT] ranges; during a step the row minima; then what goes into the parent
     double* w1;            // [nmax][L] first leg (or straight) wire cost

@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 2) k_lshape_persistent(Tab
         int cn[kDpBuckets], g[kDpBuckets], last[kDpBuckets];  // last: end of the bucket's packs
 #pragma unroll
         for (int k = 0; k < kDpBuckets; ++k) cn[k] = bo[k + 1] - bo[k];
-        pack_sizes(cn, tune.per_grab, nwarps, nmax, g);
+        pack_sizes(cn, tune.per_pack, nwarps, nmax, g);
         int packs = 0;
 #pragma unroll
         for (int k = kDpBuckets - 1; k >= 0; --k) {
@@ -871,7 +871,10 @@ constexpr int kPersistThreads = kChunkMax;
 // raster, empty and set bits.  k_batch_persistent with gather/publish threads
 // of 256/256, 320/320, 448/192, 512/256, 576/256, 640/192, 640/256: 800x800x10
 // (900K nets) 8.3, 7.7, 7.3, 7.1, 7.0, 6.9, 7.0 ms; 1600x1600x10 (1.5M nets)
-// 20.2, 19.4, 20.1, 17.9, 18.4, 18.5, 20.8 ms.
+// 20.2, 19.4, 20.1, 17.9, 18.4, 18.5, 20.8 ms.  Whole batchings with 512/256,
+// 576/256, 640/192: 320x320x10 (120K) 1.99, 1.99, 2.00 ms, 800x800x10 8.97, 8.97,
+// 8.96, 1200x1200x10 (900K) 8.90, 8.86, 8.87, 1600x1600x10 23.1, 23.7, 23.9: the
+// split matters where the worker rounds are the longer side, on the large grid.
 constexpr int kGatherThreads = 512, kPublishThreads = 256;
 template <int CH>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_batch_persistent(BatchState B, GridSync S, Tables T) {
@@ -1087,7 +1090,11 @@ static __device__ __align__(256) int g_noalloc_scratch[kNoAllocWords];
 // ---------------------------------------------------------------------------
 // Until grb_set_flt_block_width is called the width follows the batch: while
 // every net can have a CTA to itself, one pays as soon as a level is more than
-// two rounds of a warp's kFltSlots nodes; beyond that only for the widest.
+// two rounds of a warp's kFltSlots nodes; beyond that only for the widest.  Stage
+// with widths 3, 6, 9, 12 and never, ms: 120x120x10 (180 nets, 13 batches) 1.83,
+// 1.91, 1.93, 1.93, 1.94; 200x200x10 (800, 24) 3.85, 4.05, 4.18, 4.21, 4.21;
+// 320x320x10 (2,400, 35) 6.79, 7.27, 7.34, 7.40, 7.40; 340x340x10 (400, 9) 1.54,
+// 1.63, 1.69, 1.69, 1.70.
 constexpr int kFltWidthAuto = INT_MAX;
 constexpr int kFltNarrow = 2 * kFltSlots, kFltWide = 32;
 
@@ -1123,7 +1130,7 @@ struct grb_ctx {
     size_t gscratch_bytes = 0;
     int* work = nullptr;
     int work_cap = 0;
-    unsigned* sync = nullptr;   // [count, generation]
+    unsigned* sync = nullptr;   // barrier arrivals
     // batching buffers
     unsigned *cellmask = nullptr, *fmask = nullptr, *fullmask = nullptr;
     unsigned* lmask[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // chunk-local masks
@@ -1437,7 +1444,7 @@ int refresh_plain(grb_ctx* c) {
 }
 
 // Batch b in the per-batch DP form: one launch for all its size buckets (or
-// only bucket `only` when only >= 0), each bucket with its tuned nets per CTA
+// only bucket `only` when only >= 0), each bucket with its tuned warps per CTA
 // and an arena sized to the bucket.
 int launch_buckets(grb_ctx* c, int b, int stamp, int only) {
     const int* bo = c->h_bucket_off.data() + size_t(b) * (kDpBuckets + 1);
@@ -1562,7 +1569,7 @@ int stage_plain(grb_ctx* c, int stamp0) {
 }
 
 // --- Z-shape stage executors (pipeline_ggr.hpp:119-134) ---------------------
-int z_blocks(const grb_ctx* c) { return c->sms * 8; }  // CTAs with a scratch slot
+int z_blocks(const grb_ctx* c) { return c->sms * 8; }  // most CTAs of a launch (ZTrees::most)
 constexpr size_t z_smem_bytes(int LY, int fit) {
     return sizeof(int) * (size_t(kZThreads / 32) * 2 * LY * LY + size_t(fit) * znet_ints(LY));
 }
@@ -1626,11 +1633,11 @@ int z_stage_persistent(grb_ctx* c, int stamp0) {
     GRB_CUDA(c, allow_smem((const void*)k_zshape_persistent, kZSmemMax));
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zshape_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent Z-shape kernel does not fit on an SM");
-    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
+    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, sizeof(unsigned), c->stream));
     Tables T = c->T;
     ZTrees Z = c->Z;
     Plan P = make_plan(c);
-    GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
+    GridSync S{c->sync, c->wait_ns, c->profiling ? c->d_phase : nullptr};
     void* args[] = {&T, &Z, &P, &S, &stamp0};
     GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_zshape_persistent, dim3(std::min(per_sm * c->sms, z_blocks(c))),
                                             dim3(kPersistentThreads), args, smem, c->stream));
@@ -1826,11 +1833,11 @@ int flt_stage_persistent(grb_ctx* c, int stamp0, int remove) {
     GRB_CUDA(c, allow_smem((const void*)k_flt_persistent, smem));
     GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flt_persistent, kPersistentThreads, smem));
     if (per_sm < 1) return fail(c, GRB_EINVAL, "persistent FLT kernel does not fit on an SM");
-    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
+    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, sizeof(unsigned), c->stream));
     Tables T = c->T;
     Flt F = c->F;
     Plan P1 = make_plan(c), P2 = make_plan2(c);
-    GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
+    GridSync S{c->sync, c->wait_ns, c->profiling ? c->d_phase : nullptr};
     void* args[] = {&T, &F, &P1, &P2, &S, &stamp0, &remove};
     GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_flt_persistent, dim3(per_sm * c->sms), dim3(kPersistentThreads),
                                             args, smem, c->stream));
@@ -1893,10 +1900,10 @@ int stage_persistent(grb_ctx* c, int stamp0) {
     if (rc) return rc;
     if ((rc = ensure_buckets(c))) return rc;
     if ((rc = ensure_work(c))) return rc;
-    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
+    GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, sizeof(unsigned), c->stream));
     Tables T = c->T;
     Plan P = make_plan(c);
-    GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr};
+    GridSync S{c->sync, c->wait_ns, c->profiling ? c->d_phase : nullptr};
     char* gs = c->gscratch;
     DpTune tune = c->tune;
     if ((rc = ensure_tail(c))) return rc;
@@ -1938,8 +1945,8 @@ static int launch_batching(grb_ctx* c, BatchState& B, int mode, size_t smem) {
     if (mode == GRB_MODE_PERSISTENT)
         GRB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persistent<CH>, kPersistThreads, smem));
     if (mode == GRB_MODE_PERSISTENT && per_sm * c->sms >= 2) {
-        GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned), c->stream));
-        GridSync S{c->sync, c->sync + 1, c->wait_ns, c->profiling ? c->d_phase : nullptr, 0};
+        GRB_CUDA(c, cudaMemsetAsync(c->sync, 0, sizeof(unsigned), c->stream));
+        GridSync S{c->sync, c->wait_ns, c->profiling ? c->d_phase : nullptr, 0};
         Tables T = c->T;
         void* args[] = {&B, &S, &T};
         GRB_CUDA(c, cudaLaunchCooperativeKernel((void*)k_batch_persistent<CH>, dim3(per_sm * c->sms), dim3(kPersistThreads),
@@ -2031,7 +2038,9 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
         !g->unit_length_short_costs || !g->x_edge_len || !g->y_edge_len)
         return GRB_EINVAL;
     if (size_t(g->L) * g->X * g->Y >= (size_t(1) << 31)) return GRB_EINVAL;
-    if (std::max(g->X, g->Y) > 8192) return GRB_EINVAL;  // prefix tree depth (kChunkPos << 8)
+    // The longest track whose block totals the refresh's stack holds (cost.cuh).
+    static_assert((kScanBlock << kScanLevels) == 8192, "ScanStack");
+    if (std::max(g->X, g->Y) > (kScanBlock << kScanLevels)) return GRB_EINVAL;
     auto c = std::make_unique<grb_ctx>();
     c->device = device;
     GRB_CUDA(c.get(), cudaSetDevice(device));
@@ -2077,7 +2086,7 @@ int grb_create(const grb_grid* g, int32_t device, grb_ctx** out) {
     rc |= dalloc(cp, &T.wirelength, 1, cp->owned);
     rc |= dalloc(cp, &T.vias, 1, cp->owned);
     rc |= dalloc(cp, &T.error, 2, cp->owned);
-    rc |= dalloc(cp, &c->sync, 2, cp->owned);
+    rc |= dalloc(cp, &c->sync, 1, cp->owned);
     if (rc) { free_all(cp->owned); return GRB_ENOMEM; }
     T.error_info = T.error + 1;
     T.short_costs = sc; T.xlen = xl; T.ylen = yl; T.capacity = cap; T.xdist = xd; T.ydist = yd;
@@ -2723,6 +2732,7 @@ int grb_upload_zshape(grb_ctx* c, const grb_zshape_trees* t) {
     const int n = c->n_nets, XY = T.XY;
     const int N = std::max(T.X, T.Y), LAYER = T.L + 1;
     const long long NN = (long long)N * N, LNN = LAYER * NN;
+    // Back-pointers are plane indexes; the limit is the one the planes had.
     if (16 * LNN >= (1ll << 31)) return fail(c, GRB_EINVAL, "Z-shape planes exceed 32-bit indexing");
     if (t->node_off[0] != 0) return fail(c, GRB_EINVAL, "Z-shape offsets must start at 0");
     for (int i = 0; i < n; ++i) if (t->node_off[i + 1] < t->node_off[i]) return fail(c, GRB_EINVAL, "Z-shape offsets must be non-decreasing");
@@ -3531,7 +3541,7 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
     if (what & 1) {
         // Per-batch DP form: coordinate descent over the buckets -- for each
         // bucket in turn, time the whole per-batch launch of the three largest
-        // batches with each nets-per-CTA choice (DP only, on refreshed tables).
+        // batches with each choice of warps per CTA (DP only, on refreshed tables).
         if ((rc = refresh_plain(c))) { c->profiling = prof; return rc; }
         std::vector<int> order(c->n_batches);
         for (int b = 0; b < c->n_batches; ++b) order[b] = b;
@@ -3570,7 +3580,7 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
         float best = 1e30f;
         int pick = 0;
         for (int k = 0; k < kCands; ++k) {
-            for (int q = 0; q < kDpBuckets; ++q) c->tune.per_grab[q] = cands[k][q];
+            for (int q = 0; q < kDpBuckets; ++q) c->tune.per_pack[q] = cands[k][q];
             if ((rc = grb_reset(c))) { c->profiling = prof; return rc; }
             GRB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
             if ((rc = stage_persistent(c, 0))) { c->profiling = prof; return rc; }
@@ -3581,7 +3591,7 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
             if ((rc = check_device_error(c))) { c->profiling = prof; return rc; }
             if (t < best) { best = t; pick = k; }
         }
-        for (int q = 0; q < kDpBuckets; ++q) c->tune.per_grab[q] = cands[pick][q];
+        for (int q = 0; q < kDpBuckets; ++q) c->tune.per_pack[q] = cands[pick][q];
     }
     c->profiling = prof;
     if ((rc = grb_reset(c))) return rc;
@@ -3594,7 +3604,7 @@ int grb_autotune(grb_ctx* c, int32_t what, int32_t* per_cta, int32_t* per_grab) 
         const int* bo = c->h_bucket_off.data() + size_t(largest) * (kDpBuckets + 1);
         cn[q] = bo[q + 1] - bo[q];
     }
-    pack_sizes(cn, c->tune.per_grab, c->sms * 16, pack_nmax(c->T.L), packs);
+    pack_sizes(cn, c->tune.per_pack, c->sms * 16, pack_nmax(c->T.L), packs);
     for (int q = 0; q < kDpBuckets; ++q) {
         if (per_cta) per_cta[q] = c->tune.per_cta[q];
         if (per_grab) per_grab[q] = packs[q];

@@ -309,9 +309,10 @@ class Router:
         return out
 
     def autotune(self, plain: bool = True, persistent: bool = True) -> dict:
-        """Pick nets-per-CTA (per-batch DP launch) and nets-per-grab (persistent
-        work queue) by size bucket (<= 2, <= 8, <= 16, > 16 tree nodes) on the
-        current plan; leaves the context reset."""
+        """Pick the warps per CTA of the per-batch DP launch ("nets_per_cta") and
+        the nets a warp of the persistent form takes together ("nets_per_grab") by
+        size bucket (<= 2, <= 8, <= 16, > 16 tree nodes) on the current plan;
+        leaves the context reset."""
         per_cta = np.zeros(4, np.int32)
         per_grab = np.zeros(4, np.int32)
         what = (1 if plain else 0) | (2 if persistent else 0)
@@ -431,8 +432,9 @@ class Router:
         return _stats_dict(st)
 
     # Batching: plain form raster / gather / solve / publish; persistent form
-    # a worker round / solve and the waits.  Stages: cost refresh (cost_pass1),
-    # DP, commit.
+    # a worker round (batch_gather) / solve and the waits.  Stages: cost refresh
+    # (cost_pass1), DP, commit.  prefix_tree_pass2 and unused11 stay 0; net_ms and
+    # longest_net_ms count packs.
     PHASES = ("batch_raster", "batch_gather", "batch_solve", "batch_publish", "cost_pass1", "dp", "commit",
               "prefix_tree_pass2", "batch_solver_wait", "batch_worker_wait", "flt_edge_tables", "unused11",
               "net_ms_bucket0", "net_ms_bucket1", "net_ms_bucket2", "net_ms_bucket3",

@@ -350,7 +350,8 @@ typedef struct grb_zshape_trees {
 } grb_zshape_trees;
 
 /* Upload Z-shape trees (host buffers); also derives every net's bounding box
- * and allocates the DP planes (22 int planes of (L+1) * max(X,Y)^2). */
+ * and allocates scratch for nets of more than 96 nodes (at most 832 bytes per
+ * node of theirs, and no more than the largest one's for each block). */
 int grb_upload_zshape(grb_ctx* ctx, const grb_zshape_trees* trees);
 
 /* Refine every batch of the current plan into bounding-box batches
@@ -387,9 +388,10 @@ int grb_softmin_forward(grb_ctx* ctx, int32_t dtype, double tau, const void* cap
 /* Hand-written adjoint of grb_softmin_forward: grad_total * d(total)/d(capacity)
  * into dcap, d(total)/d(unit_wire) per edge into dunit_wire (device arrays
  * like the inputs) and d(total)/d(unit_via) into *dunit_via.  Each net's DP
- * tables are recomputed in a per-thread slot (memory bounded by the threads
- * in flight, not by the nets); as tau -> 0 the gradient tends to the
- * indicator of the chosen routes. */
+ * tables are recomputed, in shared memory up to 32 tree nodes (designs with
+ * larger nets: in scratch of 2 * L * L values per tree node of the design); as
+ * tau -> 0 the gradient tends to the indicator of the chosen routes.  A
+ * candidate whose cost is NaN, infinite or at least 1e21 does not exist. */
 int grb_softmin_backward(grb_ctx* ctx, int32_t dtype, double tau, const void* capacity, const void* unit_wire,
                          double unit_via, double grad_total, void* dcap, void* dunit_wire, double* dunit_via);
 
@@ -476,10 +478,11 @@ int grb_set_wait_limit(grb_ctx* ctx, double seconds);
  * (plain form only); stages [4] cost refresh, [5] DP (persistent: + wire
  * commit), [6] commit (persistent: vias), [7] unused; persistent batching [8]
  * solver waiting for a gathered chunk, [9] other blocks waiting for a solved
- * chunk; [10] and [11] unused; persistent L-shape stage, per size bucket k of
- * the DP (tree nodes <= 2, <= 8, <= 16, more): [12+k] warp time summed over
- * its packs, [16+k] the longest single pack (a maximum, not a sum).  The reference prints its stage timings as BATCH_TIMING /
- * DAG_TIMING records (router_state.hpp:259-264). */
+ * chunk; [10] FLT layer-change tables (persistent); [11] unused; persistent
+ * L-shape stage, per size bucket k of the DP (tree nodes <= 2, <= 8, <= 16,
+ * more): [12+k] warp time summed over its packs, [16+k] the longest single pack
+ * (a maximum, not a sum).  The reference prints its stage timings as
+ * BATCH_TIMING / DAG_TIMING records (router_state.hpp:259-264). */
 int grb_set_profiling(grb_ctx* ctx, int32_t on);
 int grb_phase_times(grb_ctx* ctx, double* ms, int32_t n, int32_t reset);
 

@@ -16,7 +16,7 @@ Per workload (a seeded synthetic design written as CAP/NET files):
      batches, routes, demand and statistics are compared with the reference's.
 
 Usage:  python oracle/ref_stage_timing.py [--workloads medium_320x320x10,large_800x800x10]
-                                          [--out gpurun_out/ref_stage_timing.json] [--reps 3]
+                                          [--out ref_stage_timing.json] [--reps 3]
 """
 from __future__ import annotations
 
