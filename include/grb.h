@@ -145,7 +145,9 @@ int grb_read_topology(grb_ctx* ctx, int32_t* node_off, int32_t* nodes, int32_t* 
 int grb_plan_batches(grb_ctx* ctx, const int32_t* order, int32_t n, int32_t limit, int32_t sparsity,
                      int32_t mode, int32_t* batch_of, int32_t* n_batches);
 
-/* Set an explicit plan: net ids in execution order and batch offsets. */
+/* Set an explicit plan: net ids in execution order and batch offsets (from 0 to
+ * n, not decreasing).  A plan stays when other nets are uploaded; calls that use
+ * it are refused while it names nets that are not there. */
 int grb_set_plan(grb_ctx* ctx, const int32_t* ids, int32_t n, const int32_t* batch_off, int32_t n_batches);
 /* Copy the current plan out (ids[n], batch_off[n_batches+1]). */
 int grb_get_plan(grb_ctx* ctx, int32_t* ids, int32_t* batch_off, int32_t* n, int32_t* n_batches);
